@@ -326,10 +326,10 @@ void launch_pdl(void (*kernel)(KArgs...), int grid, int block, size_t smem, Args
 }
 
 template <typename... KArgs, typename... Args>
-void launch_pdl_grid(void (*kernel)(KArgs...), dim3 grid, int block, Args... args) {
+void launch_pdl_grid(void (*kernel)(KArgs...), dim3 grid, int block, size_t smem, Args... args) {
 	same_carveout((const void*)kernel);
 	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = grid, cfg.blockDim = dim3(block), cfg.dynamicSmemBytes = 0, cfg.stream = g.stream;
+	cfg.gridDim = grid, cfg.blockDim = dim3(block), cfg.dynamicSmemBytes = smem, cfg.stream = g.stream;
 	cudaLaunchAttribute at[1];
 	at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
 	at[0].val.programmaticStreamSerializationAllowed = g.use_pdl ? 1 : 0;
@@ -1339,11 +1339,13 @@ static void pf_gemm(const CUtensorMap* tm, const PfGemmArgs& a, int rows, int n)
 }
 
 template <typename KVT, int HD>
-static void pf_attn(const PfAttnArgs& a, int n) {
-	const dim3 grid(cdiv(n, PFA_WARPS), g.cfg.n_kv_heads);
-	if (g.kv_mul % 4 == 0) launch_pdl_grid(k_pf_attn<KVT, HD, 4>, grid, PFA_WARPS * 32, a);
-	else if (g.kv_mul % 2 == 0) launch_pdl_grid(k_pf_attn<KVT, HD, 2>, grid, PFA_WARPS * 32, a);
-	else launch_pdl_grid(k_pf_attn<KVT, HD, 1>, grid, PFA_WARPS * 32, a);
+static void pf_attn(PfAttnArgs a, int n) {
+	static bool opted = false;
+	if (!opted) smem_optin(k_pf_attn<KVT, HD>, pfa_smem_bytes<HD>()), opted = true;
+	for (a.km = 8; g.kv_mul % a.km; --a.km) { // the largest divisor of the group up to 8 heads
+	}
+	a.tb = 8 / a.km;
+	launch_pdl_grid(k_pf_attn<KVT, HD>, dim3(cdiv(n, 16 * a.tb), g.cfg.n_kv_heads * (g.kv_mul / a.km)), 32 * a.km * a.tb, pfa_smem_bytes<HD>(), a);
 	++g_launches;
 }
 

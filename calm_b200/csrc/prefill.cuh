@@ -12,8 +12,8 @@
 //               through mbarriers (tcgen05.commit), the epilogue reads TMEM with tcgen05.ld and applies what the
 //               decode kernels apply: bias / clip / RoPE / KV-cache append (QKV), residual add (wo, w2),
 //               act(w1 x) * (w3 x) with both accumulators side by side in TMEM (FFN up).
-//   k_pf_attn   causal attention of the block against the cache (fp32 math on the cached fp16 / e5m2 entries, online
-//               softmax; reference infer.c:238-267), one warp per query token, K/V tiles staged in shared memory.
+//   k_pf_attn   causal attention of the block against the cache (online softmax in fp32; reference infer.c:238-267), scores and
+//               values on warp-level tensor cores with hi + lo queries and weights against the cached fp16 / e5m2 entries.
 //   k_pf_norm   RMSNorm / LayerNorm per token (reference infer.c:183-207) -> hi / lo f16 rows.
 //
 // Parity contract (tests/test_prefill_gpu.py): after forward_prefill_cuda(tokens, n, pos0) the KV cache and the logits of
@@ -320,8 +320,16 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_pf_gemm(const __grid_constant
 }
 
 // ---------------------------------------------------------------- causal attention of the block against the cache
-#define PFA_WARPS 8
-#define PFA_TILE 32 // keys per shared-memory tile: one per lane
+// Flash attention on warp-level tensor cores (mma.m16n8k16, fp32 accumulators).  A CTA serves KM of the query heads that share a kv
+// head: warp = (head, 16 consecutive tokens), so one 64-key tile of K and V in shared memory feeds up to 128 rows.  The cache
+// entries (fp16, or e5m2 widened on the way in) are exact f16 operands; queries and softmax weights travel as an f16 hi + lo
+// pair, two MMAs into the same fp32 accumulator, so they keep 22 bits.  A query row is first scaled by the power of two that
+// brings its largest entry into [1, 2) (exact; the score is scaled back), so no query leaves the f16 range.  Running maximum,
+// exponentials and the denominator are fp32.
+// Bound: the MMA rate (4 x 64 MMAs per warp and tile against 32 KB of ldmatrix traffic).  Tokens are taken 16 per warp and not 32 because
+// 64 accumulator and 64 query registers per 16 rows already fill the file at 8 warps; the last blocks of the prompt, which see
+// the most keys, are started first.  2047 tokens, 32 / 8 heads of 128: 1550 us a layer as fp32 FMAs, one token per warp; about 360 us here.
+#define PFA_TILE 64 // keys per tile
 
 struct PfAttnArgs {
 	const float* Q; // [T][q_dim]
@@ -330,128 +338,173 @@ struct PfAttnArgs {
 	__half* Ohi;    // [T][q_dim]
 	__half* Olo;
 	int n_tokens, pos0, seq_len, q_dim, kv_mul;
+	int km, tb; // query heads and 16-token blocks per CTA: km * tb warps, km divides kv_mul
 	float inv_sqrt_hd;
 };
 
-// DPL (2 or 4) consecutive cache elements -> floats with a single shared-memory load
-template <int DPL>
-__device__ __forceinline__ void pf_load_dims(const __half* p, float (&o)[DPL]) {
-	if constexpr (DPL == 4) {
-		const uint2 r = *reinterpret_cast<const uint2*>(p);
-		const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&r.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&r.y));
-		o[0] = a.x, o[1] = a.y, o[2] = b.x, o[3] = b.y;
-	} else {
-		const float2 a = __half22float2(*reinterpret_cast<const __half2*>(p));
-		o[0] = a.x, o[1] = a.y;
-	}
-}
-template <int DPL>
-__device__ __forceinline__ void pf_load_dims(const uint8_t* p, float (&o)[DPL]) {
-	if constexpr (DPL == 4) {
-		const uint32_t r = *reinterpret_cast<const uint32_t*>(p);
-		const float2 a = e5m2x2_lo(r), b = e5m2x2_hi(r);
-		o[0] = a.x, o[1] = a.y, o[2] = b.x, o[3] = b.y;
-	} else {
-		const uint32_t r = *reinterpret_cast<const unsigned short*>(p);
-		const float2 a = e5m2x2_lo(r);
-		o[0] = a.x, o[1] = a.y;
-	}
+template <int HD>
+__host__ __device__ constexpr size_t pfa_smem_bytes() { // two buffers of K and V
+	return (size_t)2 * 2 * PFA_TILE * HD * sizeof(__half);
 }
 
-// CTA = (kv head, 8 consecutive query tokens); warp = one token with all kv_mul query heads of the kv head (KM of them per pass)
-template <typename KVT, int HD, int KM>
-__global__ void __launch_bounds__(PFA_WARPS * 32) k_pf_attn(const PfAttnArgs a) {
+__device__ __forceinline__ void ldsm_x4(const void* p, uint32_t (&r)[4]) {
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
+}
+__device__ __forceinline__ void ldsm_x4_t(const void* p, uint32_t (&r)[4]) {
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
+}
+__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+	asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+	             : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+	             : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool in) { // 16 bytes, zeros when !in
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+// two floats -> (hi, lo) f16 pairs
+__device__ __forceinline__ void split_hl2(float x, float y, uint32_t& hi, uint32_t& lo) {
+	const __half2 h = __floats2half2_rn(x, y);
+	const float2 f = __half22float2(h);
+	const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+	hi = *reinterpret_cast<const uint32_t*>(&h), lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+template <typename KVT, int HD>
+__global__ void __launch_bounds__(256, 1) k_pf_attn(const PfAttnArgs a) {
 	pdl_enter();
-	constexpr int DPL = HD / 32;               // head dims owned by a lane in the value pass
-	constexpr int KSTR = HD * sizeof(KVT) + 16; // padded key row: 16-byte reads of one row per lane are conflict-free per quarter warp
-	__shared__ __align__(16) unsigned char ks[PFA_TILE * KSTR];
-	__shared__ __align__(16) unsigned char vs[PFA_TILE * HD * sizeof(KVT)];
-	__shared__ __align__(16) float qs[PFA_WARPS][KM * HD];
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	const int kvh = blockIdx.y, t = blockIdx.x * PFA_WARPS + warp;
-	const bool live = t < a.n_tokens;
-	const int last = a.pos0 + min(a.n_tokens - 1, (int)blockIdx.x * PFA_WARPS + PFA_WARPS - 1); // last key position any warp of the CTA needs
-	const int mypos = a.pos0 + t;
+	constexpr int CH = HD / 8;   // 16-byte chunks of a tile row
+	constexpr int NT = PFA_TILE / 8, KS = HD / 16, TILE = PFA_TILE * HD;
+	extern __shared__ __align__(128) __half sm[];
+	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+	const int per_kv = a.kv_mul / a.km; // CTAs per kv head and token block
+	const int kvh = blockIdx.y / per_kv, head = kvh * a.kv_mul + (blockIdx.y % per_kv) * a.km + warp % a.km;
+	const int c0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * 16 * a.tb; // first token of the CTA (the longest rows first)
+	const int t0 = c0 + (warp / a.km) * 16;                            // first token of the warp
+	const int last = a.pos0 + min(a.n_tokens, c0 + 16 * a.tb) - 1;     // last key position any row of the CTA sees
+	const int wlast = a.pos0 + min(a.n_tokens, t0 + 16) - 1;           // ... of this warp (below pos0 + t0: no live row)
 	const KVT* kbase = reinterpret_cast<const KVT*>(a.kc) + (size_t)kvh * a.seq_len * HD;
 	const KVT* vbase = reinterpret_cast<const KVT*>(a.vc) + (size_t)kvh * a.seq_len * HD;
-	for (int hg = 0; hg < a.kv_mul; hg += KM) { // KM query heads per pass over the keys
-		const int h0 = kvh * a.kv_mul + hg;
-		for (int i = lane; i < KM * HD; i += 32) qs[warp][i] = live ? a.Q[(size_t)t * a.q_dim + (size_t)h0 * HD + i] : 0.f;
-		float m[KM], l[KM], acc[KM][DPL];
-#pragma unroll
-		for (int h = 0; h < KM; ++h) {
-			m[h] = -FLT_MAX, l[h] = 0.f;
-#pragma unroll
-			for (int d = 0; d < DPL; ++d) acc[h][d] = 0.f;
-		}
-		for (int k0 = 0; k0 <= last; k0 += PFA_TILE) {
-			__syncthreads(); // the previous tile is no longer being read
-			for (int i = threadIdx.x; i < PFA_TILE * HD * (int)sizeof(KVT) / 16; i += blockDim.x) {
-				const int row = i / (HD * (int)sizeof(KVT) / 16), c = i % (HD * (int)sizeof(KVT) / 16);
-				const bool in = k0 + row <= last;
-				const uint4 z = make_uint4(0, 0, 0, 0);
-				*reinterpret_cast<uint4*>(ks + row * KSTR + c * 16) = in ? __ldcg(reinterpret_cast<const uint4*>(kbase + (size_t)(k0 + row) * HD) + c) : z;
-				*reinterpret_cast<uint4*>(vs + row * HD * sizeof(KVT) + c * 16) = in ? __ldcg(reinterpret_cast<const uint4*>(vbase + (size_t)(k0 + row) * HD) + c) : z;
-			}
-			__syncthreads();
-			if (!live || k0 > mypos) continue; // (warp-uniform) causal: nothing of this tile is visible to this token
-			const bool vis = k0 + lane <= mypos;
-			// scores of key (k0 + lane) against the KM heads
-			float sc[KM];
-#pragma unroll
-			for (int h = 0; h < KM; ++h) sc[h] = 0.f;
-			const unsigned char* krow = ks + lane * KSTR;
-#pragma unroll 4
-			for (int c = 0; c < HD / 8; ++c) {
-				float kf[8];
-				kv_load8(reinterpret_cast<const KVT*>(krow) + c * 8, kf);
-#pragma unroll
-				for (int h = 0; h < KM; ++h) {
-					const float4 q0 = *reinterpret_cast<const float4*>(&qs[warp][h * HD + c * 8]), q1 = *reinterpret_cast<const float4*>(&qs[warp][h * HD + c * 8 + 4]);
-					float s = sc[h];
-					s = fmaf(q0.x, kf[0], s), s = fmaf(q0.y, kf[1], s), s = fmaf(q0.z, kf[2], s), s = fmaf(q0.w, kf[3], s);
-					s = fmaf(q1.x, kf[4], s), s = fmaf(q1.y, kf[5], s), s = fmaf(q1.z, kf[6], s), s = fmaf(q1.w, kf[7], s);
-					sc[h] = s;
-				}
-			}
-			float p[KM];
-#pragma unroll
-			for (int h = 0; h < KM; ++h) {
-				const float s = vis ? sc[h] * a.inv_sqrt_hd : -FLT_MAX;
-				const float mn = fmaxf(m[h], warp_max(s));
-				const float corr = expf(m[h] - mn);
-				p[h] = vis ? expf(s - mn) : 0.f;
-				l[h] = fmaf(l[h], corr, warp_sum(p[h]));
-				m[h] = mn;
-#pragma unroll
-				for (int d = 0; d < DPL; ++d) acc[h][d] *= corr;
-			}
-			// values: lane owns head dims [lane * DPL, lane * DPL + DPL)
-			const int nk = min(PFA_TILE, mypos - k0 + 1);
-			for (int j = 0; j < nk; ++j) {
-				float vf[DPL];
-				pf_load_dims<DPL>(reinterpret_cast<const KVT*>(vs) + (size_t)j * HD + lane * DPL, vf); // one 8- / 4- / 2-byte load
-#pragma unroll
-				for (int h = 0; h < KM; ++h) {
-					const float pj = __shfl_sync(0xffffffffu, p[h], j);
-#pragma unroll
-					for (int d = 0; d < DPL; ++d) acc[h][d] = fmaf(pj, vf[d], acc[h][d]);
-				}
+	// row r, chunk c of a tile lies at chunk c ^ (r & 7): ldmatrix reads 8 rows of one chunk without bank conflicts
+	auto at = [&](int buf, int which, int r, int c) { return sm + (size_t)(buf * 2 + which) * TILE + r * HD + ((c ^ (r & 7)) << 3); };
+	auto fetch = [&](int buf, int k0) {
+		for (int i = tid; i < 2 * PFA_TILE * CH; i += blockDim.x) {
+			const int which = i / (PFA_TILE * CH), r = (i / CH) % PFA_TILE, c = i % CH;
+			const bool in = k0 + r <= last;
+			const KVT* src = (which ? vbase : kbase) + (size_t)(in ? k0 + r : 0) * HD + c * 8;
+			if constexpr (sizeof(KVT) == 2) {
+				cp_async16(at(buf, which, r, c), src, in);
+			} else { // an e5m2 byte is the high byte of the f16
+				const uint2 w = in ? __ldcg(reinterpret_cast<const uint2*>(src)) : make_uint2(0, 0);
+				*reinterpret_cast<uint4*>(at(buf, which, r, c)) = make_uint4(__byte_perm(w.x, 0, 0x1404), __byte_perm(w.x, 0, 0x3424), __byte_perm(w.y, 0, 0x1404), __byte_perm(w.y, 0, 0x3424));
 			}
 		}
-		if (live) {
+		asm volatile("cp.async.commit_group;" ::: "memory");
+	};
+	fetch(0, 0);
+
+	// queries of rows t0 + g and t0 + g + 8 as MMA fragments
+	uint32_t qh[KS][4], ql[KS][4];
+	float smul[2]; // score factor of the two rows
+	{
+		float2 q[2][KS][2];
 #pragma unroll
-			for (int h = 0; h < KM; ++h) {
-				const float inv = 1.0f / l[h];
+		for (int r = 0; r < 2; ++r) {
+			const int t = t0 + g + 8 * r;
+			const float* qp = a.Q + (size_t)t * a.q_dim + (size_t)head * HD + 2 * t4;
+			float mx = 0.f;
 #pragma unroll
-				for (int d = 0; d < DPL; ++d) {
-					__half hh, hl;
-					split_hl(acc[h][d] * inv, hh, hl);
-					const size_t o = (size_t)t * a.q_dim + (size_t)(h0 + h) * HD + lane * DPL + d;
-					a.Ohi[o] = hh, a.Olo[o] = hl;
+			for (int k = 0; k < KS; ++k)
+#pragma unroll
+				for (int j = 0; j < 2; ++j) {
+					q[r][k][j] = t < a.n_tokens ? __ldcg(reinterpret_cast<const float2*>(qp + 16 * k + 8 * j)) : make_float2(0.f, 0.f);
+					mx = fmaxf(mx, fmaxf(fabsf(q[r][k][j].x), fabsf(q[r][k][j].y)));
 				}
+			mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1)), mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+			const uint32_t e = __float_as_uint(mx) >> 23; // biased exponent of the largest entry
+			const bool normal = e > 0 && e < 254;
+			const float down = normal ? __uint_as_float((254 - e) << 23) : 1.f; // 2^(127 - e)
+			smul[r] = (normal ? __uint_as_float(e << 23) : 1.f) * a.inv_sqrt_hd;
+#pragma unroll
+			for (int k = 0; k < KS; ++k)
+#pragma unroll
+				for (int j = 0; j < 2; ++j) split_hl2(q[r][k][j].x * down, q[r][k][j].y * down, qh[k][2 * j + r], ql[k][2 * j + r]);
+		}
+	}
+	float o[HD / 8][4], m[2] = {-FLT_MAX, -FLT_MAX}, l[2] = {0.f, 0.f};
+#pragma unroll
+	for (int n = 0; n < HD / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+
+	for (int k0 = 0, buf = 0; k0 <= last; k0 += PFA_TILE, buf ^= 1) {
+		asm volatile("cp.async.wait_group 0;" ::: "memory");
+		__syncthreads(); // the tile has arrived, and the other buffer is no longer being read
+		if (k0 + PFA_TILE <= last) fetch(buf ^ 1, k0 + PFA_TILE);
+		if (k0 > wlast) continue; // (warp-uniform) nothing of this tile is visible to this warp's rows
+		float s[NT][4];
+#pragma unroll
+		for (int n = 0; n < NT; ++n) {
+			s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+#pragma unroll
+			for (int k = 0; k < KS; k += 2) {
+				uint32_t b[4]; // key block n, dims 16k .. 16k + 31
+				ldsm_x4(at(buf, 0, n * 8 + (lane & 7), 2 * k + (lane >> 3)), b);
+				mma_f16(s[n], qh[k], b[0], b[1]), mma_f16(s[n], ql[k], b[0], b[1]);
+				mma_f16(s[n], qh[k + 1], b[2], b[3]), mma_f16(s[n], ql[k + 1], b[2], b[3]);
 			}
 		}
-		__syncwarp();
+		float mx[2] = {-FLT_MAX, -FLT_MAX};
+		const int p0 = a.pos0 + t0 + g; // position of row 0
+		const bool whole = k0 + PFA_TILE - 1 <= a.pos0 + t0; // every row of the warp sees every key of the tile
+#pragma unroll
+		for (int n = 0; n < NT; ++n)
+#pragma unroll
+			for (int e = 0; e < 4; ++e) {
+				const int r = e >> 1, key = k0 + n * 8 + 2 * t4 + (e & 1);
+				s[n][e] = whole || key <= p0 + 8 * r ? s[n][e] * smul[r] : -FLT_MAX;
+				mx[r] = fmaxf(mx[r], s[n][e]);
+			}
+		float corr[2];
+#pragma unroll
+		for (int r = 0; r < 2; ++r) {
+			mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1)), mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
+			const float mn = fmaxf(m[r], mx[r]);
+			corr[r] = expf(m[r] - mn);
+			m[r] = mn, l[r] *= corr[r];
+		}
+#pragma unroll
+		for (int n = 0; n < HD / 8; ++n) o[n][0] *= corr[0], o[n][1] *= corr[0], o[n][2] *= corr[1], o[n][3] *= corr[1];
+#pragma unroll
+		for (int kk = 0; kk < PFA_TILE / 16; ++kk) { // 16 keys: their weights, then their values
+			uint32_t ph[4], pl[4];
+#pragma unroll
+			for (int j = 0; j < 2; ++j)
+#pragma unroll
+				for (int r = 0; r < 2; ++r) {
+					const float x = s[2 * kk + j][2 * r], y = s[2 * kk + j][2 * r + 1];
+					const float px = x == -FLT_MAX ? 0.f : expf(x - m[r]), py = y == -FLT_MAX ? 0.f : expf(y - m[r]);
+					l[r] += px + py;
+					split_hl2(px, py, ph[2 * j + r], pl[2 * j + r]);
+				}
+#pragma unroll
+			for (int n = 0; n < HD / 8; n += 2) {
+				uint32_t b[4]; // (keys 0-7, dims n), (keys 8-15, dims n), (keys 0-7, dims n + 1), (keys 8-15, dims n + 1)
+				ldsm_x4_t(at(buf, 1, kk * 16 + (lane & 15), n + (lane >> 4)), b);
+				mma_f16(o[n], ph, b[0], b[1]), mma_f16(o[n], pl, b[0], b[1]);
+				mma_f16(o[n + 1], ph, b[2], b[3]), mma_f16(o[n + 1], pl, b[2], b[3]);
+			}
+		}
+	}
+#pragma unroll
+	for (int r = 0; r < 2; ++r) {
+		l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1), l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
+		const int t = t0 + g + 8 * r;
+		if (t >= a.n_tokens) continue;
+		const float inv = 1.0f / l[r];
+		const size_t at0 = (size_t)t * a.q_dim + (size_t)head * HD + 2 * t4;
+#pragma unroll
+		for (int n = 0; n < HD / 8; ++n) {
+			uint32_t hi, lo;
+			split_hl2(o[n][2 * r] * inv, o[n][2 * r + 1] * inv, hi, lo);
+			*reinterpret_cast<uint32_t*>(a.Ohi + at0 + 8 * n) = hi, *reinterpret_cast<uint32_t*>(a.Olo + at0 + 8 * n) = lo;
+		}
 	}
 }
