@@ -376,8 +376,24 @@ __device__ __forceinline__ float dot_vec<4>(const uint4& w, const float4 (&xv)[8
 	return acc;
 }
 
-__device__ __forceinline__ uint32_t pack_h2(__half a, __half b) {
-	return (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16);
+// gf4 word -> its eight weights as four f16 pairs, exact (at most 6 significant bits).  A 3-bit code at bit p of a half whose upper bits are
+// those of 1024.0 reads as 1024 + q 2^p: the four pairs are picked so that both codes lie at some p <= 7 of their halves (one
+// byte permute, one masked or), one fma takes the offset and the 2^p off (q - 4, exact) and one multiplication applies -s/4:
+// 19 instructions for 8 weights.
+__device__ __forceinline__ uint32_t gf4_pair(uint32_t v, uint32_t mask, __half2 mul, __half2 sub, __half2 sc) {
+	uint32_t r;
+	asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(v), "r"(mask), "r"(0x64006400u)); // (v & mask) | 1024.0 in both halves
+	const __half2 h = __hmul2(__hfma2(*reinterpret_cast<__half2*>(&r), mul, sub), sc);
+	return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ void gf4_to_h2(uint32_t w, uint32_t (&h)[4]) {
+	const uint32_t x = w >> 8, s2 = __byte_perm(w, 0, 0x0404);
+	const __half2 sc = __hmul2(*reinterpret_cast<const __half2*>(&s2), __half2half2(__ushort_as_half(0xB400))); // -s / 4
+	auto c = [](float a, float b) { return __floats2half2_rn(a, b); };
+	h[0] = gf4_pair(__byte_perm(x, 0, 0x1010), 0x00380007u, c(1.f, 0.125f), c(-1028.f, -132.f), sc);     // codes at bits 0 and 3 of w >> 8
+	h[1] = gf4_pair(__byte_perm(x, w, 0x7610), 0x000E01C0u, c(0.015625f, 0.5f), c(-20.f, -516.f), sc);   // bit 6 of w >> 8, bit 17 of w
+	h[2] = gf4_pair(__byte_perm(w, 0, 0x3232), 0x03800070u, c(0.0625f, 0.0078125f), c(-68.f, -12.f), sc); // bits 20 and 23 of w
+	h[3] = gf4_pair(__byte_perm(x, 0, 0x3232), 0x00E0001Cu, c(0.25f, 0.03125f), c(-260.f, -36.f), sc);   // bits 18 and 21 of w >> 8
 }
 
 // single weight decode (embedding row)

@@ -141,7 +141,10 @@ struct Prefill {
 	__half *Nhi = nullptr, *Nlo = nullptr, *Ahi = nullptr, *Alo = nullptr, *Hhi = nullptr, *Hlo = nullptr;
 	float2* rope = nullptr;
 	int* tokens = nullptr;
-	CUtensorMap tmN[2], tmA[2], tmH[2]; // (hi, lo) views of the three activation matrices the GEMMs read
+	CUtensorMap tmN[3][2], tmA[3][2], tmH[3][2]; // views of the three activation matrices the GEMMs read: [64- / 128- / 256-row boxes][hi, lo]
+	std::vector<CUtensorMap> tmW;       // per layer: wq, wk, wv, wo, w1, w3, w2
+	float* ws = nullptr;                // partial sums of K-split products
+	unsigned* counter = nullptr;
 };
 Prefill pf;
 int g_device_override = -1;
@@ -1102,7 +1105,7 @@ extern "C" void calm_b200_release(struct Transformer* transformer) {
 	cudaFree(g.stamps), cudaFree(g.stamp_acc), cudaFree(g.attn_cells);
 	if (g.dev_err) cudaFreeHost(g.dev_err);
 	if (pf.cap) {
-		cudaFree(pf.X), cudaFree(pf.Q), cudaFree(pf.Nhi), cudaFree(pf.Nlo), cudaFree(pf.Ahi), cudaFree(pf.Alo), cudaFree(pf.Hhi), cudaFree(pf.Hlo), cudaFree(pf.rope), cudaFree(pf.tokens);
+		cudaFree(pf.X), cudaFree(pf.Q), cudaFree(pf.Nhi), cudaFree(pf.Nlo), cudaFree(pf.Ahi), cudaFree(pf.Alo), cudaFree(pf.Hhi), cudaFree(pf.Hlo), cudaFree(pf.rope), cudaFree(pf.tokens), cudaFree(pf.ws), cudaFree(pf.counter);
 		pf = Prefill();
 	}
 	cudaFree(g.x), cudaFree(g.xb), cudaFree(g.q), cudaFree(g.att), cudaFree(g.hb), cudaFree(g.logits_dev);
@@ -1273,7 +1276,8 @@ extern "C" int calm_b200_sample_logits(const float* logits_host, int vocab, floa
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                                   CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-static void pf_make_map(CUtensorMap* map, void* base, int rows, int cols) { // f16 [rows][cols], box = 128 rows x 64 columns, 128-byte swizzle
+// [rows][cols] of `type`, box = box_rows x box_cols
+static void pf_make_map(CUtensorMap* map, const void* base, int rows, int cols, CUtensorMapDataType type, int box_rows, int box_cols, CUtensorMapSwizzle swizzle) {
 	static EncodeTiledFn encode = nullptr;
 	if (!encode) {
 		cudaDriverEntryPointQueryResult qres;
@@ -1283,16 +1287,36 @@ static void pf_make_map(CUtensorMap* map, void* base, int rows, int cols) { // f
 		encode = (EncodeTiledFn)fn;
 	}
 	const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-	const cuuint64_t strides[1] = {(cuuint64_t)cols * sizeof(__half)};
-	const cuuint32_t box[2] = {PF_BK, PF_BN}, estr[2] = {1, 1};
-	CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+	const cuuint64_t strides[1] = {(cuuint64_t)cols * (type == CU_TENSOR_MAP_DATA_TYPE_FLOAT16 ? 2 : 1)};
+	const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows}, estr[2] = {1, 1};
+	CUresult r = encode(map, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
 	                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-	if (r != CUDA_SUCCESS) CALM_FATAL("cuTensorMapEncodeTiled failed (%d) for a %d x %d f16 matrix", (int)r, rows, cols);
+	if (r != CUDA_SUCCESS) CALM_FATAL("cuTensorMapEncodeTiled failed (%d) for a %d x %d matrix", (int)r, rows, cols);
+}
+static void pf_act_maps(CUtensorMap (&map)[3][2], const __half* hi, const __half* lo, int rows, int cols) {
+	for (int b = 0; b < 3; ++b)
+		for (int h = 0; h < 2; ++h) pf_make_map(&map[b][h], h ? lo : hi, rows, cols, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 64 << b, PF_BK, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+static void pf_weight_map(CUtensorMap* map, const void* base, int rows, int cols) { // a k-stage of 128 rows; the swizzles are those k_pf_gemm's readers expect
+	if (g.w.dbits == 16) pf_make_map(map, base, rows, cols, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, PF_BM, PF_BK, CU_TENSOR_MAP_SWIZZLE_128B);
+	else pf_make_map(map, base, rows, cols * g.w.dbits / 8, CU_TENSOR_MAP_DATA_TYPE_UINT8, PF_BM, PF_BK * g.w.dbits / 8, g.w.dbits == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
 
 static void pf_reserve(int n) {
 	const Config& c = g.cfg;
-	int cap = cdiv(n, PF_BN) * PF_BN;
+	if (pf.tmW.empty()) { // once per model
+		pf.tmW.resize((size_t)c.n_layers * 7);
+		for (int l = 0; l < c.n_layers; ++l) {
+			CUtensorMap* t = &pf.tmW[(size_t)l * 7];
+			pf_weight_map(t, g.w.wq[l], g.q_dim, c.dim), pf_weight_map(t + 1, g.w.wk[l], g.kv_dim, c.dim), pf_weight_map(t + 2, g.w.wv[l], g.kv_dim, c.dim);
+			pf_weight_map(t + 3, g.w.wo[l], c.dim, g.q_dim);
+			pf_weight_map(t + 4, g.w.w1[l], c.hidden_dim, c.dim), pf_weight_map(t + 5, g.w.w3[l], c.hidden_dim, c.dim), pf_weight_map(t + 6, g.w.w2[l], c.dim, c.hidden_dim);
+		}
+		pf.ws = (float*)dev_alloc((size_t)g.sms * 256 * PF_BM * sizeof(float)); // an item's accumulators: at most 256 columns
+		pf.counter = (unsigned*)dev_alloc(g.sms * sizeof(unsigned));
+		CUDA_CHECK(cudaMemset(pf.counter, 0, g.sms * sizeof(unsigned)));
+	}
+	int cap = cdiv(n, PF_PAD) * PF_PAD;
 	if (cap <= pf.cap) return;
 	if (pf.cap) {
 		CUDA_CHECK(cudaStreamSynchronize(g.stream));
@@ -1311,9 +1335,9 @@ static void pf_reserve(int n) {
 	pf.Hhi = (__half*)zalloc((size_t)cap * c.hidden_dim * sizeof(__half)), pf.Hlo = (__half*)zalloc((size_t)cap * c.hidden_dim * sizeof(__half));
 	pf.rope = (float2*)zalloc((size_t)cap * (c.head_dim / 2) * sizeof(float2));
 	pf.tokens = (int*)zalloc((size_t)cap * sizeof(int));
-	pf_make_map(&pf.tmN[0], pf.Nhi, cap, c.dim), pf_make_map(&pf.tmN[1], pf.Nlo, cap, c.dim);
-	pf_make_map(&pf.tmA[0], pf.Ahi, cap, g.q_dim), pf_make_map(&pf.tmA[1], pf.Alo, cap, g.q_dim);
-	pf_make_map(&pf.tmH[0], pf.Hhi, cap, c.hidden_dim), pf_make_map(&pf.tmH[1], pf.Hlo, cap, c.hidden_dim);
+	pf_act_maps(pf.tmN, pf.Nhi, pf.Nlo, cap, c.dim);
+	pf_act_maps(pf.tmA, pf.Ahi, pf.Alo, cap, g.q_dim);
+	pf_act_maps(pf.tmH, pf.Hhi, pf.Hlo, cap, c.hidden_dim);
 }
 
 // which models the tensor-core pass serves; everything else is fed token by token (still on the GPU)
@@ -1323,18 +1347,44 @@ static bool pf_supported() {
 	       (c.head_dim == 64 || c.head_dim == 128) && !(getenv("CALM_B200_PREFILL") && atoi(getenv("CALM_B200_PREFILL")) == 0);
 }
 
-template <int MODE, int DBITS, typename KVT>
-static void pf_gemm(const CUtensorMap* tm, const PfGemmArgs& a, int rows, int n) {
+// Row tiles and tokens per item and K-slices of a product of `rows` weight rows over n tokens: the choice with the least estimated time, in cycles.
+// A k-stage was measured at 1600 / 1880 / 2660 cycles for one row tile and 64 / 128 / 256 tokens, at 2000 / 2550 for two (fp8, 4096 x 4096 x 2048
+// tokens; 370 / 260 / 184 / 276 / 176 us), so the widest item wins while every SM has one and smaller ones win below; K is sliced only
+// while an item per SM is left over, and a slice pays for its way through memory.
+static void pf_tiles(int mode, int rows, int n, int nkb, PfGemmArgs& a) {
+	long best = -1;
+	for (int na = mode == PF_UP ? 2 : 1; na <= 2; ++na)
+		for (int bn = 64; bn * na <= 256; bn *= 2) {
+			const int tiles = (mode == PF_UP ? rows / PF_BM : cdiv(rows / PF_BM, na)) * cdiv(n, bn);
+			const int stage = 900 + na * bn * 5;
+			for (int sp = 1; sp == 1 || (tiles * sp <= g.sms && sp * 2 <= nkb && sp <= 16); ++sp) {
+				const long cost = (long)cdiv(tiles * sp, g.sms) * cdiv(nkb, sp) * stage + na * bn * 20 + (sp > 1 ? 5000 + na * bn * (20 + 15 * sp) : 0);
+				if (best < 0 || cost < best) best = cost, a.na = na, a.bn = bn, a.splits = sp;
+			}
+		}
+}
+
+template <int MODE, int DBITS>
+static void pf_gemm(const CUtensorMap (&tx)[3][2], const CUtensorMap* tw, PfGemmArgs a, int rows, int n) {
+	constexpr size_t fixed = pf_fixed_bytes<DBITS>(), limit = 226 * 1024;
 	static bool opted = false;
-	if (!opted) smem_optin(k_pf_gemm<MODE, DBITS, KVT>, pf_smem_bytes<MODE>()), opted = true;
-	same_carveout((const void*)k_pf_gemm<MODE, DBITS, KVT>);
+	if (!opted) smem_optin(k_pf_gemm<MODE, DBITS>, limit), opted = true;
+	same_carveout((const void*)k_pf_gemm<MODE, DBITS>);
+	pf_tiles(MODE, rows, n, a.K / PF_BK, a);
+	PfMaps m;
+	memcpy(m.x, tx[a.bn / 128], sizeof(m.x)); // 64, 128, 256 -> 0, 1, 2
+	memcpy(m.w, tw, (MODE == PF_QKV ? 3 : MODE == PF_UP ? 2 : 1) * sizeof(CUtensorMap));
+	a.n_tokens = n, a.rows = rows, a.ws = pf.ws, a.counter = pf.counter, a.err = g.dev_err;
+	a.nb = imin(PF_MAX_B, (int)((limit - fixed) / (a.bn * 128)) & ~1);
+	const int row_items = MODE == PF_UP ? rows / PF_BM : cdiv(rows / PF_BM, a.na);
 	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3(rows / PF_BM, cdiv(n, PF_BN)), cfg.blockDim = dim3(PF_THREADS), cfg.dynamicSmemBytes = pf_smem_bytes<MODE>(), cfg.stream = g.stream;
+	cfg.gridDim = dim3(imin(g.sms, row_items * a.splits * cdiv(n, a.bn))), cfg.blockDim = dim3(pf_threads<DBITS>()), cfg.stream = g.stream;
+	cfg.dynamicSmemBytes = fixed + (size_t)a.nb * a.bn * 128;
 	cudaLaunchAttribute at[1];
 	at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
 	at[0].val.programmaticStreamSerializationAllowed = g.use_pdl ? 1 : 0;
 	cfg.attrs = at, cfg.numAttrs = 1;
-	CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_pf_gemm<MODE, DBITS, KVT>, tm[0], tm[1], a));
+	CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_pf_gemm<MODE, DBITS>, m, a));
 	++g_launches;
 }
 
@@ -1360,13 +1410,13 @@ static void pf_run(int n, int pos0) {
 	for (int l = 0; l < c.n_layers; ++l) {
 		launch_pdl(k_pf_norm, n, 256, 0, (const float*)pf.X, (const float*)w.rms_att_weight[l], pf.Nhi, pf.Nlo, n, c.dim, c.norm_eps, (int)c.norm_ln);
 		++g_launches;
+		const CUtensorMap* tw = &pf.tmW[(size_t)l * 7];
 		PfGemmArgs a = {};
-		a.n_tokens = n;
-		a.w[0] = w.wq[l], a.w[1] = w.wk[l], a.w[2] = w.wv[l], a.K = c.dim;
+		a.K = c.dim, a.kvbits = g.kvbits;
 		a.Q = pf.Q, a.q_dim = g.q_dim, a.kv_dim = g.kv_dim, a.head_dim = c.head_dim, a.seq_len = c.seq_len, a.pos0 = pos0;
 		a.bias = w.bqkv[l], a.clip = c.qkv_clip, a.rope = pf.rope;
 		a.kc = (KVT*)g.kc + l * kv_layer, a.vc = (KVT*)g.vc + l * kv_layer;
-		pf_gemm<PF_QKV, DBITS, KVT>(pf.tmN, a, g.q_dim + 2 * g.kv_dim, n);
+		pf_gemm<PF_QKV, DBITS>(pf.tmN, tw, a, g.q_dim + 2 * g.kv_dim, n);
 
 		PfAttnArgs aa = {};
 		aa.Q = pf.Q, aa.kc = a.kc, aa.vc = a.vc, aa.Ohi = pf.Ahi, aa.Olo = pf.Alo;
@@ -1375,20 +1425,20 @@ static void pf_run(int n, int pos0) {
 		else pf_attn<KVT, 64>(aa, n);
 
 		PfGemmArgs b = {};
-		b.n_tokens = n, b.w[0] = w.wo[l], b.K = g.q_dim, b.X = pf.X, b.dim = c.dim;
-		pf_gemm<PF_WO, DBITS, KVT>(pf.tmA, b, c.dim, n);
+		b.K = g.q_dim, b.X = pf.X, b.dim = c.dim;
+		pf_gemm<PF_RES, DBITS>(pf.tmA, tw + 3, b, c.dim, n);
 
 		if (!c.norm_par) { // (parallel-norm models reuse the attention-norm output, reference infer.c:417-420)
 			launch_pdl(k_pf_norm, n, 256, 0, (const float*)pf.X, (const float*)w.rms_ffn_weight[l], pf.Nhi, pf.Nlo, n, c.dim, c.norm_eps, (int)c.norm_ln);
 			++g_launches;
 		}
 		PfGemmArgs u = {};
-		u.n_tokens = n, u.w[0] = w.w1[l], u.w[1] = w.w3[l], u.K = c.dim, u.Hhi = pf.Hhi, u.Hlo = pf.Hlo, u.hidden = c.hidden_dim, u.gelu = c.act_gelu;
-		pf_gemm<PF_UP, DBITS, KVT>(pf.tmN, u, c.hidden_dim, n);
+		u.K = c.dim, u.Hhi = pf.Hhi, u.Hlo = pf.Hlo, u.hidden = c.hidden_dim, u.gelu = c.act_gelu;
+		pf_gemm<PF_UP, DBITS>(pf.tmN, tw + 4, u, c.hidden_dim, n);
 
 		PfGemmArgs d = {};
-		d.n_tokens = n, d.w[0] = w.w2[l], d.K = c.hidden_dim, d.X = pf.X, d.dim = c.dim;
-		pf_gemm<PF_DOWN, DBITS, KVT>(pf.tmH, d, c.dim, n);
+		d.K = c.hidden_dim, d.X = pf.X, d.dim = c.dim;
+		pf_gemm<PF_RES, DBITS>(pf.tmH, tw + 6, d, c.dim, n);
 	}
 }
 
@@ -1423,6 +1473,7 @@ extern "C" int forward_prefill_cuda(struct Transformer* transformer, const int* 
 		default: pf_run<4, uint8_t>(m, pos0 + o); break;
 		}
 		CUDA_CHECK(cudaStreamSynchronize(g.stream)); // `tokens` is the caller's memory (pageable): the copy above must have left it
+		if (*(volatile int*)g.dev_err) CALM_FATAL("prompt pass: a wait inside a product gave up (code %d)", *(volatile int*)g.dev_err);
 	}
 	CUDA_CHECK(cudaGetLastError());
 	return 1;

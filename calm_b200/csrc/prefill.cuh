@@ -3,14 +3,11 @@
 // matrix is read once per 128-token tile instead of once per token and the projections become real GEMMs on the
 // 5th-generation tensor cores:
 //
-//   k_pf_gemm   D[128 weight rows][128 tokens] (+)= W_tile . X_tile^T with tcgen05.mma (kind::f16, cta_group::1), fp32
-//               accumulators in TMEM.  A = the weight tile, dequantised ON THE FLY by four warps from the model's own
-//               format (fp16 / e5m2 / gf4: all exact in f16) into the 128-byte-swizzled K-major shared-memory layout
-//               the MMA reads; B = the activations as TWO f16 matrices hi + lo (x = hi + lo to 22 bits, so the result
-//               carries fp32-grade inputs: two MMAs per k-step into the same accumulator), brought in by 2-D TMA
-//               (cp.async.bulk.tensor, SWIZZLE_128B).  One warp issues TMA, one thread issues MMAs, completion flows
-//               through mbarriers (tcgen05.commit), the epilogue reads TMEM with tcgen05.ld and applies what the
-//               decode kernels apply: bias / clip / RoPE / KV-cache append (QKV), residual add (wo, w2),
+//   k_pf_gemm   D[128 weight rows][<= 256 tokens] = W_tile . X_tile^T with tcgen05.mma (kind::f16, cta_group::1), fp32
+//               accumulators in TMEM.  A = the weight tile, widened ON THE FLY from the model's own format (fp16 / e5m2 /
+//               gf4: all exact in f16); B = the activations as TWO f16 matrices hi + lo (x = hi + lo to 22 bits, so the
+//               result carries fp32-grade inputs: two MMAs per k-step into the same accumulator).  The epilogue applies
+//               what the decode kernels apply: bias / clip / RoPE / KV-cache append (QKV), residual add (wo, w2),
 //               act(w1 x) * (w3 x) with both accumulators side by side in TMEM (FFN up).
 //   k_pf_attn   causal attention of the block against the cache (online softmax in fp32; reference infer.c:238-267), scores and
 //               values on warp-level tensor cores with hi + lo queries and weights against the cached fp16 / e5m2 entries.
@@ -25,14 +22,10 @@
 #include "stages.cuh"
 #include "tc05.cuh"
 
-#define PF_BM 128 // weight rows per tile  (TMEM lanes)
-#define PF_BN 128 // tokens per tile       (TMEM columns per accumulator)
-#define PF_BK 64  // k per stage: 64 f16 = 128 bytes = one swizzle atom
-#define PF_THREADS 192
-enum { PF_QKV = 0, PF_WO = 1, PF_UP = 2, PF_DOWN = 3 };
-
-// instruction descriptor, kind::f16: D = f32, A = B = f16, both K-major, M = 128, N = 128
-#define PF_IDESC ((1u << 4) | ((uint32_t)(PF_BN >> 3) << 17) | ((uint32_t)(PF_BM >> 4) << 24))
+#define PF_BM 128  // weight rows per tile  (TMEM lanes)
+#define PF_BK 64   // k per stage: 64 f16 = 128 bytes = one swizzle atom
+#define PF_PAD 128 // activation rows are allocated in multiples of this
+enum { PF_QKV = 0, PF_RES = 1 /* wo, w2 */, PF_UP = 2 };
 
 // ---------------------------------------------------------------- small kernels
 
@@ -91,13 +84,32 @@ __global__ void __launch_bounds__(256) k_pf_norm(const float* X, const float* no
 }
 
 // ---------------------------------------------------------------- the GEMM
+//
+// Persistent: a CTA walks work items = (one or two tiles of 128 weight rows, K-slice, bn tokens), token tiles fastest, so that
+// the CTAs running at one time share a weight tile's bytes in L2.  Roles, each with its own ring so that none waits for another's
+// latency: two warps stream the hi and the lo activation tiles and one the weight bytes in the model's format (TMA; a warp gets one
+// copy on its way every 300 cycles or so, hence three of them), warps 6-9 widen them to f16 in the swizzled layout of the MMA (fp16 weights arrive in it), warp 1 issues the MMAs, warps 2-5
+// drain one of two TMEM accumulators while the other is being filled.
+// Bound: the hand-overs of a k-stage, about 900 cycles of waits, commits and issue in the MMA warp that its MMAs (1150 cycles for two row tiles
+// and 128 tokens) only partly cover; loads with fixed addresses, no loads at all, or no widening measured the same.  So an item is as large as
+// TMEM allows.  14336 x 2 rows, K 4096, 2048 tokens: fp8 900 us, fp16 850 us; 4096 rows: 174 and 158 us.  (1324 and 387 us (fp8) before, when
+// every thread loaded its weight row one stage ahead.)
+struct PfMaps {
+	CUtensorMap x[2]; // activations, hi and lo: f16 [tokens][K], box = bn rows x 64 columns, 128-byte swizzle
+	CUtensorMap w[3]; // weights: QKV: wq, wk, wv   UP: w1, w3   WO / DOWN: w
+};
 
 struct PfGemmArgs {
-	const void* w[3]; // QKV: wq, wk, wv   UP: w1, w3   WO / DOWN: w
 	int K, n_tokens;
+	// work items
+	int rows, na, bn, splits; // weight rows; row tiles per item (UP: 2, w1 and w3); tokens per tile (64, 128 or 256, na * bn <= 256); K-slices
+	int nb;                   // activation slots (even: hi, lo, hi, lo ...)
+	float* ws;            // splits > 1: [item][na][bn][128] partial sums
+	unsigned* counter;    // splits > 1: [row tiles x token tiles], zero between launches
+	int* err;             // mapped host word: code of a wait that gave up
 	// QKV epilogue
 	float* Q;         // [T][q_dim]
-	int q_dim, kv_dim, head_dim, seq_len, pos0;
+	int q_dim, kv_dim, head_dim, seq_len, pos0, kvbits;
 	const float* bias;
 	float clip;
 	const float2* rope; // [T][head_dim / 2]
@@ -112,210 +124,363 @@ struct PfGemmArgs {
 	int hidden, gelu;
 };
 
-// 64 weights of one row (one k-stage) -> 8 swizzled 16-byte chunks of f16 in the A tile
+#define PF_TILE_BYTES (PF_BM * 128)
+#define PF_MAX_B 8
 template <int DBITS>
-__device__ __forceinline__ void pf_load_raw(const unsigned char* row, int kb, uint4 (&raw)[DBITS / 2]) {
-	const uint4* p = reinterpret_cast<const uint4*>(row + (size_t)kb * (PF_BK * DBITS / 8));
-#pragma unroll
-	for (int i = 0; i < DBITS / 2; ++i) raw[i] = ldg_stream(p + i);
+__host__ __device__ constexpr int pf_raw_bytes() {
+	return PF_BM * PF_BK * DBITS / 8;
 }
+// shared memory: widened weight tiles, weight tiles as stored (fp16: none), the rest activation slots
+template <int DBITS>
+__host__ __device__ constexpr int pf_a_tiles() {
+	return DBITS == 16 ? 6 : 4;
+}
+template <int DBITS>
+__host__ __device__ constexpr int pf_raw_tiles() {
+	return DBITS == 16 ? 0 : 32768 / pf_raw_bytes<DBITS>();
+}
+template <int DBITS>
+__host__ __device__ constexpr size_t pf_fixed_bytes() { // everything but the activation slots
+	return (size_t)pf_a_tiles<DBITS>() * PF_TILE_BYTES + pf_raw_tiles<DBITS>() * pf_raw_bytes<DBITS>() + 1024; // + alignment slack
+}
+template <int DBITS>
+__host__ __device__ constexpr int pf_threads() {
+	return DBITS == 16 ? 8 * 32 : 12 * 32;
+}
+
+// 64 weights of row r (one k-stage) out of the copied bytes.  The copy swizzles them (64-byte pattern for fp8, 32-byte for gf4), so that
+// a row per lane reads without bank conflicts.
+template <int DBITS>
+__device__ __forceinline__ void pf_load_raw(const unsigned char* raw, int r, uint4 (&w)[DBITS / 2]) {
+#pragma unroll
+	for (int i = 0; i < DBITS / 2; ++i) {
+		const int c = DBITS == 8 ? i ^ ((r >> 1) & 3) : i ^ ((r >> 2) & 1);
+		// volatile: these reads stay ahead of the arrival that lets the copy engine overwrite the slot
+		asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[i].x), "=r"(w[i].y), "=r"(w[i].z), "=r"(w[i].w) : "r"(smem_u32(raw + r * (PF_BK * DBITS / 8) + (c << 4))) : "memory");
+	}
+}
+// ... into 8 swizzled 16-byte chunks of f16 in the A tile
 template <int DBITS>
 __device__ __forceinline__ void pf_store_a(unsigned char* tile, int r, const uint4 (&raw)[DBITS / 2]) {
 	unsigned char* rowp = tile + r * 128;
 	auto put = [&](int c, uint4 v) { *reinterpret_cast<uint4*>(rowp + ((c ^ (r & 7)) << 4)) = v; };
-	if constexpr (DBITS == 16) {
 #pragma unroll
-		for (int c = 0; c < 8; ++c) put(c, raw[c]);
-	} else if constexpr (DBITS == 8) { // an e5m2 byte is the high byte of the f16 (reference infer.c:28-35)
-#pragma unroll
-		for (int i = 0; i < 4; ++i) {
-			const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+	for (int i = 0; i < DBITS / 2; ++i) {
+		const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+		if constexpr (DBITS == 8) { // an e5m2 byte is the high byte of the f16 (reference infer.c:28-35)
 			put(2 * i, make_uint4(__byte_perm(w[0], 0, 0x1404), __byte_perm(w[0], 0, 0x3424), __byte_perm(w[1], 0, 0x1404), __byte_perm(w[1], 0, 0x3424)));
 			put(2 * i + 1, make_uint4(__byte_perm(w[2], 0, 0x1404), __byte_perm(w[2], 0, 0x3424), __byte_perm(w[3], 0, 0x1404), __byte_perm(w[3], 0, 0x3424)));
-		}
-	} else { // gf4: (q - 4) * s / -4 (reference infer.c:37-40); at most 6 significant bits: exact in f16
-#pragma unroll
-		for (int i = 0; i < 2; ++i) {
-			const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+		} else { // gf4 (reference infer.c:37-40)
 #pragma unroll
 			for (int j = 0; j < 4; ++j) {
-				const float sf = e5m2_to_float((uint8_t)(w[j] & 0xff)) * -0.25f;
 				uint32_t h[4];
-#pragma unroll
-				for (int k = 0; k < 4; ++k) {
-					const float a0 = (float)((int)((w[j] >> (8 + 6 * k)) & 7) - 4) * sf, a1 = (float)((int)((w[j] >> (11 + 6 * k)) & 7) - 4) * sf;
-					h[k] = pack_h2(__float2half_rn(a0), __float2half_rn(a1));
-				}
+				gf4_to_h2(w[j], h);
 				put(4 * i + j, make_uint4(h[0], h[1], h[2], h[3]));
 			}
 		}
 	}
 }
 
+// What the decode kernels apply, on 32 tokens of one weight row: gr = row (lanes = consecutive rows), t0 = first token, v (v3: FFN up's second matrix) the sums.
 template <int MODE>
-__host__ __device__ constexpr int pf_stages() {
-	return MODE == PF_UP ? 3 : 4;
-}
-template <int MODE>
-__host__ __device__ constexpr size_t pf_stage_bytes() {
-	return (size_t)(MODE == PF_UP ? 2 : 1) * PF_BM * 128 + 2 * PF_BN * 128; // A tile(s) + B hi + B lo
-}
-template <int MODE>
-__host__ __device__ constexpr size_t pf_smem_bytes() {
-	return pf_stages<MODE>() * pf_stage_bytes<MODE>() + 1024; // + alignment slack
+__device__ __forceinline__ void pf_epilogue(const PfGemmArgs& a, int gr, int lane, int t0, const float (&v)[32], const float (&v3)[32]) {
+	if constexpr (MODE == PF_QKV) { // bias / clip / RoPE / KV-cache append
+		const bool is_q = gr < a.q_dim, is_k = !is_q && gr < a.q_dim + a.kv_dim; // uniform over a tile: the dims are multiples of 128
+		const int k = is_q ? gr : (is_k ? gr - a.q_dim : gr - a.q_dim - a.kv_dim);
+		const int d = k % a.head_dim, h = k / a.head_dim;
+		const float b = a.bias ? a.bias[gr] : 0.f;
+		const size_t kv0 = ((size_t)h * a.seq_len + a.pos0) * a.head_dim + d;
+#pragma unroll
+		for (int j = 0; j < 32; ++j) {
+			const int t = t0 + j;
+			float x = fminf(fmaxf(v[j] + b, -a.clip), a.clip);
+			const float other = __shfl_xor_sync(0xffffffffu, x, 1); // the row pair a rotation mixes sits in adjacent lanes
+			if (t < a.n_tokens) {
+				if (is_q || is_k) {
+					const float2 cs = a.rope[(size_t)t * (a.head_dim / 2) + (d >> 1)];
+					x = (lane & 1) ? fmaf(other, cs.y, x * cs.x) : fmaf(-other, cs.y, x * cs.x);
+				}
+				const size_t o = kv0 + (size_t)t * a.head_dim;
+				if (is_q) a.Q[(size_t)t * a.q_dim + k] = x;
+				else if (a.kvbits == 16) kv_store(reinterpret_cast<__half*>(is_k ? a.kc : a.vc) + o, x);
+				else kv_store(reinterpret_cast<uint8_t*>(is_k ? a.kc : a.vc) + o, x);
+			}
+		}
+	} else if constexpr (MODE == PF_UP) { // act(w1 x) * (w3 x)
+#pragma unroll
+		for (int j = 0; j < 32; ++j) {
+			const int t = t0 + j;
+			if (t < a.n_tokens) {
+				const float hv = (a.gelu ? act_gelu(v[j]) : act_silu(v[j])) * v3[j];
+				__half hh, hl;
+				split_hl(hv, hh, hl);
+				a.Hhi[(size_t)t * a.hidden + gr] = hh, a.Hlo[(size_t)t * a.hidden + gr] = hl;
+			}
+		}
+	} else { // residual add: all loads before the first store
+		float x[32];
+		float* p = a.X + (size_t)t0 * a.dim + gr;
+#pragma unroll
+		for (int j = 0; j < 32; ++j) x[j] = t0 + j < a.n_tokens ? __ldcg(p + (size_t)j * a.dim) : 0.f;
+#pragma unroll
+		for (int j = 0; j < 32; ++j)
+			if (t0 + j < a.n_tokens) p[(size_t)j * a.dim] = x[j] + v[j];
+	}
 }
 
-template <int MODE, int DBITS, typename KVT>
-__global__ void __launch_bounds__(PF_THREADS, 1) k_pf_gemm(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CUtensorMap tm_lo, const PfGemmArgs a) {
-	constexpr int STAGES = pf_stages<MODE>(), NA = MODE == PF_UP ? 2 : 1;
-	constexpr uint32_t TMEM_COLS = NA * PF_BN;
+// named barrier of `threads` threads that also tells whether `p` held for all of them
+__device__ __forceinline__ bool bar_and(int id, int threads, bool p) {
+	int all;
+	asm volatile(
+	    "{\n\t.reg .pred p, q;\n\t"
+	    "setp.ne.s32 p, %3, 0;\n\t"
+	    "barrier.cta.red.and.pred q, %1, %2, p;\n\t"
+	    "selp.s32 %0, 1, 0, q;\n\t}"
+	    : "=r"(all)
+	    : "r"(id), "r"(threads), "r"((int)p)
+	    : "memory");
+	return all != 0;
+}
+
+__device__ __forceinline__ bool elect_one() { // one lane of a converged warp
+	uint32_t p;
+	asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+	return p != 0;
+}
+
+template <int MODE, int DBITS>
+__global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid_constant__ PfMaps m, const PfGemmArgs a) {
+	constexpr int W_WARP = DBITS == 16 ? 6 : 10, LO_WARP = W_WARP + 1;
+	constexpr int AT = pf_a_tiles<DBITS>(), RT = pf_raw_tiles<DBITS>(), RAW = pf_raw_bytes<DBITS>();
 	extern __shared__ unsigned char smem_dyn[];
-	__shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], accum;
+	__shared__ __align__(8) uint64_t a_full[AT], a_empty[AT], r_full[RT ? RT : 1], r_empty[RT ? RT : 1], b_full[PF_MAX_B], b_empty[PF_MAX_B], acc_full[2], acc_empty[2];
 	__shared__ uint32_t tmem_base_s;
+	__shared__ int last_s;
 	unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-	const int row0 = blockIdx.x * PF_BM, tok0 = blockIdx.y * PF_BN;
-	const int nkb = a.K / PF_BK;
-	auto a_tile = [&](int s, int i) { return smem + (size_t)s * pf_stage_bytes<MODE>() + (size_t)i * PF_BM * 128; };
-	auto b_tile = [&](int s, int i) { return smem + (size_t)s * pf_stage_bytes<MODE>() + (size_t)NA * PF_BM * 128 + (size_t)i * PF_BN * 128; };
+	const int nkb = a.K / PF_BK, nb = a.nb, bn = a.bn, splits = a.splits, na = MODE == PF_UP ? 2 : a.na;
+	const int as = AT / na, rs = RT / na; // slots of na tiles
+	const int row_tiles = a.rows / PF_BM, tok_tiles = (a.n_tokens + bn - 1) / bn;
+	const int items = (MODE == PF_UP ? row_tiles : (row_tiles + na - 1) / na) * splits * tok_tiles;
+	const int b_bytes = bn * 128;
+	auto a_tile = [&](int s, int i) { return smem + (size_t)(s * na + i) * PF_TILE_BYTES; };
+	auto r_tile = [&](int s, int i) { return smem + (size_t)AT * PF_TILE_BYTES + (size_t)(s * na + i) * RAW; };
+	auto b_tile = [&](int s) { return smem + (size_t)AT * PF_TILE_BYTES + (size_t)RT * RAW + (size_t)s * b_bytes; };
+	// item -> first weight row, tiles, first token, k-stages [k0, k1)
+	struct Item {
+		int row0, cnt, tok0, k0, k1;
+	};
+	auto item_of = [&](int it) {
+		Item r;
+		const int q = it / tok_tiles, sp = q % splits, rt = q / splits * (MODE == PF_UP ? 1 : na);
+		r.tok0 = (it % tok_tiles) * bn, r.row0 = rt * PF_BM, r.cnt = MODE == PF_UP ? 2 : min(na, row_tiles - rt);
+		r.k0 = (int)((long)nkb * sp / splits), r.k1 = (int)((long)nkb * (sp + 1) / splits);
+		return r;
+	};
+	// every wait is bounded: a role whose wait gives up records a code and leaves its loop, the others follow, and the host reads the code
+	auto gave_up = [&](int code) {
+		if (a.err) *reinterpret_cast<volatile int*>(a.err) = code;
+		return false;
+	};
 
 	pdl_launch_next();
 	if (tid == 0) {
-		for (int s = 0; s < STAGES; ++s) mbar_init(&full[s], 1 + 4), mbar_init(&empty[s], 1);
-		mbar_init(&accum, 1);
+		for (int s = 0; s < AT; ++s) mbar_init(&a_full[s], DBITS == 16 ? 1 : 4), mbar_init(&a_empty[s], 1);
+		for (int s = 0; s < RT; ++s) mbar_init(&r_full[s], 1), mbar_init(&r_empty[s], 4);
+		for (int s = 0; s < nb; ++s) mbar_init(&b_full[s], 1), mbar_init(&b_empty[s], 1);
+		for (int s = 0; s < 2; ++s) mbar_init(&acc_full[s], 1), mbar_init(&acc_empty[s], 4);
 		mbar_init_fence();
 	}
-	if (warp == 1) tmem_alloc(&tmem_base_s, TMEM_COLS);
+	if (warp == 1) tmem_alloc(&tmem_base_s, 512);
 	tc_fence_before();
 	__syncthreads();
 	tc_fence_after();
-	const uint32_t tmem_base = tmem_base_s;
-	pdl_wait_prev(); // activations (and, for the KV rows, the cache) come from the previous kernels of the layer
+	const uint32_t tmem_base = tmem_base_s; // accumulator i of buffer b: columns 256 b + bn i
 
-	if (warp == 0) {
-		// ===== TMA producer: the two activation tiles of every k-stage
-		if (lane == 0) {
-			for (int kb = 0; kb < nkb; ++kb) {
-				const int s = kb % STAGES;
-				mbar_wait_guard(&empty[s], ((kb / STAGES) & 1) ^ 1);
-				mbar_expect_tx(&full[s], 2 * PF_BN * 128);
-				tma_load_2d(b_tile(s, 0), &tm_hi, kb * PF_BK, tok0, &full[s]);
-				tma_load_2d(b_tile(s, 1), &tm_lo, kb * PF_BK, tok0, &full[s]);
-			}
-		}
-	} else if (warp == 1) {
-		// ===== MMA issuer
-		if (lane == 0) {
-			for (int kb = 0; kb < nkb; ++kb) {
-				const int s = kb % STAGES;
-				mbar_wait_guard(&full[s], (kb / STAGES) & 1);
-				tc_fence_after();
-#pragma unroll
-				for (int k = 0; k < PF_BK / 16; ++k) { // 16 f16 = 32 bytes along K inside the swizzle atom: +2 in the 16-byte address field
-					const uint64_t db_hi = umma_desc_sw128(b_tile(s, 0)) + 2 * k, db_lo = umma_desc_sw128(b_tile(s, 1)) + 2 * k;
-#pragma unroll
-					for (int i = 0; i < NA; ++i) {
-						const uint64_t da = umma_desc_sw128(a_tile(s, i)) + 2 * k;
-						umma_f16(tmem_base + i * PF_BN, da, db_hi, PF_IDESC, (kb | k) ? 1u : 0u);
-						umma_f16(tmem_base + i * PF_BN, da, db_lo, PF_IDESC, 1u);
-					}
+	// The one-thread roles keep their warp together and elect a lane for the issuing: addresses and descriptors then live in uniform registers
+	// (one lane in a branch of its own spent 60 cycles per MMA on moving them).
+	bool ok = true;
+	if (warp == 0 || warp == LO_WARP) { // ===== activations: hi tiles in the even slots, lo tiles in the odd ones
+		pdl_wait_prev();
+		const bool el = elect_one();
+		const int lo = warp != 0;
+		int s = lo;
+		unsigned ph = 1;
+		for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+			const Item t = item_of(it);
+			for (int kb = t.k0; kb < t.k1; ++kb) {
+				if (!__all_sync(0xffffffffu, mbar_wait_bounded(&b_empty[s], ph))) {
+					ok = gave_up(9301);
+					break;
 				}
-				umma_commit(&empty[s]); // frees the stage when these MMAs have read it
-			}
-			umma_commit(&accum);
-		}
-	} else {
-		// ===== dequantising producers (one tile row per thread), then the epilogue (one accumulator row per thread)
-		const int r = tid - 64; // 0..127
-		const unsigned char* rowp[NA];
-		{
-			const size_t rowbytes = (size_t)a.K * DBITS / 8;
-			const int gr = row0 + r;
-			if constexpr (MODE == PF_QKV) {
-				const void* w = gr < a.q_dim ? a.w[0] : (gr < a.q_dim + a.kv_dim ? a.w[1] : a.w[2]);
-				const int k = gr < a.q_dim ? gr : (gr < a.q_dim + a.kv_dim ? gr - a.q_dim : gr - a.q_dim - a.kv_dim);
-				rowp[0] = reinterpret_cast<const unsigned char*>(w) + (size_t)k * rowbytes;
-			} else if constexpr (MODE == PF_UP) {
-				rowp[0] = reinterpret_cast<const unsigned char*>(a.w[0]) + (size_t)gr * rowbytes;
-				rowp[1] = reinterpret_cast<const unsigned char*>(a.w[1]) + (size_t)gr * rowbytes;
-			} else {
-				rowp[0] = reinterpret_cast<const unsigned char*>(a.w[0]) + (size_t)gr * rowbytes;
+				if (el) {
+					mbar_expect_tx(&b_full[s], b_bytes);
+					tma_load_2d(b_tile(s), &m.x[lo], kb * PF_BK, t.tok0, &b_full[s]);
+				}
+				if ((s += 2) >= nb) s = lo, ph ^= 1;
 			}
 		}
-		uint4 raw[NA][DBITS / 2];
+	} else if (warp == 1) { // ===== MMAs
+		// kind::f16: D = f32, A = B = f16, both K-major, M = 128, N = bn
+		const uint32_t idesc = (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(PF_BM >> 4) << 24);
+		const bool el = elect_one();
+		int s = 0, sa = 0;
+		unsigned ph = 0, pa = 0, q = 0;
+		for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++q) {
+			const Item t = item_of(it);
+			const uint32_t acc = tmem_base + (q & 1) * 256;
+			if (!__all_sync(0xffffffffu, mbar_wait_bounded(&acc_empty[q & 1], ((q >> 1) & 1) ^ 1))) ok = gave_up(9302);
+			tc_fence_after();
+			for (int kb = t.k0; kb < t.k1 && ok; ++kb) {
+				if (!__all_sync(0xffffffffu, mbar_wait_bounded(&a_full[sa], pa))) ok = gave_up(9303);
+				for (int half = 0; half < 2 && ok; ++half) {
+					if (!__all_sync(0xffffffffu, mbar_wait_bounded(&b_full[s], ph))) {
+						ok = gave_up(9304);
+						break;
+					}
+					if (el) {
+						const uint64_t db = umma_desc_sw128(b_tile(s)), da = umma_desc_sw128(a_tile(sa, 0));
 #pragma unroll
-		for (int i = 0; i < NA; ++i) pf_load_raw<DBITS>(rowp[i], 0, raw[i]);
-		for (int kb = 0; kb < nkb; ++kb) {
-			const int s = kb % STAGES;
-			mbar_wait_guard(&empty[s], ((kb / STAGES) & 1) ^ 1);
-#pragma unroll
-			for (int i = 0; i < NA; ++i) pf_store_a<DBITS>(a_tile(s, i), r, raw[i]);
-			if (kb + 1 < nkb) { // the next stage's bytes travel while this one is being multiplied
-#pragma unroll
-				for (int i = 0; i < NA; ++i) pf_load_raw<DBITS>(rowp[i], kb + 1, raw[i]);
+						for (int k = 0; k < PF_BK / 16; ++k) { // 16 f16 = 32 bytes along K inside the swizzle atom: +2 in the 16-byte address field
+							const uint32_t add = (kb > t.k0 || half || k) ? 1u : 0u;
+							umma_f16(acc, da + 2 * k, db + 2 * k, idesc, add);
+							if (t.cnt == 2) umma_f16(acc + bn, da + (PF_TILE_BYTES >> 4) + 2 * k, db + 2 * k, idesc, add);
+						}
+						umma_commit(&b_empty[s]); // frees the slot when these MMAs have read it
+						if (half) umma_commit(&a_empty[sa]);
+					}
+					__syncwarp();
+					if (++s == nb) s = 0, ph ^= 1;
+				}
+				if (++sa == as) sa = 0, pa ^= 1;
 			}
-			fence_async_smem();
+			if (el) umma_commit(&acc_full[q & 1]);
 			__syncwarp();
-			if (lane == 0) mbar_arrive(&full[s]);
 		}
-
-		mbar_wait_guard(&accum, 0);
-		tc_fence_after();
-		const int q4 = warp & 3; // the TMEM lane quarter this warp may read
-		const int lr = q4 * 32 + lane, gr = row0 + lr;
-		for (int c0 = 0; c0 < PF_BN; c0 += 32) {
-			float v[32];
-			tmem_ld32(tmem_base + ((uint32_t)(q4 * 32) << 16) + c0, v);
-			if constexpr (MODE == PF_QKV) {
-				const bool is_q = gr < a.q_dim, is_k = !is_q && gr < a.q_dim + a.kv_dim;
-				const int k = is_q ? gr : (is_k ? gr - a.q_dim : gr - a.q_dim - a.kv_dim);
-				const int d = k % a.head_dim, h = k / a.head_dim;
-				const float b = a.bias ? a.bias[gr] : 0.f;
-#pragma unroll
-				for (int j = 0; j < 32; ++j) {
-					const int t = tok0 + c0 + j;
-					float x = fminf(fmaxf(v[j] + b, -a.clip), a.clip);
-					const float other = __shfl_xor_sync(0xffffffffu, x, 1); // the row pair a rotation mixes sits in adjacent lanes
-					if (t < a.n_tokens) {
-						if (is_q || is_k) {
-							const float2 cs = a.rope[(size_t)t * (a.head_dim / 2) + (d >> 1)];
-							x = (lane & 1) ? fmaf(other, cs.y, x * cs.x) : fmaf(-other, cs.y, x * cs.x);
-						}
-						if (is_q) {
-							a.Q[(size_t)t * a.q_dim + k] = x;
-						} else {
-							KVT* dst = reinterpret_cast<KVT*>(is_k ? a.kc : a.vc) + ((size_t)h * a.seq_len + a.pos0 + t) * a.head_dim + d;
-							kv_store(dst, x);
-						}
+	} else if (warp < 6) { // ===== epilogue: one accumulator row per thread
+		pdl_wait_prev();
+		const int q4 = warp & 3, lr = q4 * 32 + lane; // the TMEM lane quarter this warp may read
+		unsigned q = 0;
+		for (int it = blockIdx.x; it < items; it += gridDim.x, ++q) {
+			const Item t = item_of(it);
+			const uint32_t acc = tmem_base + (q & 1) * 256 + ((uint32_t)(q4 * 32) << 16);
+			// the four warps go on together or leave together: none is left alone at a named barrier
+			if (!bar_and(1, 128, mbar_wait_bounded(&acc_full[q & 1], (q >> 1) & 1))) {
+				gave_up(9305);
+				break;
+			}
+			tc_fence_after();
+			const int cols = min(bn, a.n_tokens - t.tok0);
+			float v[32], v3[32];
+			if (splits == 1) {
+				for (int i = 0; i < (MODE == PF_UP ? 1 : t.cnt); ++i)
+					for (int c0 = 0; c0 < cols; c0 += 32) {
+						tmem_ld32(acc + i * bn + c0, v);
+						if (MODE == PF_UP) tmem_ld32(acc + bn + c0, v3);
+						pf_epilogue<MODE>(a, t.row0 + i * PF_BM + lr, lane, t.tok0 + c0, v, v3);
 					}
-				}
-			} else if constexpr (MODE == PF_UP) {
-				float v3[32];
-				tmem_ld32(tmem_base + ((uint32_t)(q4 * 32) << 16) + PF_BN + c0, v3);
-#pragma unroll
-				for (int j = 0; j < 32; ++j) {
-					const int t = tok0 + c0 + j;
-					if (t < a.n_tokens) {
-						const float hv = (a.gelu ? act_gelu(v[j]) : act_silu(v[j])) * v3[j];
-						__half hh, hl;
-						split_hl(hv, hh, hl);
-						a.Hhi[(size_t)t * a.hidden + gr] = hh, a.Hlo[(size_t)t * a.hidden + gr] = hl;
-					}
-				}
 			} else {
+				for (int i = 0; i < t.cnt; ++i)
+					for (int c0 = 0; c0 < cols; c0 += 32) {
+						tmem_ld32(acc + i * bn + c0, v);
+						float* p = a.ws + ((size_t)(it * na + i) * bn + c0) * PF_BM + lr;
 #pragma unroll
-				for (int j = 0; j < 32; ++j) {
-					const int t = tok0 + c0 + j;
-					if (t < a.n_tokens) a.X[(size_t)t * a.dim + gr] += v[j];
+						for (int j = 0; j < 32; ++j) __stcg(p + j * PF_BM, v[j]);
+					}
+			}
+			tc_fence_before();
+			__syncwarp();
+			if (lane == 0) mbar_arrive(&acc_empty[q & 1]);
+			if (splits > 1) { // the last slice of a tile to arrive adds all of them up in slice order
+				const int tile = it / tok_tiles / splits * tok_tiles + it % tok_tiles;
+				__threadfence();
+				asm volatile("bar.sync 1, 128;" ::: "memory");
+				if (tid == 64) {
+					const bool last = atomicAdd(a.counter + tile, 1u) == (unsigned)splits - 1;
+					if (last) a.counter[tile] = 0;
+					last_s = last;
 				}
+				asm volatile("bar.sync 1, 128;" ::: "memory");
+				const bool last = last_s;
+				asm volatile("bar.sync 1, 128;" ::: "memory");
+				if (!last) continue;
+				__threadfence();
+				const int first = it / tok_tiles / splits * splits * tok_tiles + it % tok_tiles; // item of slice 0
+				auto fold = [&](int i, int c0, float(&sum)[32]) {
+#pragma unroll
+					for (int j = 0; j < 32; ++j) sum[j] = 0.f;
+					for (int sp = 0; sp < splits; ++sp) {
+						const float* p = a.ws + ((size_t)((first + sp * tok_tiles) * na + i) * bn + c0) * PF_BM + lr;
+#pragma unroll
+						for (int j = 0; j < 32; ++j) sum[j] += __ldcg(p + j * PF_BM);
+					}
+				};
+				for (int i = 0; i < (MODE == PF_UP ? 1 : t.cnt); ++i)
+					for (int c0 = 0; c0 < cols; c0 += 32) {
+						fold(i, c0, v);
+						if (MODE == PF_UP) fold(1, c0, v3);
+						pf_epilogue<MODE>(a, t.row0 + i * PF_BM + lr, lane, t.tok0 + c0, v, v3);
+					}
 			}
 		}
-		tc_fence_before();
+	} else if (warp == W_WARP) { // ===== weights: immutable, so the first tiles are requested before the previous kernel has finished
+		uint64_t* full = DBITS == 16 ? a_full : r_full;
+		uint64_t* empty = DBITS == 16 ? a_empty : r_empty;
+		const int ws = DBITS == 16 ? as : rs;
+		const bool el = elect_one();
+		int s = 0;
+		unsigned ph = 1;
+		for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+			const Item t = item_of(it);
+			for (int kb = t.k0; kb < t.k1; ++kb) {
+				if (!__all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], ph))) {
+					ok = gave_up(9306);
+					break;
+				}
+				if (el) {
+					mbar_expect_tx(&full[s], t.cnt * RAW);
+					for (int i = 0; i < t.cnt; ++i) {
+						int row = t.row0 + (MODE == PF_UP ? 0 : i * PF_BM), which = MODE == PF_UP ? i : 0;
+						if (MODE == PF_QKV && row >= a.q_dim) {
+							row -= a.q_dim, which = 1;
+							if (row >= a.kv_dim) row -= a.kv_dim, which = 2;
+						}
+						tma_load_2d(DBITS == 16 ? a_tile(s, i) : r_tile(s, i), &m.w[which], kb * (DBITS == 16 ? PF_BK : PF_BK * DBITS / 8), row, &full[s]);
+					}
+				}
+				if (++s == ws) s = 0, ph ^= 1;
+			}
+		}
+	} else if constexpr (DBITS != 16) { // ===== widening: one tile row per thread
+		const int r = tid - 192;
+		int sr = 0, sa = 0;
+		unsigned pr = 0, pe = 1;
+		for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+			const Item t = item_of(it);
+			for (int kb = t.k0; kb < t.k1 && ok; ++kb) {
+				uint4 raw[2][DBITS / 2];
+				if (!mbar_wait_bounded(&r_full[sr], pr)) ok = gave_up(9307);
+				pf_load_raw<DBITS>(r_tile(sr, 0), r, raw[0]);
+				if (t.cnt == 2) pf_load_raw<DBITS>(r_tile(sr, 1), r, raw[1]);
+				fence_async_smem(); // the copy engine writes next what was read here
+				__syncwarp();
+				if (lane == 0) mbar_arrive(&r_empty[sr]);
+				if (!mbar_wait_bounded(&a_empty[sa], pe)) ok = gave_up(9308);
+				pf_store_a<DBITS>(a_tile(sa, 0), r, raw[0]);
+				if (t.cnt == 2) pf_store_a<DBITS>(a_tile(sa, 1), r, raw[1]);
+				fence_async_smem();
+				__syncwarp();
+				if (lane == 0) mbar_arrive(&a_full[sa]);
+				if (++sr == rs) sr = 0, pr ^= 1;
+				if (++sa == as) sa = 0, pe ^= 1;
+			}
+		}
 	}
+	tc_fence_before();
 	__syncthreads();
 	if (warp == 1) {
 		tc_fence_after();
-		tmem_dealloc(tmem_base, TMEM_COLS);
+		tmem_dealloc(tmem_base, 512);
 	}
 }
 

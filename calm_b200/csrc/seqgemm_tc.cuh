@@ -31,13 +31,6 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
 	             "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
 	             : "memory");
 }
-// about a second at most; false = gave up
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity) {
-	for (unsigned spins = 0; spins < (1u << 24); ++spins)
-		if (mbar_try_wait(bar, parity)) return true;
-	return false;
-}
-
 // The epilogue of one warp: its 32 weight rows (lane = row m) against the tile's tokens, 32 at a time.  E: what the epilogue does when it is one
 // of the plain ones -- a bias at most, and for EPI_F32 columns past `split` in the activation type -- with everything that does not depend on
 // the token worked out before the loop; TG_ANY: gemm_store decides per element.

@@ -53,15 +53,11 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 	             "r"(c0), "r"(c1), "r"(smem_u32(bar))
 	             : "memory");
 }
-// bounded wait (about 2 s): a broken pipeline traps with a message instead of hanging the GPU
-__device__ __forceinline__ void mbar_wait_guard(uint64_t* bar, uint32_t parity) {
-	unsigned spins = 0;
-	while (!mbar_try_wait(bar, parity)) {
-		if (++spins > (1u << 26)) {
-			printf("calm_b200: k_pf_gemm pipeline stalled (block %d,%d thread %d)\n", blockIdx.x, blockIdx.y, threadIdx.x);
-			__trap();
-		}
-	}
+// about a second at most; false = gave up
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity) {
+	for (unsigned spins = 0; spins < (1u << 24); ++spins)
+		if (mbar_try_wait(bar, parity)) return true;
+	return false;
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 	asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");

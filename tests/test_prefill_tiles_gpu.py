@@ -23,3 +23,14 @@ def test_attention_groups_and_edges(heads, kv, hd, n, pos0, kvbits):
     toks = mg.teacher_tokens(spec.vocab_size, n + 1)
     serial, batched = _both(spec, mg.generate(spec, seed=4), toks, pos0, 256, kvbits, warm=mg.teacher_tokens(spec.vocab_size, pos0, start=500))
     _check(spec, serial, batched, kvbits, f"heads {heads}/{kv}x{hd}, {n} at {pos0}, kv{kvbits}")
+
+
+# Products: one and two row tiles per item (an odd number of row tiles leaves a single one), 64 / 128 / 256 tokens per tile with ragged last tiles, K cut into
+# slices (small models) and not, many items per CTA, all three weight formats.  The cache after two layers sees every product.
+@pytest.mark.parametrize("dtype", ["fp8", "gf4", "fp16"])
+@pytest.mark.parametrize("dim,heads,kv,hidden,n", [(384, 3, 1, 1152, 1), (896, 7, 1, 2432, 61), (1024, 8, 2, 3456, 65), (2048, 16, 4, 5504, 257), (4096, 32, 8, 14336, 130)])
+def test_product_tiles(dtype, dim, heads, kv, hidden, n):
+    spec = replace(mg.SPECS["pf-tiny"], name="tiles", dtype=dtype, dim=dim, n_heads=heads, n_kv_heads=kv, head_dim=128, hidden_dim=hidden, max_seq_len=512)
+    toks = mg.teacher_tokens(spec.vocab_size, n + 1)
+    serial, batched = _both(spec, mg.generate(spec, seed=6), toks, 0, 512, 16)
+    _check(spec, serial, batched, 16, f"{dtype} dim {dim} hidden {hidden}, {n} tokens")
