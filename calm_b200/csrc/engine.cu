@@ -1348,15 +1348,15 @@ static bool pf_supported() {
 }
 
 // Row tiles and tokens per item and K-slices of a product of `rows` weight rows over n tokens: the choice with the least estimated time, in cycles.
-// A k-stage was measured at 1600 / 1880 / 2660 cycles for one row tile and 64 / 128 / 256 tokens, at 2000 / 2550 for two (fp8, 4096 x 4096 x 2048
-// tokens; 370 / 260 / 184 / 276 / 176 us), so the widest item wins while every SM has one and smaller ones win below; K is sliced only
-// while an item per SM is left over, and a slice pays for its way through memory.
+// A k-stage was measured at 1040 / 1290 / 2070 cycles for one row tile and 64 / 128 / 256 tokens, at 2010 for two and 128 (fp8, 4096 x 4096 x 2048
+// tokens: 251 / 178 / 143 / 139 us), so wide items win while every SM has one, two row tiles (half the activation bytes) first; K
+// is sliced only while an item per SM is left over, and a slice pays for its way through memory.
 static void pf_tiles(int mode, int rows, int n, int nkb, PfGemmArgs& a) {
 	long best = -1;
-	for (int na = mode == PF_UP ? 2 : 1; na <= 2; ++na)
+	for (int na = 2; na >= (mode == PF_UP ? 2 : 1); --na)
 		for (int bn = 64; bn * na <= 256; bn *= 2) {
 			const int tiles = (mode == PF_UP ? rows / PF_BM : cdiv(rows / PF_BM, na)) * cdiv(n, bn);
-			const int stage = 900 + na * bn * 5;
+			const int stage = 650 + na * bn * 5;
 			for (int sp = 1; sp == 1 || (tiles * sp <= g.sms && sp * 2 <= nkb && sp <= 16); ++sp) {
 				const long cost = (long)cdiv(tiles * sp, g.sms) * cdiv(nkb, sp) * stage + na * bn * 20 + (sp > 1 ? 5000 + na * bn * (20 + 15 * sp) : 0);
 				if (best < 0 || cost < best) best = cost, a.na = na, a.bn = bn, a.splits = sp;
@@ -1375,11 +1375,11 @@ static void pf_gemm(const CUtensorMap (&tx)[3][2], const CUtensorMap* tw, PfGemm
 	memcpy(m.x, tx[a.bn / 128], sizeof(m.x)); // 64, 128, 256 -> 0, 1, 2
 	memcpy(m.w, tw, (MODE == PF_QKV ? 3 : MODE == PF_UP ? 2 : 1) * sizeof(CUtensorMap));
 	a.n_tokens = n, a.rows = rows, a.ws = pf.ws, a.counter = pf.counter, a.err = g.dev_err;
-	a.nb = imin(PF_MAX_B, (int)((limit - fixed) / (a.bn * 128)) & ~1);
+	a.stages = imin(PF_MAX_STAGES, (int)((limit - fixed) / pf_stage_bytes(a.na, a.bn)));
 	const int row_items = MODE == PF_UP ? rows / PF_BM : cdiv(rows / PF_BM, a.na);
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3(imin(g.sms, row_items * a.splits * cdiv(n, a.bn))), cfg.blockDim = dim3(pf_threads<DBITS>()), cfg.stream = g.stream;
-	cfg.dynamicSmemBytes = fixed + (size_t)a.nb * a.bn * 128;
+	cfg.dynamicSmemBytes = fixed + a.stages * pf_stage_bytes(a.na, a.bn);
 	cudaLaunchAttribute at[1];
 	at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
 	at[0].val.programmaticStreamSerializationAllowed = g.use_pdl ? 1 : 0;

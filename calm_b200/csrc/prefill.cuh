@@ -87,13 +87,13 @@ __global__ void __launch_bounds__(256) k_pf_norm(const float* X, const float* no
 //
 // Persistent: a CTA walks work items = (one or two tiles of 128 weight rows, K-slice, bn tokens), token tiles fastest, so that
 // the CTAs running at one time share a weight tile's bytes in L2.  Roles, each with its own ring so that none waits for another's
-// latency: two warps stream the hi and the lo activation tiles and one the weight bytes in the model's format (TMA; a warp gets one
-// copy on its way every 300 cycles or so, hence three of them), warps 6-9 widen them to f16 in the swizzled layout of the MMA (fp16 weights arrive in it), warp 1 issues the MMAs, warps 2-5
-// drain one of two TMEM accumulators while the other is being filled.
-// Bound: the hand-overs of a k-stage, about 900 cycles of waits, commits and issue in the MMA warp that its MMAs (1150 cycles for two row tiles
-// and 128 tokens) only partly cover; loads with fixed addresses, no loads at all, or no widening measured the same.  So an item is as large as
-// TMEM allows.  14336 x 2 rows, K 4096, 2048 tokens: fp8 900 us, fp16 850 us; 4096 rows: 174 and 158 us.  (1324 and 387 us (fp8) before, when
-// every thread loaded its weight row one stage ahead.)
+// latency: two warps stream the hi and the lo activation tiles and one the weight bytes in the model's format (TMA; a warp gets one copy on its
+// way every 300 cycles or so), four or eight widen them to f16 in the swizzled layout of the MMA (fp16 weights arrive in it), warp 1
+// issues the MMAs, warps 2-5 drain one of two TMEM accumulators while the other is being filled.
+// Bound: the MMA warp's hand-overs.  A stage's MMAs take 1150 cycles for two row tiles and 128 tokens; with a wait and a commit for the weights,
+// for hi and for lo a stage cost 2000, with one of each 1550, so everything a stage needs arrives on one barrier and an item is as
+// large as TMEM allows.  14336 x 2 rows, K 4096, 2048 tokens: fp8 696 us, fp16 683 us (1380 TFLOP/s, hi and lo counted; 900 and 850 us with
+// three barriers; 1324 us (fp8) when every thread loaded its weight row one stage ahead); 4096 rows: 139 and 128 us (387 us).
 struct PfMaps {
 	CUtensorMap x[2]; // activations, hi and lo: f16 [tokens][K], box = bn rows x 64 columns, 128-byte swizzle
 	CUtensorMap w[3]; // weights: QKV: wq, wk, wv   UP: w1, w3   WO / DOWN: w
@@ -103,7 +103,7 @@ struct PfGemmArgs {
 	int K, n_tokens;
 	// work items
 	int rows, na, bn, splits; // weight rows; row tiles per item (UP: 2, w1 and w3); tokens per tile (64, 128 or 256, na * bn <= 256); K-slices
-	int nb;                   // activation slots (even: hi, lo, hi, lo ...)
+	int stages;               // in flight
 	float* ws;            // splits > 1: [item][na][bn][128] partial sums
 	unsigned* counter;    // splits > 1: [row tiles x token tiles], zero between launches
 	int* err;             // mapped host word: code of a wait that gave up
@@ -125,58 +125,55 @@ struct PfGemmArgs {
 };
 
 #define PF_TILE_BYTES (PF_BM * 128)
-#define PF_MAX_B 8
+#define PF_MAX_STAGES 6
 template <int DBITS>
 __host__ __device__ constexpr int pf_raw_bytes() {
 	return PF_BM * PF_BK * DBITS / 8;
 }
-// shared memory: widened weight tiles, weight tiles as stored (fp16: none), the rest activation slots
-template <int DBITS>
-__host__ __device__ constexpr int pf_a_tiles() {
-	return DBITS == 16 ? 6 : 4;
-}
+// shared memory: weight tiles as stored (fp16: none), then stages = widened weight tiles, hi tile, lo tile
 template <int DBITS>
 __host__ __device__ constexpr int pf_raw_tiles() {
 	return DBITS == 16 ? 0 : 32768 / pf_raw_bytes<DBITS>();
 }
 template <int DBITS>
-__host__ __device__ constexpr size_t pf_fixed_bytes() { // everything but the activation slots
-	return (size_t)pf_a_tiles<DBITS>() * PF_TILE_BYTES + pf_raw_tiles<DBITS>() * pf_raw_bytes<DBITS>() + 1024; // + alignment slack
+__host__ __device__ constexpr size_t pf_fixed_bytes() { // everything but the stages
+	return (size_t)pf_raw_tiles<DBITS>() * pf_raw_bytes<DBITS>() + 1024; // + alignment slack
+}
+__host__ __device__ inline size_t pf_stage_bytes(int na, int bn) {
+	return (size_t)na * PF_TILE_BYTES + 2 * bn * 128;
+}
+template <int DBITS>
+__host__ __device__ constexpr int pf_widen_warps() { // FFN up as below: fp8 696 us with four warps and 802 with eight (more arrivals per stage), gf4 871 and 825 (19 instructions per 8 weights)
+	return DBITS == 16 ? 0 : DBITS == 8 ? 4 : 8;
 }
 template <int DBITS>
 __host__ __device__ constexpr int pf_threads() {
-	return DBITS == 16 ? 8 * 32 : 12 * 32;
+	return (8 + pf_widen_warps<DBITS>()) * 32;
 }
 
-// 64 weights of row r (one k-stage) out of the copied bytes.  The copy swizzles them (64-byte pattern for fp8, 32-byte for gf4), so that
-// a row per lane reads without bank conflicts.
+// 16 bytes i of row r (one k-stage of it) out of the copied bytes.  The copy swizzles them (64-byte pattern for fp8, 32-byte for gf4), so that a
+// row per lane reads without bank conflicts.
 template <int DBITS>
-__device__ __forceinline__ void pf_load_raw(const unsigned char* raw, int r, uint4 (&w)[DBITS / 2]) {
-#pragma unroll
-	for (int i = 0; i < DBITS / 2; ++i) {
-		const int c = DBITS == 8 ? i ^ ((r >> 1) & 3) : i ^ ((r >> 2) & 1);
-		// volatile: these reads stay ahead of the arrival that lets the copy engine overwrite the slot
-		asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[i].x), "=r"(w[i].y), "=r"(w[i].z), "=r"(w[i].w) : "r"(smem_u32(raw + r * (PF_BK * DBITS / 8) + (c << 4))) : "memory");
-	}
+__device__ __forceinline__ uint4 pf_load_raw(const unsigned char* raw, int r, int i) {
+	const int c = DBITS == 8 ? i ^ ((r >> 1) & 3) : i ^ ((r >> 2) & 1);
+	uint4 w;
+	// volatile: these reads stay ahead of the arrival that lets the copy engine overwrite the slot
+	asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "r"(smem_u32(raw + r * (PF_BK * DBITS / 8) + (c << 4))) : "memory");
+	return w;
 }
-// ... into 8 swizzled 16-byte chunks of f16 in the A tile
+// ... widened: 16 / 32 weights are 2 / 4 16-byte chunks of f16
 template <int DBITS>
-__device__ __forceinline__ void pf_store_a(unsigned char* tile, int r, const uint4 (&raw)[DBITS / 2]) {
-	unsigned char* rowp = tile + r * 128;
-	auto put = [&](int c, uint4 v) { *reinterpret_cast<uint4*>(rowp + ((c ^ (r & 7)) << 4)) = v; };
+__device__ __forceinline__ void pf_widen(const uint4& raw, uint4* out) {
+	const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+	if constexpr (DBITS == 8) { // an e5m2 byte is the high byte of the f16 (reference infer.c:28-35)
+		out[0] = make_uint4(__byte_perm(w[0], 0, 0x1404), __byte_perm(w[0], 0, 0x3424), __byte_perm(w[1], 0, 0x1404), __byte_perm(w[1], 0, 0x3424));
+		out[1] = make_uint4(__byte_perm(w[2], 0, 0x1404), __byte_perm(w[2], 0, 0x3424), __byte_perm(w[3], 0, 0x1404), __byte_perm(w[3], 0, 0x3424));
+	} else { // gf4 (reference infer.c:37-40)
 #pragma unroll
-	for (int i = 0; i < DBITS / 2; ++i) {
-		const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
-		if constexpr (DBITS == 8) { // an e5m2 byte is the high byte of the f16 (reference infer.c:28-35)
-			put(2 * i, make_uint4(__byte_perm(w[0], 0, 0x1404), __byte_perm(w[0], 0, 0x3424), __byte_perm(w[1], 0, 0x1404), __byte_perm(w[1], 0, 0x3424)));
-			put(2 * i + 1, make_uint4(__byte_perm(w[2], 0, 0x1404), __byte_perm(w[2], 0, 0x3424), __byte_perm(w[3], 0, 0x1404), __byte_perm(w[3], 0, 0x3424)));
-		} else { // gf4 (reference infer.c:37-40)
-#pragma unroll
-			for (int j = 0; j < 4; ++j) {
-				uint32_t h[4];
-				gf4_to_h2(w[j], h);
-				put(4 * i + j, make_uint4(h[0], h[1], h[2], h[3]));
-			}
+		for (int j = 0; j < 4; ++j) {
+			uint32_t h[4];
+			gf4_to_h2(w[j], h);
+			out[j] = make_uint4(h[0], h[1], h[2], h[3]);
 		}
 	}
 }
@@ -191,19 +188,23 @@ __device__ __forceinline__ void pf_epilogue(const PfGemmArgs& a, int gr, int lan
 		const float b = a.bias ? a.bias[gr] : 0.f;
 		const size_t kv0 = ((size_t)h * a.seq_len + a.pos0) * a.head_dim + d;
 #pragma unroll
-		for (int j = 0; j < 32; ++j) {
-			const int t = t0 + j;
-			float x = fminf(fmaxf(v[j] + b, -a.clip), a.clip);
-			const float other = __shfl_xor_sync(0xffffffffu, x, 1); // the row pair a rotation mixes sits in adjacent lanes
-			if (t < a.n_tokens) {
-				if (is_q || is_k) {
-					const float2 cs = a.rope[(size_t)t * (a.head_dim / 2) + (d >> 1)];
-					x = (lane & 1) ? fmaf(other, cs.y, x * cs.x) : fmaf(-other, cs.y, x * cs.x);
+		for (int j0 = 0; j0 < 32; j0 += 16) { // the angles of 16 tokens at a time, all loads before the first store (one by one they cost a round trip each)
+			float2 cs[16];
+#pragma unroll
+			for (int j = 0; j < 16; ++j)
+				cs[j] = (is_q || is_k) && t0 + j0 + j < a.n_tokens ? __ldcg(a.rope + (size_t)(t0 + j0 + j) * (a.head_dim / 2) + (d >> 1)) : make_float2(1.f, 0.f);
+#pragma unroll
+			for (int j = 0; j < 16; ++j) {
+				const int t = t0 + j0 + j;
+				float x = fminf(fmaxf(v[j0 + j] + b, -a.clip), a.clip);
+				const float other = __shfl_xor_sync(0xffffffffu, x, 1); // the row pair a rotation mixes sits in adjacent lanes
+				if (is_q || is_k) x = (lane & 1) ? fmaf(other, cs[j].y, x * cs[j].x) : fmaf(-other, cs[j].y, x * cs[j].x);
+				if (t < a.n_tokens) {
+					const size_t o = kv0 + (size_t)t * a.head_dim;
+					if (is_q) a.Q[(size_t)t * a.q_dim + k] = x;
+					else if (a.kvbits == 16) kv_store(reinterpret_cast<__half*>(is_k ? a.kc : a.vc) + o, x);
+					else kv_store(reinterpret_cast<uint8_t*>(is_k ? a.kc : a.vc) + o, x);
 				}
-				const size_t o = kv0 + (size_t)t * a.head_dim;
-				if (is_q) a.Q[(size_t)t * a.q_dim + k] = x;
-				else if (a.kvbits == 16) kv_store(reinterpret_cast<__half*>(is_k ? a.kc : a.vc) + o, x);
-				else kv_store(reinterpret_cast<uint8_t*>(is_k ? a.kc : a.vc) + o, x);
 			}
 		}
 	} else if constexpr (MODE == PF_UP) { // act(w1 x) * (w3 x)
@@ -250,22 +251,23 @@ __device__ __forceinline__ bool elect_one() { // one lane of a converged warp
 
 template <int MODE, int DBITS>
 __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid_constant__ PfMaps m, const PfGemmArgs a) {
-	constexpr int W_WARP = DBITS == 16 ? 6 : 10, LO_WARP = W_WARP + 1;
-	constexpr int AT = pf_a_tiles<DBITS>(), RT = pf_raw_tiles<DBITS>(), RAW = pf_raw_bytes<DBITS>();
+	constexpr int WIDEN = pf_widen_warps<DBITS>(), W_WARP = 6 + WIDEN, LO_WARP = W_WARP + 1;
+	constexpr int RT = pf_raw_tiles<DBITS>(), RAW = pf_raw_bytes<DBITS>();
 	extern __shared__ unsigned char smem_dyn[];
-	__shared__ __align__(8) uint64_t a_full[AT], a_empty[AT], r_full[RT ? RT : 1], r_empty[RT ? RT : 1], b_full[PF_MAX_B], b_empty[PF_MAX_B], acc_full[2], acc_empty[2];
+	__shared__ __align__(8) uint64_t full[PF_MAX_STAGES], empty[PF_MAX_STAGES], r_full[RT ? RT : 1], r_empty[RT ? RT : 1], acc_full[2], acc_empty[2];
 	__shared__ uint32_t tmem_base_s;
 	__shared__ int last_s;
 	unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-	const int nkb = a.K / PF_BK, nb = a.nb, bn = a.bn, splits = a.splits, na = MODE == PF_UP ? 2 : a.na;
-	const int as = AT / na, rs = RT / na; // slots of na tiles
+	const int nkb = a.K / PF_BK, ns = a.stages, bn = a.bn, splits = a.splits, na = MODE == PF_UP ? 2 : a.na;
+	const int rs = RT / na; // slots of na weight tiles
 	const int row_tiles = a.rows / PF_BM, tok_tiles = (a.n_tokens + bn - 1) / bn;
 	const int items = (MODE == PF_UP ? row_tiles : (row_tiles + na - 1) / na) * splits * tok_tiles;
 	const int b_bytes = bn * 128;
-	auto a_tile = [&](int s, int i) { return smem + (size_t)(s * na + i) * PF_TILE_BYTES; };
-	auto r_tile = [&](int s, int i) { return smem + (size_t)AT * PF_TILE_BYTES + (size_t)(s * na + i) * RAW; };
-	auto b_tile = [&](int s) { return smem + (size_t)AT * PF_TILE_BYTES + (size_t)RT * RAW + (size_t)s * b_bytes; };
+	const size_t stage_bytes = pf_stage_bytes(na, bn);
+	auto r_tile = [&](int s, int i) { return smem + (size_t)(s * na + i) * RAW; };
+	auto a_tile = [&](int s, int i) { return smem + (size_t)RT * RAW + s * stage_bytes + (size_t)i * PF_TILE_BYTES; };
+	auto b_tile = [&](int s) { return smem + (size_t)RT * RAW + s * stage_bytes + (size_t)na * PF_TILE_BYTES; };
 	// item -> first weight row, tiles, first token, k-stages [k0, k1)
 	struct Item {
 		int row0, cnt, tok0, k0, k1;
@@ -285,9 +287,8 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 
 	pdl_launch_next();
 	if (tid == 0) {
-		for (int s = 0; s < AT; ++s) mbar_init(&a_full[s], DBITS == 16 ? 1 : 4), mbar_init(&a_empty[s], 1);
-		for (int s = 0; s < RT; ++s) mbar_init(&r_full[s], 1), mbar_init(&r_empty[s], 4);
-		for (int s = 0; s < nb; ++s) mbar_init(&b_full[s], 1), mbar_init(&b_empty[s], 1);
+		for (int s = 0; s < RT; ++s) mbar_init(&r_full[s], 1), mbar_init(&r_empty[s], WIDEN);
+		for (int s = 0; s < ns; ++s) mbar_init(&full[s], 2 + (DBITS == 16 ? 1 : WIDEN)), mbar_init(&empty[s], 1); // hi, lo, weights: the copy or the widening warps
 		for (int s = 0; s < 2; ++s) mbar_init(&acc_full[s], 1), mbar_init(&acc_empty[s], 4);
 		mbar_init_fence();
 	}
@@ -300,59 +301,57 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 	// The one-thread roles keep their warp together and elect a lane for the issuing: addresses and descriptors then live in uniform registers
 	// (one lane in a branch of its own spent 60 cycles per MMA on moving them).
 	bool ok = true;
-	if (warp == 0 || warp == LO_WARP) { // ===== activations: hi tiles in the even slots, lo tiles in the odd ones
+	if (warp == 0 || warp == LO_WARP) { // ===== activations: one warp the hi, one the lo tile of a stage
 		pdl_wait_prev();
 		const bool el = elect_one();
 		const int lo = warp != 0;
-		int s = lo;
+		int s = 0;
 		unsigned ph = 1;
 		for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
 			const Item t = item_of(it);
 			for (int kb = t.k0; kb < t.k1; ++kb) {
-				if (!__all_sync(0xffffffffu, mbar_wait_bounded(&b_empty[s], ph))) {
+				if (!__all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], ph))) {
 					ok = gave_up(9301);
 					break;
 				}
 				if (el) {
-					mbar_expect_tx(&b_full[s], b_bytes);
-					tma_load_2d(b_tile(s), &m.x[lo], kb * PF_BK, t.tok0, &b_full[s]);
+					mbar_expect_tx(&full[s], b_bytes);
+					tma_load_2d(b_tile(s) + lo * b_bytes, &m.x[lo], kb * PF_BK, t.tok0, &full[s]);
 				}
-				if ((s += 2) >= nb) s = lo, ph ^= 1;
+				if (++s == ns) s = 0, ph ^= 1;
 			}
 		}
 	} else if (warp == 1) { // ===== MMAs
 		// kind::f16: D = f32, A = B = f16, both K-major, M = 128, N = bn
 		const uint32_t idesc = (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(PF_BM >> 4) << 24);
 		const bool el = elect_one();
-		int s = 0, sa = 0;
-		unsigned ph = 0, pa = 0, q = 0;
+		int s = 0;
+		unsigned ph = 0, q = 0;
 		for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++q) {
 			const Item t = item_of(it);
 			const uint32_t acc = tmem_base + (q & 1) * 256;
 			if (!__all_sync(0xffffffffu, mbar_wait_bounded(&acc_empty[q & 1], ((q >> 1) & 1) ^ 1))) ok = gave_up(9302);
 			tc_fence_after();
 			for (int kb = t.k0; kb < t.k1 && ok; ++kb) {
-				if (!__all_sync(0xffffffffu, mbar_wait_bounded(&a_full[sa], pa))) ok = gave_up(9303);
-				for (int half = 0; half < 2 && ok; ++half) {
-					if (!__all_sync(0xffffffffu, mbar_wait_bounded(&b_full[s], ph))) {
-						ok = gave_up(9304);
-						break;
-					}
-					if (el) {
-						const uint64_t db = umma_desc_sw128(b_tile(s)), da = umma_desc_sw128(a_tile(sa, 0));
-#pragma unroll
-						for (int k = 0; k < PF_BK / 16; ++k) { // 16 f16 = 32 bytes along K inside the swizzle atom: +2 in the 16-byte address field
-							const uint32_t add = (kb > t.k0 || half || k) ? 1u : 0u;
-							umma_f16(acc, da + 2 * k, db + 2 * k, idesc, add);
-							if (t.cnt == 2) umma_f16(acc + bn, da + (PF_TILE_BYTES >> 4) + 2 * k, db + 2 * k, idesc, add);
-						}
-						umma_commit(&b_empty[s]); // frees the slot when these MMAs have read it
-						if (half) umma_commit(&a_empty[sa]);
-					}
-					__syncwarp();
-					if (++s == nb) s = 0, ph ^= 1;
+				if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full[s], ph))) {
+					ok = gave_up(9303);
+					break;
 				}
-				if (++sa == as) sa = 0, pa ^= 1;
+				if (el) {
+					const uint64_t db = umma_desc_sw128(b_tile(s)), da = umma_desc_sw128(a_tile(s, 0));
+#pragma unroll
+					for (int k = 0; k < PF_BK / 16; ++k) // 16 f16 = 32 bytes along K inside the swizzle atom: +2 in the 16-byte address field
+#pragma unroll
+						for (int i = 0; i < 2; ++i)
+							if (i < t.cnt) {
+								const uint64_t dw = da + i * (PF_TILE_BYTES >> 4) + 2 * k;
+								umma_f16(acc + i * bn, dw, db + 2 * k, idesc, (kb > t.k0 || k) ? 1u : 0u);
+								umma_f16(acc + i * bn, dw, db + (b_bytes >> 4) + 2 * k, idesc, 1u);
+							}
+					umma_commit(&empty[s]); // frees the stage when these MMAs have read it
+				}
+				__syncwarp();
+				if (++s == ns) s = 0, ph ^= 1;
 			}
 			if (el) umma_commit(&acc_full[q & 1]);
 			__syncwarp();
@@ -424,55 +423,75 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 			}
 		}
 	} else if (warp == W_WARP) { // ===== weights: immutable, so the first tiles are requested before the previous kernel has finished
-		uint64_t* full = DBITS == 16 ? a_full : r_full;
-		uint64_t* empty = DBITS == 16 ? a_empty : r_empty;
-		const int ws = DBITS == 16 ? as : rs;
+		uint64_t* wfull = DBITS == 16 ? full : r_full;
+		uint64_t* wempty = DBITS == 16 ? empty : r_empty;
+		const int ws = DBITS == 16 ? ns : rs;
 		const bool el = elect_one();
 		int s = 0;
 		unsigned ph = 1;
 		for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
 			const Item t = item_of(it);
 			for (int kb = t.k0; kb < t.k1; ++kb) {
-				if (!__all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], ph))) {
+				if (!__all_sync(0xffffffffu, mbar_wait_bounded(&wempty[s], ph))) {
 					ok = gave_up(9306);
 					break;
 				}
 				if (el) {
-					mbar_expect_tx(&full[s], t.cnt * RAW);
+					mbar_expect_tx(&wfull[s], t.cnt * RAW);
 					for (int i = 0; i < t.cnt; ++i) {
 						int row = t.row0 + (MODE == PF_UP ? 0 : i * PF_BM), which = MODE == PF_UP ? i : 0;
 						if (MODE == PF_QKV && row >= a.q_dim) {
 							row -= a.q_dim, which = 1;
 							if (row >= a.kv_dim) row -= a.kv_dim, which = 2;
 						}
-						tma_load_2d(DBITS == 16 ? a_tile(s, i) : r_tile(s, i), &m.w[which], kb * (DBITS == 16 ? PF_BK : PF_BK * DBITS / 8), row, &full[s]);
+						tma_load_2d(DBITS == 16 ? a_tile(s, i) : r_tile(s, i), &m.w[which], kb * (DBITS == 16 ? PF_BK : PF_BK * DBITS / 8), row, &wfull[s]);
 					}
 				}
 				if (++s == ws) s = 0, ph ^= 1;
 			}
 		}
-	} else if constexpr (DBITS != 16) { // ===== widening: one tile row per thread
-		const int r = tid - 192;
+	} else if constexpr (DBITS != 16) { // ===== widening: a row per thread; with eight warps a tile each of two, or half the row each of one
+		constexpr int NV = DBITS / 2, PER = 8 / NV, NT = WIDEN == 4 ? 2 : 1; // 16-byte vectors of a row's k-stage, chunks of f16 from each, tiles per thread
+		const int r = (tid - 192) & 127, part = (tid - 192) >> 7;
+		const bool whole = WIDEN == 4 || na == 2;
+		const int tile0 = WIDEN == 8 && na == 2 ? part : 0, i0 = whole ? 0 : part * (NV / 2);
 		int sr = 0, sa = 0;
 		unsigned pr = 0, pe = 1;
 		for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
 			const Item t = item_of(it);
+			const int nt = min(NT, t.cnt - tile0);
 			for (int kb = t.k0; kb < t.k1 && ok; ++kb) {
-				uint4 raw[2][DBITS / 2];
+				uint4 raw[NT][NV];
 				if (!mbar_wait_bounded(&r_full[sr], pr)) ok = gave_up(9307);
-				pf_load_raw<DBITS>(r_tile(sr, 0), r, raw[0]);
-				if (t.cnt == 2) pf_load_raw<DBITS>(r_tile(sr, 1), r, raw[1]);
+#pragma unroll
+				for (int j = 0; j < NT; ++j)
+					if (j < nt) {
+#pragma unroll
+						for (int i = 0; i < NV; ++i)
+							if (whole || i < NV / 2) raw[j][i] = pf_load_raw<DBITS>(r_tile(sr, tile0 + j), r, i0 + i);
+					}
 				fence_async_smem(); // the copy engine writes next what was read here
 				__syncwarp();
 				if (lane == 0) mbar_arrive(&r_empty[sr]);
-				if (!mbar_wait_bounded(&a_empty[sa], pe)) ok = gave_up(9308);
-				pf_store_a<DBITS>(a_tile(sa, 0), r, raw[0]);
-				if (t.cnt == 2) pf_store_a<DBITS>(a_tile(sa, 1), r, raw[1]);
+				if (!mbar_wait_bounded(&empty[sa], pe)) ok = gave_up(9308);
+#pragma unroll
+				for (int j = 0; j < NT; ++j)
+					if (j < nt) {
+						unsigned char* const dst = a_tile(sa, tile0 + j) + r * 128;
+#pragma unroll
+						for (int i = 0; i < NV; ++i)
+							if (whole || i < NV / 2) {
+								uint4 out[PER];
+								pf_widen<DBITS>(raw[j][i], out);
+#pragma unroll
+								for (int c = 0; c < PER; ++c) *reinterpret_cast<uint4*>(dst + ((((i0 + i) * PER + c) ^ (r & 7)) << 4)) = out[c];
+							}
+					}
 				fence_async_smem();
 				__syncwarp();
-				if (lane == 0) mbar_arrive(&a_full[sa]);
+				if (lane == 0) mbar_arrive(&full[sa]);
 				if (++sr == rs) sr = 0, pr ^= 1;
-				if (++sa == as) sa = 0, pe ^= 1;
+				if (++sa == ns) sa = 0, pe ^= 1;
 			}
 		}
 	}
