@@ -35,6 +35,14 @@ __device__ __forceinline__ void split_hl(float x, __half& hi, __half& lo) {
 	lo = __float2half_rn(x - __half2float(hi));
 }
 
+// two floats -> (hi, lo) f16 pairs
+__device__ __forceinline__ void split_hl2(float x, float y, uint32_t& hi, uint32_t& lo) {
+	const __half2 h = __floats2half2_rn(x, y);
+	const float2 f = __half22float2(h);
+	const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+	hi = *reinterpret_cast<const uint32_t*>(&h), lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
 // X[t][:] = decode(E[tokens[t]])  (reference infer.c:335-347)
 template <int DBITS>
 __global__ void k_pf_embed(float* X, const void* table, const int* tokens, int n, int dim) {
@@ -55,32 +63,47 @@ __global__ void k_pf_rope(float2* rope, const float* freq, int n, int half_hd, i
 	rope[i] = make_float2(c, s);
 }
 
-// one CTA per token: norm (infer.c:183-207) then hi / lo split; rows beyond n (tile padding) are zeroed once at allocation
+// one CTA per token: norm (infer.c:183-207) then hi / lo split; rows beyond n (tile padding) are zeroed once at allocation.  dim is a multiple of 4;
+// a row of up to 8192 is read once, 16 bytes at a time, and stays in registers (the 64 norms of a 333-token Mistral-7B prompt: 0.9 of its 18.7 ms saved)
+#define PFN_REGS 8
 __global__ void __launch_bounds__(256) k_pf_norm(const float* X, const float* normw, __half* hi, __half* lo, int n, int dim, float eps, int ln) {
 	pdl_enter();
 	__shared__ float red[32];
-	const int t = blockIdx.x;
+	const int t = blockIdx.x, n4 = dim >> 2;
 	if (t >= n) return;
-	const float* x = X + (size_t)t * dim;
+	const float4* x = reinterpret_cast<const float4*>(X + (size_t)t * dim);
+	float4 v[PFN_REGS];
+#pragma unroll
+	for (int k = 0; k < PFN_REGS; ++k) {
+		const int i = threadIdx.x + k * 256;
+		if (i < n4) v[k] = __ldcg(x + i);
+	}
+	auto each = [&](auto&& f) { // f(group, value of the group)
+#pragma unroll
+		for (int k = 0; k < PFN_REGS; ++k)
+			if ((int)threadIdx.x + k * 256 < n4) f(threadIdx.x + k * 256, v[k]);
+		for (int i = threadIdx.x + PFN_REGS * 256; i < n4; i += 256) f(i, __ldcg(x + i));
+	};
 	float mean = 0.f;
 	if (ln) {
 		float s = 0.f;
-		for (int i = threadIdx.x; i < dim; i += blockDim.x) s += x[i];
+		each([&](int, float4 a) { s += (a.x + a.y) + (a.z + a.w); });
 		mean = block_sum(s, red) / dim;
 	}
 	float ss = 0.f;
-	for (int i = threadIdx.x; i < dim; i += blockDim.x) {
-		const float d = x[i] - mean;
-		ss = fmaf(d, d, ss);
-	}
+	each([&](int, float4 a) {
+		a.x -= mean, a.y -= mean, a.z -= mean, a.w -= mean;
+		ss += (a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w);
+	});
 	ss = block_sum(ss, red);
 	const float scale = 1.0f / sqrtf(ss / dim + eps);
-	for (int i = threadIdx.x; i < dim; i += blockDim.x) {
-		const float v = (x[i] - mean) * scale * normw[i];
-		__half h, l;
-		split_hl(v, h, l);
-		hi[(size_t)t * dim + i] = h, lo[(size_t)t * dim + i] = l;
-	}
+	each([&](int i, float4 a) {
+		const float4 w = __ldg(reinterpret_cast<const float4*>(normw) + i);
+		uint2 h, l;
+		split_hl2((a.x - mean) * scale * w.x, (a.y - mean) * scale * w.y, h.x, l.x);
+		split_hl2((a.z - mean) * scale * w.z, (a.w - mean) * scale * w.w, h.y, l.y);
+		reinterpret_cast<uint2*>(hi + (size_t)t * dim)[i] = h, reinterpret_cast<uint2*>(lo + (size_t)t * dim)[i] = l;
+	});
 }
 
 // ---------------------------------------------------------------- the GEMM
@@ -545,14 +568,6 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], u
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool in) { // 16 bytes, zeros when !in
 	asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
 }
-// two floats -> (hi, lo) f16 pairs
-__device__ __forceinline__ void split_hl2(float x, float y, uint32_t& hi, uint32_t& lo) {
-	const __half2 h = __floats2half2_rn(x, y);
-	const float2 f = __half22float2(h);
-	const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
-	hi = *reinterpret_cast<const uint32_t*>(&h), lo = *reinterpret_cast<const uint32_t*>(&l);
-}
-
 template <typename KVT, int HD>
 __global__ void __launch_bounds__(256, 1) k_pf_attn(const PfAttnArgs a) {
 	pdl_enter();
