@@ -15,6 +15,9 @@
 // ([position][head_dim] is contiguous per (layer, kv head)).  The slot written this step and the attention sinks that
 // k_embed re-rotates are read from global memory after the wait instead of from the early copy.
 //
+// Groups of 3, 5, 6 or 7 heads run as 4 or 8 with zero queries in the rest: with positions dealt out to many CTAs the spare arithmetic is hidden
+// by the fold (Qwen2-0.5B, 14 heads on 2, 131 positions: 16.7 us a layer in k_attn, 10.3 here).
+//
 // Lane layout and arithmetic are k_attn's transposing score path: LPP = head_dim / 8 lanes own a position (8 dims per
 // lane), P = LPP / HG positions per lane group and step, so the HG * P partial dot products of a step transpose onto the
 // LPP lanes of the group (one complete score per lane), the two exponentials are evaluated once per lane, and the
@@ -111,7 +114,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) k_attn2(const AttnArgs a) {
 	const int nbmax = a.nbmax, nsplit = a.nsplit;
 	const int unit = blockIdx.x / nsplit, split = blockIdx.x % nsplit;
 	const int kvh = unit / a.qgroups;
-	const int hbase = kvh * a.kv_mul + (unit % a.qgroups) * HG;
+	const int hbase = kvh * a.kv_mul + (unit % a.qgroups) * a.hg; // a.hg heads of the unit are real, the rest of HG are zero queries
 	constexpr uint32_t BLK = ATTN2_BP * HD * sizeof(KVT); // bytes of a whole block
 	KVT* Ks = reinterpret_cast<KVT*>(smem_raw);
 	KVT* Vs = Ks + (size_t)nbmax * ATTN2_BP * HD;
@@ -153,7 +156,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) k_attn2(const AttnArgs a) {
 	constexpr int QPT = (HG * HD + ATTN_THREADS - 1) / ATTN_THREADS;
 	float qreg[QPT];
 #pragma unroll
-	for (int i = 0; i < QPT; ++i) qreg[i] = (tid + i * ATTN_THREADS < HG * HD) ? __ldcg(a.q + (size_t)hbase * HD + tid + i * ATTN_THREADS) : 0.f;
+	for (int i = 0; i < QPT; ++i) qreg[i] = (tid + i * ATTN_THREADS < a.hg * HD) ? __ldcg(a.q + (size_t)hbase * HD + tid + i * ATTN_THREADS) : 0.f;
 	const int kv_len = a.tp->kv_len, kv_pos = a.tp->kv_pos, kv_sink = a.tp->kv_sink;
 	const unsigned epoch = (unsigned)a.tp->tp_seq * a.epoch_stride + a.epoch_idx;
 	if (tid < nbmax && !issued && (split + tid * nsplit) * ATTN2_BP < kv_len) request(tid), issued = true;
@@ -191,8 +194,11 @@ __global__ void __launch_bounds__(ATTN_THREADS) k_attn2(const AttnArgs a) {
 	for (int sb = (warp * G + grp) * P; sb - grp * P < nslots; sb += SC * STEP) { // warp-uniform trip count (full-warp shuffles inside)
 		float sc[SC];
 		bool val[SC], fast[SC];
+		const int live = min(SC, (nslots - (sb - grp * P) + STEP - 1) / STEP); // steps of the chunk that reach a slot (warp-uniform): contexts of 777 / 2049 positions have one / two of four (14.2 -> 9.1, 15.2 -> 10.4 us)
 #pragma unroll
 		for (int c = 0; c < SC; ++c) {
+			sc[c] = -FLT_MAX, val[c] = false, fast[c] = false;
+			if (c >= live) continue;
 			const int s0 = sb + c * STEP;
 			const bool inr = s0 < nslots;
 			int j = 0, o = 0, t0 = 0;
@@ -268,6 +274,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) k_attn2(const AttnArgs a) {
 		}
 #pragma unroll
 		for (int c = 0; c < SC; ++c) {
+			if (c >= live) continue;
 			const int s0 = sb + c * STEP;
 			const bool inr = s0 < nslots;
 			int j = 0, o = 0, t0 = 0;
@@ -333,7 +340,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) k_attn2(const AttnArgs a) {
 		}
 		__syncthreads();
 		// CTA `split` normalises outputs [split * per, (split + 1) * per): 8 adjacent lanes share an output, each sums every 8th slice
-		const int nout = HG * HD, per = (nout + nsplit - 1) / nsplit;
+		const int nout = a.hg * HD, per = (nout + nsplit - 1) / nsplit;
 		const int o_end = min(nout, (split + 1) * per);
 		for (int o0 = split * per; o0 < o_end; o0 += ATTN_THREADS / 8) {
 			const int o = o0 + tid / 8, sg = tid & 7;
@@ -383,7 +390,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) k_attn2(const AttnArgs a) {
 		__syncthreads();
 		ATTN_DBG(6);
 		// CTA `split` normalises outputs [split * per, (split + 1) * per): 8 adjacent lanes share an output, each sums every 8th slice
-		const int nout = HG * HD, per = (nout + nsplit - 1) / nsplit;
+		const int nout = a.hg * HD, per = (nout + nsplit - 1) / nsplit;
 		const int o_end = min(nout, (split + 1) * per);
 		for (int o0 = split * per; o0 < o_end; o0 += ATTN_THREADS / 8) {
 			const int o = o0 + tid / 8, sg = tid & 7;

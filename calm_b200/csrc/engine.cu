@@ -57,7 +57,7 @@ struct Engine {
 	int ncand = 0;
 
 	// attention launch shape
-	int attn_hg = 1, attn_qgroups = 1, attn_nsplit = 1, attn_lpp = 1;
+	int attn_hg = 1, attn_hg2 = 1 /* k_attn2: padded to what it is instantiated for */, attn_qgroups = 1, attn_nsplit = 1, attn_lpp = 1;
 	// TMA-ring matvec kernels (ring.cuh): slots per warp / CTAs per SM for FFN-up and for wo / w2; u = 512-byte units per row and chunk (0: not used)
 	int ring_up_ns = 2, ring_up_cps = 2, ring_res_ns = 2, ring_res_warps = 16; // measured: 16 consuming warps per SM are needed (profiles/r02_sweep_ring_*.jsonl)
 	int ring_up_u = 0, ring_wo_u = 0, ring_down_u = 0, ring_wo_s = 1, ring_down_s = 1;
@@ -454,7 +454,7 @@ bool attn2_shape_ok(int hg, int lpp, int head_dim) {
 template <typename KVT>
 void dispatch_attn(const AttnArgs& a, int nunits, int* nl) {
 	if (g.attn2) {
-		switch (g.attn_lpp * 100 + g.attn_hg) {
+		switch (g.attn_lpp * 100 + g.attn_hg2) {
 		case 1604: launch_attn2<KVT, 4, 16>(a, nunits, nl); return;
 		case 1608: launch_attn2<KVT, 8, 16>(a, nunits, nl); return;
 		case 802: launch_attn2<KVT, 2, 8>(a, nunits, nl); return;
@@ -571,7 +571,7 @@ int run_token(int mode) {
 			a.q = g.q, a.kc = (KVT*)g.kc + l * kv_layer, a.vc = (KVT*)g.vc + l * kv_layer;
 			a.partial = g.attn_partial, a.counter = g.attn_counter, a.out = g.att, a.tp = g.tp;
 			a.head_dim = hd, a.seq_len = c.seq_len, a.nsplit = g.attn_nsplit, a.lpp = g.attn_lpp;
-			a.kv_mul = g.kv_mul, a.qgroups = g.attn_qgroups;
+			a.kv_mul = g.kv_mul, a.qgroups = g.attn_qgroups, a.hg = g.attn_hg;
 			a.inv_sqrt_hd = 1.0f / sqrtf((float)hd);
 			a.nbmax = g.attn_nbmax;
 			a.cells = g.attn_cells, a.epoch_stride = (unsigned)c.n_layers + 1, a.epoch_idx = (unsigned)l + 1, a.err = g.dev_err;
@@ -744,9 +744,9 @@ void make_plan() {
 	{
 		// k_attn2 when the shape is instantiated and the CTA's share of the context fits in shared memory
 		g.attn_nbmax = cdiv(cdiv(c.seq_len, ATTN2_BP), g.attn_nsplit);
-		g.attn2_smem = attn2_smem_bytes<KVT>(g.attn_hg, c.head_dim, g.attn_nbmax, g.attn_nsplit);
+		g.attn2_smem = attn2_smem_bytes<KVT>(g.attn_hg2, c.head_dim, g.attn_nbmax, g.attn_nsplit);
 		const bool want = !(getenv("CALM_B200_ATTN2") && atoi(getenv("CALM_B200_ATTN2")) == 0);
-		g.attn2 = want && attn2_shape_ok(g.attn_hg, g.attn_lpp, c.head_dim) && g.attn_nbmax <= ATTN2_MAXB && g.attn2_smem <= 200 * 1024;
+		g.attn2 = want && attn2_shape_ok(g.attn_hg2, g.attn_lpp, c.head_dim) && g.attn_nbmax <= ATTN2_MAXB && g.attn2_smem <= 200 * 1024;
 		g.attn2_cluster = g.attn2 && g.attn_nsplit <= ATTN2_MAX_CLUSTER && getenv("CALM_B200_ATTN_CLUSTER") && atoi(getenv("CALM_B200_ATTN_CLUSTER")) != 0;
 		AttnArgs aa = {};
 		aa.head_dim = c.head_dim, aa.nsplit = g.attn_nsplit;
@@ -1007,6 +1007,7 @@ extern "C" void prepare_cuda(struct Transformer* transformer) {
 			g.attn_hg = h;
 			break;
 		}
+	g.attn_hg2 = g.attn_hg == 3 ? 4 : g.attn_hg > 4 ? 8 : g.attn_hg;
 	g.attn_qgroups = g.kv_mul / g.attn_hg;
 	g.attn_lpp = 1;
 	while (g.attn_lpp * 8 < c.head_dim) g.attn_lpp *= 2;
@@ -1019,14 +1020,14 @@ extern "C" void prepare_cuda(struct Transformer* transformer) {
 	// still-resident q/k/v CTAs delay; kept selectable for the record -- profiles/r02_sweep_ring_and_attention_variants.jsonl)
 	if (g.attn_nsplit > ATTN2_MAXB + 4) g.attn_nsplit = ATTN2_MAXB + 4; // k_attn2 keeps one (m, l) pair per slice in static shared memory
 	const bool want_cluster = getenv("CALM_B200_ATTN_CLUSTER") && atoi(getenv("CALM_B200_ATTN_CLUSTER")) != 0;
-	if (want_cluster && attn2_shape_ok(g.attn_hg, g.attn_lpp, c.head_dim) && !(getenv("CALM_B200_ATTN2") && atoi(getenv("CALM_B200_ATTN2")) == 0)) {
+	if (want_cluster && attn2_shape_ok(g.attn_hg2, g.attn_lpp, c.head_dim) && !(getenv("CALM_B200_ATTN2") && atoi(getenv("CALM_B200_ATTN2")) == 0)) {
 		int ns = 1; // the slices of a unit will be one thread-block cluster: a power of two, at most 16 CTAs
 		while (ns * 2 <= g.attn_nsplit && ns * 2 <= ATTN2_MAX_CLUSTER) ns *= 2;
 		g.attn_nsplit = ns;
 	}
 	g.attn_partial = (float*)dev_alloc((size_t)units * g.attn_nsplit * g.attn_hg * (c.head_dim + 2) * sizeof(float));
 	{
-		const size_t cell_bytes = (size_t)units * (g.sms / units > g.attn_nsplit ? g.sms / units : g.attn_nsplit) * g.attn_hg * (c.head_dim + 2) * sizeof(unsigned long long);
+		const size_t cell_bytes = (size_t)units * (g.sms / units > g.attn_nsplit ? g.sms / units : g.attn_nsplit) * g.attn_hg2 * (c.head_dim + 2) * sizeof(unsigned long long);
 		// (the attention grid must be co-resident for the cell fold: units * nsplit CTAs of <= 1/2 SM each)
 		g.attn_cells = (unsigned long long*)dev_alloc(cell_bytes);
 		CUDA_CHECK(cudaMemset(g.attn_cells, 0, cell_bytes));

@@ -404,7 +404,7 @@ struct AttnArgs {
 	float* out;       // [n_heads*head_dim]
 	const TokenParams* tp;
 	int head_dim, seq_len, nsplit, lpp; // lpp: lanes per position (power of two >= head_dim/8)
-	int kv_mul, qgroups;                // query heads per kv head; qgroups = kv_mul / HG
+	int kv_mul, qgroups, hg;            // query heads per kv head; heads per unit; qgroups = kv_mul / hg
 	float inv_sqrt_hd;
 	int nbmax;                          // k_attn2: 16-position blocks per CTA = ceil(ceil(seq_len / 16) / nsplit)
 	unsigned long long* cells;          // k_attn2: [units][nsplit][HG][head_dim + 2] {value, epoch} cells of the slice fold
