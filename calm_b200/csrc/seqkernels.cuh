@@ -946,6 +946,179 @@ __global__ void __launch_bounds__(256) k_seq_attn_softmax(AttSoftmax a) {
 	}
 }
 
+// ---------------------------------------------------------------- prompt attention in one kernel
+// Flash attention for sequences that bring many tokens to a step: attentions over cached keys and values of the same width HD, scores in bf16
+// products (not scores_f32, no distance bias, one map).  A CTA serves km of the query heads that share a key head and tb blocks of
+// 16 tokens, a warp one of each; a tile of 64 cached rows (fp32, through the page table) is copied to shared memory while the
+// previous one is multiplied, rounded to bf16 once for all its warps, and read as mma.m16n8k16 fragments.  Scores, the running maximum,
+// exponentials and the denominator are fp32; queries, keys and values are bf16 with fp32 accumulation, as in the products that this replaces,
+// and the weights a bf16 value and its remainder (one bf16 there).  Those were: gather, score product, softmax and value product per sequence, key head and block of queries, with scores
+// and weights going through memory.
+// Bound: the MMAs and, with few query heads per key head, the fp32 rows (64 KB a tile from L2).  A 2048-token
+// step: 638 us in 16 launches before, 308 here; three sequences of 700 tokens: 700 us in 48 launches, 146 here.
+#define AFL_TILE 64
+template <int HD>
+__host__ __device__ constexpr size_t afl_smem() { // the rows as cached (K, V), then as bf16 (K, V)
+	return (size_t)2 * AFL_TILE * HD * (sizeof(float) + sizeof(bf16));
+}
+__device__ __forceinline__ void afl_ldsm(const void* p, uint32_t (&r)[4]) {
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
+}
+__device__ __forceinline__ void afl_ldsm_t(const void* p, uint32_t (&r)[4]) {
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
+}
+__device__ __forceinline__ uint32_t afl_pack(float x, float y) {
+	const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+	return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+template <int HD>
+__global__ void __launch_bounds__(256, 1) k_seq_attn_flash(const AttArgs a, const bf16* __restrict__ Q, bf16* __restrict__ out, const SeqBatch sb, int km, int tb, int min_count) {
+	pdl_enter();
+	constexpr int C4 = HD / 4, KS = HD / 16, NT = AFL_TILE / 8;
+	extern __shared__ __align__(128) unsigned char afl_sm[];
+	float* const raw = reinterpret_cast<float*>(afl_sm);                                   // [K, V][64][HD]
+	bf16* const tile = reinterpret_cast<bf16*>(afl_sm + (size_t)2 * AFL_TILE * HD * sizeof(float)); // the same, 16-byte chunks c of row r at c ^ (r & 7)
+	const int b = blockIdx.z, cnt = sb.scount[b], c0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * 16 * tb; // first token of the CTA in its sequence (the longest rows first)
+	if (cnt < min_count || c0 >= cnt) return;
+	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+	const int first = sb.sstart[b], pos0 = sb.spos0[b], slot = sb.sslot[b], per = a.group / km;
+	const int kvh = blockIdx.y / per, head = kvh * a.group + (blockIdx.y % per) * km + warp % km;
+	const int t0 = c0 + (warp / km) * 16; // first token of the warp
+	const float* const kbase = a.kc + kvh * HD;
+	const float* const vbase = a.vc + kvh / a.vshare * HD;
+	const int keep = a.window > 0 ? a.keep_first : 0;
+	auto low = [&](int p) { // first position that a query at p sees (but for the kept ones)
+		int l = a.window > 0 ? max(0, p - a.window + 1) : 0;
+		return a.chunk > 0 ? max(l, p / a.chunk * a.chunk) : l;
+	};
+	const int pa = pos0 + c0, pb = pos0 + min(cnt, c0 + 16 * tb) - 1;       // the CTA's positions
+	const int wa = pos0 + t0, wb = pos0 + min(cnt, t0 + 16) - 1;            // the warp's (wb < wa: none)
+	const int from = low(pa) & ~(AFL_TILE - 1);                             // tiles from here on, and before them those of the kept positions
+	auto next = [&](int k) { // the tile after k
+		k += AFL_TILE;
+		return k < from && k >= keep ? from : k;
+	};
+	auto fetch = [&](int k0) {
+		for (int i = tid; i < 2 * AFL_TILE * C4; i += blockDim.x) {
+			const int which = i / (AFL_TILE * C4), r = i / C4 % AFL_TILE, c = i % C4, pos = k0 + r;
+			if (pos > pb) continue; // the rest of the tile is never visible
+			const long row = cache_row(sb, slot, pos);
+			cp_async16(raw + ((size_t)which * AFL_TILE + r) * HD + 4 * c, (which ? vbase + row * a.vld : kbase + row * a.kld) + 4 * c);
+		}
+		asm volatile("cp.async.commit_group;" ::: "memory");
+	};
+	auto at = [&](int which, int r, int c) { return tile + ((size_t)which * AFL_TILE + r) * HD + ((c ^ (r & 7)) << 3); };
+	int k0 = keep > 0 ? 0 : from;
+	if (k0 < from && k0 >= keep) k0 = from;
+	fetch(k0);
+
+	uint32_t q[KS][4];
+#pragma unroll
+	for (int r = 0; r < 2; ++r) {
+		const int t = t0 + g + 8 * r;
+		const uint32_t* qp = reinterpret_cast<const uint32_t*>(Q + ((size_t)(first + t) * a.heads + head) * HD) + t4;
+#pragma unroll
+		for (int k = 0; k < KS; ++k) q[k][r] = t < cnt ? qp[8 * k] : 0u, q[k][2 + r] = t < cnt ? qp[8 * k + 4] : 0u;
+	}
+	float o[HD / 8][4], m[2], l[2];
+#pragma unroll
+	for (int n = 0; n < HD / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+	m[0] = m[1] = a.add_one ? 0.f : a.sink ? ldf(a.sink + head) : -FLT_MAX;
+	if (m[0] == -INFINITY) m[0] = m[1] = -FLT_MAX; // a sink of no weight
+	l[0] = l[1] = (a.add_one || a.sink) && t4 == 0 ? 1.f : 0.f; // a lane's share of the denominator
+	const int wlow = low(wa);
+	while (k0 <= pb) {
+		asm volatile("cp.async.wait_group 0;" ::: "memory");
+		__syncthreads(); // the tile has arrived, and the bf16 one is no longer being read
+		for (int i = tid; i < 2 * AFL_TILE * (HD / 8); i += blockDim.x) {
+			const int which = i / (AFL_TILE * (HD / 8)), r = i / (HD / 8) % AFL_TILE, c = i % (HD / 8);
+			const float4* s = reinterpret_cast<const float4*>(raw + ((size_t)which * AFL_TILE + r) * HD + 8 * c);
+			const bool in = k0 + r <= pb; // rows past the last position are zero: a weight of zero must not meet a NaN
+			const float4 z = make_float4(0.f, 0.f, 0.f, 0.f), x = in ? s[0] : z, y = in ? s[1] : z;
+			*reinterpret_cast<uint4*>(at(which, r, c)) = make_uint4(afl_pack(x.x, x.y), afl_pack(x.z, x.w), afl_pack(y.x, y.y), afl_pack(y.z, y.w));
+		}
+		__syncthreads();
+		const int kt = k0;
+		k0 = next(k0);
+		if (k0 <= pb) fetch(k0);
+		if (kt > wb || (kt + AFL_TILE <= wlow && kt >= keep)) continue; // (warp-uniform) nothing of this tile is visible to this warp's rows
+		float s[NT][4];
+#pragma unroll
+		for (int n = 0; n < NT; ++n) {
+			s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+#pragma unroll
+			for (int k = 0; k < KS; k += 2) {
+				uint32_t bb[4];
+				afl_ldsm(at(0, n * 8 + (lane & 7), 2 * k + (lane >> 3)), bb);
+				const uint32_t b0[2] = {bb[0], bb[1]}, b1[2] = {bb[2], bb[3]};
+				mma_bf16_16816(s[n], q[k], b0), mma_bf16_16816(s[n], q[k + 1], b1);
+			}
+		}
+		float mx[2] = {-FLT_MAX, -FLT_MAX};
+#pragma unroll
+		for (int r = 0; r < 2; ++r) {
+			const int p = wa + g + 8 * r, lo = low(p);
+#pragma unroll
+			for (int n = 0; n < NT; ++n)
+#pragma unroll
+				for (int e = 0; e < 2; ++e) {
+					const int key = kt + n * 8 + 2 * t4 + e;
+					float& x = s[n][2 * r + e];
+					x = key <= p && (key >= lo || key < keep) ? att_cap(x * a.scale, a.softcap) : -INFINITY;
+					mx[r] = fmaxf(mx[r], x);
+				}
+		}
+		float corr[2];
+#pragma unroll
+		for (int r = 0; r < 2; ++r) {
+			mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1)), mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
+			const float mn = fmaxf(m[r], mx[r]);
+			corr[r] = expf(m[r] - mn);
+			m[r] = mn, l[r] *= corr[r];
+		}
+#pragma unroll
+		for (int n = 0; n < HD / 8; ++n) o[n][0] *= corr[0], o[n][1] *= corr[0], o[n][2] *= corr[1], o[n][3] *= corr[1];
+#pragma unroll
+		for (int kk = 0; kk < AFL_TILE / 16; ++kk) {
+			uint32_t p[4], pl[4];
+#pragma unroll
+			for (int j = 0; j < 2; ++j)
+#pragma unroll
+				for (int r = 0; r < 2; ++r) {
+					const float x = expf(s[2 * kk + j][2 * r] - m[r]), y = expf(s[2 * kk + j][2 * r + 1] - m[r]);
+					l[r] += x + y;
+					const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+					p[2 * j + r] = *reinterpret_cast<const uint32_t*>(&h);
+					pl[2 * j + r] = afl_pack(x - __bfloat162float(h.x), y - __bfloat162float(h.y));
+				}
+#pragma unroll
+			for (int n = 0; n < HD / 8; n += 2) {
+				uint32_t bb[4];
+				afl_ldsm_t(at(1, kk * 16 + (lane & 15), n + (lane >> 4)), bb);
+				const uint32_t b0[2] = {bb[0], bb[1]}, b1[2] = {bb[2], bb[3]};
+				mma_bf16_16816(o[n], p, b0), mma_bf16_16816(o[n + 1], p, b1);
+				mma_bf16_16816(o[n], pl, b0), mma_bf16_16816(o[n + 1], pl, b1);
+			}
+		}
+	}
+#pragma unroll
+	for (int r = 0; r < 2; ++r) {
+		l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1), l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
+		const int t = t0 + g + 8 * r;
+		if (t >= cnt) continue;
+		const float* gp = a.gate ? a.gate + (size_t)(first + t) * a.ldg + (size_t)head * a.ghs : nullptr;
+		const float inv = (gp && a.ges == 0 ? sigmoidf_(gp[0]) : 1.f) / l[r];
+		bf16* dst = out + ((size_t)(first + t) * a.heads + head) * HD + 2 * t4;
+#pragma unroll
+		for (int n = 0; n < HD / 8; ++n) {
+			float x = o[n][2 * r] * inv, y = o[n][2 * r + 1] * inv;
+			if (gp && a.ges != 0) x *= sigmoidf_(gp[(size_t)(8 * n + 2 * t4) * a.ges]), y *= sigmoidf_(gp[(size_t)(8 * n + 2 * t4 + 1) * a.ges]);
+			*reinterpret_cast<uint32_t*>(dst + 8 * n) = afl_pack(x, y);
+		}
+	}
+}
+
 // ---------------------------------------------------------------- differential attention: two maps of one head
 // Head h of key group g has two maps over the same values; the attention kernels run them as query heads (g * 2 + map) * group + j
 // of 2 x key heads (j: the head's place in its group).  With their outputs a1, a2: o = a1 - lambda a2, o / sqrt(mean(o^2) + eps) * mul.

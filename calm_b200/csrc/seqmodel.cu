@@ -660,6 +660,29 @@ void attention_products(Seq& s, int kind, const AttArgs& a, bf16* out, float* fu
 	}
 }
 
+// attentions that k_seq_attn_flash computes: keys and values of one instantiated width in rows of their own, plain scores in bf16 products
+bool flash_fits(const AttArgs& a) {
+	return (a.kd == 64 || a.kd == 128) && a.vd == a.kd && a.kc != a.vc && a.kld % 4 == 0 && a.vld % 4 == 0 && !a.split && !a.slopes && !a.qr;
+}
+// all sequences with at least kAttnGemmMin new tokens in one launch; queries wait in a3
+void attention_flash(Seq& s, int kind, const AttArgs& a, bf16* out, const SeqBatch& sb) {
+	int km = 8, longest = 0;
+	while (a.group % km) --km; // the largest divisor of the group up to 8 heads
+	const int tb = 8 / km;
+	double pairs = 0;
+	for (int b = 0; b < sb.B; ++b)
+		if (s.hb_count[b] >= kAttnGemmMin) {
+			longest = std::max(longest, s.hb_count[b]);
+			const double span = a.window > 0 ? a.window + a.keep_first : 1e18;
+			pairs += s.hb_count[b] * std::min(s.hb_pos0[b] + s.hb_count[b] * 0.5, span);
+		}
+	const dim3 grid(cdiv(longest, 16 * tb), a.heads / km, sb.B);
+	run_kernel(s, kind, (double)s.tok_on_products * (a.heads * a.kd * 4.0 + (a.heads / a.group) * a.kd * 8.0), 4.0 * pairs * a.heads * a.kd, [&] {
+		if (a.kd == 128) launch_k(s, k_seq_attn_flash<128>, grid, 32 * km * tb, afl_smem<128>(), a, (const bf16*)s.a3, out, sb, km, tb, kAttnGemmMin);
+		else launch_k(s, k_seq_attn_flash<64>, grid, 32 * km * tb, afl_smem<64>(), a, (const bf16*)s.a3, out, sb, km, tb, kAttnGemmMin);
+	});
+}
+
 // q_ready: the queries already wait in a3, in the form the product path reads.  diff: a.heads are the maps of diff->heads heads, which a last kernel
 // combines: from fp32 rows in `full` where they were computed as products, from the shares of the keys elsewhere
 void attention(Seq& s, int kind, AttArgs a, void* out, const SeqBatch& sb, double kv_rows, int longest, bool q_ready = false, const AttDiff* diff = nullptr, float* full = nullptr) {
@@ -670,7 +693,8 @@ void attention(Seq& s, int kind, AttArgs a, void* out, const SeqBatch& sb, doubl
 		if (q_ready) {
 		} else if (a.split) run_kernel(s, KD_ELEMENT, n * 10.0, 0, [&] { launch_k(s, k_seq_split_q, cdiv(n, 256), 256, 0, (bf16*)s.a3, a.q, a.kd, (size_t)sb.N * a.heads); });
 		else run_kernel(s, KD_ELEMENT, n * 6.0, 0, [&] { launch_k(s, k_seq_cast_cols<bf16>, cdiv(n, 256), 256, 0, (bf16*)s.a3, a.q, a.heads * a.kd, 0, a.heads * a.kd, sb.N); });
-		for (int b = 0; b < sb.B; ++b)
+		if (!diff && flash_fits(a)) attention_flash(s, kind, a, (bf16*)out, sb);
+		else for (int b = 0; b < sb.B; ++b)
 			if (s.hb_count[b] >= kAttnGemmMin) attention_products(s, kind, a, (bf16*)out, diff ? full : nullptr, sb, s.hb_slot[b], s.hb_start[b], s.hb_count[b], s.hb_pos0[b]);
 		a.skip = s.d_skip;
 		rest = s.n_on_products < sb.B;
@@ -1443,6 +1467,8 @@ extern "C" void* calm_b200_seq_prepare(const struct SeqModel* model) {
 		CUDA_CHECK(cudaFuncSetAttribute(k_seq_gla_scan<R, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gla_smem(R, P)));
 	});
 	CUDA_CHECK(cudaFuncSetAttribute(k_seq_attn_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+	CUDA_CHECK(cudaFuncSetAttribute(k_seq_attn_flash<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)afl_smem<128>()));
+	CUDA_CHECK(cudaFuncSetAttribute(k_seq_attn_flash<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)afl_smem<64>()));
 	CUDA_CHECK(cudaFuncSetAttribute(k_seq_attention<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
 	CUDA_CHECK(cudaFuncSetAttribute(k_seq_attention<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
 	// rotation tables of the grouped-query and latent attentions: angle step per rotated pair (in double), rescaled between two wavelengths
