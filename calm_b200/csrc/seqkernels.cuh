@@ -1267,130 +1267,165 @@ __global__ void k_seq_delta_scan(DeltaArgs a, SeqBatch sb) {
 	__syncthreads();
 	for (int i = tid; i < D * V; i += blockDim.x) Sg[i] = S[i];
 }
-// The same recurrence with the state in registers: four lanes share a value column, each holding D/4 of its rows.  Tokens are
-// staged DELTA_TB at a time: while one block of tokens is applied (no barrier between its tokens, only shuffles inside a
-// column's four lanes), the next block's k, q, decay, v and beta travel from global memory into the other half of a double
-// buffer; k, q and the decay are read back as float4 (quarters padded by 4 floats: the four lanes hit different banks).
+// The same recurrence with the state in registers.  Value columns are independent: a CTA takes DELTA_VC of them, eight lanes share a
+// pair of columns and each holds D/8 rows of both.  Tokens are staged DELTA_TB at a time: while one block of tokens is applied (no
+// barrier between its tokens, only shuffles inside a pair's eight lanes), the next block's k, q, decay, v and beta travel from global
+// memory into the other half of a double buffer; k, q and the decay are read back as float4 (eighths padded so that the eight lanes
+// hit different banks).  The lanes' shares of a block's read-outs are folded together at its end, so that lane i ends with the i-th of
+// the pair's 2 DELTA_TB values.
+// Bound: shared-memory reads, D/4 float4 of k and q and D/8 of the decay per lane group and token, and the chain of a token (dot,
+// shuffles, update).  With all columns of a head in one CTA and a column per four lanes, 48 CTAs took 845 us
+// for 3 x 700 tokens of 16 heads of 128; 192 CTAs of a quarter of the columns and half the reads per column take 522.
 #define DELTA_TB 4
+#define DELTA_VC 32
+__host__ __device__ constexpr int delta_qp(int D) { return D / 8 == 4 ? 4 : D / 8 + 4; }
+__host__ __device__ constexpr int delta_tok(int D) { return 3 * 8 * delta_qp(D) + DELTA_VC + 4; } // k, q, g (padded eighths), v, beta
 template <int D>
-__global__ void __launch_bounds__(512) k_seq_delta_scan_reg(DeltaArgs a, SeqBatch sb) {
+__global__ void __launch_bounds__(128) k_seq_delta_scan_reg(DeltaArgs a, SeqBatch sb) {
 	pdl_enter(); // programmatic dependent launch: let the next kernel's launch overlap this one, then wait for the previous one
-	constexpr int Q = D / 4, QP = Q + 4;
-	extern __shared__ __align__(16) float sm[];
-	const int b = blockIdx.x, h = blockIdx.y, V = a.vdim;
+	constexpr int Q = D / 8, QP = delta_qp(D), TOK = delta_tok(D), VAT = 3 * 8 * QP, BAT = VAT + DELTA_VC;
+	constexpr int ITEMS = (3 * D + DELTA_VC) / 4 + 1, ROUNDS = (DELTA_TB * ITEMS + 127) / 128;
+	__shared__ __align__(16) float sm[2 * DELTA_TB * TOK];
+	const int b = blockIdx.x, h = blockIdx.y, V = a.vdim, v0 = blockIdx.z * DELTA_VC;
 	const int kh = h / (a.heads / a.kv_heads);
-	const int tid = threadIdx.x, part = tid & 3;
-	const bool live = (tid >> 2) < V;          // lanes past the last column run along on a copy of it (whole warps shuffle)
-	const int col = live ? tid >> 2 : V - 1;
-	const int vpad = (V + 1 + 3) & ~3;         // v and beta of a token, rounded so that the next token stays 16-byte aligned
-	const int tok_len = 3 * 4 * QP + vpad;     // k, q, g (padded quarters), v, beta
-	float* buf[2] = {sm, sm + DELTA_TB * tok_len};
-	float S[Q];
-	float* Sg = a.state + ((size_t)sb.sslot[b] * a.heads + h) * D * V;
+	const int tid = threadIdx.x, part = tid & 7, cl = (tid >> 3) * 2;
+	const bool live = v0 + cl < V; // (V is a multiple of 4: both columns or none) lanes past the last column run along on a copy of it
+	const int col = live ? v0 + cl : V - 2;
+	float S[Q][2];
+	float* Sg = a.state + ((size_t)sb.sslot[b] * a.heads + h) * D * V + (size_t)part * Q * V + col;
 #pragma unroll
-	for (int i = 0; i < Q; ++i) S[i] = Sg[(size_t)(part * Q + i) * V + col];
+	for (int i = 0; i < Q; ++i) {
+		const float2 t = *(const float2*)(Sg + (size_t)i * V);
+		S[i][0] = t.x, S[i][1] = t.y;
+	}
 	const float A = expf(ldf(a.a_log + h));
 	const int start = sb.sstart[b], cnt = sb.scount[b];
-	// Staging.  A token's inputs are 3 D / 4 + V / 4 float4 items (k, q, raw decay input, v) and one scalar (beta's input); item e of a
-	// block belongs to token e / items4.  Thread tid serves items tid and tid + blockDim of every block, so where an item comes from
-	// and where it goes is worked out once; per block a thread issues its (at most two) 16-byte loads before the running block's
-	// arithmetic and finishes them (decay, beta) into the other buffer after it.
-	const int items4 = (3 * D + V) / 4 + 1;
-	const float* src[2];
-	const bf16* biasp[2];            // decay items: their four dt_bias entries
-	int stride[2], slot[2], kind[2]; // kind: 0 plain float4, 1 decay input, 2 beta input (scalar), -1 none
+	// Staging.  A token's inputs are 3 D / 4 + DELTA_VC / 4 float4 items (k, q, raw decay input, v) and one scalar (beta's input); item e
+	// of a block belongs to token e / ITEMS.  A thread serves the same items of every block, so where they come from and go to is worked
+	// out once; per block it issues its 16-byte loads before the running block's arithmetic and finishes them (decay, beta) after it.
+	const float* src[ROUNDS];
+	float4 bias[ROUNDS];                                // decay items: their dt_bias entries
+	int stride[ROUNDS], slot[ROUNDS], kind[ROUNDS];     // kind: 0 plain float4, 1 decay input, 2 beta input (scalar), -1 none
 #pragma unroll
-	for (int r = 0; r < 2; ++r) {
-		const int e = tid + r * (int)blockDim.x, tt = e / items4, it4 = e % items4;
-		kind[r] = -1, src[r] = a.k, stride[r] = 0, slot[r] = 0, biasp[r] = a.dt_bias;
-		if (tt < DELTA_TB) {
-			const int i0 = 4 * it4;
-			if (i0 < 3 * D) {
-				const int seg = i0 / D, w = i0 % D;
-				kind[r] = seg == 2 ? 1 : 0;
-				biasp[r] = a.dt_bias + h * D + w;
-				stride[r] = seg == 2 ? a.heads * D : a.kv_heads * D;
-				src[r] = (seg == 0 ? a.k + (size_t)kh * D : seg == 1 ? a.q + (size_t)kh * D : a.dt + (size_t)h * D) + w + (size_t)(start + tt) * stride[r];
-				slot[r] = tt * tok_len + seg * 4 * QP + (w / Q) * QP + w % Q;
-			} else if (i0 < 3 * D + V) {
-				kind[r] = 0, stride[r] = a.heads * V;
-				src[r] = a.v + (size_t)h * V + (i0 - 3 * D) + (size_t)(start + tt) * stride[r];
-				slot[r] = tt * tok_len + 3 * 4 * QP + i0 - 3 * D;
-			} else {
-				kind[r] = 2, stride[r] = a.ldp;
-				src[r] = a.proj + a.bcol + h + (size_t)(start + tt) * stride[r];
-				slot[r] = tt * tok_len + 3 * 4 * QP + V;
+	for (int r = 0; r < ROUNDS; ++r) {
+		const int e = tid + r * 128, tt = e / ITEMS, i0 = 4 * (e % ITEMS);
+		kind[r] = -1, src[r] = a.k, stride[r] = 0, slot[r] = 0, bias[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+		if (tt >= DELTA_TB) continue;
+		if (i0 < 3 * D) {
+			const int seg = i0 / D, w = i0 % D;
+			kind[r] = seg == 2 ? 1 : 0;
+			stride[r] = seg == 2 ? a.heads * D : a.kv_heads * D;
+			src[r] = (seg == 0 ? a.k + (size_t)kh * D : seg == 1 ? a.q + (size_t)kh * D : a.dt + (size_t)h * D) + w + (size_t)(start + tt) * stride[r];
+			slot[r] = tt * TOK + seg * 8 * QP + (w / Q) * QP + w % Q;
+			if (seg == 2) {
+				const bf16* bp = a.dt_bias + h * D + w;
+				bias[r] = make_float4(ldf(bp), ldf(bp + 1), ldf(bp + 2), ldf(bp + 3));
 			}
+		} else if (i0 < 3 * D + DELTA_VC) {
+			const int i = i0 - 3 * D;
+			if (v0 + i >= V) continue;
+			kind[r] = 0, stride[r] = a.heads * V;
+			src[r] = a.v + (size_t)h * V + v0 + i + (size_t)(start + tt) * stride[r];
+			slot[r] = tt * TOK + VAT + i;
+		} else {
+			kind[r] = 2, stride[r] = a.ldp;
+			src[r] = a.proj + a.bcol + h + (size_t)(start + tt) * stride[r];
+			slot[r] = tt * TOK + BAT;
 		}
 	}
-	const int tt_of[2] = {tid / items4, (tid + (int)blockDim.x) / items4};
-	auto fetch_block = [&](int blk, float4 (&pre)[2]) {
+	auto fetch_block = [&](int blk, float4 (&pre)[ROUNDS]) {
 		const int nt = min(DELTA_TB, cnt - blk * DELTA_TB);
 #pragma unroll
-		for (int r = 0; r < 2; ++r) {
+		for (int r = 0; r < ROUNDS; ++r) {
 			pre[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-			if (kind[r] >= 0 && tt_of[r] < nt) {
+			if (kind[r] >= 0 && (tid + r * 128) / ITEMS < nt) {
 				const float* p = src[r] + (size_t)blk * DELTA_TB * stride[r];
 				if (kind[r] == 2) pre[r].x = __ldg(p);
 				else pre[r] = __ldg((const float4*)p);
 			}
 		}
 	};
-	auto put_block = [&](float* st, int blk, const float4 (&pre)[2]) {
+	auto put_block = [&](float* st, int blk, const float4 (&pre)[ROUNDS]) {
 		const int nt = min(DELTA_TB, cnt - blk * DELTA_TB);
 #pragma unroll
-		for (int r = 0; r < 2; ++r) {
-			if (kind[r] >= 0 && tt_of[r] < nt) {
+		for (int r = 0; r < ROUNDS; ++r) {
+			if (kind[r] >= 0 && (tid + r * 128) / ITEMS < nt) {
 				float4 v = pre[r];
 				if (kind[r] == 1) {
-					const bf16* bias = biasp[r];
-					v.x = expf(-A * softplusf_(v.x + ldf(bias))), v.y = expf(-A * softplusf_(v.y + ldf(bias + 1)));
-					v.z = expf(-A * softplusf_(v.z + ldf(bias + 2))), v.w = expf(-A * softplusf_(v.w + ldf(bias + 3)));
+					v.x = expf(-A * softplusf_(v.x + bias[r].x)), v.y = expf(-A * softplusf_(v.y + bias[r].y));
+					v.z = expf(-A * softplusf_(v.z + bias[r].z)), v.w = expf(-A * softplusf_(v.w + bias[r].w));
 				}
 				if (kind[r] == 2) st[slot[r]] = sigmoidf_(v.x);
 				else *(float4*)(st + slot[r]) = v;
 			}
 		}
 	};
-	const int nblk = (cnt + DELTA_TB - 1) / DELTA_TB;
-	float4 pre[2];
+	const int nblk = (cnt + DELTA_TB - 1) / DELTA_TB, vcol = live ? cl : 0; // (a staged column; what the others compute goes nowhere)
+	float4 pre[ROUNDS];
 	fetch_block(0, pre);
-	put_block(buf[0], 0, pre);
+	put_block(sm, 0, pre);
 	__syncthreads();
 	for (int blk = 0; blk < nblk; ++blk) {
-		const float* cur = buf[blk & 1];
+		const float* __restrict__ cur = sm + (blk & 1) * DELTA_TB * TOK;
 		if (blk + 1 < nblk) fetch_block(blk + 1, pre);
 		const int nt = min(DELTA_TB, cnt - blk * DELTA_TB);
-		for (int tt = 0; tt < nt; ++tt) {
-			const float* tk = cur + tt * tok_len;
-			const float4 *ks = (const float4*)(tk + part * QP), *qs = (const float4*)(tk + 4 * QP + part * QP), *gs = (const float4*)(tk + 8 * QP + part * QP);
-			float dot = 0.f;
+		float o[2 * DELTA_TB];
+		auto apply = [&](int tt, float& oa, float& ob) { // one token: decay, correction, this lane's share of the read-out
+			const float* tk = cur + tt * TOK;
+			const float4 *ks = (const float4*)(tk + part * QP), *qs = (const float4*)(tk + 8 * QP + part * QP), *gs = (const float4*)(tk + 16 * QP + part * QP);
+			const float2 v = *(const float2*)(tk + VAT + vcol);
+			float dot[2][2] = {};
 #pragma unroll
 			for (int i = 0; i < Q / 4; ++i) {
 				const float4 g4 = gs[i], k4 = ks[i];
-				S[4 * i] *= g4.x, S[4 * i + 1] *= g4.y, S[4 * i + 2] *= g4.z, S[4 * i + 3] *= g4.w;
-				dot = fmaf(S[4 * i], k4.x, dot), dot = fmaf(S[4 * i + 1], k4.y, dot), dot = fmaf(S[4 * i + 2], k4.z, dot), dot = fmaf(S[4 * i + 3], k4.w, dot);
+				const float g[4] = {g4.x, g4.y, g4.z, g4.w}, k[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+				for (int e = 0; e < 4; ++e)
+#pragma unroll
+					for (int c = 0; c < 2; ++c) S[4 * i + e][c] *= g[e], dot[c][e & 1] = fmaf(S[4 * i + e][c], k[e], dot[c][e & 1]);
 			}
-			dot += __shfl_xor_sync(0xffffffffu, dot, 1);
-			dot += __shfl_xor_sync(0xffffffffu, dot, 2);
-			const float u = tk[3 * 4 * QP + V] * (tk[3 * 4 * QP + col] - dot);
-			float o = 0.f;
+			float u[2] = {dot[0][0] + dot[0][1], dot[1][0] + dot[1][1]};
+#pragma unroll
+			for (int w = 1; w < 8; w <<= 1) u[0] += __shfl_xor_sync(0xffffffffu, u[0], w), u[1] += __shfl_xor_sync(0xffffffffu, u[1], w);
+			u[0] = tk[BAT] * (v.x - u[0]), u[1] = tk[BAT] * (v.y - u[1]);
+			float r[2][2] = {};
 #pragma unroll
 			for (int i = 0; i < Q / 4; ++i) {
 				const float4 k4 = ks[i], q4 = qs[i];
-				S[4 * i] = fmaf(k4.x, u, S[4 * i]), S[4 * i + 1] = fmaf(k4.y, u, S[4 * i + 1]), S[4 * i + 2] = fmaf(k4.z, u, S[4 * i + 2]), S[4 * i + 3] = fmaf(k4.w, u, S[4 * i + 3]);
-				o = fmaf(S[4 * i], q4.x, o), o = fmaf(S[4 * i + 1], q4.y, o), o = fmaf(S[4 * i + 2], q4.z, o), o = fmaf(S[4 * i + 3], q4.w, o);
+				const float k[4] = {k4.x, k4.y, k4.z, k4.w}, q[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+				for (int e = 0; e < 4; ++e)
+#pragma unroll
+					for (int c = 0; c < 2; ++c) S[4 * i + e][c] = fmaf(k[e], u[c], S[4 * i + e][c]), r[c][e & 1] = fmaf(S[4 * i + e][c], q[e], r[c][e & 1]);
 			}
-			o += __shfl_xor_sync(0xffffffffu, o, 1);
-			o += __shfl_xor_sync(0xffffffffu, o, 2);
-			if (part == 0 && live) a.o[((size_t)(start + blk * DELTA_TB + tt) * a.heads + h) * V + col] = o;
+			oa = r[0][0] + r[0][1], ob = r[1][0] + r[1][1];
+		};
+		if (nt == DELTA_TB) { // no branch between the tokens: loads of later ones move up past the arithmetic of earlier ones
+#pragma unroll
+			for (int tt = 0; tt < DELTA_TB; ++tt) apply(tt, o[2 * tt], o[2 * tt + 1]);
+		} else {
+#pragma unroll
+			for (int tt = 0; tt < DELTA_TB; ++tt) {
+				o[2 * tt] = o[2 * tt + 1] = 0.f;
+				if (tt < nt) apply(tt, o[2 * tt], o[2 * tt + 1]);
+			}
 		}
-		if (blk + 1 < nblk) put_block(buf[(blk + 1) & 1], blk + 1, pre);
+#pragma unroll
+		for (int w = 4; w > 0; w >>= 1) { // lane bit w keeps the half of the values that has it
+			const bool up = part & w;
+#pragma unroll
+			for (int i = 0; i < w; ++i) {
+				const float other = __shfl_xor_sync(0xffffffffu, up ? o[i] : o[i + w], w);
+				o[i] = (up ? o[i + w] : o[i]) + other;
+			}
+		}
+		if (live && (part >> 1) < nt) a.o[((size_t)(start + blk * DELTA_TB + (part >> 1)) * a.heads + h) * V + col + (part & 1)] = o[0];
+		if (blk + 1 < nblk) put_block(sm + ((blk + 1) & 1) * DELTA_TB * TOK, blk + 1, pre);
 		__syncthreads();
 	}
 	if (live) {
 #pragma unroll
-		for (int i = 0; i < Q; ++i) Sg[(size_t)(part * Q + i) * V + col] = S[i];
+		for (int i = 0; i < Q; ++i) *(float2*)(Sg + (size_t)i * V) = make_float2(S[i][0], S[i][1]);
 	}
 }
 // read-out: o / rms(o) (per head) * w * sigmoid(gate); one warp per (token, head)

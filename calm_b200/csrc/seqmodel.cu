@@ -919,14 +919,12 @@ void mixer_typed(Seq& s, const SeqLayer& L, RunState& r, const SeqBatch& sb, dou
 		d.state = r.delta, d.o = s.f[5], d.heads = H, d.kv_heads = G, d.dim = D, d.vdim = Dv;
 		const size_t smem = ((size_t)D * Dv + 3 * D) * sizeof(float);
 		const int threads = std::max(64, cdiv(Dv, 32) * 32);
-		const size_t smem_reg = 2 * (size_t)DELTA_TB * (3 * (D + 16) + ((Dv + 4) & ~3)) * sizeof(float);
-		const int threads_reg = std::max(256, cdiv(4 * Dv, 32) * 32); // two staging rounds cover DELTA_TB * ((3 D + Dv) / 4 + 1) items
-		const bool reg = (D == 32 || D == 64 || D == 128) && 4 * Dv <= 512 && Dv % 4 == 0 && !getenv("CALM_B200_SEQ_DELTA_SMEM");
+		const bool reg = (D == 32 || D == 64 || D == 128) && Dv <= 128 && Dv % 4 == 0 && !getenv("CALM_B200_SEQ_DELTA_SMEM");
 		run_kernel(s, KD_DELTA, (double)N * H * (3.0 * D + 2.0 * Dv) * 4 + 2.0 * sb.B * H * D * Dv * 4, (double)N * H * D * Dv * 6.0, [&] {
-			const dim3 grid(sb.B, H);
-			if (reg && D == 32) launch_k(s, k_seq_delta_scan_reg<32>, grid, threads_reg, smem_reg, d, sb);
-			else if (reg && D == 64) launch_k(s, k_seq_delta_scan_reg<64>, grid, threads_reg, smem_reg, d, sb);
-			else if (reg && D == 128) launch_k(s, k_seq_delta_scan_reg<128>, grid, threads_reg, smem_reg, d, sb);
+			const dim3 grid(sb.B, H, cdiv(Dv, DELTA_VC));
+			if (reg && D == 32) launch_k(s, k_seq_delta_scan_reg<32>, grid, 128, 0, d, sb);
+			else if (reg && D == 64) launch_k(s, k_seq_delta_scan_reg<64>, grid, 128, 0, d, sb);
+			else if (reg && D == 128) launch_k(s, k_seq_delta_scan_reg<128>, grid, 128, 0, d, sb);
 			else launch_k(s, k_seq_delta_scan, dim3(sb.B, H), threads, smem, d, sb);
 		});
 		run_kernel(s, KD_NORM, (double)N * H * Dv * 10, 0,
