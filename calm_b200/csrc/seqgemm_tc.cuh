@@ -32,8 +32,12 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
 	             : "memory");
 }
 // The epilogue of one warp: its 32 weight rows (lane = row m) against the tile's tokens, 32 at a time.  E: what the epilogue does when it is one
-// of the plain ones -- a bias at most, and for EPI_F32 columns past `split` in the activation type -- with everything that does not depend on
-// the token worked out before the loop; TG_ANY: gemm_store decides per element.
+// of the plain ones -- a bias and a factor at most, and for EPI_F32 columns past `split` in the activation type -- with everything that does not
+// depend on the token worked out before the loop.  The additions to the residual stream load 16 tokens' rows ahead of the stores: one after the
+// other, each store bars the next load (164 us for 2048 x 2048 x 5632).  TG_ANY: gemm_store decides per element, in a loop that is not
+// unrolled: 32 copies of every epilogue do not fit the instruction cache (a 2048 x 2048 x 64 decay product through them took 124 us).
+// All products of a 2048-token step with attention and two linear attentions: 1735 us with residual additions, decays and squared rectifiers in the
+// unrolled TG_ANY, 747 in instances of their own.
 #define TG_ANY (-1)
 #define TG_ACT_GATE 100 // EPI_ACT times sigmoid(gate)
 template <int E>
@@ -41,7 +45,9 @@ __device__ __forceinline__ void tg_epilogue(const GemmArgs& a, int z, const Gemm
 	const int rows = min(TG_BN, gr.count - n0);
 	const bool live = m < a.M;
 	const float bias = E != TG_ANY && a.bias && live ? ldf(a.bias + (size_t)z * a.M + m) : 0.f;
+	const float scale = a.out_scale != 0.f ? a.out_scale : 1.f;
 	const bool aside = E == EPI_F32 && a.split > 0 && m >= a.split; // this weight row's results go to Y2
+	const bool f32 = (E == EPI_F32 && !aside) || E == EPI_DECAY;    // fp32 results
 	const long ld = aside ? a.ldy2 : a.ldy;
 	const size_t o = aside ? (size_t)(gr.base + n0) * a.ldy2 + (m - a.split) : (size_t)z * a.ybs + (size_t)(gr.base + n0) * a.ldy + (E == EPI_GLU ? m >> 1 : m);
 	float* const yf = (float*)a.Y + o;
@@ -52,13 +58,34 @@ __device__ __forceinline__ void tg_epilogue(const GemmArgs& a, int z, const Gemm
 		float v[32];
 		tmem_ld32(tmem + c0, v);
 		if constexpr (E == TG_ANY) {
-#pragma unroll
+#pragma unroll 1
 			for (int j = 0; j < 32; ++j) gemm_store<bf16>(a, z, gr, n0 + c0 + j, m, v[j]); // lanes = consecutive weight rows: coalesced
+		} else if constexpr (E == EPI_RES || E == EPI_DYT_RES) {
+			const int left = live ? rows - c0 : 0;
+			float* p = yf + (size_t)c0 * ld;
+			const float* rp = E == EPI_RES && a.res ? a.res + o + (size_t)c0 * ld : nullptr;
+			const float na = E == EPI_DYT_RES ? ldf(a.na) : 0.f, nw = E == EPI_DYT_RES && live ? ldf(a.nw + m) : 0.f, nb = E == EPI_DYT_RES && live ? ldf(a.nb + m) : 0.f;
+#pragma unroll
+			for (int j0 = 0; j0 < 32; j0 += 16) {
+				float y[16], r[16];
+				float* py = p;
+#pragma unroll
+				for (int i = 0; i < 16; ++i, py += ld) y[i] = j0 + i < left ? *py : 0.f;
+				if (rp) {
+#pragma unroll
+					for (int i = 0; i < 16; ++i, rp += ld) r[i] = j0 + i < left ? *rp : 0.f;
+				}
+#pragma unroll
+				for (int i = 0; i < 16; ++i, p += ld) {
+					const float x = (v[j0 + i] + bias) * scale;
+					if (j0 + i < left) *p = y[i] + (E == EPI_DYT_RES ? tanhf(na * x) * nw + nb : rp ? r[i] + x : x);
+				}
+			}
 		} else {
 			const int left = rows - c0;
 			// the row pointer advances by one addition per token: 32 separate row offsets would cost the kernel its second CTA per SM
-			unsigned char* q = (unsigned char*)(E == EPI_F32 && !aside ? (void*)yf : (void*)yb) + (size_t)c0 * ld * (E == EPI_F32 && !aside ? 4 : 2);
-			const size_t step = (size_t)ld * (E == EPI_F32 && !aside ? 4 : 2);
+			unsigned char* q = (unsigned char*)(f32 ? (void*)yf : (void*)yb) + (size_t)c0 * ld * (f32 ? 4 : 2);
+			const size_t step = (size_t)ld * (f32 ? 4 : 2);
 			if constexpr (E == EPI_GLU) { // lanes 2c (gate) and 2c + 1 (up) share the unit's tokens: the even lane forms token j, the odd one token j + 1
 				const int odd = lane & 1;
 				q += odd ? step : 0;
@@ -71,12 +98,15 @@ __device__ __forceinline__ void tg_epilogue(const GemmArgs& a, int z, const Gemm
 			} else {
 #pragma unroll
 				for (int j = 0; j < 32; ++j, q += step, gate += gstep) {
-					const float x = v[j] + bias;
+					const float x = (v[j] + bias) * scale;
 					if (j >= left || !live) continue;
+					const float pos = fmaxf(x, 0.f);
 					if constexpr (E == EPI_F32) {
-						if (aside) *(bf16*)q = __float2bfloat16_rn(x);
+						if (aside) *(bf16*)q = __float2bfloat16_rn(a.split_act ? x : pos * pos);
 						else *(float*)q = x;
-					} else if constexpr (E == EPI_ACT) *(bf16*)q = __float2bfloat16_rn(x);
+					} else if constexpr (E == EPI_DECAY) *(float*)q = expf(-softplusf_(-x) * a.epi_f);
+					else if constexpr (E == EPI_ACT_RELU2) *(bf16*)q = __float2bfloat16_rn(pos * pos);
+					else if constexpr (E == EPI_ACT) *(bf16*)q = __float2bfloat16_rn(x);
 					else if constexpr (E == TG_ACT_GATE) *(bf16*)q = __float2bfloat16_rn(x * sigmoidf_(*gate));
 					else {
 						const bf16 h = __float2bfloat16_rn(x);
@@ -90,9 +120,9 @@ __device__ __forceinline__ void tg_epilogue(const GemmArgs& a, int z, const Gemm
 }
 // which instance serves a product
 static inline int tg_kind(const GemmArgs& a) {
-	const bool plain = a.out_scale == 0.f && a.out_cap == 0.f && !a.rs && (a.split == 0 || (a.epi == EPI_F32 && a.split_act == 1));
+	const bool plain = a.out_cap == 0.f && !a.rs && (a.split == 0 || a.epi == EPI_F32) && (a.out_scale == 0.f || a.epi != EPI_GLU);
 	if (a.gate) return plain && a.epi == EPI_ACT ? TG_ACT_GATE : TG_ANY;
-	return plain && (a.epi == EPI_F32 || a.epi == EPI_ACT || a.epi == EPI_SPLIT3 || a.epi == EPI_GLU) ? a.epi : TG_ANY;
+	return plain ? a.epi : TG_ANY;
 }
 
 template <int E>
@@ -202,7 +232,8 @@ static inline void gemm_tc_setup() {
 	CUDA_CHECK(cudaHostAlloc((void**)&g_tg.err_host, sizeof(int), cudaHostAllocMapped));
 	*g_tg.err_host = 0;
 	CUDA_CHECK(cudaHostGetDevicePointer((void**)&g_tg.err_dev, g_tg.err_host, 0));
-	for (auto k : {k_seq_gemm_tc<TG_ANY>, k_seq_gemm_tc<EPI_F32>, k_seq_gemm_tc<EPI_ACT>, k_seq_gemm_tc<EPI_SPLIT3>, k_seq_gemm_tc<EPI_GLU>, k_seq_gemm_tc<TG_ACT_GATE>})
+	for (auto k : {k_seq_gemm_tc<TG_ANY>, k_seq_gemm_tc<EPI_F32>, k_seq_gemm_tc<EPI_ACT>, k_seq_gemm_tc<EPI_SPLIT3>, k_seq_gemm_tc<EPI_GLU>, k_seq_gemm_tc<TG_ACT_GATE>, k_seq_gemm_tc<EPI_RES>,
+	               k_seq_gemm_tc<EPI_DYT_RES>, k_seq_gemm_tc<EPI_ACT_RELU2>, k_seq_gemm_tc<EPI_DECAY>})
 		CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TG_SMEM));
 }
 // a stalled pipeline leaves its code here; read after the stream has been synchronised
@@ -254,6 +285,10 @@ static inline bool gemm_tc_launch(const GemmArgs& a, int batch, cudaStream_t str
 	case EPI_ACT: go(k_seq_gemm_tc<EPI_ACT>); break;
 	case EPI_SPLIT3: go(k_seq_gemm_tc<EPI_SPLIT3>); break;
 	case EPI_GLU: go(k_seq_gemm_tc<EPI_GLU>); break;
+	case EPI_RES: go(k_seq_gemm_tc<EPI_RES>); break;
+	case EPI_DYT_RES: go(k_seq_gemm_tc<EPI_DYT_RES>); break;
+	case EPI_ACT_RELU2: go(k_seq_gemm_tc<EPI_ACT_RELU2>); break;
+	case EPI_DECAY: go(k_seq_gemm_tc<EPI_DECAY>); break;
 	case TG_ACT_GATE: go(k_seq_gemm_tc<TG_ACT_GATE>); break;
 	default: go(k_seq_gemm_tc<TG_ANY>);
 	}
