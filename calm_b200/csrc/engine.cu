@@ -1315,7 +1315,7 @@ static void pf_reserve(int n) {
 		}
 		pf.ws = (float*)dev_alloc((size_t)g.sms * 256 * PF_BM * sizeof(float)); // an item's accumulators: at most 256 columns
 		pf.counter = (unsigned*)dev_alloc(g.sms * sizeof(unsigned));
-		CUDA_CHECK(cudaMemset(pf.counter, 0, g.sms * sizeof(unsigned)));
+		CUDA_CHECK(cudaMemsetAsync(pf.counter, 0, g.sms * sizeof(unsigned), g.stream));
 	}
 	int cap = cdiv(n, PF_PAD) * PF_PAD;
 	if (cap <= pf.cap) return;
@@ -1326,7 +1326,7 @@ static void pf_reserve(int n) {
 	pf.cap = cap;
 	auto zalloc = [&](size_t bytes) {
 		void* p = dev_alloc(bytes);
-		CUDA_CHECK(cudaMemset(p, 0, bytes)); // padding rows of a partial token tile stay zero
+		CUDA_CHECK(cudaMemsetAsync(p, 0, bytes, g.stream)); // padding rows of a partial token tile stay zero.  On the stream of the pass: it does not wait for the default one
 		return p;
 	};
 	pf.X = (float*)zalloc((size_t)cap * c.dim * sizeof(float));
@@ -1605,7 +1605,7 @@ extern "C" void calm_b200_set_perf(int on) {
 	g.perf = on != 0;
 	if (!on) return;
 	CUDA_CHECK(cudaStreamSynchronize(g.stream));
-	CUDA_CHECK(cudaMemset(g.stamp_acc, 0, (size_t)(MAX_STAMPS + 2) * sizeof(unsigned long long)));
+	CUDA_CHECK(cudaMemsetAsync(g.stamp_acc, 0, (size_t)(MAX_STAMPS + 2) * sizeof(unsigned long long), g.stream));
 	for (int i = 0; i < ST_COUNT; ++i) g.stage_ms[i] = 0, g.stage_bytes[i] = 0, g.stage_launches[i] = 0;
 	g.perf_runs = 0, g.token_span_ms = 0;
 }
