@@ -56,6 +56,7 @@ struct Engine {
 	int* last_token = nullptr; // pinned + mapped
 	int ncand = 0;
 
+	unsigned pf_wait_limit = MBAR_SPINS; // tries of a wait in the prompt products
 	// attention launch shape
 	int attn_hg = 1, attn_hg2 = 1 /* k_attn2: padded to what it is instantiated for */, attn_qgroups = 1, attn_nsplit = 1, attn_lpp = 1;
 	// TMA-ring matvec kernels (ring.cuh): slots per warp / CTAs per SM for FFN-up and for wo / w2; u = 512-byte units per row and chunk (0: not used)
@@ -950,6 +951,7 @@ extern "C" void prepare_cuda(struct Transformer* transformer) {
 	g.use_graph = !(getenv("CALM_B200_GRAPH") && atoi(getenv("CALM_B200_GRAPH")) == 0);
 	g.use_pdl = !(getenv("CALM_B200_PDL") && atoi(getenv("CALM_B200_PDL")) == 0);
 	g.carveout = getenv("CALM_B200_CARVEOUT") ? atoi(getenv("CALM_B200_CARVEOUT")) : -1;
+	if (const char* e = getenv("CALM_B200_PREFILL_WAIT")) g.pf_wait_limit = (unsigned)atoi(e);
 	g.debug = getenv("CALM_B200_DEBUG") && atoi(getenv("CALM_B200_DEBUG"));
 	if (g.debug) g.use_graph = false;
 	g.perf = (getenv("CALM_B200_PERF") && atoi(getenv("CALM_B200_PERF"))) || getenv("CUDA_INJECTION64_PATH");
@@ -1375,7 +1377,7 @@ static void pf_gemm(const CUtensorMap (&tx)[3][2], const CUtensorMap* tw, PfGemm
 	PfMaps m;
 	memcpy(m.x, tx[a.bn / 128], sizeof(m.x)); // 64, 128, 256 -> 0, 1, 2
 	memcpy(m.w, tw, (MODE == PF_QKV ? 3 : MODE == PF_UP ? 2 : 1) * sizeof(CUtensorMap));
-	a.n_tokens = n, a.rows = rows, a.ws = pf.ws, a.counter = pf.counter, a.err = g.dev_err;
+	a.n_tokens = n, a.rows = rows, a.ws = pf.ws, a.counter = pf.counter, a.err = g.dev_err, a.wait_limit = g.pf_wait_limit;
 	a.stages = imin(PF_MAX_STAGES, (int)((limit - fixed) / pf_stage_bytes(a.na, a.bn)));
 	const int row_items = MODE == PF_UP ? rows / PF_BM : cdiv(rows / PF_BM, a.na);
 	cudaLaunchConfig_t cfg = {};

@@ -130,6 +130,7 @@ struct PfGemmArgs {
 	float* ws;            // splits > 1: [item][na][bn][128] partial sums
 	unsigned* counter;    // splits > 1: [row tiles x token tiles], zero between launches
 	int* err;             // mapped host word: code of a wait that gave up
+	unsigned wait_limit;  // tries of a wait before it gives up
 	// QKV epilogue
 	float* Q;         // [T][q_dim]
 	int q_dim, kv_dim, head_dim, seq_len, pos0, kvbits;
@@ -275,11 +276,13 @@ __device__ __forceinline__ bool elect_one() { // one lane of a converged warp
 template <int MODE, int DBITS>
 __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid_constant__ PfMaps m, const PfGemmArgs a) {
 	constexpr int WIDEN = pf_widen_warps<DBITS>(), W_WARP = 6 + WIDEN, LO_WARP = W_WARP + 1;
+	constexpr int ROLES = 2 + (DBITS == 16 ? 1 : WIDEN); // arrivals that make a stage full: hi, lo, then the weight copy or the widening warps
 	constexpr int RT = pf_raw_tiles<DBITS>(), RAW = pf_raw_bytes<DBITS>();
 	extern __shared__ unsigned char smem_dyn[];
 	__shared__ __align__(8) uint64_t full[PF_MAX_STAGES], empty[PF_MAX_STAGES], r_full[RT ? RT : 1], r_empty[RT ? RT : 1], acc_full[2], acc_empty[2];
 	__shared__ uint32_t tmem_base_s;
 	__shared__ int last_s;
+	__shared__ int handed[ROLES], raw_handed, multiplied, accumulated; // stages and items that each role got to (read when a wait has given up)
 	unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 	const int nkb = a.K / PF_BK, ns = a.stages, bn = a.bn, splits = a.splits, na = MODE == PF_UP ? 2 : a.na;
@@ -302,7 +305,8 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 		r.k0 = (int)((long)nkb * sp / splits), r.k1 = (int)((long)nkb * (sp + 1) / splits);
 		return r;
 	};
-	// every wait is bounded: a role whose wait gives up records a code and leaves its loop, the others follow, and the host reads the code
+	// every wait is bounded: a role whose wait gives up (whole warps at a time) records a code and leaves its loop, the others follow, what is on its
+	// way into shared memory or TMEM is waited for, and the host reads the code
 	auto gave_up = [&](int code) {
 		if (a.err) *reinterpret_cast<volatile int*>(a.err) = code;
 		return false;
@@ -311,7 +315,7 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 	pdl_launch_next();
 	if (tid == 0) {
 		for (int s = 0; s < RT; ++s) mbar_init(&r_full[s], 1), mbar_init(&r_empty[s], WIDEN);
-		for (int s = 0; s < ns; ++s) mbar_init(&full[s], 2 + (DBITS == 16 ? 1 : WIDEN)), mbar_init(&empty[s], 1); // hi, lo, weights: the copy or the widening warps
+		for (int s = 0; s < ns; ++s) mbar_init(&full[s], ROLES), mbar_init(&empty[s], 1);
 		for (int s = 0; s < 2; ++s) mbar_init(&acc_full[s], 1), mbar_init(&acc_empty[s], 4);
 		mbar_init_fence();
 	}
@@ -328,12 +332,12 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 		pdl_wait_prev();
 		const bool el = elect_one();
 		const int lo = warp != 0;
-		int s = 0;
+		int s = 0, n = 0;
 		unsigned ph = 1;
 		for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
 			const Item t = item_of(it);
 			for (int kb = t.k0; kb < t.k1; ++kb) {
-				if (!__all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], ph))) {
+				if (!mbar_wait_warp(&empty[s], ph, a.wait_limit)) {
 					ok = gave_up(9301);
 					break;
 				}
@@ -341,22 +345,24 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 					mbar_expect_tx(&full[s], b_bytes);
 					tma_load_2d(b_tile(s) + lo * b_bytes, &m.x[lo], kb * PF_BK, t.tok0, &full[s]);
 				}
+				++n;
 				if (++s == ns) s = 0, ph ^= 1;
 			}
 		}
+		if (lane == 0) handed[lo] = n;
 	} else if (warp == 1) { // ===== MMAs
 		// kind::f16: D = f32, A = B = f16, both K-major, M = 128, N = bn
 		const uint32_t idesc = (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(PF_BM >> 4) << 24);
 		const bool el = elect_one();
-		int s = 0;
+		int s = 0, n = 0;
 		unsigned ph = 0, q = 0;
-		for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++q) {
+		for (int it = blockIdx.x; it < items; it += gridDim.x, ++q) {
 			const Item t = item_of(it);
 			const uint32_t acc = tmem_base + (q & 1) * 256;
-			if (!__all_sync(0xffffffffu, mbar_wait_bounded(&acc_empty[q & 1], ((q >> 1) & 1) ^ 1))) ok = gave_up(9302);
+			if (!mbar_wait_warp(&acc_empty[q & 1], ((q >> 1) & 1) ^ 1, a.wait_limit)) ok = gave_up(9302);
 			tc_fence_after();
 			for (int kb = t.k0; kb < t.k1 && ok; ++kb) {
-				if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full[s], ph))) {
+				if (!mbar_wait_warp(&full[s], ph, a.wait_limit)) {
 					ok = gave_up(9303);
 					break;
 				}
@@ -374,11 +380,14 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 					umma_commit(&empty[s]); // frees the stage when these MMAs have read it
 				}
 				__syncwarp();
+				++n;
 				if (++s == ns) s = 0, ph ^= 1;
 			}
+			if (!ok) break;
 			if (el) umma_commit(&acc_full[q & 1]);
 			__syncwarp();
 		}
+		if (lane == 0) multiplied = n, accumulated = q;
 	} else if (warp < 6) { // ===== epilogue: one accumulator row per thread
 		pdl_wait_prev();
 		const int q4 = warp & 3, lr = q4 * 32 + lane; // the TMEM lane quarter this warp may read
@@ -387,8 +396,8 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 			const Item t = item_of(it);
 			const uint32_t acc = tmem_base + (q & 1) * 256 + ((uint32_t)(q4 * 32) << 16);
 			// the four warps go on together or leave together: none is left alone at a named barrier
-			if (!bar_and(1, 128, mbar_wait_bounded(&acc_full[q & 1], (q >> 1) & 1))) {
-				gave_up(9305);
+			if (!bar_and(1, 128, mbar_wait_bounded(&acc_full[q & 1], (q >> 1) & 1, a.wait_limit))) {
+				ok = gave_up(9305);
 				break;
 			}
 			tc_fence_after();
@@ -450,12 +459,12 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 		uint64_t* wempty = DBITS == 16 ? empty : r_empty;
 		const int ws = DBITS == 16 ? ns : rs;
 		const bool el = elect_one();
-		int s = 0;
+		int s = 0, n = 0;
 		unsigned ph = 1;
 		for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
 			const Item t = item_of(it);
 			for (int kb = t.k0; kb < t.k1; ++kb) {
-				if (!__all_sync(0xffffffffu, mbar_wait_bounded(&wempty[s], ph))) {
+				if (!mbar_wait_warp(&wempty[s], ph, a.wait_limit)) {
 					ok = gave_up(9306);
 					break;
 				}
@@ -470,22 +479,27 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 						tma_load_2d(DBITS == 16 ? a_tile(s, i) : r_tile(s, i), &m.w[which], kb * (DBITS == 16 ? PF_BK : PF_BK * DBITS / 8), row, &wfull[s]);
 					}
 				}
+				++n;
 				if (++s == ws) s = 0, ph ^= 1;
 			}
 		}
+		if (lane == 0) (DBITS == 16 ? handed[2] : raw_handed) = n;
 	} else if constexpr (DBITS != 16) { // ===== widening: a row per thread; with eight warps a tile each of two, or half the row each of one
 		constexpr int NV = DBITS / 2, PER = 8 / NV, NT = WIDEN == 4 ? 2 : 1; // 16-byte vectors of a row's k-stage, chunks of f16 from each, tiles per thread
 		const int r = (tid - 192) & 127, part = (tid - 192) >> 7;
 		const bool whole = WIDEN == 4 || na == 2;
 		const int tile0 = WIDEN == 8 && na == 2 ? part : 0, i0 = whole ? 0 : part * (NV / 2);
-		int sr = 0, sa = 0;
+		int sr = 0, sa = 0, n = 0;
 		unsigned pr = 0, pe = 1;
 		for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
 			const Item t = item_of(it);
 			const int nt = min(NT, t.cnt - tile0);
-			for (int kb = t.k0; kb < t.k1 && ok; ++kb) {
+			for (int kb = t.k0; kb < t.k1; ++kb) {
 				uint4 raw[NT][NV];
-				if (!mbar_wait_bounded(&r_full[sr], pr)) ok = gave_up(9307);
+				if (!mbar_wait_warp(&r_full[sr], pr, a.wait_limit)) {
+					ok = gave_up(9307);
+					break;
+				}
 #pragma unroll
 				for (int j = 0; j < NT; ++j)
 					if (j < nt) {
@@ -496,7 +510,10 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 				fence_async_smem(); // the copy engine writes next what was read here
 				__syncwarp();
 				if (lane == 0) mbar_arrive(&r_empty[sr]);
-				if (!mbar_wait_bounded(&empty[sa], pe)) ok = gave_up(9308);
+				if (!mbar_wait_warp(&empty[sa], pe, a.wait_limit)) {
+					ok = gave_up(9308);
+					break;
+				}
 #pragma unroll
 				for (int j = 0; j < NT; ++j)
 					if (j < nt) {
@@ -513,13 +530,32 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 				fence_async_smem();
 				__syncwarp();
 				if (lane == 0) mbar_arrive(&full[sa]);
+				++n;
 				if (++sr == rs) sr = 0, pr ^= 1;
 				if (++sa == ns) sa = 0, pe ^= 1;
 			}
 		}
+		if (lane == 0) handed[warp - 4] = n;
 	}
 	tc_fence_before();
-	__syncthreads();
+	if (__syncthreads_or(!ok)) { // a wait gave up: the copies and MMAs already issued end before the CTA does
+		if (tid == 0) {
+			int most = 0;
+			for (int r = 0; r < ROLES; ++r) most = max(most, handed[r]);
+			// no role is ns stages ahead of another, so each barrier is in the phase of one of the last ns stages; it gets the arrivals of the roles that
+			// did not come that far and then completes with its copies
+			for (int i = max(0, most - ns); i < most; ++i) {
+				for (int r = 0; r < ROLES; ++r)
+					if (handed[r] <= i) mbar_arrive(&full[i % ns]);
+				mbar_wait_bounded(&full[i % ns], (i / ns) & 1);
+			}
+			if constexpr (RT > 0)
+				for (int i = max(0, raw_handed - rs); i < raw_handed; ++i) mbar_wait_bounded(&r_full[i % rs], (i / rs) & 1);
+			if (multiplied) mbar_wait_bounded(&empty[(multiplied - 1) % ns], ((multiplied - 1) / ns) & 1);
+			if (accumulated) mbar_wait_bounded(&acc_full[(accumulated - 1) & 1], ((accumulated - 1) >> 1) & 1);
+		}
+		__syncthreads();
+	}
 	if (warp == 1) {
 		tc_fence_after();
 		tmem_dealloc(tmem_base, 512);

@@ -53,11 +53,16 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 	             "r"(c0), "r"(c1), "r"(smem_u32(bar))
 	             : "memory");
 }
-// about a second at most; false = gave up
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity) {
-	for (unsigned spins = 0; spins < (1u << 24); ++spins)
+#define MBAR_SPINS (1u << 24) // about a second at most
+// false = gave up
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, unsigned limit = MBAR_SPINS) {
+	for (unsigned spins = 0; spins < limit; ++spins)
 		if (mbar_try_wait(bar, parity)) return true;
 	return false;
+}
+// the same for a whole warp, which goes on or gives up together: a lane that left alone would be missing at the warp's next barrier
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, unsigned limit = MBAR_SPINS) {
+	return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, limit));
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 	asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
