@@ -157,16 +157,20 @@ __global__ void __launch_bounds__(TG_THREADS, 2) k_seq_gemm_tc(const __grid_cons
 	__syncthreads();
 	tc_fence_after();
 	const uint32_t tmem_base = tmem_base_s;
+	bool ok = true;
+	int copied = 0; // thread 0: stages requested
 
 	if (warp == 0) {
 		if (lane == 0) {
-			for (int kb = 0, it = 0; kb < nkb; ++kb) {
+			for (int kb = 0; kb < nkb; ++kb) {
 				if (skips(kb)) continue;
-				const int s = it % TG_STAGES;
-				if (!mbar_wait_bounded(&empty[s], ((it++ / TG_STAGES) & 1) ^ 1)) {
+				const int s = copied % TG_STAGES;
+				if (!mbar_wait_bounded(&empty[s], ((copied / TG_STAGES) & 1) ^ 1)) {
 					atomicExch(err, 1);
+					ok = false;
 					break;
 				}
+				++copied;
 				mbar_expect_tx(&full[s], TG_STAGE_BYTES);
 				if (w3d) tma_load_3d(a_tile(s), &tm_w, kb * TG_BK, m0, z, &full[s]);
 				else tma_load_2d(a_tile(s), &tm_w, kb * TG_BK, m0, &full[s]);
@@ -176,8 +180,7 @@ __global__ void __launch_bounds__(TG_THREADS, 2) k_seq_gemm_tc(const __grid_cons
 		}
 	} else if (warp == 1) {
 		if (lane == 0) {
-			bool ok = true;
-			for (int kb = 0, it = 0; kb < nkb && ok; ++kb) {
+			for (int kb = 0, it = 0; kb < nkb; ++kb) {
 				if (skips(kb)) continue;
 				const int s = it % TG_STAGES;
 				if (!mbar_wait_bounded(&full[s], (it / TG_STAGES) & 1)) {
@@ -195,7 +198,7 @@ __global__ void __launch_bounds__(TG_THREADS, 2) k_seq_gemm_tc(const __grid_cons
 			umma_commit(&accum); // arrives when everything issued so far has completed, also after a stall
 		}
 	} else {
-		const bool ok = mbar_wait_bounded(&accum, 0);
+		ok = mbar_wait_warp(&accum, 0);
 		if (!ok && lane == 0) atomicExch(err, 3);
 		tc_fence_after();
 		if (ok) {
@@ -204,7 +207,13 @@ __global__ void __launch_bounds__(TG_THREADS, 2) k_seq_gemm_tc(const __grid_cons
 		}
 		tc_fence_before();
 	}
-	__syncthreads();
+	if (__syncthreads_or(!ok)) { // a wait gave up: the copies and MMAs already issued end before the CTA does
+		if (tid == 0) {
+			for (int i = max(0, copied - TG_STAGES); i < copied; ++i) mbar_wait_bounded(&full[i % TG_STAGES], (i / TG_STAGES) & 1);
+			mbar_wait_bounded(&accum, 0);
+		}
+		__syncthreads();
+	}
 	if (warp == 1) {
 		tc_fence_after();
 		tmem_dealloc(tmem_base, TG_BN);

@@ -24,6 +24,9 @@ def test_warps_give_up_together():
     roles = src[src.index("k_pf_gemm(const __grid_constant__"):src.index("__syncthreads_or(!ok)")]
     assert "mbar_wait_warp(" in roles
     assert not re.findall(r"(?<!bar_and\(1, 128, )mbar_wait_bounded\(", roles)
+    src = open(os.path.join(ROOT, "calm_b200", "csrc", "seqgemm_tc.cuh")).read()
+    epilogue = src[src.index("} else {\n\t\tok = "):src.index("__syncthreads_or(!ok)")]  # the roles before it are one lane each
+    assert "mbar_wait_warp(" in epilogue and "mbar_wait_bounded(" not in epilogue
 
 
 @pytest.mark.gpu
