@@ -567,12 +567,14 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 // head: warp = (head, 16 consecutive tokens), so one 64-key tile of K and V in shared memory feeds up to 128 rows.  The cache
 // entries (fp16, or e5m2 widened on the way in) are exact f16 operands; queries and softmax weights travel as an f16 hi + lo
 // pair, two MMAs into the same fp32 accumulator, so they keep 22 bits.  A query row is first scaled by the power of two that
-// brings its largest entry into [1, 2) (exact; the score is scaled back), so no query leaves the f16 range.  Running maximum,
-// exponentials and the denominator are fp32.
+// brings its largest entry into [1, 2) (exact; the score is scaled back), so no query leaves the f16 range.  The weights (at most 1) carry a factor
+// of 2^15, which the denominator shares: 22 bits down to 2^-18 of the largest, steps of 2^-39 of it below (without the factor 2^-24: a
+// thousand keys of 2^-26 were lost).  Running maximum, exponentials and the denominator are fp32.
 // Bound: the MMA rate (4 x 64 MMAs per warp and tile against 32 KB of ldmatrix traffic).  Tokens are taken 16 per warp and not 32 because
 // 64 accumulator and 64 query registers per 16 rows already fill the file at 8 warps; the last blocks of the prompt, which see
 // the most keys, are started first.  2047 tokens, 32 / 8 heads of 128: 1550 us a layer as fp32 FMAs, one token per warp; about 360 us here.
 #define PFA_TILE 64 // keys per tile
+#define PFA_ONE 32768.f // weight of the largest score
 
 struct PfAttnArgs {
 	const float* Q; // [T][q_dim]
@@ -715,7 +717,7 @@ __global__ void __launch_bounds__(256, 1) k_pf_attn(const PfAttnArgs a) {
 #pragma unroll
 				for (int r = 0; r < 2; ++r) {
 					const float x = s[2 * kk + j][2 * r], y = s[2 * kk + j][2 * r + 1];
-					const float px = x == -FLT_MAX ? 0.f : expf(x - m[r]), py = y == -FLT_MAX ? 0.f : expf(y - m[r]);
+					const float px = x == -FLT_MAX ? 0.f : expf(x - m[r]) * PFA_ONE, py = y == -FLT_MAX ? 0.f : expf(y - m[r]) * PFA_ONE;
 					l[r] += px + py;
 					split_hl2(px, py, ph[2 * j + r], pl[2 * j + r]);
 				}
