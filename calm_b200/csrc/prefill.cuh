@@ -711,6 +711,8 @@ __global__ void __launch_bounds__(256, 1) k_pf_attn(const PfAttnArgs a) {
 		for (int n = 0; n < HD / 8; ++n) o[n][0] *= corr[0], o[n][1] *= corr[0], o[n][2] *= corr[1], o[n][3] *= corr[1];
 #pragma unroll
 		for (int kk = 0; kk < PFA_TILE / 16; ++kk) { // 16 keys: their weights, then their values
+			const int kb = k0 + kk * 16;
+			if (kb > wlast) continue; // (warp-uniform) seen by no row of the warp
 			uint32_t ph[4], pl[4];
 #pragma unroll
 			for (int j = 0; j < 2; ++j)
@@ -721,6 +723,36 @@ __global__ void __launch_bounds__(256, 1) k_pf_attn(const PfAttnArgs a) {
 					l[r] += px + py;
 					split_hl2(px, py, ph[2 * j + r], pl[2 * j + r]);
 				}
+			if (sizeof(KVT) == 2 && kb + 15 > a.pos0 + t0) { // some rows do not see some of the keys: a weight of zero must not meet an infinity (e5m2 entries are finite)
+				bool finite = true;
+#pragma unroll
+				for (int n = 0; n < HD / 8; n += 2) {
+					uint32_t b[4];
+					ldsm_x4_t(at(buf, 1, kk * 16 + (lane & 15), n + (lane >> 4)), b);
+#pragma unroll
+					for (int i = 0; i < 4; ++i) finite &= __vcmpeq2(b[i] & 0x7c007c00u, 0x7c007c00u) == 0;
+				}
+				if (!__all_sync(0xffffffffu, finite)) { // key by key, for the rows that see it
+#pragma unroll 1
+					for (int i = 0; i < 16; ++i) {
+						float p[2];
+						const int key = kb + i, half = i >> 3, src = (lane & ~3) | ((i & 7) >> 1); // the lane of the quad that has the key's weights
+#pragma unroll
+						for (int r = 0; r < 2; ++r) {
+							const uint32_t hw = __shfl_sync(0xffffffffu, half ? ph[2 + r] : ph[r], src), lw = __shfl_sync(0xffffffffu, half ? pl[2 + r] : pl[r], src);
+							const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hw)), l2 = __half22float2(*reinterpret_cast<const __half2*>(&lw));
+							p[r] = i & 1 ? h.y + l2.y : h.x + l2.x;
+						}
+#pragma unroll
+						for (int n = 0; n < HD / 8; ++n) {
+							const float2 v = __half22float2(*reinterpret_cast<const __half2*>(at(buf, 1, kk * 16 + i, n) + 2 * t4));
+							if (key <= p0) o[n][0] = fmaf(p[0], v.x, o[n][0]), o[n][1] = fmaf(p[0], v.y, o[n][1]);
+							if (key <= p0 + 8) o[n][2] = fmaf(p[1], v.x, o[n][2]), o[n][3] = fmaf(p[1], v.y, o[n][3]);
+						}
+					}
+					continue;
+				}
+			}
 #pragma unroll
 			for (int n = 0; n < HD / 8; n += 2) {
 				uint32_t b[4]; // (keys 0-7, dims n), (keys 8-15, dims n), (keys 0-7, dims n + 1), (keys 8-15, dims n + 1)

@@ -37,10 +37,10 @@ def _model(hd, value, gain, delta):
     return spec, t
 
 
-def _both(spec, tensors, toks, kvbits):
+def _both(spec, tensors, toks):
     out = []
     for batched in (False, True):
-        with lib.DeviceModel(spec, tensors, seq_len=1200, kvbits=kvbits) as dm:
+        with lib.DeviceModel(spec, tensors, seq_len=1200) as dm:
             if batched:
                 assert dm.prefill(toks, 0) == 1
             else:
@@ -56,7 +56,20 @@ def test_long_tail_of_small_weights(hd, bits):
     """A first key without a value, and a thousand keys of 2^-bits of its weight that hold all there is."""
     value = 2.0 ** min(15, bits - 8)  # large enough that what is left of it is an ordinary activation
     spec, t = _model(hd, {1: 0.0, 2: value}, 2.0 ** (bits - 9) / value, bits * math.log(2.0))
-    serial, batched = _both(spec, t, [1] + [2] * 1030, 16)
+    serial, batched = _both(spec, t, [1] + [2] * 1030)
     assert np.abs(serial[40:]).min() > 1e-3
     # a weight keeps 22 bits or, where that is coarser, steps of 2^-39 of the largest (half a step: 2^-40); two roundings to fp16
     np.testing.assert_allclose(batched[40:], serial[40:], rtol=2.0 ** -10 + 2.0 ** -22 + 2.0 ** (bits - 40))
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("at", [5, 15, 16, 70, 97])  # inside a 16-key block, at its ends, in later tiles
+def test_an_infinite_value_reaches_no_earlier_token(hd, at):
+    spec, t = _model(hd, {1: 3.0, 2: 1.0}, 0.5, 1.0)
+    t["model.layers.0.attn.wv.weight"][:, 3] = 60000.0  # token 3: beyond what an fp16 cache holds (an e5m2 one saturates)
+    toks = [1] + [2] * 99
+    toks[at] = 3
+    serial, batched = _both(spec, t, toks)
+    assert np.isfinite(serial[:at]).all() and np.abs(serial[:at]).min() > 1e-3 and not np.isfinite(serial[at:]).any()
+    np.testing.assert_allclose(batched[:at], serial[:at], rtol=2.0 ** -10)  # two roundings to fp16
+    assert not np.isfinite(batched[at:]).any()
