@@ -592,12 +592,6 @@ __host__ __device__ constexpr size_t pfa_smem_bytes() { // two buffers of K and 
 	return (size_t)2 * 2 * PFA_TILE * HD * sizeof(__half);
 }
 
-__device__ __forceinline__ void ldsm_x4(const void* p, uint32_t (&r)[4]) {
-	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
-}
-__device__ __forceinline__ void ldsm_x4_t(const void* p, uint32_t (&r)[4]) {
-	asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
-}
 __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
 	asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
 	             : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])

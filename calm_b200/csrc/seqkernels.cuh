@@ -9,6 +9,7 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "tc05.cuh"
 
 typedef __nv_bfloat16 bf16;
 
@@ -948,7 +949,7 @@ __global__ void __launch_bounds__(256) k_seq_attn_softmax(AttSoftmax a) {
 
 // ---------------------------------------------------------------- prompt attention in one kernel
 // Flash attention for sequences that bring many tokens to a step: attentions over cached keys and values of the same width HD, scores in bf16
-// products (not scores_f32, no distance bias, one map).  A CTA serves km of the query heads that share a key head and tb blocks of
+// products (not scores_f32, no distance bias, one map), at most with a window, a sink and a gate per channel.  A CTA serves km of the query heads that share a key head and tb blocks of
 // 16 tokens, a warp one of each; a tile of 64 cached rows (fp32, through the page table) is copied to shared memory while the
 // previous one is multiplied, rounded to bf16 once for all its warps, and read as mma.m16n8k16 fragments.  Scores, the running maximum,
 // exponentials and the denominator are fp32; queries, keys and values are bf16 with fp32 accumulation, as in the products that this replaces,
@@ -960,12 +961,6 @@ __global__ void __launch_bounds__(256) k_seq_attn_softmax(AttSoftmax a) {
 template <int HD>
 __host__ __device__ constexpr size_t afl_smem() { // the rows as cached (K, V), then as bf16 (K, V)
 	return (size_t)2 * AFL_TILE * HD * (sizeof(float) + sizeof(bf16));
-}
-__device__ __forceinline__ void afl_ldsm(const void* p, uint32_t (&r)[4]) {
-	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
-}
-__device__ __forceinline__ void afl_ldsm_t(const void* p, uint32_t (&r)[4]) {
-	asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
 }
 __device__ __forceinline__ uint32_t afl_pack(float x, float y) {
 	const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
@@ -986,12 +981,9 @@ __global__ void __launch_bounds__(256, 1) k_seq_attn_flash(const AttArgs a, cons
 	const int kvh = blockIdx.y / per, head = kvh * a.group + (blockIdx.y % per) * km + warp % km;
 	const int t0 = c0 + (warp / km) * 16; // first token of the warp
 	const float* const kbase = a.kc + kvh * HD;
-	const float* const vbase = a.vc + kvh / a.vshare * HD;
+	const float* const vbase = a.vc + kvh * HD;
 	const int keep = a.window > 0 ? a.keep_first : 0;
-	auto low = [&](int p) { // first position that a query at p sees (but for the kept ones)
-		int l = a.window > 0 ? max(0, p - a.window + 1) : 0;
-		return a.chunk > 0 ? max(l, p / a.chunk * a.chunk) : l;
-	};
+	auto low = [&](int p) { return a.window > 0 ? max(0, p - a.window + 1) : 0; }; // first position that a query at p sees (but for the kept ones)
 	const int pa = pos0 + c0, pb = pos0 + min(cnt, c0 + 16 * tb) - 1;       // the CTA's positions
 	const int wa = pos0 + t0, wb = pos0 + min(cnt, t0 + 16) - 1;            // the warp's (wb < wa: none)
 	const int from = low(pa) & ~(AFL_TILE - 1);                             // tiles from here on, and before them those of the kept positions
@@ -1024,9 +1016,9 @@ __global__ void __launch_bounds__(256, 1) k_seq_attn_flash(const AttArgs a, cons
 	float o[HD / 8][4], m[2], l[2];
 #pragma unroll
 	for (int n = 0; n < HD / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
-	m[0] = m[1] = a.add_one ? 0.f : a.sink ? ldf(a.sink + head) : -FLT_MAX;
+	m[0] = m[1] = a.sink ? ldf(a.sink + head) : -FLT_MAX;
 	if (m[0] == -INFINITY) m[0] = m[1] = -FLT_MAX; // a sink of no weight
-	l[0] = l[1] = (a.add_one || a.sink) && t4 == 0 ? 1.f : 0.f; // a lane's share of the denominator
+	l[0] = l[1] = a.sink && t4 == 0 ? 1.f : 0.f; // a lane's share of the denominator
 	const int wlow = low(wa);
 	while (k0 <= pb) {
 		asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -1050,7 +1042,7 @@ __global__ void __launch_bounds__(256, 1) k_seq_attn_flash(const AttArgs a, cons
 #pragma unroll
 			for (int k = 0; k < KS; k += 2) {
 				uint32_t bb[4];
-				afl_ldsm(at(0, n * 8 + (lane & 7), 2 * k + (lane >> 3)), bb);
+				ldsm_x4(at(0, n * 8 + (lane & 7), 2 * k + (lane >> 3)), bb);
 				const uint32_t b0[2] = {bb[0], bb[1]}, b1[2] = {bb[2], bb[3]};
 				mma_bf16_16816(s[n], q[k], b0), mma_bf16_16816(s[n], q[k + 1], b1);
 			}
@@ -1065,7 +1057,7 @@ __global__ void __launch_bounds__(256, 1) k_seq_attn_flash(const AttArgs a, cons
 				for (int e = 0; e < 2; ++e) {
 					const int key = kt + n * 8 + 2 * t4 + e;
 					float& x = s[n][2 * r + e];
-					x = key <= p && (key >= lo || key < keep) ? att_cap(x * a.scale, a.softcap) : -INFINITY;
+					x = key <= p && (key >= lo || key < keep) ? x * a.scale : -INFINITY;
 					mx[r] = fmaxf(mx[r], x);
 				}
 		}
@@ -1095,7 +1087,7 @@ __global__ void __launch_bounds__(256, 1) k_seq_attn_flash(const AttArgs a, cons
 #pragma unroll
 			for (int n = 0; n < HD / 8; n += 2) {
 				uint32_t bb[4];
-				afl_ldsm_t(at(1, kk * 16 + (lane & 15), n + (lane >> 4)), bb);
+				ldsm_x4_t(at(1, kk * 16 + (lane & 15), n + (lane >> 4)), bb);
 				const uint32_t b0[2] = {bb[0], bb[1]}, b1[2] = {bb[2], bb[3]};
 				mma_bf16_16816(o[n], p, b0), mma_bf16_16816(o[n + 1], p, b1);
 				mma_bf16_16816(o[n], pl, b0), mma_bf16_16816(o[n + 1], pl, b1);
@@ -1108,12 +1100,12 @@ __global__ void __launch_bounds__(256, 1) k_seq_attn_flash(const AttArgs a, cons
 		const int t = t0 + g + 8 * r;
 		if (t >= cnt) continue;
 		const float* gp = a.gate ? a.gate + (size_t)(first + t) * a.ldg + (size_t)head * a.ghs : nullptr;
-		const float inv = (gp && a.ges == 0 ? sigmoidf_(gp[0]) : 1.f) / l[r];
+		const float inv = 1.f / l[r];
 		bf16* dst = out + ((size_t)(first + t) * a.heads + head) * HD + 2 * t4;
 #pragma unroll
 		for (int n = 0; n < HD / 8; ++n) {
 			float x = o[n][2 * r] * inv, y = o[n][2 * r + 1] * inv;
-			if (gp && a.ges != 0) x *= sigmoidf_(gp[(size_t)(8 * n + 2 * t4) * a.ges]), y *= sigmoidf_(gp[(size_t)(8 * n + 2 * t4 + 1) * a.ges]);
+			if (gp) x *= sigmoidf_(gp[(size_t)(8 * n + 2 * t4) * a.ges]), y *= sigmoidf_(gp[(size_t)(8 * n + 2 * t4 + 1) * a.ges]);
 			*reinterpret_cast<uint32_t*>(dst + 8 * n) = afl_pack(x, y);
 		}
 	}

@@ -660,9 +660,11 @@ void attention_products(Seq& s, int kind, const AttArgs& a, bf16* out, float* fu
 	}
 }
 
-// attentions that k_seq_attn_flash computes: keys and values of one instantiated width in rows of their own, plain scores in bf16 products
+// attentions that k_seq_attn_flash computes: keys and values of one instantiated width in rows of their own, plain scores in bf16 products, at most a
+// window, a sink and a gate per channel (the other options of a layer come with scores_f32 or a distance bias in every family)
 bool flash_fits(const AttArgs& a) {
-	return (a.kd == 64 || a.kd == 128) && a.vd == a.kd && a.kc != a.vc && a.kld % 4 == 0 && a.vld % 4 == 0 && !a.split && !a.slopes && !a.qr;
+	return (a.kd == 64 || a.kd == 128) && a.vd == a.kd && a.kc != a.vc && a.kld % 4 == 0 && a.vld % 4 == 0 && !a.split && !a.slopes && !a.qr && a.chunk <= 0 && a.softcap == 0.f &&
+	       !a.add_one && a.vshare == 1 && (!a.gate || a.ges != 0);
 }
 // all sequences with at least kAttnGemmMin new tokens in one launch; queries wait in a3
 void attention_flash(Seq& s, int kind, const AttArgs& a, bf16* out, const SeqBatch& sb) {

@@ -75,3 +75,10 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(const void* tile) {
 	const uint64_t addr = (uint64_t)(smem_u32(tile) & 0x3FFFF) >> 4;
 	return addr | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
+// warp-level tensor cores: four 8 x 8 tiles of 16-bit elements from shared memory, as they lie and transposed (lane l names row l % 8 of tile l / 8)
+__device__ __forceinline__ void ldsm_x4(const void* p, uint32_t (&r)[4]) {
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
+}
+__device__ __forceinline__ void ldsm_x4_t(const void* p, uint32_t (&r)[4]) {
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
+}
