@@ -391,6 +391,7 @@ struct AttArgs {
 	float softcap = 0.f; // > 0: score = softcap tanh(score / softcap), after the scale
 	int vshare = 1;      // neighbouring key heads that read one value head
 	int parts = 0;       // 1: results go to `part` whatever nsplit is (k_seq_attn_diff_merge finishes)
+	int merge_skipped = 0; // 1: k_seq_attention_merge takes the tokens that `skip` names, not the others
 };
 __device__ __forceinline__ float att_cap(float s, float cap) { return cap > 0.f ? cap * tanhf(s / cap) : s; }
 // channel c of the query of (token, head)
@@ -569,7 +570,7 @@ __global__ void __launch_bounds__(128) k_seq_attention_merge(AttArgs a, AT* out)
 	pdl_enter(); // programmatic dependent launch: let the next kernel's launch overlap this one, then wait for the previous one
 	__shared__ float wz[ATT_MAXSPLIT], red[2][4];
 	const int n = blockIdx.x, h = blockIdx.y, pw = a.vd + 2, z = threadIdx.x, d = blockIdx.z * 128 + threadIdx.x;
-	if (a.skip && a.skip[n]) return;
+	if (a.skip && (a.skip[n] != 0) != (a.merge_skipped != 0)) return;
 	const float* p = a.part + ((size_t)n * a.heads + h) * a.nsplit * pw;
 	const float m = z < a.nsplit ? p[z * pw + a.vd] : -INFINITY, lz = z < a.nsplit ? p[z * pw + a.vd + 1] : 0.f;
 	float mx = warp_max(m);
@@ -949,12 +950,14 @@ __global__ void __launch_bounds__(256) k_seq_attn_softmax(AttSoftmax a) {
 
 // ---------------------------------------------------------------- prompt attention in one kernel
 // Flash attention for sequences that bring many tokens to a step: attentions over cached keys and values of the same width HD, scores in bf16
-// products (not scores_f32, no distance bias, one map), at most with a window, a sink and a gate per channel.  A CTA serves km of the query heads that share a key head and tb blocks of
-// 16 tokens, a warp one of each; a tile of 64 cached rows (fp32, through the page table) is copied to shared memory while the
-// previous one is multiplied, rounded to bf16 once for all its warps, and read as mma.m16n8k16 fragments.  Scores, the running maximum,
-// exponentials and the denominator are fp32; queries, keys and values are bf16 with fp32 accumulation, as in the products that this replaces,
-// and the weights a bf16 value and its remainder (one bf16 there).  Those were: gather, score product, softmax and value product per sequence, key head and block of queries, with scores
-// and weights going through memory.
+// products (not scores_f32, no distance bias, one map), at most with a window, a sink and a gate per channel.  A CTA serves km of
+// the query heads that share a key head and tb blocks of 16 tokens, a warp one of each, over one of nsplit shares of the keys
+// (flash_shares; partial results then, which k_seq_attention_merge folds in share order); a tile of 64 cached rows (fp32, through the page
+// table) is copied to shared memory while the previous one is multiplied, rounded to bf16 once for all its warps, and read as
+// mma.m16n8k16 fragments.  Scores, the running maximum, exponentials and the denominator are fp32; queries, keys and values are bf16
+// with fp32 accumulation, as in the products that this replaces, and the weights a bf16 value and its remainder (one bf16 there).  Those
+// were: gather, score product, softmax and value product per sequence, key head and block of queries, with scores and weights going
+// through memory.
 // Bound: the MMAs and, with few query heads per key head, the fp32 rows (64 KB a tile from L2).  A 2048-token
 // step: 638 us in 16 launches before, 308 here; three sequences of 700 tokens: 700 us in 48 launches, 146 here.
 #define AFL_TILE 64
@@ -978,7 +981,8 @@ __global__ void __launch_bounds__(256, 1) k_seq_attn_flash(const AttArgs a, cons
 	if (cnt < min_count || c0 >= cnt) return;
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
 	const int first = sb.sstart[b], pos0 = sb.spos0[b], slot = sb.sslot[b], per = a.group / km;
-	const int kvh = blockIdx.y / per, head = kvh * a.group + (blockIdx.y % per) * km + warp % km;
+	const int hg = blockIdx.y / a.nsplit, share = blockIdx.y % a.nsplit;
+	const int kvh = hg / per, head = kvh * a.group + (hg % per) * km + warp % km;
 	const int t0 = c0 + (warp / km) * 16; // first token of the warp
 	const float* const kbase = a.kc + kvh * HD;
 	const float* const vbase = a.vc + kvh * HD;
@@ -986,11 +990,10 @@ __global__ void __launch_bounds__(256, 1) k_seq_attn_flash(const AttArgs a, cons
 	auto low = [&](int p) { return a.window > 0 ? max(0, p - a.window + 1) : 0; }; // first position that a query at p sees (but for the kept ones)
 	const int pa = pos0 + c0, pb = pos0 + min(cnt, c0 + 16 * tb) - 1;       // the CTA's positions
 	const int wa = pos0 + t0, wb = pos0 + min(cnt, t0 + 16) - 1;            // the warp's (wb < wa: none)
-	const int from = low(pa) & ~(AFL_TILE - 1);                             // tiles from here on, and before them those of the kept positions
-	auto next = [&](int k) { // the tile after k
-		k += AFL_TILE;
-		return k < from && k >= keep ? from : k;
-	};
+	// the CTA's tiles: those of the kept positions, then all from the first query's window on; this share of them
+	const int from = low(pa) & ~(AFL_TILE - 1), kept = min((keep + AFL_TILE - 1) / AFL_TILE, from / AFL_TILE);
+	const int tiles = kept + (pb - from) / AFL_TILE + 1, each = (tiles + a.nsplit - 1) / a.nsplit, end = min(tiles, (share + 1) * each);
+	auto key0 = [&](int i) { return i < kept ? i * AFL_TILE : from + (i - kept) * AFL_TILE; };
 	auto fetch = [&](int k0) {
 		for (int i = tid; i < 2 * AFL_TILE * C4; i += blockDim.x) {
 			const int which = i / (AFL_TILE * C4), r = i / C4 % AFL_TILE, c = i % C4, pos = k0 + r;
@@ -1001,9 +1004,8 @@ __global__ void __launch_bounds__(256, 1) k_seq_attn_flash(const AttArgs a, cons
 		asm volatile("cp.async.commit_group;" ::: "memory");
 	};
 	auto at = [&](int which, int r, int c) { return tile + ((size_t)which * AFL_TILE + r) * HD + ((c ^ (r & 7)) << 3); };
-	int k0 = keep > 0 ? 0 : from;
-	if (k0 < from && k0 >= keep) k0 = from;
-	fetch(k0);
+	int ti = share * each;
+	if (ti < end) fetch(key0(ti));
 
 	uint32_t q[KS][4];
 #pragma unroll
@@ -1016,24 +1018,24 @@ __global__ void __launch_bounds__(256, 1) k_seq_attn_flash(const AttArgs a, cons
 	float o[HD / 8][4], m[2], l[2];
 #pragma unroll
 	for (int n = 0; n < HD / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
-	m[0] = m[1] = a.sink ? ldf(a.sink + head) : -FLT_MAX;
+	const bool sink = a.sink && share == 0; // counts once
+	m[0] = m[1] = sink ? ldf(a.sink + head) : -FLT_MAX;
 	if (m[0] == -INFINITY) m[0] = m[1] = -FLT_MAX; // a sink of no weight
-	l[0] = l[1] = a.sink && t4 == 0 ? 1.f : 0.f; // a lane's share of the denominator
+	l[0] = l[1] = sink && t4 == 0 ? 1.f : 0.f; // a lane's share of the denominator
 	const int wlow = low(wa);
-	while (k0 <= pb) {
+	for (; ti < end; ++ti) {
+		const int kt = key0(ti);
 		asm volatile("cp.async.wait_group 0;" ::: "memory");
 		__syncthreads(); // the tile has arrived, and the bf16 one is no longer being read
 		for (int i = tid; i < 2 * AFL_TILE * (HD / 8); i += blockDim.x) {
 			const int which = i / (AFL_TILE * (HD / 8)), r = i / (HD / 8) % AFL_TILE, c = i % (HD / 8);
 			const float4* s = reinterpret_cast<const float4*>(raw + ((size_t)which * AFL_TILE + r) * HD + 8 * c);
-			const bool in = k0 + r <= pb; // rows past the last position are zero: a weight of zero must not meet a NaN
+			const bool in = kt + r <= pb; // rows past the last position are zero: a weight of zero must not meet a NaN
 			const float4 z = make_float4(0.f, 0.f, 0.f, 0.f), x = in ? s[0] : z, y = in ? s[1] : z;
 			*reinterpret_cast<uint4*>(at(which, r, c)) = make_uint4(afl_pack(x.x, x.y), afl_pack(x.z, x.w), afl_pack(y.x, y.y), afl_pack(y.z, y.w));
 		}
 		__syncthreads();
-		const int kt = k0;
-		k0 = next(k0);
-		if (k0 <= pb) fetch(k0);
+		if (ti + 1 < end) fetch(key0(ti + 1));
 		if (kt > wb || (kt + AFL_TILE <= wlow && kt >= keep)) continue; // (warp-uniform) nothing of this tile is visible to this warp's rows
 		float s[NT][4];
 #pragma unroll
@@ -1099,6 +1101,13 @@ __global__ void __launch_bounds__(256, 1) k_seq_attn_flash(const AttArgs a, cons
 		l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1), l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
 		const int t = t0 + g + 8 * r;
 		if (t >= cnt) continue;
+		if (a.nsplit > 1) {
+			float* p = a.part + (((size_t)(first + t) * a.heads + head) * a.nsplit + share) * (HD + 2);
+#pragma unroll
+			for (int n = 0; n < HD / 8; ++n) *reinterpret_cast<float2*>(p + 8 * n + 2 * t4) = make_float2(o[n][2 * r], o[n][2 * r + 1]);
+			if (t4 == 0) *reinterpret_cast<float2*>(p + HD) = make_float2(l[r] > 0.f ? m[r] : -INFINITY, l[r]); // (no key of the share visible: counts nothing)
+			continue;
+		}
 		const float* gp = a.gate ? a.gate + (size_t)(first + t) * a.ldg + (size_t)head * a.ghs : nullptr;
 		const float inv = 1.f / l[r];
 		bf16* dst = out + ((size_t)(first + t) * a.heads + head) * HD + 2 * t4;

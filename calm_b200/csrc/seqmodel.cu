@@ -666,9 +666,24 @@ bool flash_fits(const AttArgs& a) {
 	return (a.kd == 64 || a.kd == 128) && a.vd == a.kd && a.kc != a.vc && a.kld % 4 == 0 && a.vld % 4 == 0 && !a.split && !a.slopes && !a.qr && a.chunk <= 0 && a.softcap == 0.f &&
 	       !a.add_one && a.vshare == 1 && (!a.gate || a.ges != 0);
 }
-// all sequences with at least kAttnGemmMin new tokens in one launch; queries wait in a3
-void attention_flash(Seq& s, int kind, const AttArgs& a, bf16* out, const SeqBatch& sb) {
-	int km = 8, longest = 0;
+// Shares of the keys for `ctas` CTAs with up to `tiles` tiles of keys each, `rows` floats of partial results a share: the number with the least estimated
+// time, in tiles.  A CTA costs its tiles and about one more, and CTAs run in waves of one per SM; folding costs a launch, about one tile, and a
+// share's results their way through memory (a tile takes 9.4 us at width 128, 5.8 at 64).  Two tiles a share at least, and a gain of a tenth.
+// 16 new tokens behind 4000 positions, 16 / 4 heads of 128: 529 us a layer without shares, 65 with (gather + products + softmax, which this kernel
+// replaced: 149 and more); 300 with 32 / 2 heads, 76 CTAs on 148 SMs: 714, 450 (572); 64 behind 8000, 16 / 2 heads of 64: 758, 100 (301).
+int flash_shares(int ctas, int tiles, size_t rows, int sms) {
+	const int most = std::min({tiles / 2, ATT_MAXSPLIT, (int)(((size_t)16 << 20) / rows)});
+	int best = 1;
+	double least = 0.9 * cdiv(ctas, sms) * (tiles + 1);
+	for (int n = 2; n <= most; ++n) {
+		const double cost = cdiv(ctas * n, sms) * (cdiv(tiles, n) + 1) + 1 + rows * n / 7e6;
+		if (cost < least) least = cost, best = n;
+	}
+	return best;
+}
+// all sequences with at least kAttnGemmMin new tokens in one launch, and the fold of the shares in a second; queries wait in a3
+void attention_flash(Seq& s, int kind, AttArgs a, bf16* out, const SeqBatch& sb) {
+	int km = 8, longest = 0, ctas = 0, tiles = 0;
 	while (a.group % km) --km; // the largest divisor of the group up to 8 heads
 	const int tb = 8 / km;
 	double pairs = 0;
@@ -677,12 +692,20 @@ void attention_flash(Seq& s, int kind, const AttArgs& a, bf16* out, const SeqBat
 			longest = std::max(longest, s.hb_count[b]);
 			const double span = a.window > 0 ? a.window + a.keep_first : 1e18;
 			pairs += s.hb_count[b] * std::min(s.hb_pos0[b] + s.hb_count[b] * 0.5, span);
+			ctas += cdiv(s.hb_count[b], 16 * tb) * (a.heads / km);
+			tiles = std::max(tiles, cdiv((int)std::min<double>(s.hb_pos0[b] + s.hb_count[b], span + 16 * tb), AFL_TILE));
 		}
-	const dim3 grid(cdiv(longest, 16 * tb), a.heads / km, sb.B);
+	const size_t rows = (size_t)sb.N * a.heads * (a.vd + 2); // (decoded tokens of the step have room in `part` too)
+	a.nsplit = flash_shares(ctas, tiles, rows, s.sms);
+	if (a.nsplit > 1) ensure_part(s, rows * a.nsplit), a.part = s.part;
+	const dim3 grid(cdiv(longest, 16 * tb), a.heads / km * a.nsplit, sb.B);
 	run_kernel(s, kind, (double)s.tok_on_products * (a.heads * a.kd * 4.0 + (a.heads / a.group) * a.kd * 8.0), 4.0 * pairs * a.heads * a.kd, [&] {
 		if (a.kd == 128) launch_k(s, k_seq_attn_flash<128>, grid, 32 * km * tb, afl_smem<128>(), a, (const bf16*)s.a3, out, sb, km, tb, kAttnGemmMin);
 		else launch_k(s, k_seq_attn_flash<64>, grid, 32 * km * tb, afl_smem<64>(), a, (const bf16*)s.a3, out, sb, km, tb, kAttnGemmMin);
 	});
+	if (a.nsplit == 1) return;
+	a.skip = s.d_skip, a.merge_skipped = 1;
+	run_kernel(s, kind, 0, 0, [&] { launch_k(s, k_seq_attention_merge<bf16>, dim3(sb.N, a.heads, cdiv(a.vd, 128)), 128, 0, a, out); });
 }
 
 // q_ready: the queries already wait in a3, in the form the product path reads.  diff: a.heads are the maps of diff->heads heads, which a last kernel
