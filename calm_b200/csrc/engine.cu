@@ -1351,20 +1351,27 @@ static bool pf_supported() {
 }
 
 // Row tiles and tokens per item and K-slices of a product of `rows` weight rows over n tokens: the choice with the least estimated time, in cycles.
-// A k-stage was measured at 1040 / 1290 / 2070 cycles for one row tile and 64 / 128 / 256 tokens, at 2010 for two and 128 (fp8, 4096 x 4096 x 2048
-// tokens: 251 / 178 / 143 / 139 us), so wide items win while every SM has one, two row tiles (half the activation bytes) first; K
-// is sliced only while an item per SM is left over, and a slice pays for its way through memory.
-static void pf_tiles(int mode, int rows, int n, int nkb, PfGemmArgs& a) {
+// Kernel time over k-stages, 4096 x 4096 x 2047 tokens, in cycles at 1.9 GHz, for 64 / 128 / 256 tokens of one row tile and 64 / 128 of two: fp8
+// 1150 / 1250 / 1920 and 1720 / 2050 (271 / 169 / 129 and 232 / 138 us), fp16 910 / 1150 / 2150 and 1260 / 1810 (214 / 155 / 145 and 170 / 122 us);
+// the estimate has 970 / 1290 / 1930 and 1290 / 1930 for all formats.  So wide items win while every SM has one, two row tiles (half the
+// activation bytes) first; K is sliced only while an item per SM is left over, and a slice pays for its way through memory.
+// Where it misses: two row tiles and 64 tokens of weights that are widened cost a third more than estimated, and two K-slices more than the
+// fold's share (FFN up 14336 x 4096, 130 tokens, fp8: 171 us, 128 with 128 tokens a tile; q/k/v 6144 x 4096, 333 tokens, gf4: 94 us, 69 unsliced);
+// over 48 products of four models the choice is within a tenth of the best in 40.
+static void pf_tiles(int mode, int rows, int n, int nkb, int sms, int& na_out, int& bn_out, int& splits_out) {
 	long best = -1;
 	for (int na = 2; na >= (mode == PF_UP ? 2 : 1); --na)
 		for (int bn = 64; bn * na <= 256; bn *= 2) {
 			const int tiles = (mode == PF_UP ? rows / PF_BM : cdiv(rows / PF_BM, na)) * cdiv(n, bn);
 			const int stage = 650 + na * bn * 5;
-			for (int sp = 1; sp == 1 || (tiles * sp <= g.sms && sp * 2 <= nkb && sp <= 16); ++sp) {
-				const long cost = (long)cdiv(tiles * sp, g.sms) * cdiv(nkb, sp) * stage + na * bn * 20 + (sp > 1 ? 5000 + na * bn * (20 + 15 * sp) : 0);
-				if (best < 0 || cost < best) best = cost, a.na = na, a.bn = bn, a.splits = sp;
+			for (int sp = 1; sp == 1 || (tiles * sp <= sms && sp * 2 <= nkb && sp <= 16); ++sp) {
+				const long cost = (long)cdiv(tiles * sp, sms) * cdiv(nkb, sp) * stage + na * bn * 20 + (sp > 1 ? 5000 + na * bn * (20 + 15 * sp) : 0);
+				if (best < 0 || cost < best) best = cost, na_out = na, bn_out = bn, splits_out = sp;
 			}
 		}
+}
+extern "C" void calm_b200_prefill_tiles(int product, int rows, int n, int k, int sms, int* out3) {
+	pf_tiles(product == 0 ? PF_QKV : product == 1 ? PF_RES : PF_UP, rows, n, k / PF_BK, sms, out3[0], out3[1], out3[2]);
 }
 
 template <int MODE, int DBITS>
@@ -1373,7 +1380,7 @@ static void pf_gemm(const CUtensorMap (&tx)[3][2], const CUtensorMap* tw, PfGemm
 	static bool opted = false;
 	if (!opted) smem_optin(k_pf_gemm<MODE, DBITS>, limit), opted = true;
 	same_carveout((const void*)k_pf_gemm<MODE, DBITS>);
-	pf_tiles(MODE, rows, n, a.K / PF_BK, a);
+	pf_tiles(MODE, rows, n, a.K / PF_BK, g.sms, a.na, a.bn, a.splits);
 	PfMaps m;
 	memcpy(m.x, tx[a.bn / 128], sizeof(m.x)); // 64, 128, 256 -> 0, 1, 2
 	memcpy(m.w, tw, (MODE == PF_QKV ? 3 : MODE == PF_UP ? 2 : 1) * sizeof(CUtensorMap));

@@ -103,6 +103,9 @@ int calm_b200_tp_mode(void);
  * tokens were fed one by one instead -- same result either way.  A host integrates it by replacing the prompt loop:
  * forward_prefill_cuda(t, prompt, n - 1, 0); logits = forward_cuda(t, prompt[n - 1], n - 1, 0);  (INTEGRATION.md). */
 int forward_prefill_cuda(struct Transformer* transformer, const int* tokens, int n, int pos0);
+/* How a product of the pass over n tokens is cut on a GPU of `sms` SMs (no GPU needed; for tests and measurements): product 0 q/k/v, 1 wo and w2, 2 FFN
+ * up (rows of one of its matrices); out3 = row tiles of 128 per item, tokens per item, slices of k. */
+void calm_b200_prefill_tiles(int product, int rows, int n, int k, int sms, int* out3);
 
 /* forward + device-side greedy sample.  Returns argmax(logits) with the
  * reference's tie rule (lowest index, sampler.c:34-42).  The logits are still

@@ -1,0 +1,72 @@
+"""How the products of a prompt are cut (calm_b200_prefill_tiles) and that every cut it makes computes the same: each combination of row tiles and tokens per item
+and sliced or whole k that the rule picks anywhere in the range is run by one of the shapes here or in test_prefill_tiles_gpu.py."""
+import ctypes as C
+import os
+import sys
+from dataclasses import replace
+
+import pytest
+import torch
+
+sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
+from test_prefill_gpu import _both, _check  # noqa: E402
+
+from calm_b200 import build as cbuild  # noqa: E402
+from calm_b200 import lib  # noqa: E402
+from calm_b200 import modelgen as mg  # noqa: E402
+
+SMS = 148
+# dim, heads, kv heads, head_dim, hidden, tokens, and the cuts that only this shape reaches
+SHAPES = [(896, 14, 2, 64, 4864, 449, {("res", 1, 128, True)}), (896, 14, 2, 64, 4864, 1537, {("qkv", 2, 64, False), ("res", 1, 256, True), ("res", 2, 64, False)}),
+          (768, 6, 2, 128, 2688, 1550, {("res", 2, 128, True)}), (384, 3, 3, 128, 384, 1900, {("qkv", 1, 128, False)}), (896, 7, 7, 128, 896, 1717, {("qkv", 1, 256, False)}),
+          (1536, 12, 12, 128, 1536, 1595, {("qkv", 2, 128, False), ("res", 2, 128, False)}), (3072, 24, 8, 128, 6144, 67, {("up", 2, 128, True)}),
+          (4096, 32, 32, 128, 1024, 70, {("qkv", 2, 128, True), ("up", 2, 64, True)})]
+ELSEWHERE = [(384, 384, 128, 1152, 1), (896, 896, 128, 2432, 61), (1024, 1024, 256, 3456, 65), (2048, 2048, 512, 5504, 257), (4096, 4096, 1024, 14336, 130)]
+
+
+@pytest.fixture(scope="module")
+def cuts():
+    cbuild.build()
+    L, out = lib.load(), (C.c_int * 3)()
+
+    def of(dim, q_dim, kv_dim, hidden, n):
+        got = set()
+        for name, product, rows, k in (("qkv", 0, q_dim + 2 * kv_dim, dim), ("res", 1, dim, q_dim), ("up", 2, hidden, dim), ("res", 1, dim, hidden)):
+            L.calm_b200_prefill_tiles(product, rows, n, k, SMS, out)
+            na, bn, sp = out
+            items = (rows // 128 if name == "up" else -(-rows // 128 // na)) * -(-n // bn)
+            # the accumulators fit half of TMEM; a slice is not empty; partial sums and counters of sliced products have one place per SM
+            assert na in (1, 2) and bn in (64, 128, 256) and na * bn <= 256 and (name != "up" or na == 2) and 1 <= sp <= k // 64 and (sp == 1 or items * sp <= SMS)
+            got.add((name, na, bn, sp > 1))
+        return got
+
+    return of
+
+
+def test_every_cut_is_run_by_a_test(cuts):
+    run = set()
+    for s in ELSEWHERE:
+        run |= cuts(*s)
+    for dim, heads, kv, hd, hidden, n, only in SHAPES:
+        here = cuts(dim, heads * hd, kv * hd, hidden, n)
+        assert only <= here
+        run |= here
+    picked = set()
+    for dim in (384, 512, 768, 896, 1024, 1536, 2048, 3072, 4096, 5120, 8192):
+        for kv in {max(128, dim // f // 128 * 128) for f in (1, 2, 4, 8)}:
+            for hidden in {max(128, int(dim * f) // 128 * 128) for f in (1, 1.5, 2, 2.7, 3.5, 5.4)}:
+                for n in list(range(1, 130, 9)) + list(range(130, 2049, 61)):
+                    picked |= cuts(dim, dim, kv, hidden, n)
+    assert picked <= run, sorted(picked - run)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["fp8", "gf4", "fp16"])
+@pytest.mark.parametrize("dim,heads,kv,hd,hidden,n", [s[:6] for s in SHAPES])
+def test_cuts(dtype, dim, heads, kv, hd, hidden, n):
+    assert torch.cuda.get_device_properties(0).multi_processor_count == SMS
+    spec = replace(mg.SPECS["pf-tiny"], name="cuts", dtype=dtype, dim=dim, n_heads=heads, n_kv_heads=kv, head_dim=hd, hidden_dim=hidden, max_seq_len=2048)
+    tensors = mg.generate(spec, seed=6, device="cuda")
+    torch.cuda.synchronize()
+    serial, batched = _both(spec, tensors, mg.teacher_tokens(spec.vocab_size, n + 1), 0, 2048, 16)
+    _check(spec, serial, batched, 16, f"{dtype} dim {dim} hidden {hidden}, {n} tokens")

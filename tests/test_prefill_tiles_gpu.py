@@ -25,8 +25,9 @@ def test_attention_groups_and_edges(heads, kv, hd, n, pos0, kvbits):
     _check(spec, serial, batched, kvbits, f"heads {heads}/{kv}x{hd}, {n} at {pos0}, kv{kvbits}")
 
 
-# Products: one and two row tiles per item (an odd number of row tiles leaves a single one), 64 / 128 / 256 tokens per tile with ragged last tiles, K cut into
-# slices (small models) and not, many items per CTA, all three weight formats.  The cache after two layers sees every product.
+# Products: one and two row tiles per item (an odd number of row tiles leaves a single one), 64 tokens per tile and in FFN up 128, with ragged last tiles, K cut
+# into slices (small models) and not, many items per CTA, all three weight formats; the other cuts are in test_prefill_choice.py.  The cache after two layers sees
+# every product.
 @pytest.mark.parametrize("dtype", ["fp8", "gf4", "fp16"])
 @pytest.mark.parametrize("dim,heads,kv,hidden,n", [(384, 3, 1, 1152, 1), (896, 7, 1, 2432, 61), (1024, 8, 2, 3456, 65), (2048, 16, 4, 5504, 257), (4096, 32, 8, 14336, 130)])
 def test_product_tiles(dtype, dim, heads, kv, hidden, n):
