@@ -668,11 +668,12 @@ bool flash_fits(const AttArgs& a) {
 }
 // Shares of the keys for `ctas` CTAs with up to `tiles` tiles of keys each, `rows` floats of partial results a share: the number with the least estimated
 // time, in tiles.  A CTA costs its tiles and about one more, and CTAs run in waves of one per SM; folding costs a launch, about one tile, and a
-// share's results their way through memory (a tile takes 9.4 us at width 128, 5.8 at 64).  Two tiles a share at least, and a gain of a tenth.
+// share's results their way through memory (a tile takes 9.4 us at width 128, 5.8 at 64).  Two tiles a share at least, a gain of a tenth, and eight
+// tiles in all: with five, 300 tokens of 16 / 4 heads of 128 take 143 us a layer either way.
 // 16 new tokens behind 4000 positions, 16 / 4 heads of 128: 529 us a layer without shares, 65 with (gather + products + softmax, which this kernel
 // replaced: 149 and more); 300 with 32 / 2 heads, 76 CTAs on 148 SMs: 714, 450 (572); 64 behind 8000, 16 / 2 heads of 64: 758, 100 (301).
 int flash_shares(int ctas, int tiles, size_t rows, int sms) {
-	const int most = std::min({tiles / 2, ATT_MAXSPLIT, (int)(((size_t)16 << 20) / rows)});
+	const int most = tiles < 8 ? 1 : std::min({tiles / 2, ATT_MAXSPLIT, (int)(((size_t)16 << 20) / rows)});
 	int best = 1;
 	double least = 0.9 * cdiv(ctas, sms) * (tiles + 1);
 	for (int n = 2; n <= most; ++n) {
