@@ -15,8 +15,9 @@
 // ([position][head_dim] is contiguous per (layer, kv head)).  The slot written this step and the attention sinks that
 // k_embed re-rotates are read from global memory after the wait instead of from the early copy.
 //
-// Groups of 3, 5, 6 or 7 heads run as 4 or 8 with zero queries in the rest: with positions dealt out to many CTAs the spare arithmetic is hidden
-// by the fold (Qwen2-0.5B, 14 heads on 2, 131 positions: 16.7 us a layer in k_attn, 10.3 here).
+// Groups of 3, 5, 6 or 7 heads run as 4 or 8 with zero queries in the rest.  The spare arithmetic costs less than k_attn at every context: 100 /
+// 2049 / 4086 positions, k_attn against this kernel: 12.0 / 15.6 / 21.5 and 8.0 / 9.0 / 11.8 us for 24 / 8 heads of 128, 15.3 / 22.5 / 31.6
+// and 10.1 / 13.8 / 19.3 for 40 / 8, 16.6 / 17.1 / 20.3 and 8.9 / 11.3 / 12.3 for 14 / 2 of 64.
 //
 // Lane layout and arithmetic are k_attn's transposing score path: LPP = head_dim / 8 lanes own a position (8 dims per
 // lane), P = LPP / HG positions per lane group and step, so the HG * P partial dot products of a step transpose onto the
@@ -54,7 +55,7 @@ __host__ __device__ inline size_t attn2_smem_bytes(int hg, int head_dim, int nbm
 	return kv + ((size_t)hg * head_dim + scratch + (size_t)hg * (head_dim + 2)) * sizeof(float);
 }
 
-// How the slices of a unit are folded (measured on the in-kernel timeline, profiles/README.md round 2: with global partials,
+// How the slices of a unit are folded (measured on the in-kernel timeline: with global partials,
 // a grid-scope fence, an atomic counter and a last-CTA pass the fold cost the last CTA 5.5 us of a 15 us kernel):
 //   CLUSTER = false (default): every CTA publishes its record as 8-byte {value, epoch} cells -- no fence, no atomic: a reader
 //     that sees the epoch sees the value -- and then normalises 1/nsplit of the unit's outputs itself, polling the cells
@@ -194,7 +195,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) k_attn2(const AttnArgs a) {
 	for (int sb = (warp * G + grp) * P; sb - grp * P < nslots; sb += SC * STEP) { // warp-uniform trip count (full-warp shuffles inside)
 		float sc[SC];
 		bool val[SC], fast[SC];
-		const int live = min(SC, (nslots - (sb - grp * P) + STEP - 1) / STEP); // steps of the chunk that reach a slot (warp-uniform): contexts of 777 / 2049 positions have one / two of four (14.2 -> 9.1, 15.2 -> 10.4 us)
+		const int live = min(SC, (nslots - (sb - grp * P) + STEP - 1) / STEP); // steps of the chunk that reach a slot (warp-uniform): contexts of 777 / 2049 positions have one / two of four (13.6 -> 8.9, 14.5 -> 9.7 us)
 #pragma unroll
 		for (int c = 0; c < SC; ++c) {
 			sc[c] = -FLT_MAX, val[c] = false, fast[c] = false;

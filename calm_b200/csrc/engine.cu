@@ -60,7 +60,7 @@ struct Engine {
 	// attention launch shape
 	int attn_hg = 1, attn_hg2 = 1 /* k_attn2: padded to what it is instantiated for */, attn_qgroups = 1, attn_nsplit = 1, attn_lpp = 1;
 	// TMA-ring matvec kernels (ring.cuh): slots per warp / CTAs per SM for FFN-up and for wo / w2; u = 512-byte units per row and chunk (0: not used)
-	int ring_up_ns = 2, ring_up_cps = 2, ring_res_ns = 2, ring_res_warps = 16; // measured: 16 consuming warps per SM are needed (profiles/r02_sweep_ring_*.jsonl)
+	int ring_up_ns = 2, ring_up_cps = 2, ring_res_ns = 2, ring_res_warps = 16; // measured: 16 consuming warps per SM are needed
 	int ring_up_u = 0, ring_wo_u = 0, ring_down_u = 0, ring_wo_s = 1, ring_down_s = 1;
 	int grid_up_ring = 0, grid_wo_ring = 0, grid_down_ring = 0;
 	size_t smem_up_ring = 0, smem_wo_ring = 0, smem_down_ring = 0;
@@ -77,7 +77,7 @@ struct Engine {
 	int attn_nsplit_cap = 1 << 30;
 
 	// L2 prefetch schedule (common.cuh Prefetch): what each stage requests for the stages after it.  Bytes, or flags.
-	// Measured (profiles/r02_sweep_l2_prefetch_schedule.jsonl): no setting beats "off" -- the stage kernels are not waiting for
+	// Measured: no setting beats "off" -- the stage kernels are not waiting for
 	// DRAM behind their boundaries, and requests for later stages only compete with the running one -- so the default is off;
 	// CALM_B200_PF keeps the experiment reproducible.
 	bool pf_kv = false;           // k_qkv / w2 request the KV prefix the next attention kernel reads
@@ -689,7 +689,7 @@ int run_token(int mode) {
 }
 
 
-// Tensor-parallel view of the model for rank r of N (Megatron split; SURVEY.md s.8e): query/kv heads and FFN rows
+// Tensor-parallel view of the model for rank r of N (Megatron split): query/kv heads and FFN rows
 // are divided, so wq/wk/wv/w1/w3 shards are contiguous row ranges of the uploaded tensors (no copy), while wo and w2
 // need their COLUMN range, packed once into a contiguous (dim x n/N) matrix.  Embedding, norms and the classifier
 // are replicated.  After this the engine runs unchanged on the "local" shapes; the two partial projections per layer
@@ -1019,7 +1019,7 @@ extern "C" void prepare_cuda(struct Transformer* transformer) {
 	int maxsplit = cdiv(c.seq_len, 64);                 // at least 64 positions per slice at full context
 	g.attn_nsplit = want < 1 ? 1 : (want > maxsplit ? maxsplit : want);
 	// (measured 9 us per launch SLOWER than the global-partial fold: a 16-CTA cluster needs 16 SMs of one GPC at once, which the
-	// still-resident q/k/v CTAs delay; kept selectable for the record -- profiles/r02_sweep_ring_and_attention_variants.jsonl)
+	// still-resident q/k/v CTAs delay; kept selectable for the record)
 	if (g.attn_nsplit > ATTN2_MAXB + 4) g.attn_nsplit = ATTN2_MAXB + 4; // k_attn2 keeps one (m, l) pair per slice in static shared memory
 	const bool want_cluster = getenv("CALM_B200_ATTN_CLUSTER") && atoi(getenv("CALM_B200_ATTN_CLUSTER")) != 0;
 	if (want_cluster && attn2_shape_ok(g.attn_hg2, g.attn_lpp, c.head_dim) && !(getenv("CALM_B200_ATTN2") && atoi(getenv("CALM_B200_ATTN2")) == 0)) {
@@ -1273,7 +1273,7 @@ extern "C" int calm_b200_sample_logits(const float* logits_host, int vocab, floa
 }
 
 // ---------------------------------------------------------------------------------------------
-// forward_prefill_cuda: the prompt as one batched pass (SURVEY.md s.8b "additive entry points"; reference run.c:206-209 calls
+// forward_prefill_cuda: the prompt as one batched pass (an additive entry point; reference run.c:206-209 calls
 // forward(..., FF_UPDATE_KV_ONLY) once per prompt token).
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
@@ -1351,13 +1351,13 @@ static bool pf_supported() {
 }
 
 // Row tiles and tokens per item and K-slices of a product of `rows` weight rows over n tokens: the choice with the least estimated time, in cycles.
-// Kernel time over k-stages, 4096 x 4096 x 2047 tokens, in cycles at 1.9 GHz, for 64 / 128 / 256 tokens of one row tile and 64 / 128 of two: fp8
-// 1150 / 1250 / 1920 and 1720 / 2050 (271 / 169 / 129 and 232 / 138 us), fp16 910 / 1150 / 2150 and 1260 / 1810 (214 / 155 / 145 and 170 / 122 us);
+// Kernel time over k-stages, 4096 x 4096 x 2047 tokens, in cycles at 1.965 GHz, for 64 / 128 / 256 tokens of one row tile and 64 / 128 of two: fp8
+// 1180 / 1280 / 1960 and 1770 / 2070 (269 / 167 / 128 and 231 / 135 us), fp16 950 / 1190 / 2220 and 1280 / 1810 (217 / 155 / 145 and 166 / 118 us);
 // the estimate has 970 / 1290 / 1930 and 1290 / 1930 for all formats.  So wide items win while every SM has one, two row tiles (half the
 // activation bytes) first; K is sliced only while an item per SM is left over, and a slice pays for its way through memory.
 // Where it misses: two row tiles and 64 tokens of weights that are widened cost a third more than estimated, and two K-slices more than the
-// fold's share (FFN up 14336 x 4096, 130 tokens, fp8: 171 us, 128 with 128 tokens a tile; q/k/v 6144 x 4096, 333 tokens, gf4: 94 us, 69 unsliced);
-// over 48 products of four models the choice is within a tenth of the best in 40.
+// fold's share (FFN up 14336 x 4096, 130 tokens, fp8: 171 us, 127 with 128 tokens a tile; q/k/v 6144 x 4096, 333 tokens, gf4: 90 us, 67 unsliced);
+// over 48 products of four models the choice is within a tenth of the best in 39.
 static void pf_tiles(int mode, int rows, int n, int nkb, int sms, int& na_out, int& bn_out, int& splits_out) {
 	long best = -1;
 	for (int na = 2; na >= (mode == PF_UP ? 2 : 1); --na)

@@ -1,6 +1,6 @@
-// prefill.cuh -- batched prompt pass (SURVEY.md s.8f row 1; reference behaviour replaced: run.c:206-209 feeds the prompt one
-// token at a time through forward(), README.md:80).  T prompt tokens go through every layer together, so each weight
-// matrix is read once per 128-token tile instead of once per token and the projections become real GEMMs on the
+// prefill.cuh -- batched prompt pass (reference behaviour replaced: run.c:206-209 feeds the prompt one
+// token at a time through forward()).  T prompt tokens go through every layer together, so each weight
+// matrix is read once per tile of 64 to 256 tokens instead of once per token and the projections become real GEMMs on the
 // 5th-generation tensor cores:
 //
 //   k_pf_gemm   D[128 weight rows][<= 256 tokens] = W_tile . X_tile^T with tcgen05.mma (kind::f16, cta_group::1), fp32
@@ -113,10 +113,10 @@ __global__ void __launch_bounds__(256) k_pf_norm(const float* X, const float* no
 // latency: two warps stream the hi and the lo activation tiles and one the weight bytes in the model's format (TMA; a warp gets one copy on its
 // way every 300 cycles or so), four or eight widen them to f16 in the swizzled layout of the MMA (fp16 weights arrive in it), warp 1
 // issues the MMAs, warps 2-5 drain one of two TMEM accumulators while the other is being filled.
-// Bound: the MMA warp's hand-overs.  A stage's MMAs take 1150 cycles for two row tiles and 128 tokens; with a wait and a commit for the weights,
-// for hi and for lo a stage cost 2000, with one of each 1550, so everything a stage needs arrives on one barrier and an item is as
-// large as TMEM allows.  14336 x 2 rows, K 4096, 2048 tokens: fp8 696 us, fp16 683 us (1380 TFLOP/s, hi and lo counted; 900 and 850 us with
-// three barriers; 1324 us (fp8) when every thread loaded its weight row one stage ahead); 4096 rows: 139 and 128 us (387 us).
+// Bound: the MMA warp's hand-overs (tensor pipe 42 to 61 % active).  Everything a stage needs arrives on one barrier (with a wait and a commit for the weights,
+// for hi and for lo, FFN up took a fifth longer) and an item is as large as TMEM allows.  14336 x 2 rows, K 4096, 2047 tokens: fp8 733 us,
+// fp16 717 us (1310 and 1340 TFLOP/s, hi and lo counted; 1324 us (fp8) when every thread loaded its weight row one stage ahead); 4096 rows:
+// 135 and 118 us (387 us).
 struct PfMaps {
 	CUtensorMap x[2]; // activations, hi and lo: f16 [tokens][K], box = bn rows x 64 columns, 128-byte swizzle
 	CUtensorMap w[3]; // weights: QKV: wq, wk, wv   UP: w1, w3   WO / DOWN: w
@@ -167,7 +167,7 @@ __host__ __device__ inline size_t pf_stage_bytes(int na, int bn) {
 	return (size_t)na * PF_TILE_BYTES + 2 * bn * 128;
 }
 template <int DBITS>
-__host__ __device__ constexpr int pf_widen_warps() { // FFN up as below: fp8 696 us with four warps and 802 with eight (more arrivals per stage), gf4 871 and 825 (19 instructions per 8 weights)
+__host__ __device__ constexpr int pf_widen_warps() { // FFN up as above, side by side: fp8 696 us with four warps and 802 with eight (more arrivals per stage), gf4 871 and 825 (19 instructions per 8 weights)
 	return DBITS == 16 ? 0 : DBITS == 8 ? 4 : 8;
 }
 template <int DBITS>
@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 // thousand keys of 2^-26 were lost).  Running maximum, exponentials and the denominator are fp32.
 // Bound: the MMA rate (4 x 64 MMAs per warp and tile against 32 KB of ldmatrix traffic).  Tokens are taken 16 per warp and not 32 because
 // 64 accumulator and 64 query registers per 16 rows already fill the file at 8 warps; the last blocks of the prompt, which see
-// the most keys, are started first.  2047 tokens, 32 / 8 heads of 128: 1550 us a layer as fp32 FMAs, one token per warp; about 360 us here.
+// the most keys, are started first.  2047 tokens, 32 / 8 heads of 128: 1550 us a layer as fp32 FMAs, one token per warp; 365 us here (tensor pipe 35 % active).
 #define PFA_TILE 64 // keys per tile
 #define PFA_ONE 32768.f // weight of the largest score
 

@@ -3,8 +3,8 @@
 //   fp32 accumulators in TMEM.  Both operands are K-major bf16 matrices in global memory (weights as stored,
 //   activations as the producing kernels wrote them) and come in by TMA (cp.async.bulk.tensor, SWIZZLE_128B; edges of M,
 //   N and K are zero-filled by the copy).  One lane issues the copies, one lane the MMAs, completion flows through
-//   mbarriers (tcgen05.commit); four warps read the accumulators back (tcgen05.ld) and apply the epilogue of the product:
-//   fp32 store, activation-type store, or Dynamic-Tanh + residual add.  blockIdx.z walks a batch of per-head products
+//   mbarriers (tcgen05.commit); four warps read the accumulators back (tcgen05.ld) and apply the epilogue of the product, in an instance of
+//   the kernel for each common one (tg_epilogue; the same arithmetic as gemm_store, which serves the rest and the other kernels).  blockIdx.z walks a batch of per-head products
 //   (3-D tensor maps; an operand shared by the batch keeps a 2-D map).
 // Every wait is bounded: a stalled pipeline records a code in `err`, every role falls through to the common exit, TMEM
 // is released and the host reports the code after the step.
@@ -35,9 +35,11 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
 // of the plain ones -- a bias and a factor at most, and for EPI_F32 columns past `split` in the activation type -- with everything that does not
 // depend on the token worked out before the loop.  The additions to the residual stream load 16 tokens' rows ahead of the stores: one after the
 // other, each store bars the next load (164 us for 2048 x 2048 x 5632).  TG_ANY: gemm_store decides per element, in a loop that is not
-// unrolled: 32 copies of every epilogue do not fit the instruction cache (a 2048 x 2048 x 64 decay product through them took 124 us).
+// unrolled: 32 copies of every epilogue do not fit the instruction cache, which costs more than the accumulators' way through local memory.  What is left to it,
+// as a loop and unrolled: factors per row, all products of a Sopepel step of 2048 / 700 tokens 1194 / 763 and 1286 / 823 us; capped logits, of
+// a Tabisun step with 512 tokens' logits 838 and 852 us.
 // All products of a 2048-token step with attention and two linear attentions: 1735 us with residual additions, decays and squared rectifiers in the
-// unrolled TG_ANY, 747 in instances of their own.
+// unrolled TG_ANY, 743 in instances of their own.
 #define TG_ANY (-1)
 #define TG_ACT_GATE 100 // EPI_ACT times sigmoid(gate)
 template <int E>

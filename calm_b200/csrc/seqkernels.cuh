@@ -959,7 +959,7 @@ __global__ void __launch_bounds__(256) k_seq_attn_softmax(AttSoftmax a) {
 // were: gather, score product, softmax and value product per sequence, key head and block of queries, with scores and weights going
 // through memory.
 // Bound: the MMAs and, with few query heads per key head, the fp32 rows (64 KB a tile from L2).  A 2048-token
-// step: 638 us in 16 launches before, 308 here; three sequences of 700 tokens: 700 us in 48 launches, 146 here.
+// step: 638 us in 16 launches before, 293 here (tensor pipe 13 % active); three sequences of 700 tokens: 700 us in 48 launches, 140 here.
 #define AFL_TILE 64
 template <int HD>
 __host__ __device__ constexpr size_t afl_smem() { // the rows as cached (K, V), then as bf16 (K, V)

@@ -316,7 +316,7 @@ struct QkvArgs {
 #define QKV_THREADS 256
 // One warp per row pair (the whole 2 x rowbytes pair is requested in one batch), 3 CTAs per SM.  (A one-CTA-per-SM form with
 // equal contiguous shares, meant to leave half the register file to an early attention CTA, measured 2.8 us slower per
-// launch: most warps then need a second DRAM round trip -- profiles/README.md, round 2.)
+// launch: most warps then need a second DRAM round trip.)
 template <int DBITS, typename KVT>
 __global__ void __launch_bounds__(QKV_THREADS, 3) k_qkv(const QkvArgs<KVT> a) {
 	pdl_launch_next();
@@ -1075,7 +1075,7 @@ struct OutputArgs {
 	float eps;
 	int ln;
 	unsigned long long* stamp;
-	// tensor parallelism ("lm_head: rows split by vocab"): this rank owns classifier rows [row0, row1) and
+	// tensor parallelism (rows split by vocabulary): this rank owns classifier rows [row0, row1) and
 	// stores its logits and per-CTA greedy candidates straight into EVERY rank's gather area over NVLink (peer[rank] is
 	// its own); k_tp_gather then waits for all slices.  world <= 1: rows [0, vocab) into `logits` / `cand_*`.
 	int row0, row1, world, rank;
