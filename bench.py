@@ -1,12 +1,11 @@
 #!/usr/bin/env python
-"""bench.py -- tokens/s of single-batch decode through libcalm_b200.so (BASELINE.json metric).
+"""bench.py -- tokens/s of single-batch decode through libcalm_b200.so.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference] [--workload NAME] [--engine E]
 
 One "step" = one token of single-sequence decode (one pass of the per-token forward() path).  The
-N = 1 workload is BASELINE.json configs[1]: Llama-3-8B shape, random-init fp8 (e5m2) weights, 4096-token
-context, the timed tokens sitting at the END of the context (the reference's own "last tokens" protocol,
-README.md:86) so attention reads the whole KV cache.  Every token streams all 7.5 GB of weights, far more
+N = 1 workload is the Llama-3-8B shape, random-init fp8 (e5m2) weights, 4096-token
+context, the timed tokens sitting at the END of the context (the reference's own "last tokens" protocol) so attention reads the whole KV cache.  Every token streams all 7.5 GB of weights, far more
 than the 126 MB L2, so no L2 flush is needed between steps.
 
 Printed JSON (one line, rank 0):
@@ -301,7 +300,7 @@ def main():
     barrier, max_over_ranks = agg.barrier, agg.max_over_ranks
 
     os.environ.setdefault("CALM_B200_QUIET", "1")  # keep stdout to the one JSON line
-    sampler = ClockSampler(local)  # started well ahead of the timed region: nvidia-smi needs a second to come up on an 8-GPU box
+    sampler = ClockSampler(local)  # started well ahead of the timed region: nvidia-smi needs a second to come up on an 8-GPU machine
     sampler.start()
     cbuild.build()
     L = lib.load()
@@ -398,7 +397,7 @@ def main():
     dm.close()
 
     if rank == 0 and world == 1 and not args.no_ref_cuda and os.path.exists(os.path.join(ROOT, "oracle", "_ref", "libcalm_ref_cuda.so")):
-        # the kernel to beat (SURVEY.md s.6): the UNMODIFIED reference infer.cu on this GPU, same model, same positions, same
+        # the kernel to beat: the UNMODIFIED reference infer.cu on this GPU, same model, same positions, same
         # host-stepped protocol as the e2e leg; its own process (global statics, abort() on error), after ours released the device
         try:
             del tensors

@@ -1,4 +1,4 @@
-"""Build the shared libraries in-tree with nvcc for sm_100a (no JIT cache: the .so files ship to the GPU box).
+"""Build the shared libraries in-tree with nvcc for sm_100a (no JIT cache: the .so files travel with the tree).
 
 Two targets, each its own library so that a host compiles only what its model family needs:
   engine  libcalm_b200.so      the calm backend boundary (single-sequence Llama-shaped models)

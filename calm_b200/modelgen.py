@@ -1,6 +1,6 @@
 """Seeded synthetic models in calm's formats.
 
-There is no network in the build or on the GPU box, so every model in the
+Checkpoints are not part of the repository, so every model in the
 tests and in bench.py is random-initialised here with the SHAPES the reference
 expects (reference run.c:71-117 lists every tensor name, dtype and shape) and,
 when written to disk, in the reference's `.calm` container (a safetensors-like
@@ -53,7 +53,7 @@ class ModelSpec:
     tied: bool = False  # no model.output.weight: classifier = embedding
     max_seq_len: int = 4096
     init_std: float = 0.02
-    gate_std: float = 0.2  # wider router init keeps top-k margins healthy (SURVEY.md s.9)
+    gate_std: float = 0.2  # wider router init keeps top-k margins healthy
     bos_id: int = 0
     eos_id: int = 1
 
@@ -70,7 +70,7 @@ class ModelSpec:
         return self.n_kv_heads * self.head_dim
 
 
-# The five BASELINE.json configurations (shapes from SURVEY.md s.8) ...
+# The five model shapes the benchmark names ...
 SPECS: Dict[str, ModelSpec] = {
     "qwen2-0.5b-fp16": ModelSpec("qwen2-0.5b-fp16", 896, 4864, 24, 14, 2, 64, 151936, "fp16", rope_theta=1e6,
                                  norm_eps=1e-6, qkv_bias=True, tied=True, bos_id=2, eos_id=1),
@@ -98,7 +98,7 @@ SPECS.update({
     # Mixtral flavour: 8 experts, top-2
     "tiny-moe": replace(_T, name="tiny-moe", n_experts=8, n_experts_active=2, hidden_dim=512),
     "tiny-moe-gf4": replace(_T, name="tiny-moe-gf4", dtype="gf4", n_experts=8, n_experts_active=2, hidden_dim=512),
-    # model switches of the reference that the five configs do not exercise
+    # model switches of the reference that the five shapes do not exercise
     "tiny-gelu-clip": replace(_T, name="tiny-gelu-clip", act_type="gelu", qkv_clip=1.0, rotary_dim=16),
     "tiny-ln": replace(_T, name="tiny-ln", norm_type="layernorm", dtype="fp16"),
     "tiny-lnpar": replace(_T, name="tiny-lnpar", norm_type="layernorm_par", dtype="fp16"),
@@ -392,7 +392,7 @@ class HostModel:
 
 
 def teacher_tokens(vocab_size: int, n: int, start: int = 0) -> list:
-    """Fixed token list for teacher-forced parity runs: tok_i = (7919 i + 13) mod vocab (SURVEY.md s.8d)."""
+    """Fixed token list for teacher-forced parity runs: tok_i = (7919 i + 13) mod vocab."""
     return [((7919 * (i + start)) + 13) % vocab_size for i in range(n)]
 
 

@@ -1,4 +1,4 @@
-"""Host side of tensor parallelism (SURVEY.md s.8e; the reference is single-device, src/infer.cu:79).
+"""Host side of tensor parallelism (the reference is single-device, src/infer.cu:79).
 
 The split itself happens inside prepare_cuda (csrc/engine.cu tp_shard_model): rank r of N keeps query heads
 [r*n_heads/N, (r+1)*n_heads/N), the kv heads they attend to, and FFN rows [r*hidden/N, (r+1)*hidden/N); the output

@@ -6,8 +6,8 @@
  * reference driver declares exactly these prototypes (reference src/run.c:22-25)
  * and the reference backend defines them extern "C" (src/infer.cu:69, 73, 743,
  * 761).  Linking the unmodified reference run.c/tensors.c/tokenizer.c/sampler.c
- * against this library instead of infer.cu gives a working `run` binary -- see
- * INTEGRATION.md.  Everything prefixed calm_b200_ is additive.
+ * against this library instead of infer.cu gives a working `run` binary.
+ * Everything prefixed calm_b200_ is additive.
  *
  * Error behaviour follows the reference (infer.cu:12-20, 755): there are no
  * error codes; a CUDA failure or an unsupported configuration prints one line
@@ -75,8 +75,8 @@ void calm_b200_free(void* device_ptr);
  * never frees, run.c:636) so another model can be prepared in this process. */
 void calm_b200_release(struct Transformer* transformer);
 
-/* Tensor parallelism for models that do not fit (or should not sit on) one GPU -- the 70B shape of
- * BASELINE.json configs[4]; the reference has no counterpart (single device, infer.cu:79).  One process per GPU.
+/* Tensor parallelism for models that do not fit (or should not sit on) one GPU -- the 70B shape;
+ * the reference has no counterpart (single device, infer.cu:79).  One process per GPU.
  * Rank 0 obtains a 128-byte NCCL id with calm_b200_tp_unique_id() and hands it to the other ranks by any means
  * (file, pipe, torch.distributed broadcast); every rank then calls calm_b200_tp_init(rank, world, id) BEFORE
  * prepare_cuda() and afterwards drives the library exactly as a single-GPU host does: upload the FULL tensors,
@@ -94,14 +94,14 @@ int calm_b200_tp_mode(void);
 
 
 /* The prompt as ONE batched pass (the reference feeds prompt tokens one at a time through forward(.., FF_UPDATE_KV_ONLY),
- * run.c:206-209, README.md:80): n tokens at positions pos0 .. pos0+n-1 go through every layer together; the projections
+ * run.c:206-209): n tokens at positions pos0 .. pos0+n-1 go through every layer together; the projections
  * are tensor-core GEMMs (tcgen05.mma, TMEM accumulators, weights dequantised on the fly, activations as an f16 hi + lo
  * pair so inputs keep 22 bits), attention is causal over the block and the cache.  Afterwards the KV cache holds what n
  * serial KV-only calls would have left (within the stated tolerance); no logits, no synchronisation with the host beyond
  * reading `tokens`.  Returns 1 when the batched pass ran, 0 when the model shape is not served by it (MoE, tensor
  * parallelism, dims not multiples of 128, head_dim other than 64 / 128, a block that would roll the cache over) and the
  * tokens were fed one by one instead -- same result either way.  A host integrates it by replacing the prompt loop:
- * forward_prefill_cuda(t, prompt, n - 1, 0); logits = forward_cuda(t, prompt[n - 1], n - 1, 0);  (INTEGRATION.md). */
+ * forward_prefill_cuda(t, prompt, n - 1, 0); logits = forward_cuda(t, prompt[n - 1], n - 1, 0). */
 int forward_prefill_cuda(struct Transformer* transformer, const int* tokens, int n, int pos0);
 /* How a product of the pass over n tokens is cut on a GPU of `sms` SMs (no GPU needed; for tests and measurements): product 0 q/k/v, 1 wo and w2, 2 FFN
  * up (rows of one of its matrices); out3 = row tiles of 128 per item, tokens per item, slices of k. */

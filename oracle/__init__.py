@@ -33,7 +33,7 @@ _PATHS = {
 
 
 def build(ref: bool = True) -> None:
-    """Compile the restatement and, when /root/reference is present, the reference itself."""
+    """Compile the restatement and, where its sources are present, the reference itself."""
     targets = ["all"] + (["ref"] if ref else [])
     subprocess.run(["make", "-C", HERE, "--no-print-directory"] + targets, check=True, stdout=subprocess.DEVNULL)
 

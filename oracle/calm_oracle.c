@@ -15,12 +15,12 @@
  * compiler flags or thread count.
  *
  * How it is pinned: the reference has no golden vectors or unit tests
- * (SURVEY.md section 4), so parity is pinned by EXECUTING the reference:
- * oracle/Makefile compiles the unmodified reference sources from
- * /root/reference/src into oracle/_ref/, tests/test_oracle.py runs
+ * so parity is pinned by EXECUTING the reference:
+ * oracle/Makefile compiles the unmodified reference sources into
+ * oracle/_ref/, tests/test_oracle.py runs
  * both on the same seeded synthetic models, and tools/make_golden.py stores
- * reference outputs as fixtures under tests/golden/ for boxes that do not
- * have /root/reference.
+ * reference outputs as fixtures under tests/golden/ for machines that do
+ * not have them.
  *
  * Two builds (see oracle/Makefile):
  *   libcalm_oracle.so      acc_t = float : the reference's arithmetic

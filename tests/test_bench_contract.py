@@ -1,6 +1,6 @@
-"""The JSON line bench.py prints (the driver's contract) checked on the committed round-2 lines: keys, types and the internal
+"""The JSON line bench.py prints checked on committed lines: keys, types and the internal
 arithmetic (value <-> ms_per_step, roofline.frac = achieved / peak, e2e declares its copies).  CPU only: the lines were
-produced on the GPU box by the committed command and live under profiles/."""
+produced on a B200 by the committed command and live under profiles/."""
 import json
 import os
 import sys

@@ -1,4 +1,4 @@
-"""The drop-in proof on the GPU box: the UNMODIFIED reference driver (run.c, tensors.c, tokenizer.c, sampler.c) linked
+"""The drop-in proof: the UNMODIFIED reference driver (run.c, tensors.c, tokenizer.c, sampler.c) linked
 against libcalm_b200.so (oracle/_ref/run_b200, built by `make -C oracle dropin`) loads a .calm file, decodes greedily on
 the GPU and prints the same tokens as the reference's own CPU path (CALM_CPU=1, same binary) and as the oracle."""
 import os
@@ -17,7 +17,7 @@ pytestmark = pytest.mark.gpu
 EXE = os.path.join(ROOT, "oracle", "_ref", "run_b200")
 
 
-@pytest.mark.skipif(not os.path.exists(EXE), reason="oracle/_ref/run_b200 did not travel (needs /root/reference at build time)")
+@pytest.mark.skipif(not os.path.exists(EXE), reason="oracle/_ref/run_b200 is not there (needs the reference sources at build time)")
 @pytest.mark.parametrize("name", ["tiny-llama", "tiny-gf4", "tiny-moe"])
 def test_reference_driver_with_our_backend(tmp_path, oracle_pkg, name):
     spec = mg.SPECS[name]
@@ -57,7 +57,7 @@ def test_reference_driver_with_our_backend(tmp_path, oracle_pkg, name):
     assert got[2:2 + len(gen)] == gen[:len(got) - 2]
 
 
-@pytest.mark.skipif(not os.path.exists(EXE), reason="oracle/_ref/run_b200 did not travel (needs /root/reference at build time)")
+@pytest.mark.skipif(not os.path.exists(EXE), reason="oracle/_ref/run_b200 is not there (needs the reference sources at build time)")
 def test_perf_table_through_the_reference_driver(tmp_path):
     """CALM_B200_PERF=1: the unmodified reference driver, linked to our backend, ends with perf_cuda()'s per-stage table (the
     reference prints its own under a CUPTI injection, run.c:630-632, infer.cu:761-801); timings come from inside the production graph."""

@@ -41,7 +41,7 @@ def test_oracle_matches_golden(oracle_pkg, name):
     ck.release(model)
 
 
-@pytest.mark.skipif(not HAVE_REF, reason="oracle/_ref not built and /root/reference absent")
+@pytest.mark.skipif(not HAVE_REF, reason="oracle/_ref not built and the reference absent")
 @pytest.mark.parametrize("name", ["tiny-fp8", "tiny-gf4", "tiny-qwen", "tiny-moe"])
 def test_oracle_matches_reference_live(oracle_pkg, name):
     """Same comparison against the reference executed now, on a different seed and at a position offset."""
@@ -116,7 +116,7 @@ def test_gf4_quantiser_properties():
 
 
 def test_algorithmic_bytes_table():
-    """n_bandwidth (run.c:523-532) of the five named shapes == BASELINE.md section 2."""
+    """n_bandwidth (run.c:523-532) of the five named shapes, in GB."""
     exp = {"qwen2-0.5b-fp16": 0.988, "llama3-8b-fp8": 7.506, "llama3-8b-fp16": 15.010, "mistral-7b-gf4": 3.556,
            "mixtral-8x7b-fp8": 12.750, "llama3-70b-fp8": 69.507}
     for name, gb in exp.items():

@@ -3,7 +3,7 @@ backend (upload_cuda -> prepare_cuda -> forward_cuda per token), against
   (1) the CPU oracle (oracle/calm_oracle.c) on the same seeded model,
   (2) the committed golden fixtures produced by the unmodified reference, and
   (3) the unmodified reference itself (oracle/_ref/libcalm_ref_cpu.so) when it travelled to this box.
-Tolerance (stated): |dlogit| <= 5e-3 * std(logits); argmax identical on every step whose
+Tolerance: |dlogit| <= 5e-3 * std(logits); argmax identical on every step whose
 reference top-2 margin exceeds twice that; KV entries within fp16 rounding."""
 import os
 import sys
@@ -142,7 +142,7 @@ def test_matvec_kernel_vs_oracle(oracle_pkg, dbits, n, d):
 
 
 def test_full_size_matvec_properties(oracle_pkg):
-    """BASELINE-sized matrix (Llama-3-8B w1: 14336 x 4096 fp8): size-independent properties --
+    """A matrix of the benchmark (Llama-3-8B w1: 14336 x 4096 fp8): size-independent properties --
     linearity in x, a row subset against the oracle, and zero input -> exact zeros."""
     n, d = 4096, 14336
     g = torch.Generator(device="cuda").manual_seed(0)

@@ -1,4 +1,4 @@
-"""Sampler row: the restatement of reference sampler.c against the unmodified reference
+"""Sampler: the restatement of reference sampler.c against the unmodified reference
 (when it is mounted) and against the committed fixture made from it; on the GPU, the device-side sampler against
 the restatement on the same logits and generator state."""
 import os

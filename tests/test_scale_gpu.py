@@ -1,4 +1,4 @@
-"""GPU parity at the scale of the headline configuration (VERDICT r01 #1): the full 4096-position context through the
+"""GPU parity at the scale of the headline configuration: the full 4096-position context through the
 multi-slice attention merge, the fp8 (e5m2) KV cache, and the 32-layer Llama-3-8B shape itself.
 
 Checkers:

@@ -2,8 +2,8 @@
 """Generate tests/golden/*.npz by RUNNING THE REFERENCE (oracle/_ref/libcalm_ref_cpu.so, i.e. the
 unmodified reference src/infer.c compiled with the reference's flags by oracle/Makefile).
 
-The reference ships no golden vectors or unit tests (SURVEY.md s.4), so these fixtures are what pins
-the oracle and the CUDA path on machines without /root/reference (the GPU box).  Each fixture holds,
+The reference ships no golden vectors or unit tests, so these fixtures are what pins
+the oracle and the CUDA path on machines without its sources.  Each fixture holds,
 for one seeded synthetic model (calm_b200.modelgen, seed 0) and the fixed teacher-forced token list:
   sha256     of the generated tensors (guards against a generator that drifted)
   tokens     the token list

@@ -5,7 +5,7 @@
   oracle/_ref/run_b200  the same reference program linked against libcalm_b200.so (the drop-in)
 
 Writes the synthetic model as a .calm file (calm_b200.modelgen.write_calm) into /dev/shm, runs both binaries with
-the reference's own protocol (README.md:86: first tokens at pos 0.., last tokens with CALM_POSO) and prints the
+the reference's own protocol (first tokens at pos 0.., last tokens with CALM_POSO) and prints the
 reference's stats lines (run.c:249-253).  Usage: python tools/ref_cuda_bench.py [workload] [n_tokens]"""
 import json
 import os
