@@ -4,9 +4,10 @@
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference] [--workload NAME] [--engine E]
 
 One "step" = one token of single-sequence decode (one pass of the per-token forward() path).  The
-N = 1 workload is the Llama-3-8B shape, random-init fp8 (e5m2) weights, 4096-token
-context, the timed tokens sitting at the END of the context (the reference's own "last tokens" protocol) so attention reads the whole KV cache.  Every token streams all 7.5 GB of weights, far more
-than the 126 MB L2, so no L2 flush is needed between steps.
+N = 1 workload is the Llama-3-8B shape, random-init fp8 (e5m2) weights, 4096-token context, the timed
+tokens sitting at the END of the context (the reference's own "last tokens" protocol) so attention reads
+the whole KV cache.  Every token streams all 7.5 GB of weights, far more than the 126 MB L2, so no L2
+flush is needed between steps.
 
 Printed JSON (one line, rank 0):
   value      tokens/s with everything resident in HBM: device-side greedy loop (forward + argmax feeding
