@@ -1599,6 +1599,247 @@ __global__ void __launch_bounds__(128) k_seq_gla_scan(GlaArgs a, SeqBatch sb) {
 	}
 }
 
+// The same recurrence for long portions, cut into chunks of tokens that run side by side: (1) k_seq_gla_local forms what a chunk adds to a zero
+// state and the product of its decays, (2) k_seq_gla_starts walks a state element through the chunks, leaving every chunk's first state in place
+// of what it adds, and updates the slot's state, (3) k_seq_gla_apply runs each chunk's tokens from there for the read-outs.
+// k_seq_gla_scan is a chain over all tokens on as many SMs as sequences x heads x columns give (2048 tokens of 16 heads of 128 x 128: 469 us,
+// 230 ns a token whatever the arithmetic); here (1) and (3) fill the SMs: 140 us, each launch alone with cold caches 47 + 16 + 94.
+struct GlaChunks {
+	float* add;  // [B][count][heads][vdim][dim]: what a chunk adds, then the state it starts from
+	float* keep; // [B][count][heads][dim]: product of the chunk's decays
+	int len, count;
+};
+// (1): S[v][d] = sum over tokens of v (x) k scaled by the decays that follow, a block of GLC_TB tokens at a time: inside a block the keys carry the
+// product of the later tokens' decays (nothing is divided), so that an element costs one FMA per token and one multiplication per block.
+// One CTA per (chunk, head, 128 value columns), 2 D threads of 8 x 8 elements each, multiplied in pairs (an FMA pipe is as fast on single ones, but pairs
+// leave every second issue slot to the loads).  Blocks travel two ahead by asynchronous copies, and a block's keys are scaled while the one before is
+// multiplied.
+#define GLC_TB 8
+#define GLC_STAGES 4
+__host__ __device__ constexpr int glc_tok(int D) { return 2 * D + 128; } // k, decay, v
+__host__ __device__ constexpr size_t glc_smem(int D) { return ((size_t)GLC_STAGES * GLC_TB * glc_tok(D) + 2 * (GLC_TB + 1) * D) * sizeof(float); }
+template <int D>
+__global__ void __launch_bounds__(2 * D, 256 / D) k_seq_gla_local(GlaArgs a, GlaChunks c, SeqBatch sb) {
+	pdl_enter(); // programmatic dependent launch: let the next kernel's launch overlap this one, then wait for the previous one
+	constexpr int TX = D / 8, TOK = glc_tok(D), ITEMS = TOK / 4, ROUNDS = (ITEMS + 2 * D - 1) / (2 * D);
+	extern __shared__ __align__(16) float sm[];
+	float* const scaled = sm + GLC_STAGES * GLC_TB * TOK; // [2][GLC_TB scaled keys, then the block's decays][D]
+	const int b = blockIdx.x / c.count, ch = blockIdx.x % c.count, h = blockIdx.y, v0 = blockIdx.z * 128, V = a.vdim;
+	const int t0 = ch * c.len, nt = min(c.len, sb.scount[b] - t0);
+	if (nt <= 0) return;
+	const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX, nblk = (nt + GLC_TB - 1) / GLC_TB;
+	const size_t first = (size_t)sb.sstart[b] + t0;
+	// a thread copies the same 16-byte items of every token; columns past the last one are zero
+	const float* src[ROUNDS];
+	long stride[ROUNDS];
+#pragma unroll
+	for (int r = 0; r < ROUNDS; ++r) {
+		const int i = 4 * (tid + r * 2 * D);
+		src[r] = nullptr, stride[r] = a.ldp;
+		if (i < D) src[r] = a.proj + first * a.ldp + a.kcol + h * D + i;
+		else if (i < 2 * D) src[r] = a.decay + (first * a.heads + h) * D + i - D, stride[r] = (long)a.heads * D;
+		else if (i < TOK && v0 + i - 2 * D < V) src[r] = a.proj + first * a.ldp + a.vcol + h * V + v0 + i - 2 * D;
+		else if (i < TOK)
+			for (int t = 0; t < GLC_STAGES * GLC_TB; ++t) *(float4*)(sm + t * TOK + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+	}
+	auto issue = [&](int blk) {
+		const int n = min(GLC_TB, nt - blk * GLC_TB);
+		float* dst = sm + blk % GLC_STAGES * GLC_TB * TOK;
+#pragma unroll
+		for (int r = 0; r < ROUNDS; ++r)
+			if (src[r])
+				for (int t = 0; t < n; ++t) cp_async16(dst + t * TOK + 4 * (tid + r * 2 * D), src[r] + (blk * GLC_TB + t) * stride[r]);
+		asm volatile("cp.async.commit_group;" ::: "memory"); // (an empty group past the last block)
+	};
+	float all = 1.f; // threads that scale keys: the decays of the chunk so far
+	auto scale = [&](int blk) {
+		const int n = min(GLC_TB, nt - blk * GLC_TB);
+		const float* raw = sm + blk % GLC_STAGES * GLC_TB * TOK + tid;
+		float* to = scaled + (blk & 1) * (GLC_TB + 1) * D + tid;
+		float w = 1.f;
+#pragma unroll
+		for (int t = GLC_TB - 1; t >= 0; --t) {
+			to[t * D] = t < n ? raw[t * TOK] * w : 0.f;
+			if (t < n) w *= raw[t * TOK + D];
+		}
+		to[GLC_TB * D] = w, all *= w;
+	};
+	float2 S[8][4] = {}; // [value column][pair of key channels], both as two groups of four: 4 ty + {0, 64}, 4 tx + {0, D / 2}
+	issue(0), issue(1), issue(2);
+	asm volatile("cp.async.wait_group 2;" ::: "memory");
+	__syncthreads();
+	if (tid < D) scale(0);
+	for (int blk = 0; blk < nblk; ++blk) {
+		asm volatile("cp.async.wait_group 1;" ::: "memory");
+		__syncthreads(); // block blk + 1 is there, block blk scaled, block blk - 1 done with
+		issue(blk + 3);
+		if (tid < D && blk + 1 < nblk) scale(blk + 1);
+		const float* kk = scaled + (blk & 1) * (GLC_TB + 1) * D + 4 * tx;
+		const float* vv = sm + blk % GLC_STAGES * GLC_TB * TOK + 2 * D + 4 * ty;
+		float2 k[4];
+		auto row = [&](int t) {
+			const float4 x = *(const float4*)(kk + t * D), y = *(const float4*)(kk + t * D + D / 2);
+			k[0] = make_float2(x.x, x.y), k[1] = make_float2(x.z, x.w), k[2] = make_float2(y.x, y.y), k[3] = make_float2(y.z, y.w);
+		};
+		row(GLC_TB);
+#pragma unroll
+		for (int j = 0; j < 8; ++j)
+#pragma unroll
+			for (int i = 0; i < 4; ++i) S[j][i] = __fmul2_rn(S[j][i], k[i]);
+		const int n = min(GLC_TB, nt - blk * GLC_TB);
+#pragma unroll 4
+		for (int t = 0; t < n; ++t) {
+			row(t);
+			const float4 x = *(const float4*)(vv + t * TOK), y = *(const float4*)(vv + t * TOK + 64);
+			const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+			for (int j = 0; j < 8; ++j)
+#pragma unroll
+				for (int i = 0; i < 4; ++i) S[j][i] = __ffma2_rn(make_float2(v[j], v[j]), k[i], S[j][i]);
+		}
+	}
+	const size_t unit = ((size_t)b * c.count + ch) * a.heads + h;
+#pragma unroll
+	for (int j = 0; j < 8; ++j) {
+		const int v = v0 + (j >> 2) * 64 + 4 * ty + (j & 3);
+		if (v >= V) continue;
+		float* o = c.add + (unit * V + v) * D;
+		*(float4*)(o + 4 * tx) = make_float4(S[j][0].x, S[j][0].y, S[j][1].x, S[j][1].y);
+		*(float4*)(o + D / 2 + 4 * tx) = make_float4(S[j][2].x, S[j][2].y, S[j][3].x, S[j][3].y);
+	}
+	if (tid < D && blockIdx.z == 0) c.keep[unit * D + tid] = all;
+}
+// (2): four key channels of one value column per thread
+template <int D>
+__global__ void __launch_bounds__(128) k_seq_gla_starts(GlaArgs a, GlaChunks c, SeqBatch sb) {
+	pdl_enter(); // programmatic dependent launch: let the next kernel's launch overlap this one, then wait for the previous one
+	const int b = blockIdx.y, e = blockIdx.x * 128 + threadIdx.x, d = e % (D / 4) * 4, hv = e / (D / 4);
+	if (hv >= a.heads * a.vdim) return;
+	const int h = hv / a.vdim, nc = (sb.scount[b] + c.len - 1) / c.len;
+	float4* const st = (float4*)(a.state + ((size_t)sb.sslot[b] * a.heads * a.vdim + hv) * a.ldstate + d);
+	float4* ap = (float4*)(c.add + ((size_t)b * c.count * a.heads * a.vdim + hv) * D + d);
+	const float4* kp = (const float4*)(c.keep + ((size_t)b * c.count * a.heads + h) * D + d);
+	const size_t as = (size_t)a.heads * a.vdim * D / 4, ks = (size_t)a.heads * D / 4;
+	float4 s = *st;
+	for (int i0 = 0; i0 < nc; i0 += 4, ap += 4 * as, kp += 4 * ks) {
+		float4 x[4], k[4];
+#pragma unroll
+		for (int i = 0; i < 4; ++i)
+			if (i0 + i < nc) x[i] = ap[i * as], k[i] = kp[i * ks];
+#pragma unroll
+		for (int i = 0; i < 4; ++i)
+			if (i0 + i < nc) {
+				ap[i * as] = s;
+				s = make_float4(fmaf(k[i].x, s.x, x[i].x), fmaf(k[i].y, s.y, x[i].y), fmaf(k[i].z, s.z, x[i].z), fmaf(k[i].w, s.w, x[i].w));
+			}
+	}
+	*st = s;
+}
+// (3): one CTA of four warps per (chunk, head, gla_cols(D) value columns); D / 8 lanes share four columns and hold eight key channels of each, so that
+// the seven 16-byte shared-memory reads of a token serve 96 multiplications and multiply-adds per lane (k_seq_gla_scan: six for 24).  Bound by those: the
+// FMA pipe is at two thirds, and pairs of them (half as many instructions, the same pipe time) are as fast as single ones, 94 and 96 us.
+#define GLA_TC 8
+__host__ __device__ constexpr int gla_cols(int D) { return 128 / (D / 8) * 4; }
+template <int D>
+__global__ void __launch_bounds__(128, 4) k_seq_gla_apply(GlaArgs a, GlaChunks c, SeqBatch sb) {
+	pdl_enter(); // programmatic dependent launch: let the next kernel's launch overlap this one, then wait for the previous one
+	constexpr int P = D / 8, VC = gla_cols(D), TOK = 3 * D + VC, ITEMS = TOK / 4;
+	__shared__ __align__(16) float sm[2][GLA_TC * TOK]; // per token k, q, decay, v
+	const int b = blockIdx.x / c.count, ch = blockIdx.x % c.count, h = blockIdx.y, V = a.vdim, v0 = blockIdx.z * VC;
+	const int t0 = ch * c.len, nt = min(c.len, sb.scount[b] - t0);
+	if (nt <= 0) return;
+	const int tid = threadIdx.x, part = tid % P, cl = tid / P * 4;
+	const bool live = v0 + cl < V; // (V is a multiple of 4) lanes past the last column run along on the last group's state
+	const size_t first = (size_t)sb.sstart[b] + t0;
+	float2 S[4][4]; // [value column][pairs of the key channels 4 part + {0..3}, D / 2 + 4 part + {0..3}]
+	const float* Sg = c.add + ((((size_t)b * c.count + ch) * a.heads + h) * V + (live ? v0 + cl : V - 4)) * D + 4 * part;
+#pragma unroll
+	for (int j = 0; j < 4; ++j) {
+		const float4 x = *(const float4*)(Sg + j * D), y = *(const float4*)(Sg + j * D + D / 2);
+		S[j][0] = make_float2(x.x, x.y), S[j][1] = make_float2(x.z, x.w), S[j][2] = make_float2(y.x, y.y), S[j][3] = make_float2(y.z, y.w);
+	}
+	// a thread copies the same (at most two) 16-byte items of every token
+	const float* src[2] = {nullptr, nullptr};
+	long stride[2] = {0, 0};
+#pragma unroll
+	for (int r = 0; r < 2; ++r) {
+		const int i = 4 * (tid + r * 128);
+		if (tid + r * 128 >= ITEMS) continue;
+		if (i < 2 * D) src[r] = a.proj + first * a.ldp + (i < D ? a.kcol + i : a.qcol + i - D) + h * D, stride[r] = a.ldp;
+		else if (i < 3 * D) src[r] = a.decay + (first * a.heads + h) * D + i - 2 * D, stride[r] = (long)a.heads * D;
+		else if (v0 + i - 3 * D < V) src[r] = a.proj + first * a.ldp + a.vcol + h * V + v0 + i - 3 * D, stride[r] = a.ldp;
+	}
+	auto issue = [&](int blk) {
+		const int n = min(GLA_TC, nt - blk * GLA_TC);
+#pragma unroll
+		for (int r = 0; r < 2; ++r)
+			if (src[r])
+				for (int t = 0; t < n; ++t) cp_async16(sm[blk & 1] + t * TOK + 4 * (tid + r * 128), src[r] + (blk * GLA_TC + t) * stride[r]);
+		asm volatile("cp.async.commit_group;" ::: "memory");
+	};
+	const int nblk = (nt + GLA_TC - 1) / GLA_TC;
+	issue(0);
+	for (int blk = 0; blk < nblk; ++blk) {
+		if (blk + 1 < nblk) {
+			issue(blk + 1);
+			asm volatile("cp.async.wait_group 1;" ::: "memory");
+		} else asm volatile("cp.async.wait_group 0;" ::: "memory");
+		__syncthreads();
+		const float* __restrict__ cur = sm[blk & 1];
+		const int n = min(GLA_TC, nt - blk * GLA_TC);
+		float o[4 * GLA_TC]; // this lane's shares of the read-outs [token][column]
+		auto apply = [&](int t) {
+			const float* tk = cur + t * TOK;
+			const float4 va = *(const float4*)(tk + 3 * D + cl);
+			const float v[4] = {va.x, va.y, va.z, va.w};
+			float2 r[4] = {};
+#pragma unroll
+			for (int half = 0; half < 2; ++half) {
+				const float* at = tk + half * (D / 2) + 4 * part;
+				const float4 k4 = *(const float4*)at, q4 = *(const float4*)(at + D), g4 = *(const float4*)(at + 2 * D);
+				const float2 k[2] = {make_float2(k4.x, k4.y), make_float2(k4.z, k4.w)}, q[2] = {make_float2(q4.x, q4.y), make_float2(q4.z, q4.w)}, g[2] = {make_float2(g4.x, g4.y), make_float2(g4.z, g4.w)};
+#pragma unroll
+				for (int j = 0; j < 4; ++j)
+#pragma unroll
+					for (int i = 0; i < 2; ++i) {
+						float2& s = S[j][2 * half + i];
+						s = __ffma2_rn(g[i], s, __fmul2_rn(k[i], make_float2(v[j], v[j]))), r[j] = __ffma2_rn(s, q[i], r[j]);
+					}
+			}
+#pragma unroll
+			for (int j = 0; j < 4; ++j) o[4 * t + j] = r[j].x + r[j].y;
+		};
+		if (n == GLA_TC) {
+#pragma unroll
+			for (int t = 0; t < GLA_TC; ++t) apply(t);
+		} else {
+#pragma unroll
+			for (int t = 0; t < GLA_TC; ++t) {
+				if (t < n) apply(t);
+				else o[4 * t] = o[4 * t + 1] = o[4 * t + 2] = o[4 * t + 3] = 0.f;
+			}
+		}
+		// folded over the column's lanes, each keeping half of the values at every step: lane `part` ends with values E part .. E part + E - 1
+		constexpr int E = 4 * GLA_TC / P;
+#pragma unroll
+		for (int w = P / 2, left = 2 * GLA_TC; w > 0; w >>= 1, left >>= 1) {
+			const bool up = part & w;
+#pragma unroll
+			for (int i = 0; i < left; ++i) {
+				const float other = __shfl_xor_sync(0xffffffffu, up ? o[i] : o[i + left], w);
+				o[i] = (up ? o[i + left] : o[i]) + other;
+			}
+		}
+		const int t = part * E / 4;
+		if (live && t < n) {
+			float* dst = a.o + ((first + blk * GLA_TC + t) * a.heads + h) * V + v0 + cl + part * E % 4;
+			if constexpr (E == 2) *(float2*)dst = make_float2(o[0] * a.qscale, o[1] * a.qscale);
+			else *(float4*)dst = make_float4(o[0] * a.qscale, o[1] * a.qscale, o[2] * a.qscale, o[3] * a.qscale);
+		}
+		__syncthreads(); // this half of the buffer may be filled again
+	}
+}
+
 // ---------------------------------------------------------------- query / key preparation of grouped-query attention
 // One CTA per token (or, with norms per head, several: gridDim.y slices of the heads), on the stacked (biased) projection [q | k | v | ...]: an RMS norm over the WHOLE query projection and one over
 // the whole key projection (all heads at once, weights qw / kw; null: no norm), then the first rot_dims channels of every head turn

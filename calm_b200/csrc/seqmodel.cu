@@ -79,6 +79,8 @@ struct Seq {
 	size_t w_rope = 0;
 	float2* carry = nullptr;                          // SEQ_MINGRU: chunk maps of a step's longer portions
 	size_t carry_cap = 0;
+	float* gla = nullptr;                             // gated linear attention: states and decays of a step's chunks
+	size_t gla_cap = 0;
 	void* ah = nullptr;                               // parallel blocks: a dense unit's hidden activations, written by the mixer's input product
 	size_t w_ah = 0;
 	float* mo = nullptr;                              // parallel blocks: the mixer's output until the feed-forward's is added with it; hyper blocks: a sublayer's output
@@ -828,6 +830,16 @@ void out_product(Seq& s, const AT* X, const void* Wt, int N, int K, const OutEpi
 	gemm(s, X, K, 0, Wt, K, 0, oe.dst, s.m.width, 0, N, s.m.width, K, 1, oe.epi, oe.nrm, -1, true, &gx);
 }
 
+void ensure_gla(Seq& s, size_t need) {
+	if (need <= s.gla_cap) return;
+	CUDA_CHECK(cudaStreamSynchronize(s.stream));
+	cudaFree(s.gla); // decode graphs (one token per sequence) never read it
+	s.gla = (float*)dalloc(need * sizeof(float)), s.gla_cap = need;
+}
+// Portions from this many tokens on are cut into chunks.  Scan against chunks, us a layer of 128 x 128: 16 heads, 200 tokens 57, 36; 256 66, 38; 2048 468, 140; two
+// sequences of 256 85, 52; 8 heads, 128 tokens 26, 27; 256 45, 31; 2048 298, 83.
+const int kGlaChunksMin = 160;
+
 // the gated-linear-attention scan over a step's tokens: S <- diag(decay) S + k v^T, o = S^T q * qscale per (sequence, head); g names
 // the inputs (columns of a matrix with row stride ld), the state and the output
 void gla_launch(Seq& s, GlaArgs& g, const SeqBatch& sb, int ld) {
@@ -835,6 +847,26 @@ void gla_launch(Seq& s, GlaArgs& g, const SeqBatch& sb, int ld) {
 	g.ldp = ld;
 	g.vec = D % 4 == 0 && Dv % 4 == 0 && ld % 4 == 0 && g.qcol % 4 == 0 && g.kcol % 4 == 0 && g.vcol % 4 == 0 && ((uintptr_t)g.proj & 15) == 0; // 16-byte copies
 	g.ldstate = gla_ldstate(D);
+	// long portions: chunks of tokens side by side, as many as keep every CTA of the last pass resident (four per SM)
+	int longest = 0;
+	for (int b = 0; b < sb.B; ++b) longest = std::max(longest, s.hb_count[b]);
+	const int nv = D == 64 || D == 128 ? cdiv(Dv, gla_cols(D)) : 0, room = nv ? 4 * s.sms / (sb.B * H * nv) : 0;
+	if (g.vec && longest >= kGlaChunksMin && room > 1) {
+		GlaChunks c;
+		c.len = (cdiv(longest, room) + GLC_TB - 1) / GLC_TB * GLC_TB, c.count = cdiv(longest, c.len);
+		const size_t units = (size_t)sb.B * c.count * H;
+		ensure_gla(s, units * D * (Dv + 1));
+		c.add = s.gla, c.keep = s.gla + units * D * Dv;
+		const double bytes = (double)N * H * (3.0 * D + 2.0 * Dv) * 4 + 2.0 * sb.B * H * D * Dv * 4, flops = (double)N * H * D * Dv * 4.0;
+		auto go = [&](auto local, auto starts, auto apply) {
+			run_kernel(s, KD_GLA, 0, 0, [&] { launch_k(s, local, dim3(sb.B * c.count, H, cdiv(Dv, 128)), 2 * D, glc_smem(D), g, c, sb); });
+			run_kernel(s, KD_GLA, 0, 0, [&] { launch_k(s, starts, dim3(cdiv((long)H * Dv * D / 4, 128), sb.B), 128, 0, g, c, sb); });
+			run_kernel(s, KD_GLA, bytes, flops, [&] { launch_k(s, apply, dim3(sb.B * c.count, H, nv), 128, 0, g, c, sb); });
+		};
+		if (D == 128) go(k_seq_gla_local<128>, k_seq_gla_starts<128>, k_seq_gla_apply<128>);
+		else go(k_seq_gla_local<64>, k_seq_gla_starts<64>, k_seq_gla_apply<64>);
+		return;
+	}
 	// lanes per value column: more of them while sequences x heads x columns alone would leave SMs without a CTA
 	int lanes = 4;
 	while (lanes < 16 && (long)sb.B * H * cdiv(Dv * lanes, 128) < s.sms) lanes *= 2;
@@ -1490,6 +1522,8 @@ extern "C" void* calm_b200_seq_prepare(const struct SeqModel* model) {
 		constexpr int R = decltype(r)::value, P = decltype(p)::value;
 		CUDA_CHECK(cudaFuncSetAttribute(k_seq_gla_scan<R, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gla_smem(R, P)));
 	});
+	CUDA_CHECK(cudaFuncSetAttribute(k_seq_gla_local<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)glc_smem(128)));
+	CUDA_CHECK(cudaFuncSetAttribute(k_seq_gla_local<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)glc_smem(64)));
 	CUDA_CHECK(cudaFuncSetAttribute(k_seq_attn_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
 	CUDA_CHECK(cudaFuncSetAttribute(k_seq_attn_flash<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)afl_smem<128>()));
 	CUDA_CHECK(cudaFuncSetAttribute(k_seq_attn_flash<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)afl_smem<64>()));
@@ -1586,7 +1620,7 @@ extern "C" void calm_b200_seq_release(void* handle) {
 		for (RunState& q : r.sub) drop(q);
 	};
 	for (RunState& r : s->runs) drop(r);
-	cudaFree(s->lin), cudaFree(s->fsh), cudaFree(s->hist), cudaFree(s->carry), cudaFree(s->rope_cs);
+	cudaFree(s->lin), cudaFree(s->fsh), cudaFree(s->hist), cudaFree(s->carry), cudaFree(s->gla), cudaFree(s->rope_cs);
 	cudaFree(s->table_dev), cudaFree(s->d_tok), cudaFree(s->d_want), cudaFree(s->d_argmax), cudaFree(s->logits), cudaFree(s->hW);
 	cudaFree(s->part), cudaFree(s->a3), cudaFree(s->att_kb), cudaFree(s->att_vt), cudaFree(s->att_s), cudaFree(s->att_p), cudaFree(s->x), cudaFree(s->x0), cudaFree(s->proj), cudaFree(s->hA), cudaFree(s->a1), cudaFree(s->a2), cudaFree(s->trace_buf);
 	for (float* p : s->f) cudaFree(p);
