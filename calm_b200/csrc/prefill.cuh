@@ -267,12 +267,6 @@ __device__ __forceinline__ bool bar_and(int id, int threads, bool p) {
 	return all != 0;
 }
 
-__device__ __forceinline__ bool elect_one() { // one lane of a converged warp
-	uint32_t p;
-	asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-	return p != 0;
-}
-
 template <int MODE, int DBITS>
 __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid_constant__ PfMaps m, const PfGemmArgs a) {
 	constexpr int WIDEN = pf_widen_warps<DBITS>(), W_WARP = 6 + WIDEN, LO_WARP = W_WARP + 1;

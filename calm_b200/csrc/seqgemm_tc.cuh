@@ -1,5 +1,6 @@
 // seqgemm_tc.cuh -- the layer-list products on the 5th-generation tensor cores (bf16 mode, many tokens):
-//   D[128 weight rows][128 tokens] += W_tile . X_tile^T with tcgen05.mma (kind::f16 on bf16 operands, cta_group::1),
+//   D[128 weight rows][128 tokens] += W_tile . X_tile^T with tcgen05.mma (kind::f16 on bf16 operands, cta_group::1; large products: 256 x 256 on
+//   pairs of CTAs, cta_group::2),
 //   fp32 accumulators in TMEM.  Both operands are K-major bf16 matrices in global memory (weights as stored,
 //   activations as the producing kernels wrote them) and come in by TMA (cp.async.bulk.tensor, SWIZZLE_128B; edges of M,
 //   N and K are zero-filled by the copy).  One lane issues the copies, one lane the MMAs, completion flows through
@@ -10,8 +11,10 @@
 // is released and the host reports the code after the step.
 #pragma once
 
+#include <algorithm>
 #include <map>
 #include <tuple>
+#include <type_traits>
 
 #include "seqkernels.cuh"
 #include "tc05.cuh"
@@ -39,85 +42,101 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
 // as a loop and unrolled: factors per row, all products of a Sopepel step of 2048 / 700 tokens 1194 / 763 and 1286 / 823 us; capped logits, of
 // a Tabisun step with 512 tokens' logits 838 and 852 us.
 // All products of a 2048-token step with attention and two linear attentions: 1735 us with residual additions, decays and squared rectifiers in the
-// unrolled TG_ANY, 743 in instances of their own.
+// unrolled TG_ANY, 743 in instances of their own, 652 without conditions per element, 545 with the large ones on pairs of CTAs (below).
 #define TG_ANY (-1)
 #define TG_ACT_GATE 100 // EPI_ACT times sigmoid(gate)
+// Tokens [c0, c1) of the tile.  A run of 32 tokens that are all there, for 32 rows that are all there, takes a path without a condition per element: with
+// them a warp stored one token in a hundred cycles, and a 256 x 256 tile's epilogue took as long as its products (K = 2048).
 template <int E>
-__device__ __forceinline__ void tg_epilogue(const GemmArgs& a, int z, const GemmRows& gr, int n0, int m, int lane, uint32_t tmem) {
-	const int rows = min(TG_BN, gr.count - n0);
+__device__ __forceinline__ void tg_epilogue(const GemmArgs& a, int z, const GemmRows& gr, int n0, int c0, int c1, int m, int lane, uint32_t tmem) {
+	const int rows = min(c1, gr.count - n0);
 	const bool live = m < a.M;
 	const float bias = E != TG_ANY && a.bias && live ? ldf(a.bias + (size_t)z * a.M + m) : 0.f;
 	const float scale = a.out_scale != 0.f ? a.out_scale : 1.f;
 	const bool aside = E == EPI_F32 && a.split > 0 && m >= a.split; // this weight row's results go to Y2
 	const bool f32 = (E == EPI_F32 && !aside) || E == EPI_DECAY;    // fp32 results
+	const bool alike = __all_sync(0xffffffffu, live) && (E != EPI_F32 || __all_sync(0xffffffffu, aside) || !__any_sync(0xffffffffu, aside));
 	const long ld = aside ? a.ldy2 : a.ldy;
 	const size_t o = aside ? (size_t)(gr.base + n0) * a.ldy2 + (m - a.split) : (size_t)z * a.ybs + (size_t)(gr.base + n0) * a.ldy + (E == EPI_GLU ? m >> 1 : m);
 	float* const yf = (float*)a.Y + o;
 	bf16* const yb = (bf16*)(aside ? a.Y2 : a.Y) + o;
-	const float* gate = E == TG_ACT_GATE ? a.gate + (size_t)z * a.gbs + (size_t)(gr.base + n0) * a.ldgate + m : nullptr; // advances with the row pointer
-	const size_t gstep = E == TG_ACT_GATE ? a.ldgate : 0;
-	for (int c0 = 0; c0 < rows; c0 += 32) {
+	const float* const gate = E == TG_ACT_GATE ? a.gate + (size_t)z * a.gbs + (size_t)(gr.base + n0) * a.ldgate + m : nullptr;
+	for (; c0 < rows; c0 += 32) {
 		float v[32];
 		tmem_ld32(tmem + c0, v);
 		if constexpr (E == TG_ANY) {
 #pragma unroll 1
 			for (int j = 0; j < 32; ++j) gemm_store<bf16>(a, z, gr, n0 + c0 + j, m, v[j]); // lanes = consecutive weight rows: coalesced
-		} else if constexpr (E == EPI_RES || E == EPI_DYT_RES) {
-			const int left = live ? rows - c0 : 0;
-			float* p = yf + (size_t)c0 * ld;
-			const float* rp = E == EPI_RES && a.res ? a.res + o + (size_t)c0 * ld : nullptr;
-			const float na = E == EPI_DYT_RES ? ldf(a.na) : 0.f, nw = E == EPI_DYT_RES && live ? ldf(a.nw + m) : 0.f, nb = E == EPI_DYT_RES && live ? ldf(a.nb + m) : 0.f;
+			continue;
+		}
+		auto run = [&](auto whole) { // whole: all 32 tokens and rows are there
+			constexpr bool W = decltype(whole)::value;
+			const int left = W ? 32 : live ? rows - c0 : 0; // of this row's tokens
+			if constexpr (E == EPI_RES || E == EPI_DYT_RES) {
+				float* p = yf + (size_t)c0 * ld;
+				const float* rp = E == EPI_RES && a.res ? a.res + o + (size_t)c0 * ld : nullptr;
+				const float na = E == EPI_DYT_RES ? ldf(a.na) : 0.f, nw = E == EPI_DYT_RES && live ? ldf(a.nw + m) : 0.f, nb = E == EPI_DYT_RES && live ? ldf(a.nb + m) : 0.f;
+				constexpr int B = W ? 32 : 16; // loads ahead of the stores
 #pragma unroll
-			for (int j0 = 0; j0 < 32; j0 += 16) {
-				float y[16], r[16];
-				float* py = p;
+				for (int j0 = 0; j0 < 32; j0 += B) {
+					float y[B], r[B];
+					float* py = p;
 #pragma unroll
-				for (int i = 0; i < 16; ++i, py += ld) y[i] = j0 + i < left ? *py : 0.f;
-				if (rp) {
+					for (int i = 0; i < B; ++i, py += ld) y[i] = j0 + i < left ? *py : 0.f;
+					if (rp) {
 #pragma unroll
-					for (int i = 0; i < 16; ++i, rp += ld) r[i] = j0 + i < left ? *rp : 0.f;
-				}
+						for (int i = 0; i < B; ++i, rp += ld) r[i] = j0 + i < left ? *rp : 0.f;
+					}
 #pragma unroll
-				for (int i = 0; i < 16; ++i, p += ld) {
-					const float x = (v[j0 + i] + bias) * scale;
-					if (j0 + i < left) *p = y[i] + (E == EPI_DYT_RES ? tanhf(na * x) * nw + nb : rp ? r[i] + x : x);
-				}
-			}
-		} else {
-			const int left = rows - c0;
-			// the row pointer advances by one addition per token: 32 separate row offsets would cost the kernel its second CTA per SM
-			unsigned char* q = (unsigned char*)(f32 ? (void*)yf : (void*)yb) + (size_t)c0 * ld * (f32 ? 4 : 2);
-			const size_t step = (size_t)ld * (f32 ? 4 : 2);
-			if constexpr (E == EPI_GLU) { // lanes 2c (gate) and 2c + 1 (up) share the unit's tokens: the even lane forms token j, the odd one token j + 1
-				const int odd = lane & 1;
-				q += odd ? step : 0;
-#pragma unroll
-				for (int j = 0; j < 32; j += 2, q += 2 * step) {
-					const float x0 = v[j] + bias, x1 = v[j + 1] + bias;
-					const float other = __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1);
-					if (j + odd < left && live) *(bf16*)q = __float2bfloat16_rn(glu_unit(odd ? other : x0, odd ? x1 : other, a.glu_limit, a.glu_mode));
-				}
-			} else {
-#pragma unroll
-				for (int j = 0; j < 32; ++j, q += step, gate += gstep) {
-					const float x = (v[j] + bias) * scale;
-					if (j >= left || !live) continue;
-					const float pos = fmaxf(x, 0.f);
-					if constexpr (E == EPI_F32) {
-						if (aside) *(bf16*)q = __float2bfloat16_rn(a.split_act ? x : pos * pos);
-						else *(float*)q = x;
-					} else if constexpr (E == EPI_DECAY) *(float*)q = expf(-softplusf_(-x) * a.epi_f);
-					else if constexpr (E == EPI_ACT_RELU2) *(bf16*)q = __float2bfloat16_rn(pos * pos);
-					else if constexpr (E == EPI_ACT) *(bf16*)q = __float2bfloat16_rn(x);
-					else if constexpr (E == TG_ACT_GATE) *(bf16*)q = __float2bfloat16_rn(x * sigmoidf_(*gate));
-					else {
-						const bf16 h = __float2bfloat16_rn(x);
-						bf16* d = (bf16*)q;
-						d[0] = h, d[a.split3] = h, d[2 * a.split3] = __float2bfloat16_rn(x - __bfloat162float(h));
+					for (int i = 0; i < B; ++i, p += ld) {
+						const float x = (v[j0 + i] + bias) * scale;
+						if (j0 + i < left) *p = y[i] + (E == EPI_DYT_RES ? tanhf(na * x) * nw + nb : rp ? r[i] + x : x);
 					}
 				}
+			} else if constexpr (E == EPI_GLU) { // lanes 2c (gate) and 2c + 1 (up) share the unit's tokens: the even lane forms token j, the odd one token j + 1
+				const int odd = lane & 1;
+				bf16* q = yb + (size_t)(c0 + odd) * ld;
+#pragma unroll
+				for (int j = 0; j < 32; j += 2, q += 2 * ld) {
+					const float x0 = v[j] + bias, x1 = v[j + 1] + bias;
+					const float other = __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1);
+					if (j + odd < left) *q = __float2bfloat16_rn(glu_unit(odd ? other : x0, odd ? x1 : other, a.glu_limit, a.glu_mode));
+				}
+			} else {
+				// the row pointers advance by one addition per token: 32 separate row offsets would cost k_seq_gemm_tc its second CTA per SM
+				auto each = [&](auto* q, long step, auto&& store) { // store(where, value, token)
+#pragma unroll
+					for (int j = 0; j < 32; ++j, q += step)
+						if (j < left) store(q, (v[j] + bias) * scale, j);
+				};
+				float* const qf = yf + (size_t)c0 * ld;
+				bf16* const qb = yb + (size_t)c0 * ld;
+				auto square = [](float x) { // of the positive part
+					const float pos = fmaxf(x, 0.f);
+					return pos * pos;
+				};
+				if constexpr (E == EPI_F32) {
+					if (!aside) each(qf, ld, [&](float* q, float x, int) { *q = x; });
+					else if (a.split_act) each(qb, ld, [&](bf16* q, float x, int) { *q = __float2bfloat16_rn(x); });
+					else each(qb, ld, [&](bf16* q, float x, int) { *q = __float2bfloat16_rn(square(x)); });
+				} else if constexpr (E == EPI_DECAY) each(qf, ld, [&](float* q, float x, int) { *q = expf(-softplusf_(-x) * a.epi_f); });
+				else if constexpr (E == EPI_ACT_RELU2) each(qb, ld, [&](bf16* q, float x, int) { *q = __float2bfloat16_rn(square(x)); });
+				else if constexpr (E == EPI_ACT) each(qb, ld, [&](bf16* q, float x, int) { *q = __float2bfloat16_rn(x); });
+				else if constexpr (E == TG_ACT_GATE) {
+					const float* g = gate + (size_t)c0 * a.ldgate;
+					float gv[32];
+#pragma unroll
+					for (int j = 0; j < 32; ++j, g += a.ldgate) gv[j] = j < left ? *g : 0.f;
+					each(qb, ld, [&](bf16* q, float x, int j) { *q = __float2bfloat16_rn(x * sigmoidf_(gv[j])); });
+				} else
+					each(qb, ld, [&](bf16* q, float x, int) {
+						const bf16 h = __float2bfloat16_rn(x);
+						q[0] = h, q[a.split3] = h, q[2 * a.split3] = __float2bfloat16_rn(x - __bfloat162float(h));
+					});
 			}
-		}
+		};
+		if (alike && rows - c0 >= 32) run(std::true_type{});
+		else run(std::false_type{});
 	}
 }
 // which instance serves a product
@@ -205,7 +224,7 @@ __global__ void __launch_bounds__(TG_THREADS, 2) k_seq_gemm_tc(const __grid_cons
 		tc_fence_after();
 		if (ok) {
 			const int q4 = warp & 3; // the TMEM lane quarter this warp may read
-			tg_epilogue<E>(a, z, gr, n0, m0 + q4 * 32 + lane, lane, tmem_base + ((uint32_t)(q4 * 32) << 16));
+			tg_epilogue<E>(a, z, gr, n0, 0, TG_BN, m0 + q4 * 32 + lane, lane, tmem_base + ((uint32_t)(q4 * 32) << 16));
 		}
 		tc_fence_before();
 	}
@@ -222,6 +241,129 @@ __global__ void __launch_bounds__(TG_THREADS, 2) k_seq_gemm_tc(const __grid_cons
 	}
 }
 
+// The same product with tiles of 256 weight rows x 256 tokens on pairs of CTAs (cta_group::2), persistent.  A 128 x 128 tile asks L2 for 32 KB per 64-deep
+// step, 256 cycles of the tensor core; here a CTA asks for its 128 weight rows and half of the tokens, the same 32 KB, in 512.  Roles as above, and
+// two accumulators of 256 columns, so that a tile's epilogue runs under the next tile's products.  A step takes 580 cycles where the tensor core
+// needs 512; a tile's epilogue 4300 (fp32 results) to 20000 (two addends from memory), read by eight warps.  13888 x 2048 rows and K, 2048 tokens: 83 us (1410 TFLOP/s),
+// 118 with tiles of 128.
+#define TP_BM 256
+#define TP_BN 256
+#define TP_STAGES 6
+#define TP_STAGE_BYTES (2 * 128 * TG_BK * 2) // per CTA
+#define TP_THREADS 320 // a copying and a multiplying warp, eight that read results
+#define TP_SMEM (TP_STAGES * TP_STAGE_BYTES + 1024)
+template <int E>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1) k_seq_gemm_pair(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const GemmArgs a, int* err) {
+	extern __shared__ unsigned char smem_dyn[];
+	__shared__ __align__(8) uint64_t full[TP_STAGES], empty[TP_STAGES], acc_full[2], acc_empty[2]; // full, acc_empty: rank 0's are used
+	__shared__ uint32_t tmem_base_s;
+	__shared__ int asked[2], multiplied_s; // rank 0: stages that each CTA's copies got to, stages multiplied (read when a wait has given up)
+	unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
+	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = (int)cluster_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+	const int nkb = (a.K + TG_BK - 1) / TG_BK, tok_tiles = (a.N + TP_BN - 1) / TP_BN, tiles = (a.M + TP_BM - 1) / TP_BM * tok_tiles;
+	auto a_tile = [&](int s) { return smem + (size_t)s * TP_STAGE_BYTES; };
+	auto b_tile = [&](int s) { return smem + (size_t)s * TP_STAGE_BYTES + TP_STAGE_BYTES / 2; };
+	// tokens of a tile that the MMAs run over: whole tiles, or what is left in steps of 32
+	auto width = [&](int n0) { return min(TP_BN, (a.N - n0 + 31) & ~31); };
+	pdl_launch_next();
+	if (tid == 0) {
+		for (int s = 0; s < TP_STAGES; ++s) mbar_init(&full[s], 1), mbar_init(&empty[s], 1);
+		for (int s = 0; s < 2; ++s) mbar_init(&acc_full[s], 1), mbar_init(&acc_empty[s], 16);
+		asked[0] = asked[1] = multiplied_s = 0;
+		mbar_init_fence();
+	}
+	if (warp == 1) pair_tmem_alloc(&tmem_base_s, 512);
+	tc_fence_before();
+	cluster_sync(); // the other CTA's barriers are there too
+	tc_fence_after();
+	const uint32_t tmem_base = tmem_base_s;
+	bool ok = true;
+	pdl_wait_prev();
+	if (warp == 0) {
+		int it = 0;
+		for (int t = pair; t < tiles && ok; t += pairs) {
+			const int m0 = t / tok_tiles * TP_BM + rank * 128, n0 = t % tok_tiles * TP_BN, n1 = n0 + rank * (width(n0) / 2);
+			for (int kb = 0; kb < nkb; ++kb, ++it) {
+				const int s = it % TP_STAGES;
+				ok = mbar_wait_warp(&empty[s], ((it / TP_STAGES) & 1) ^ 1);
+				if (!ok) break;
+				if (elect_one()) {
+					const uint32_t bar = cluster_addr(&full[s], 0);
+					if (rank == 0) mbar_expect_tx(&full[s], 2 * TP_STAGE_BYTES);
+					pair_tma_load_2d(a_tile(s), &tm_w, kb * TG_BK, m0, bar);
+					pair_tma_load_2d(b_tile(s), &tm_x, kb * TG_BK, n1, bar);
+				}
+				__syncwarp();
+			}
+		}
+		if (lane == 0) {
+			if (!ok) atomicExch(err, 1);
+			asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(&asked[rank], 0)), "r"(it) : "memory");
+		}
+		// the stages' last releases arrive in this CTA: they do before it ends
+		for (int i = max(0, it - TP_STAGES); i < it && ok; ++i) ok = mbar_wait_warp(&empty[i % TP_STAGES], (i / TP_STAGES) & 1);
+	} else if (warp == 1) {
+		if (rank == 0) {
+			int it = 0, n = 0;
+			for (int t = pair; t < tiles && ok; t += pairs, ++n) {
+				const int buf = n & 1;
+				const uint32_t d = tmem_base + buf * 256, idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(width(t % tok_tiles * TP_BN) >> 3) << 17) | ((uint32_t)(TP_BM >> 4) << 24);
+				ok = mbar_wait_warp(&acc_empty[buf], ((n >> 1) & 1) ^ 1);
+				tc_fence_after();
+				for (int kb = 0; kb < nkb && ok; ++kb, ++it) {
+					const int s = it % TP_STAGES;
+					ok = mbar_wait_warp(&full[s], (it / TP_STAGES) & 1);
+					if (!ok) break;
+					if (elect_one()) {
+						const uint64_t da = umma_desc_sw128(a_tile(s)), db = umma_desc_sw128(b_tile(s));
+#pragma unroll
+						for (int k = 0; k < TG_BK / 16; ++k) pair_umma_f16(d, da + 2 * k, db + 2 * k, idesc, (kb | k) ? 1u : 0u);
+						pair_umma_commit(&empty[s]);
+						if (kb + 1 == nkb) pair_umma_commit(&acc_full[buf]);
+					}
+					__syncwarp();
+				}
+			}
+			if (!ok && lane == 0) atomicExch(err, 2);
+			if (lane == 0) multiplied_s = it;
+		}
+	} else {
+		const int q4 = warp & 3, half = (warp - 2) / 4 * (TP_BN / 2); // the TMEM lane quarter this warp may read, and its half of the tokens
+		const GemmRows gr = gemm_rows(a, 0);
+		int n = 0;
+		for (int t = pair; t < tiles; t += pairs, ++n) {
+			const int buf = n & 1, m0 = t / tok_tiles * TP_BM + rank * 128, n0 = t % tok_tiles * TP_BN;
+			if constexpr (E == EPI_RES || E == EPI_DYT_RES) // what the tile's results are added to travels to L2 while they are formed (the 11 products of a 2048-token step 550 -> 545 us)
+				for (int i = n0 + half + lane; i < min(n0 + half + TP_BN / 2, a.N) && m0 + q4 * 32 < a.M; i += 32) {
+					asm volatile("prefetch.global.L2 [%0];" ::"l"((const float*)a.Y + (size_t)i * a.ldy + m0 + q4 * 32));
+					if (E == EPI_RES && a.res) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.res + (size_t)i * a.ldy + m0 + q4 * 32));
+				}
+			ok = mbar_wait_warp(&acc_full[buf], (n >> 1) & 1);
+			if (!ok) break;
+			tc_fence_after();
+			tg_epilogue<E>(a, 0, gr, n0, half, half + TP_BN / 2, m0 + q4 * 32 + lane, lane, tmem_base + buf * 256 + ((uint32_t)(q4 * 32) << 16));
+			tc_fence_before();
+			__syncwarp();
+			if (lane == 0) mbar_arrive_cluster(cluster_addr(&acc_empty[buf], 0));
+		}
+		if (!ok && lane == 0) atomicExch(err, 3);
+	}
+	const int gave_up = __syncthreads_or(!ok);
+	cluster_sync();
+	// a wait gave up: copies that are on their way end before the CTAs do (a stage that one CTA alone asked for never fills: that wait runs out), and
+	// so do the MMAs on the stages multiplied last
+	if (rank == 0 && gave_up && tid == 0) {
+		const int most = max(asked[0], asked[1]);
+		for (int i = max(0, most - TP_STAGES); i < most; ++i) mbar_wait_bounded(&full[i % TP_STAGES], (i / TP_STAGES) & 1, MBAR_SPINS / 16);
+		for (int i = max(0, multiplied_s - TP_STAGES); i < multiplied_s; ++i) mbar_wait_bounded(&empty[i % TP_STAGES], (i / TP_STAGES) & 1, MBAR_SPINS / 16);
+	}
+	cluster_sync();
+	if (warp == 1) {
+		tc_fence_after();
+		pair_tmem_dealloc(tmem_base, 512);
+	}
+}
+
 // ---------------------------------------------------------------- host side
 typedef CUresult (*TgEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                                CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -229,9 +371,17 @@ struct TgState {
 	TgEncodeFn encode = nullptr;
 	int* err_host = nullptr; // pinned + mapped
 	int* err_dev = nullptr;
+	int pairs = 0; // clusters of two CTAs that the device holds at a time
 	std::map<std::tuple<const void*, long, long, long, long, int>, CUtensorMap> maps;
 };
 static TgState g_tg;
+// f(instance) for every instance of the kernels
+template <typename F>
+static inline void tg_each(F&& f) {
+	f(std::integral_constant<int, TG_ANY>{}), f(std::integral_constant<int, EPI_F32>{}), f(std::integral_constant<int, EPI_ACT>{}), f(std::integral_constant<int, EPI_SPLIT3>{});
+	f(std::integral_constant<int, EPI_GLU>{}), f(std::integral_constant<int, TG_ACT_GATE>{}), f(std::integral_constant<int, EPI_RES>{}), f(std::integral_constant<int, EPI_DYT_RES>{});
+	f(std::integral_constant<int, EPI_ACT_RELU2>{}), f(std::integral_constant<int, EPI_DECAY>{});
+}
 
 static inline void gemm_tc_setup() {
 	if (g_tg.encode) return;
@@ -243,9 +393,14 @@ static inline void gemm_tc_setup() {
 	CUDA_CHECK(cudaHostAlloc((void**)&g_tg.err_host, sizeof(int), cudaHostAllocMapped));
 	*g_tg.err_host = 0;
 	CUDA_CHECK(cudaHostGetDevicePointer((void**)&g_tg.err_dev, g_tg.err_host, 0));
-	for (auto k : {k_seq_gemm_tc<TG_ANY>, k_seq_gemm_tc<EPI_F32>, k_seq_gemm_tc<EPI_ACT>, k_seq_gemm_tc<EPI_SPLIT3>, k_seq_gemm_tc<EPI_GLU>, k_seq_gemm_tc<TG_ACT_GATE>, k_seq_gemm_tc<EPI_RES>,
-	               k_seq_gemm_tc<EPI_DYT_RES>, k_seq_gemm_tc<EPI_ACT_RELU2>, k_seq_gemm_tc<EPI_DECAY>})
-		CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TG_SMEM));
+	tg_each([&](auto e) {
+		constexpr int E = decltype(e)::value;
+		CUDA_CHECK(cudaFuncSetAttribute(k_seq_gemm_tc<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, TG_SMEM));
+		CUDA_CHECK(cudaFuncSetAttribute(k_seq_gemm_pair<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM));
+	});
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3(2 * 74), cfg.blockDim = dim3(TP_THREADS), cfg.dynamicSmemBytes = TP_SMEM;
+	CUDA_CHECK(cudaOccupancyMaxActiveClusters(&g_tg.pairs, k_seq_gemm_pair<EPI_F32>, &cfg));
 }
 // a stalled pipeline leaves its code here; read after the stream has been synchronised
 static inline int gemm_tc_error() { return g_tg.err_host ? *g_tg.err_host : 0; }
@@ -279,29 +434,35 @@ static inline bool gemm_tc_maps(const GemmArgs& a, int batch, const CUtensorMap*
 	mx = tg_map(a.X, a.seg ? a.x_rows : a.N, a.K, a.ldx, a.xbs, batch, TG_BN);
 	return mw && mx;
 }
+// Products that run on pairs of CTAs, by estimated cycles: a 64-deep step takes a 256 x 256 tile 590 and a 128 x 128 tile 900 (two CTAs to an SM, or one), and
+// larger tiles bring 9000 more of launch, first loads and epilogue.  K = 2048, us with tiles of 128 / on pairs: 13888 rows, 2048 tokens 118 / 83; 700 tokens
+// 58 / 43; 6400 rows, 640 tokens 22.6 / 29.8 (75 tiles on 74 pairs), 2048 rows 20.1 / 20.0; K = 64: 20.3 / 21.3; K = 512: 7.4 / 9.1; K = 1024, 5632 rows, 640 tokens
+// 14.3 / 15.2, 1000 tokens 23.5 / 21.6.
+static inline bool tg_pairs(const GemmArgs& a, int batch) {
+	if (batch > 1 || a.seg || a.band_mode || g_tg.pairs < 1) return false;
+	const long steps = (a.K + TG_BK - 1) / TG_BK, slots = 4 * g_tg.pairs; // CTAs of the smaller tiles at a time
+	const long small = (long)((a.M + TG_BM - 1) / TG_BM) * ((a.N + TG_BN - 1) / TG_BN), large = (long)((a.M + TP_BM - 1) / TP_BM) * ((a.N + TP_BN - 1) / TP_BN);
+	return (large + g_tg.pairs - 1) / g_tg.pairs * steps * 590 + 9000 < (small + slots - 1) / slots * steps * 900;
+}
 // false: nothing was launched
 static inline bool gemm_tc_launch(const GemmArgs& a, int batch, cudaStream_t stream, bool pdl) {
 	const CUtensorMap *mw, *mx;
 	if (!gemm_tc_maps(a, batch, mw, mx)) return false;
-	const dim3 grid((a.M + TG_BM - 1) / TG_BM, (a.N + TG_BN - 1) / TG_BN, batch);
+	const bool pair = tg_pairs(a, batch);
+	const long tiles = (long)((a.M + TP_BM - 1) / TP_BM) * ((a.N + TP_BN - 1) / TP_BN);
 	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = grid, cfg.blockDim = dim3(TG_THREADS), cfg.dynamicSmemBytes = TG_SMEM, cfg.stream = stream;
+	cfg.gridDim = pair ? dim3(2 * (int)std::min<long>(tiles, g_tg.pairs)) : dim3((a.M + TG_BM - 1) / TG_BM, (a.N + TG_BN - 1) / TG_BN, batch);
+	cfg.blockDim = dim3(pair ? TP_THREADS : TG_THREADS), cfg.dynamicSmemBytes = pair ? TP_SMEM : TG_SMEM, cfg.stream = stream;
 	cudaLaunchAttribute at[1];
 	at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
 	at[0].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = at, cfg.numAttrs = pdl ? 1 : 0;
-	auto go = [&](auto kernel) { CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, *mw, *mx, a, (int)(a.wbs != 0 && batch > 1), (int)(a.xbs != 0 && batch > 1), g_tg.err_dev)); };
-	switch (tg_kind(a)) {
-	case EPI_F32: go(k_seq_gemm_tc<EPI_F32>); break;
-	case EPI_ACT: go(k_seq_gemm_tc<EPI_ACT>); break;
-	case EPI_SPLIT3: go(k_seq_gemm_tc<EPI_SPLIT3>); break;
-	case EPI_GLU: go(k_seq_gemm_tc<EPI_GLU>); break;
-	case EPI_RES: go(k_seq_gemm_tc<EPI_RES>); break;
-	case EPI_DYT_RES: go(k_seq_gemm_tc<EPI_DYT_RES>); break;
-	case EPI_ACT_RELU2: go(k_seq_gemm_tc<EPI_ACT_RELU2>); break;
-	case EPI_DECAY: go(k_seq_gemm_tc<EPI_DECAY>); break;
-	case TG_ACT_GATE: go(k_seq_gemm_tc<TG_ACT_GATE>); break;
-	default: go(k_seq_gemm_tc<TG_ANY>);
-	}
+	const int kind = tg_kind(a);
+	tg_each([&](auto e) {
+		constexpr int E = decltype(e)::value;
+		if (E != kind) return;
+		if (pair) CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_seq_gemm_pair<E>, *mw, *mx, a, g_tg.err_dev));
+		else CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_seq_gemm_tc<E>, *mw, *mx, a, (int)(a.wbs != 0 && batch > 1), (int)(a.xbs != 0 && batch > 1), g_tg.err_dev));
+	});
 	return true;
 }

@@ -82,3 +82,55 @@ __device__ __forceinline__ void ldsm_x4(const void* p, uint32_t (&r)[4]) {
 __device__ __forceinline__ void ldsm_x4_t(const void* p, uint32_t (&r)[4]) {
 	asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
 }
+__device__ __forceinline__ bool elect_one() { // one lane of a converged warp
+	uint32_t p;
+	asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+	return p != 0;
+}
+
+// ---------------------------------------------------------------- two CTAs of a cluster on one tile (cta_group::2)
+// Both hold their own 128 rows of A and half of B's rows at the same offsets of their shared memory; rank 0 issues the MMAs, and each finds its 128 rows of D
+// in its own TMEM.
+__device__ __forceinline__ uint32_t cluster_rank() {
+	uint32_t r;
+	asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+	return r;
+}
+__device__ __forceinline__ void cluster_sync() { // every thread of both CTAs, warps converged
+	__syncwarp();
+	asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the same variable in the shared memory of CTA `rank`
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+	uint32_t a;
+	asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+	return a;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) { // a barrier named by cluster_addr
+	asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void pair_tmem_alloc(uint32_t* smem_dst, uint32_t ncols) { // one whole warp of each CTA
+	asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols) : "memory");
+	asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void pair_tmem_dealloc(uint32_t taddr, uint32_t ncols) { // the allocating warps
+	asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+// into this CTA's shared memory; the bytes count on a barrier of either CTA (cluster_addr)
+__device__ __forceinline__ void pair_tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+	asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)), "l"(map),
+	             "r"(c0), "r"(c1), "r"(bar)
+	             : "memory");
+}
+__device__ __forceinline__ void pair_umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) { // rank 0, one thread
+	asm volatile(
+	    "{\n\t.reg .pred p;\n\t"
+	    "setp.ne.b32 p, %4, 0;\n\t"
+	    "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+	    ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+	    : "memory");
+}
+// all MMAs issued so far by this thread arrive on `bar` of both CTAs when they have completed
+__device__ __forceinline__ void pair_umma_commit(uint64_t* bar) {
+	asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
