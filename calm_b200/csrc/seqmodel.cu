@@ -1335,12 +1335,20 @@ void forward(Seq& s, const SeqBatch& sb, int n_want, double kv_rows, int longest
 	const bool post = m.block == SEQ_BLOCK_POST; // the first sublayer reads the embedding rows themselves
 	run_kernel(s, KD_EMBED, (double)N * m.width * (2.0 + (m.pos_table ? 2.0 : 0.0) + (m.bigram ? 2.0 : 0.0) + 4.0 * s.streams + (looped || s.depth ? 4.0 : 0.0) + (post ? act_size(s) : 0.0)), 0,
 	           [&] {
-		           auto go = [&](auto* act, auto kernel) {
-			           launch_k(s, kernel, N, 128, 0, s.x, looped ? s.x0 : s.depth ? s.hist : nullptr, act, (const bf16*)m.embed, s.d_tok, N, m.width, m.embed_scale != 0.f ? m.embed_scale : 1.f, (const bf16*)m.pos_table,
+		           // rows of 16-byte pieces, on bases that a caller's tables need not have
+		           auto at16 = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
+		           const bool wide = m.width % 8 == 0 && at16(m.embed) && at16(m.pos_table) && at16(m.bigram);
+		           auto go = [&](auto* act, auto kernel, int V) {
+			           launch_k(s, kernel, N, std::min(256, cdiv(m.width / V, 32) * 32), 0, s.x, looped ? s.x0 : s.depth ? s.hist : nullptr, act, (const bf16*)m.embed, s.d_tok, N, m.width, m.embed_scale != 0.f ? m.embed_scale : 1.f, (const bf16*)m.pos_table,
 			                    s.d_tpos, s.streams, EmbedBigram{(const bf16*)m.bigram, s.d_tprev, m.bigram_buckets, m.bigram_mul_prev, m.bigram_mul_cur});
 		           };
-		           if (m.exact) go(post ? (float*)s.hA : nullptr, k_seq_embed<float>);
-		           else go(post ? (bf16*)s.hA : nullptr, k_seq_embed<bf16>);
+		           auto with = [&](auto* act) {
+			           typedef std::remove_pointer_t<decltype(act)> AT;
+			           if (wide) go(act, k_seq_embed<AT, 8>, 8);
+			           else go(act, k_seq_embed<AT, 1>, 1);
+		           };
+		           if (m.exact) with(post ? (float*)s.hA : nullptr);
+		           else with(post ? (bf16*)s.hA : nullptr);
 	           });
 	s.h_ready = false;
 	for (size_t ri = 0; ri < s.runs.size(); ++ri) {
@@ -1740,7 +1748,7 @@ extern "C" int calm_b200_seq_step(void* handle, int n_seq, const int* slots, con
 extern "C" void calm_b200_seq_argmax(void* handle, int* out) {
 	Seq& s = *(Seq*)handle;
 	if (!s.last_want) return;
-	launch_k(s, k_seq_argmax, s.last_want, 256, 0, s.logits, s.m.vocab, s.d_argmax);
+	launch_k(s, k_seq_argmax, s.last_want, 1024, 0, s.logits, s.m.vocab, s.d_argmax);
 	CUDA_CHECK(cudaGetLastError());
 	++g_seq_launches;
 	CUDA_CHECK(cudaMemcpyAsync(out, s.d_argmax, s.last_want * sizeof(int), cudaMemcpyDeviceToHost, s.stream));
