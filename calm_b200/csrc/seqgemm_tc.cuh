@@ -76,6 +76,9 @@ __device__ __forceinline__ void tg_epilogue(const GemmArgs& a, int z, const Gemm
 				float* p = yf + (size_t)c0 * ld;
 				const float* rp = E == EPI_RES && a.res ? a.res + o + (size_t)c0 * ld : nullptr;
 				const float na = E == EPI_DYT_RES ? ldf(a.na) : 0.f, nw = E == EPI_DYT_RES && live ? ldf(a.nw + m) : 0.f, nb = E == EPI_DYT_RES && live ? ldf(a.nb + m) : 0.f;
+				const bool next = E == EPI_DYT_RES && a.xw;
+				const float xa = next ? ldf(a.xa) : 0.f, xw = next && live ? ldf(a.xw + m) : 0.f, xb = next && live ? ldf(a.xb + m) : 0.f;
+				bf16* px = next ? (bf16*)a.Y2 + (size_t)(gr.base + n0 + c0) * a.ldy2 + m : nullptr;
 				constexpr int B = W ? 32 : 16; // loads ahead of the stores
 #pragma unroll
 				for (int j0 = 0; j0 < 32; j0 += B) {
@@ -90,7 +93,12 @@ __device__ __forceinline__ void tg_epilogue(const GemmArgs& a, int z, const Gemm
 #pragma unroll
 					for (int i = 0; i < B; ++i, p += ld) {
 						const float x = (v[j0 + i] + bias) * scale;
-						if (j0 + i < left) *p = y[i] + (E == EPI_DYT_RES ? tanhf(na * x) * nw + nb : rp ? r[i] + x : x);
+						if (j0 + i < left) *p = y[i] += E == EPI_DYT_RES ? tanhf(na * x) * nw + nb : rp ? r[i] + x : x;
+					}
+					if (next) {
+#pragma unroll
+						for (int i = 0; i < B; ++i, px += a.ldy2)
+							if (j0 + i < left) *px = __float2bfloat16_rn(tanhf(xa * y[i]) * xw + xb);
 					}
 				}
 			} else if constexpr (E == EPI_GLU) { // lanes 2c (gate) and 2c + 1 (up) share the unit's tokens: the even lane forms token j, the odd one token j + 1

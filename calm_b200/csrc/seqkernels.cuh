@@ -2808,13 +2808,15 @@ struct GemmArgs {
 	void* Y;
 	long ldy, ybs;
 	int N, M, K;
-	int epi;                 // EPI_F32: Y fp32; EPI_ACT: Y of the activation type; EPI_DYT_RES: Y fp32 residual += tanh(alpha acc) w + b;
+	int epi;                 // EPI_F32: Y fp32; EPI_ACT: Y of the activation type; EPI_DYT_RES: Y fp32 residual += tanh(alpha acc) w + b, and
+	                         // with xw the new value's own Dynamic Tanh norm (xa, xw, xb), the next sublayer's input, to Y2 (activation type);
 	                         // EPI_RES: Y fp32 residual += (res ? res : 0) + acc; EPI_ACT_RELU2: Y of the activation type = relu(acc)^2;
 	                         // EPI_DECAY: Y fp32 = sigmoid(acc)^epi_f = exp(-softplus(-acc) * epi_f);
 	                         // EPI_SPLIT3: Y of the activation type, three columns `split3` apart: hi, hi, lo (value and remainder of its rounding);
 	                         // EPI_GLU: rows of W alternate gate and up, Y[n][m / 2] of the activation type = glu_unit(gate, up)
 	float epi_f;
 	const bf16 *nw, *nb, *na;
+	const bf16 *xw, *xb, *xa;
 	int w_immutable;         // W is a model weight: it may be read before the previous kernel has finished (products of gathered keys set 0)
 	const bf16* bias;        // [batch][M] or null: added to the accumulator first
 	const float* res;        // EPI_RES: a second addend laid out like Y, or null
@@ -2878,7 +2880,11 @@ __device__ __forceinline__ void gemm_store(const GemmArgs& a, int z, const GemmR
 	else if (a.epi == EPI_ACT_RELU2) {
 		const float r = fmaxf(acc, 0.f);
 		((AT*)a.Y)[o] = to_act<AT>(r * r);
-	} else ((float*)a.Y)[o] += tanhf(ldf(a.na) * acc) * ldf(a.nw + m) + ldf(a.nb + m);
+	} else {
+		const float y = ((float*)a.Y)[o] + (tanhf(ldf(a.na) * acc) * ldf(a.nw + m) + ldf(a.nb + m));
+		((float*)a.Y)[o] = y;
+		if (a.xw) ((AT*)a.Y2)[(size_t)(gr.base + n) * a.ldy2 + m] = to_act<AT>(tanhf(ldf(a.xa) * y) * ldf(a.xw + m) + ldf(a.xb + m));
+	}
 }
 
 // EPI_GLU: the pair of columns m (even: gate) and m + 1 (up)

@@ -457,6 +457,7 @@ struct GemmExtra {
 	long rs_ld = 1;
 	int rs_act = 0;
 	int split3 = 0;              // EPI_SPLIT3: columns between the three copies
+	const SeqNorm* next = nullptr; // EPI_DYT_RES: the norm of the sublayer that reads the new rows; its result goes to Y2
 	int glu_mode = 0;            // EPI_GLU
 	float glu_limit = 0.f;
 	const int* x_idx = nullptr;  // grouped product read through an index (gemm_skinny_fits says whether it may be given)
@@ -480,6 +481,7 @@ void gemm(Seq& s, const void* X, long ldx, long xbs, const void* W, long ldw, lo
 	a.w_immutable = w_immutable;
 	a.X = X, a.ldx = ldx, a.xbs = xbs, a.W = (const bf16*)W, a.ldw = ldw, a.wbs = wbs, a.Y = Y, a.ldy = ldy, a.ybs = ybs;
 	a.N = N, a.M = M, a.K = K, a.epi = epi;
+	a.xw = ex->next ? (const bf16*)ex->next->w : nullptr, a.xb = ex->next ? (const bf16*)ex->next->b : nullptr, a.xa = ex->next ? (const bf16*)ex->next->alpha : nullptr;
 	a.nw = nrm ? (const bf16*)nrm->w : nullptr, a.nb = nrm ? (const bf16*)nrm->b : nullptr, a.na = nrm ? (const bf16*)nrm->alpha : nullptr;
 	// a grouped product does the work of its x_rows rows, and reads at most that many groups' weights
 	const double rows = ex->seg ? (double)ex->x_rows : (double)N * batch, mats = ex->seg ? std::min((double)batch, rows) : (double)batch;
@@ -783,7 +785,7 @@ struct OutEpi {
 	float scale = 0.f; // != 0: factor on the product
 	const SeqHyper* hc = nullptr; // hyper blocks: the routed feed-forward writes the streams itself (its weighted sum is formed in that kernel)
 	const void* next_in = nullptr;      // ... and in the same kernel reads them for the sublayer that follows: its `in` weights and its norm
-	const SeqNorm* next_norm = nullptr;
+	const SeqNorm* next_norm = nullptr; // (serial blocks: the product's epilogue applies it to the new rows)
 	const SeqNorm* post = nullptr;      // post-norm blocks: the norm the routed feed-forward's sum goes through on its way into the stream
 	const Sandwich* sand = nullptr;     // sandwich blocks: how the routed feed-forward's sum goes into the stream (its routed part is filled in there)
 };
@@ -827,6 +829,7 @@ template <typename AT>
 void out_product(Seq& s, const AT* X, const void* Wt, int N, int K, const OutEpi& oe, const void* bias = nullptr) {
 	GemmExtra gx;
 	gx.res = oe.res, gx.out_scale = oe.scale, gx.bias = bias; // the factor applies to product + bias
+	if (oe.epi == EPI_DYT_RES && oe.next_norm) gx.next = oe.next_norm, gx.Y2 = s.hA, gx.ldy2 = s.m.width;
 	gemm(s, X, K, 0, Wt, K, 0, oe.dst, s.m.width, 0, N, s.m.width, K, 1, oe.epi, oe.nrm, -1, true, &gx);
 }
 
@@ -1312,14 +1315,24 @@ void layer_typed(Seq& s, const SeqLayer& L, RunState& r, const SeqBatch& sb, dou
 		s.h_ready = next != nullptr;
 		return;
 	}
-	norm(s, s.hA, s.x, nullptr, L.norm1, N);
 	if (s.m.block == SEQ_BLOCK_SERIAL) {
-		mixer_typed<AT>(s, L, r, sb, kv_rows, longest, OutEpi{EPI_DYT_RES, &L.norm1b, s.x, nullptr});
+		// a Dynamic Tanh norm needs no sum over the row: the product that changes the stream also writes the next sublayer's input (a launch of
+		// its own took 20 us for 2079 rows of 2048, and 2 of a decode step's 45 us a layer)
+		const bool elementwise = s.m.norm_kind == SEQ_NORM_DYT && L.ff_kind != SEQ_FF_MOE;
+		const SeqNorm* after = elementwise && next ? &next->norm1 : nullptr;
+		if (!s.h_ready) norm(s, s.hA, s.x, nullptr, L.norm1, N);
+		OutEpi mix{EPI_DYT_RES, &L.norm1b, s.x, nullptr}, ff{EPI_DYT_RES, &L.norm2b, s.x, nullptr};
+		mix.next_norm = L.ff > 0 ? (elementwise ? &L.norm2 : nullptr) : after, ff.next_norm = after;
+		mixer_typed<AT>(s, L, r, sb, kv_rows, longest, mix);
 		if (L.ff > 0) {
-			norm(s, s.hA, s.x, nullptr, L.norm2, N);
-			feed_forward<AT>(s, L, sb, OutEpi{EPI_DYT_RES, &L.norm2b, s.x, nullptr});
+			if (!mix.next_norm) norm(s, s.hA, s.x, nullptr, L.norm2, N);
+			feed_forward<AT>(s, L, sb, ff);
 		}
-	} else if (L.ff > 0) { // x += mixer(h) + ff(h): the mixer's output waits in `mo` for the feed-forward's last kernel
+		s.h_ready = after != nullptr;
+		return;
+	}
+	norm(s, s.hA, s.x, nullptr, L.norm1, N);
+	if (L.ff > 0) { // x += mixer(h) + ff(h): the mixer's output waits in `mo` for the feed-forward's last kernel
 		mixer_typed<AT>(s, L, r, sb, kv_rows, longest, OutEpi{EPI_F32, nullptr, s.mo, nullptr});
 		feed_forward<AT>(s, L, sb, OutEpi{EPI_RES, nullptr, s.x, s.mo});
 	} else {

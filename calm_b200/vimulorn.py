@@ -104,7 +104,10 @@ def plan(cfg: dict, tensors: Dict[str, torch.Tensor]) -> Tuple[dict, List[dict],
                 raise ValueError(f"layer {i}: feed-forward kind {ml.get('kind')} is not part of this design")
             ff = int(ml["ff"])
             rec.update(ff=ff, limit=float(ml["limit"]), norm2=norm(p + "norm2"), norm2b=norm(p + "norm2b"))
-            rec["w_gate_up"] = stack(p + "mlp.gate_up", [need(p + "mlp.gate", [ff, width]), need(p + "mlp.up", [ff, width])])
+            # alternating rows: the unit is formed in the product's epilogue
+            gate, upr = (up.pop(need(p + "mlp." + n, [ff, width])) for n in ("gate", "up"))
+            up[p + "mlp.gate_up"] = torch.stack([gate, upr], 1).reshape(2 * ff, width).contiguous()
+            rec.update(glu_rows=1, w_gate_up=p + "mlp.gate_up")
             rec["w_down"] = need(p + "mlp.down", [width, ff])
         layers.append(rec)
     lp = cfg.get("loop") or {}

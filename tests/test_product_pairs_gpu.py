@@ -32,7 +32,7 @@ def test_parallel_blocks(n):  # fp32 columns, squared rectifiers and a decay's i
 
 @pytest.mark.parametrize("n", [65, 160, 287])
 def test_dynamic_tanh(n):
-    cfg = tv.config([tv.window(mlp={"ff": 2000, "kind": "dense", "limit": 4.0})], width=2040)
+    cfg = tv.config([tv.window(mlp={"ff": 2000, "kind": "dense", "limit": 4.0}), tv.window(mlp=None)], width=2040)
     t, toks = tv.weights(cfg, 6), tv.tokens(cfg, n)
     with vimulorn.from_tensors(cfg, t, "bfloat16", max_tokens=400, max_seqs=1, page=8) as m:
         got = m.step([m.open()], [toks], list(range(n)))
