@@ -65,11 +65,14 @@ struct Seq {
 	std::vector<int> table; // host mirror of the page table
 	int* table_dev = nullptr;
 
-	// per-step batch description
-	int cap_tokens = 0, cap_seqs = 0, cap_want = 0;
+	// per-step batch description: written into page-locked memory and sent to the device in one copy (eleven small ones from a vector took a decode step
+	// 40 us); the pointers below lead into the device's, packed anew by every step.  A captured step finds them where it did: they follow from its key
+	int cap_tokens = 0, cap_want = 0;
+	int *meta = nullptr, *meta_dev = nullptr;
+	size_t cap_meta = 0;
 	int *d_tok = nullptr, *d_tslot = nullptr, *d_tpos = nullptr, *d_tfirst = nullptr, *d_tprev = nullptr, *d_sstart = nullptr, *d_scount = nullptr, *d_spos0 = nullptr, *d_sslot = nullptr,
-	    *d_want = nullptr, *d_argmax = nullptr;
-	std::vector<int> h_meta;
+	    *d_want = nullptr;
+	int *picks = nullptr, *picks_dev = nullptr; // greedy picks: page-locked memory that the device writes, and its address there
 
 	// workspace for cap_tokens tokens
 	float *x = nullptr, *x0 = nullptr, *proj = nullptr, *f[6] = {};
@@ -378,22 +381,21 @@ void drop_graphs(Seq& s) {
 }
 
 void reserve_tokens(Seq& s, int N, int B, int W) {
-	if (B > s.cap_seqs || N > s.cap_tokens || W > s.cap_want) drop_graphs(s); // captured launches hold the old addresses
-	if (B > s.cap_seqs || N > s.cap_tokens) {
-		const int cn = std::max(N, s.cap_tokens), cb = std::max(B, s.cap_seqs);
+	const size_t meta = (size_t)6 * N + 4 * B + W;
+	if (meta > s.cap_meta || N > s.cap_tokens || W > s.cap_want) drop_graphs(s); // captured launches hold the old addresses
+	if (meta > s.cap_meta) {
 		CUDA_CHECK(cudaStreamSynchronize(s.stream));
-		cudaFree(s.d_tok);
-		s.d_tok = (int*)dalloc(((size_t)6 * cn + 4 * cb) * sizeof(int));
-		s.d_tslot = s.d_tok + cn, s.d_tpos = s.d_tslot + cn, s.d_tfirst = s.d_tpos + cn, s.d_skip = s.d_tfirst + cn, s.d_tprev = s.d_skip + cn;
-		s.d_sstart = s.d_tprev + cn, s.d_scount = s.d_sstart + cb, s.d_spos0 = s.d_scount + cb, s.d_sslot = s.d_spos0 + cb;
-		s.cap_seqs = cb;
+		cudaFree(s.meta_dev), cudaFreeHost(s.meta);
+		s.meta_dev = (int*)dalloc(meta * sizeof(int));
+		CUDA_CHECK(cudaHostAlloc((void**)&s.meta, meta * sizeof(int), cudaHostAllocDefault));
+		s.cap_meta = meta;
 	}
 	if (W > s.cap_want) {
 		CUDA_CHECK(cudaStreamSynchronize(s.stream));
-		cudaFree(s.d_want), cudaFree(s.d_argmax), cudaFree(s.logits), cudaFree(s.hW);
+		cudaFreeHost(s.picks), cudaFree(s.logits), cudaFree(s.hW);
 		s.cap_want = std::max(W, 2 * s.cap_want);
-		s.d_want = (int*)dalloc(s.cap_want * sizeof(int));
-		s.d_argmax = (int*)dalloc(s.cap_want * sizeof(int));
+		CUDA_CHECK(cudaHostAlloc((void**)&s.picks, s.cap_want * sizeof(int), cudaHostAllocMapped));
+		CUDA_CHECK(cudaHostGetDevicePointer((void**)&s.picks_dev, s.picks, 0));
 		s.logits = (float*)dalloc((size_t)s.cap_want * s.m.vocab * sizeof(float));
 		s.hW = dalloc((size_t)s.cap_want * s.m.width * act_size(s));
 	}
@@ -1642,7 +1644,7 @@ extern "C" void calm_b200_seq_release(void* handle) {
 	};
 	for (RunState& r : s->runs) drop(r);
 	cudaFree(s->lin), cudaFree(s->fsh), cudaFree(s->hist), cudaFree(s->carry), cudaFree(s->gla), cudaFree(s->rope_cs);
-	cudaFree(s->table_dev), cudaFree(s->d_tok), cudaFree(s->d_want), cudaFree(s->d_argmax), cudaFree(s->logits), cudaFree(s->hW);
+	cudaFree(s->table_dev), cudaFree(s->meta_dev), cudaFreeHost(s->meta), cudaFreeHost(s->picks), cudaFree(s->logits), cudaFree(s->hW);
 	cudaFree(s->part), cudaFree(s->a3), cudaFree(s->att_kb), cudaFree(s->att_vt), cudaFree(s->att_s), cudaFree(s->att_p), cudaFree(s->x), cudaFree(s->x0), cudaFree(s->proj), cudaFree(s->hA), cudaFree(s->a1), cudaFree(s->a2), cudaFree(s->trace_buf);
 	for (float* p : s->f) cudaFree(p);
 	for (auto& kv : s->rot) cudaFree(kv.second.first);
@@ -1708,9 +1710,12 @@ extern "C" int calm_b200_seq_step(void* handle, int n_seq, const int* slots, con
 	// pages for the new tokens, then the batch description
 	double kv_rows = 0; // cache rows the causal attentions read this step
 	int longest = 0;    // longest sequence after this step
-	s.h_meta.resize((size_t)6 * N + 4 * n_seq);
-	int *tok = s.h_meta.data(), *tslot = tok + N, *tpos = tslot + N, *tfirst = tpos + N, *skip = tfirst + N, *tprev = skip + N, *sstart = tprev + N, *scount = sstart + n_seq, *spos0 = scount + n_seq,
-	    *sslot = spos0 + n_seq;
+	int *tok = s.meta, *tslot = tok + N, *tpos = tslot + N, *tfirst = tpos + N, *skip = tfirst + N, *tprev = skip + N, *sstart = tprev + N, *scount = sstart + n_seq, *spos0 = scount + n_seq,
+	    *sslot = spos0 + n_seq, *wanted = sslot + n_seq;
+	auto on_device = [&](const int* p) { return s.meta_dev + (p - s.meta); };
+	s.d_tok = on_device(tok), s.d_tslot = on_device(tslot), s.d_tpos = on_device(tpos), s.d_tfirst = on_device(tfirst), s.d_skip = on_device(skip), s.d_tprev = on_device(tprev);
+	s.d_sstart = on_device(sstart), s.d_scount = on_device(scount), s.d_spos0 = on_device(spos0), s.d_sslot = on_device(sslot), s.d_want = on_device(wanted);
+	std::copy(want, want + n_want, wanted);
 	int at = 0;
 	s.hb_start.resize(n_seq), s.hb_count.resize(n_seq), s.hb_pos0.resize(n_seq), s.hb_slot.resize(n_seq);
 	s.n_on_products = s.tok_on_products = 0;
@@ -1732,17 +1737,7 @@ extern "C" int calm_b200_seq_step(void* handle, int n_seq, const int* slots, con
 		sl.len += counts[b], sl.last_tok = tokens[at - 1];
 		longest = std::max(longest, sl.len);
 	}
-	CUDA_CHECK(cudaMemcpyAsync(s.d_tok, tok, N * sizeof(int), cudaMemcpyHostToDevice, s.stream));
-	CUDA_CHECK(cudaMemcpyAsync(s.d_tslot, tslot, N * sizeof(int), cudaMemcpyHostToDevice, s.stream));
-	CUDA_CHECK(cudaMemcpyAsync(s.d_tpos, tpos, N * sizeof(int), cudaMemcpyHostToDevice, s.stream));
-	CUDA_CHECK(cudaMemcpyAsync(s.d_tfirst, tfirst, N * sizeof(int), cudaMemcpyHostToDevice, s.stream));
-	CUDA_CHECK(cudaMemcpyAsync(s.d_skip, skip, N * sizeof(int), cudaMemcpyHostToDevice, s.stream));
-	if (m.bigram) CUDA_CHECK(cudaMemcpyAsync(s.d_tprev, tprev, N * sizeof(int), cudaMemcpyHostToDevice, s.stream));
-	CUDA_CHECK(cudaMemcpyAsync(s.d_sstart, sstart, n_seq * sizeof(int), cudaMemcpyHostToDevice, s.stream));
-	CUDA_CHECK(cudaMemcpyAsync(s.d_scount, scount, n_seq * sizeof(int), cudaMemcpyHostToDevice, s.stream));
-	CUDA_CHECK(cudaMemcpyAsync(s.d_spos0, spos0, n_seq * sizeof(int), cudaMemcpyHostToDevice, s.stream));
-	CUDA_CHECK(cudaMemcpyAsync(s.d_sslot, sslot, n_seq * sizeof(int), cudaMemcpyHostToDevice, s.stream));
-	if (n_want) CUDA_CHECK(cudaMemcpyAsync(s.d_want, want, n_want * sizeof(int), cudaMemcpyHostToDevice, s.stream));
+	CUDA_CHECK(cudaMemcpyAsync(s.meta_dev, s.meta, ((size_t)6 * N + 4 * n_seq + n_want) * sizeof(int), cudaMemcpyHostToDevice, s.stream)); // (the step before ended with a synchronisation: its copy is over)
 	SeqBatch sb;
 	sb.tok = s.d_tok, sb.tslot = s.d_tslot, sb.tpos = s.d_tpos, sb.tfirst = s.d_tfirst, sb.sstart = s.d_sstart, sb.scount = s.d_scount, sb.spos0 = s.d_spos0, sb.sslot = s.d_sslot;
 	sb.pages = s.table_dev, sb.N = N, sb.B = n_seq, sb.max_pages = s.max_pages, sb.page = m.page;
@@ -1761,11 +1756,11 @@ extern "C" int calm_b200_seq_step(void* handle, int n_seq, const int* slots, con
 extern "C" void calm_b200_seq_argmax(void* handle, int* out) {
 	Seq& s = *(Seq*)handle;
 	if (!s.last_want) return;
-	launch_k(s, k_seq_argmax, s.last_want, 1024, 0, s.logits, s.m.vocab, s.d_argmax);
+	launch_k(s, k_seq_argmax, s.last_want, 1024, 0, s.logits, s.m.vocab, s.picks_dev);
 	CUDA_CHECK(cudaGetLastError());
 	++g_seq_launches;
-	CUDA_CHECK(cudaMemcpyAsync(out, s.d_argmax, s.last_want * sizeof(int), cudaMemcpyDeviceToHost, s.stream));
 	CUDA_CHECK(cudaStreamSynchronize(s.stream));
+	std::copy(s.picks, s.picks + s.last_want, out);
 }
 extern "C" const float* calm_b200_seq_device_logits(void* handle) { return ((Seq*)handle)->logits; }
 
