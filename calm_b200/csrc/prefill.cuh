@@ -125,10 +125,11 @@ struct PfMaps {
 struct PfGemmArgs {
 	int K, n_tokens;
 	// work items
-	int rows, na, bn, splits; // weight rows; row tiles per item (UP: 2, w1 and w3); tokens per tile (64, 128 or 256, na * bn <= 256); K-slices
+	int rows, na, bn; // weight rows; row tiles per item (UP: 2, w1 and w3); tokens per tile (64, 128 or 256, na * bn <= 256)
+	int tail, splits; // the last `tail` tiles are cut into K-slices, an item each (tail * splits of them, at most one per SM); the others are one item
 	int stages;               // in flight
-	float* ws;            // splits > 1: [item][na][bn][128] partial sums
-	unsigned* counter;    // splits > 1: [row tiles x token tiles], zero between launches
+	float* ws;            // [slice of a tail tile][na][bn][128] partial sums
+	unsigned* counter;    // [tail tile] slices that have arrived, zero between launches
 	int* err;             // mapped host word: code of a wait that gave up
 	unsigned wait_limit;  // tries of a wait before it gives up
 	// QKV epilogue
@@ -166,6 +167,9 @@ __host__ __device__ constexpr size_t pf_fixed_bytes() { // everything but the st
 __host__ __device__ inline size_t pf_stage_bytes(int na, int bn) {
 	return (size_t)na * PF_TILE_BYTES + 2 * bn * 128;
 }
+// Tiles whose accumulators leave room multiply hi and lo as one operand, so that the weight tile is read from shared memory once for both: those reads, the
+// activations', the copies and the widening share its 128 bytes a cycle, which is what bounds a stage (FFN up 14336 x 4096 fp8: 135 tokens 188 -> 150 us, 20 tokens 70 -> 57).
+__host__ __device__ constexpr bool pf_side(int na, int bn) { return na * bn <= 128; }
 template <int DBITS>
 __host__ __device__ constexpr int pf_widen_warps() { // FFN up as above, side by side: fp8 696 us with four warps and 802 with eight (more arrivals per stage), gf4 871 and 825 (19 instructions per 8 weights)
 	return DBITS == 16 ? 0 : DBITS == 8 ? 4 : 8;
@@ -203,53 +207,68 @@ __device__ __forceinline__ void pf_widen(const uint4& raw, uint4* out) {
 }
 
 // What the decode kernels apply, on 32 tokens of one weight row: gr = row (lanes = consecutive rows), t0 = first token, v (v3: FFN up's second matrix) the sums.
+// Values are formed without asking whether their token is there, several at a time, and only the stores ask: a condition around each value kept the
+// values apart (q/k/v of 20 / 135 tokens, 6144 x 4096 fp8: 31 -> 26, 65 -> 50 us).
 template <int MODE>
 __device__ __forceinline__ void pf_epilogue(const PfGemmArgs& a, int gr, int lane, int t0, const float (&v)[32], const float (&v3)[32]) {
+	const int left = a.n_tokens - t0;
 	if constexpr (MODE == PF_QKV) { // bias / clip / RoPE / KV-cache append
 		const bool is_q = gr < a.q_dim, is_k = !is_q && gr < a.q_dim + a.kv_dim; // uniform over a tile: the dims are multiples of 128
 		const int k = is_q ? gr : (is_k ? gr - a.q_dim : gr - a.q_dim - a.kv_dim);
 		const int d = k % a.head_dim, h = k / a.head_dim;
 		const float b = a.bias ? a.bias[gr] : 0.f;
-		const size_t kv0 = ((size_t)h * a.seq_len + a.pos0) * a.head_dim + d;
+		const size_t kv0 = ((size_t)h * a.seq_len + a.pos0 + t0) * a.head_dim + d;
+		void* const cache = is_k ? a.kc : a.vc;
 #pragma unroll
 		for (int j0 = 0; j0 < 32; j0 += 16) { // the angles of 16 tokens at a time, all loads before the first store (one by one they cost a round trip each)
-			float2 cs[16];
+			float x[16];
 #pragma unroll
-			for (int j = 0; j < 16; ++j)
-				cs[j] = (is_q || is_k) && t0 + j0 + j < a.n_tokens ? __ldcg(a.rope + (size_t)(t0 + j0 + j) * (a.head_dim / 2) + (d >> 1)) : make_float2(1.f, 0.f);
+			for (int j = 0; j < 16; ++j) x[j] = fminf(fmaxf(v[j0 + j] + b, -a.clip), a.clip);
+			if (is_q || is_k) {
+				float2 cs[16];
 #pragma unroll
-			for (int j = 0; j < 16; ++j) {
-				const int t = t0 + j0 + j;
-				float x = fminf(fmaxf(v[j0 + j] + b, -a.clip), a.clip);
-				const float other = __shfl_xor_sync(0xffffffffu, x, 1); // the row pair a rotation mixes sits in adjacent lanes
-				if (is_q || is_k) x = (lane & 1) ? fmaf(other, cs[j].y, x * cs[j].x) : fmaf(-other, cs[j].y, x * cs[j].x);
-				if (t < a.n_tokens) {
-					const size_t o = kv0 + (size_t)t * a.head_dim;
-					if (is_q) a.Q[(size_t)t * a.q_dim + k] = x;
-					else if (a.kvbits == 16) kv_store(reinterpret_cast<__half*>(is_k ? a.kc : a.vc) + o, x);
-					else kv_store(reinterpret_cast<uint8_t*>(is_k ? a.kc : a.vc) + o, x);
+				for (int j = 0; j < 16; ++j) cs[j] = j0 + j < left ? __ldcg(a.rope + (size_t)(t0 + j0 + j) * (a.head_dim / 2) + (d >> 1)) : make_float2(1.f, 0.f);
+#pragma unroll
+				for (int j = 0; j < 16; ++j) {
+					const float other = __shfl_xor_sync(0xffffffffu, x[j], 1); // the row pair a rotation mixes sits in adjacent lanes
+					x[j] = (lane & 1) ? fmaf(other, cs[j].y, x[j] * cs[j].x) : fmaf(-other, cs[j].y, x[j] * cs[j].x);
 				}
 			}
+			auto store = [&](auto* p, size_t step, auto&& put) {
+#pragma unroll
+				for (int j = 0; j < 16; ++j)
+					if (j0 + j < left) put(p + j * step, x[j]);
+			};
+			const size_t hd = a.head_dim, o = kv0 + (size_t)j0 * hd;
+			if (is_q) store(a.Q + (size_t)(t0 + j0) * a.q_dim + k, a.q_dim, [](float* q, float y) { *q = y; });
+			else if (a.kvbits == 16) store(reinterpret_cast<__half*>(cache) + o, hd, [](__half* q, float y) { kv_store(q, y); });
+			else store(reinterpret_cast<uint8_t*>(cache) + o, hd, [](uint8_t* q, float y) { kv_store(q, y); });
 		}
 	} else if constexpr (MODE == PF_UP) { // act(w1 x) * (w3 x)
+		__half* const ph = a.Hhi + (size_t)t0 * a.hidden + gr;
+		__half* const pl = a.Hlo + (size_t)t0 * a.hidden + gr;
 #pragma unroll
-		for (int j = 0; j < 32; ++j) {
-			const int t = t0 + j;
-			if (t < a.n_tokens) {
-				const float hv = (a.gelu ? act_gelu(v[j]) : act_silu(v[j])) * v3[j];
-				__half hh, hl;
-				split_hl(hv, hh, hl);
-				a.Hhi[(size_t)t * a.hidden + gr] = hh, a.Hlo[(size_t)t * a.hidden + gr] = hl;
+		for (int j0 = 0; j0 < 32; j0 += 8) {
+			__half hh[8], hl[8];
+			if (a.gelu) {
+#pragma unroll
+				for (int j = 0; j < 8; ++j) split_hl(act_gelu(v[j0 + j]) * v3[j0 + j], hh[j], hl[j]);
+			} else {
+#pragma unroll
+				for (int j = 0; j < 8; ++j) split_hl(act_silu(v[j0 + j]) * v3[j0 + j], hh[j], hl[j]);
 			}
+#pragma unroll
+			for (int j = 0; j < 8; ++j)
+				if (j0 + j < left) ph[(size_t)(j0 + j) * a.hidden] = hh[j], pl[(size_t)(j0 + j) * a.hidden] = hl[j];
 		}
 	} else { // residual add: all loads before the first store
 		float x[32];
 		float* p = a.X + (size_t)t0 * a.dim + gr;
 #pragma unroll
-		for (int j = 0; j < 32; ++j) x[j] = t0 + j < a.n_tokens ? __ldcg(p + (size_t)j * a.dim) : 0.f;
+		for (int j = 0; j < 32; ++j) x[j] = j < left ? __ldcg(p + (size_t)j * a.dim) : 0.f;
 #pragma unroll
 		for (int j = 0; j < 32; ++j)
-			if (t0 + j < a.n_tokens) p[(size_t)j * a.dim] = x[j] + v[j];
+			if (j < left) p[(size_t)j * a.dim] = x[j] + v[j];
 	}
 }
 
@@ -279,24 +298,27 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 	__shared__ int handed[ROLES], raw_handed, multiplied, accumulated; // stages and items that each role got to (read when a wait has given up)
 	unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-	const int nkb = a.K / PF_BK, ns = a.stages, bn = a.bn, splits = a.splits, na = MODE == PF_UP ? 2 : a.na;
+	const int nkb = a.K / PF_BK, ns = a.stages, bn = a.bn, splits = a.splits, tail = a.tail, na = MODE == PF_UP ? 2 : a.na;
 	const int rs = RT / na; // slots of na weight tiles
 	const int row_tiles = a.rows / PF_BM, tok_tiles = (a.n_tokens + bn - 1) / bn;
-	const int items = (MODE == PF_UP ? row_tiles : (row_tiles + na - 1) / na) * splits * tok_tiles;
+	const int whole = (MODE == PF_UP ? row_tiles : (row_tiles + na - 1) / na) * tok_tiles - tail, items = whole + tail * splits;
 	const int b_bytes = bn * 128;
+	const bool side = pf_side(na, bn);
+	const int ac = side ? 2 * bn : bn; // accumulator columns of a weight tile: its sums with hi and with lo side by side, or both in one
 	const size_t stage_bytes = pf_stage_bytes(na, bn);
 	auto r_tile = [&](int s, int i) { return smem + (size_t)(s * na + i) * RAW; };
 	auto a_tile = [&](int s, int i) { return smem + (size_t)RT * RAW + s * stage_bytes + (size_t)i * PF_TILE_BYTES; };
 	auto b_tile = [&](int s) { return smem + (size_t)RT * RAW + s * stage_bytes + (size_t)na * PF_TILE_BYTES; };
-	// item -> first weight row, tiles, first token, k-stages [k0, k1)
+	// item -> first weight row, tiles, first token, k-stages [k0, k1), which slice of the tail it is (slices of one k next to each other; -1: none)
 	struct Item {
-		int row0, cnt, tok0, k0, k1;
+		int row0, cnt, tok0, k0, k1, part;
 	};
 	auto item_of = [&](int it) {
 		Item r;
-		const int q = it / tok_tiles, sp = q % splits, rt = q / splits * (MODE == PF_UP ? 1 : na);
-		r.tok0 = (it % tok_tiles) * bn, r.row0 = rt * PF_BM, r.cnt = MODE == PF_UP ? 2 : min(na, row_tiles - rt);
-		r.k0 = (int)((long)nkb * sp / splits), r.k1 = (int)((long)nkb * (sp + 1) / splits);
+		r.part = it < whole ? -1 : it - whole;
+		const int tile = it < whole ? it : whole + r.part % tail, sp = it < whole ? 0 : r.part / tail, of = it < whole ? 1 : splits, rt = tile / tok_tiles * (MODE == PF_UP ? 1 : na);
+		r.tok0 = (tile % tok_tiles) * bn, r.row0 = rt * PF_BM, r.cnt = MODE == PF_UP ? 2 : min(na, row_tiles - rt);
+		r.k0 = (int)((long)nkb * sp / of), r.k1 = (int)((long)nkb * (sp + 1) / of);
 		return r;
 	};
 	// every wait is bounded: a role whose wait gives up (whole warps at a time) records a code and leaves its loop, the others follow, what is on its
@@ -317,7 +339,7 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 	tc_fence_before();
 	__syncthreads();
 	tc_fence_after();
-	const uint32_t tmem_base = tmem_base_s; // accumulator i of buffer b: columns 256 b + bn i
+	const uint32_t tmem_base = tmem_base_s; // accumulator i of buffer b: columns 256 b + ac i
 
 	// The one-thread roles keep their warp together and elect a lane for the issuing: addresses and descriptors then live in uniform registers
 	// (one lane in a branch of its own spent 60 cycles per MMA on moving them).
@@ -345,8 +367,8 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 		}
 		if (lane == 0) handed[lo] = n;
 	} else if (warp == 1) { // ===== MMAs
-		// kind::f16: D = f32, A = B = f16, both K-major, M = 128, N = bn
-		const uint32_t idesc = (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(PF_BM >> 4) << 24);
+		// kind::f16: D = f32, A = B = f16, both K-major, M = 128, N = ac (the lo tile lies right behind the hi tile: as one operand they are 2 bn rows)
+		const uint32_t idesc = (1u << 4) | ((uint32_t)(ac >> 3) << 17) | ((uint32_t)(PF_BM >> 4) << 24);
 		const bool el = elect_one();
 		int s = 0, n = 0;
 		unsigned ph = 0, q = 0;
@@ -368,8 +390,8 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 						for (int i = 0; i < 2; ++i)
 							if (i < t.cnt) {
 								const uint64_t dw = da + i * (PF_TILE_BYTES >> 4) + 2 * k;
-								umma_f16(acc + i * bn, dw, db + 2 * k, idesc, (kb > t.k0 || k) ? 1u : 0u);
-								umma_f16(acc + i * bn, dw, db + (b_bytes >> 4) + 2 * k, idesc, 1u);
+								umma_f16(acc + i * ac, dw, db + 2 * k, idesc, (kb > t.k0 || k) ? 1u : 0u);
+								if (!side) umma_f16(acc + i * ac, dw, db + (b_bytes >> 4) + 2 * k, idesc, 1u);
 							}
 					umma_commit(&empty[s]); // frees the stage when these MMAs have read it
 				}
@@ -397,18 +419,27 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 			tc_fence_after();
 			const int cols = min(bn, a.n_tokens - t.tok0);
 			float v[32], v3[32];
-			if (splits == 1) {
+			auto sums = [&](int i, int c0, float(&to)[32]) { // of tile i, 32 tokens from c0
+				tmem_ld32(acc + i * ac + c0, to);
+				if (side) {
+					float lo[32];
+					tmem_ld32(acc + i * ac + bn + c0, lo);
+#pragma unroll
+					for (int j = 0; j < 32; ++j) to[j] += lo[j];
+				}
+			};
+			if (t.part < 0) {
 				for (int i = 0; i < (MODE == PF_UP ? 1 : t.cnt); ++i)
 					for (int c0 = 0; c0 < cols; c0 += 32) {
-						tmem_ld32(acc + i * bn + c0, v);
-						if (MODE == PF_UP) tmem_ld32(acc + bn + c0, v3);
+						sums(i, c0, v);
+						if (MODE == PF_UP) sums(1, c0, v3);
 						pf_epilogue<MODE>(a, t.row0 + i * PF_BM + lr, lane, t.tok0 + c0, v, v3);
 					}
 			} else {
 				for (int i = 0; i < t.cnt; ++i)
 					for (int c0 = 0; c0 < cols; c0 += 32) {
-						tmem_ld32(acc + i * bn + c0, v);
-						float* p = a.ws + ((size_t)(it * na + i) * bn + c0) * PF_BM + lr;
+						sums(i, c0, v);
+						float* p = a.ws + ((size_t)(t.part * na + i) * bn + c0) * PF_BM + lr;
 #pragma unroll
 						for (int j = 0; j < 32; ++j) __stcg(p + j * PF_BM, v[j]);
 					}
@@ -416,8 +447,8 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 			tc_fence_before();
 			__syncwarp();
 			if (lane == 0) mbar_arrive(&acc_empty[q & 1]);
-			if (splits > 1) { // the last slice of a tile to arrive adds all of them up in slice order
-				const int tile = it / tok_tiles / splits * tok_tiles + it % tok_tiles;
+			if (t.part >= 0) { // the last slice of a tile to arrive adds all of them up in slice order
+				const int tile = t.part % tail;
 				__threadfence();
 				asm volatile("bar.sync 1, 128;" ::: "memory");
 				if (tid == 64) {
@@ -430,12 +461,13 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 				asm volatile("bar.sync 1, 128;" ::: "memory");
 				if (!last) continue;
 				__threadfence();
-				const int first = it / tok_tiles / splits * splits * tok_tiles + it % tok_tiles; // item of slice 0
 				auto fold = [&](int i, int c0, float(&sum)[32]) {
 #pragma unroll
 					for (int j = 0; j < 32; ++j) sum[j] = 0.f;
+					constexpr int AHEAD = DBITS == 4 ? 1 : 2; // slices whose loads are out at a time
+#pragma unroll AHEAD
 					for (int sp = 0; sp < splits; ++sp) {
-						const float* p = a.ws + ((size_t)((first + sp * tok_tiles) * na + i) * bn + c0) * PF_BM + lr;
+						const float* p = a.ws + ((size_t)((tile + sp * tail) * na + i) * bn + c0) * PF_BM + lr;
 #pragma unroll
 						for (int j = 0; j < 32; ++j) sum[j] += __ldcg(p + j * PF_BM);
 					}
