@@ -1447,6 +1447,239 @@ __global__ void __launch_bounds__(128) k_seq_delta_scan_reg(DeltaArgs a, SeqBatc
 		for (int i = 0; i < Q; ++i) *(float2*)(Sg + (size_t)i * V) = make_float2(S[i][0], S[i][1]);
 	}
 }
+// The same recurrence, blocks of DELTA_BK tokens at a time.  Inside a block, with S the state before it, G_t the product of the decays up to token t and
+// D(t, s) that of the decays after s up to t (per key channel, nothing is divided):
+//   u_t = beta_t (v_t - (k_t G_t) S - sum_{s<t} A_ts u_s),   A_ts = k_t . D(t, s) k_s
+//   o_t = (q_t G_t) S + sum_{s<=t} B_ts u_s,                 B_ts = q_t . D(t, s) k_s
+//   S'  = G_T S + sum_s (D(T, s) k_s) u_s
+// so the corrections of a block are one triangular system, U = X (V - (K G) S) with X = (1 + diag(beta) A)^-1 diag(beta), and the read-outs are (Q G) S + (B X) (V - (K G) S).
+// X and B X depend on no value: k_seq_delta_system forms them for all blocks side by side (and turns the raw decay inputs into decays, in place), and
+// k_seq_delta_blocks walks the state from block to block with products whose terms do not wait for one another.  The scan's chain of a token (dot, shuffles,
+// update: 0.75 us) becomes a block's: 3 x 700 tokens of 16 heads of 128 x 128 522 us, now DELTA_NOW.
+#define DELTA_BK 16
+struct DeltaBlocks {
+	float* sys; // [block][heads][2][DELTA_BK][DELTA_BK]: X, B X; block j of sequence b is number sstart[b] / DELTA_BK + b + j (one more than fit a portion at most)
+	float* dt;  // DeltaArgs::dt, written
+	int count;  // blocks of the longest portion
+};
+__global__ void __launch_bounds__(512) k_seq_delta_system(DeltaArgs a, DeltaBlocks c, SeqBatch sb) {
+	pdl_enter(); // programmatic dependent launch: let the next kernel's launch overlap this one, then wait for the previous one
+	constexpr int D = 128, T = DELTA_BK; // a warp per token, four channels per lane
+	__shared__ __align__(16) float ks[T][D], qs[T][D], gs[T][D];
+	__shared__ float A[T][T + 1], Bm[T][T + 1], X[T][T + 1], beta[T];
+	const int b = blockIdx.x / c.count, blk = blockIdx.x % c.count, h = blockIdx.y, kh = h / (a.heads / a.kv_heads);
+	const int t0 = blk * T, nt = min(T, sb.scount[b] - t0);
+	if (nt <= 0) return;
+	const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, i = 4 * lane;
+	const size_t n = (size_t)sb.sstart[b] + t0 + w;
+	float4 k = make_float4(0.f, 0.f, 0.f, 0.f), q = k, g = make_float4(1.f, 1.f, 1.f, 1.f); // tokens past the portion change nothing
+	if (w < nt) {
+		k = __ldg((const float4*)(a.k + (n * a.kv_heads + kh) * D + i)), q = __ldg((const float4*)(a.q + (n * a.kv_heads + kh) * D + i));
+		float4* const dt = (float4*)(c.dt + (n * a.heads + h) * D + i);
+		const float4 z = *dt;
+		const bf16* bp = a.dt_bias + h * D + i;
+		const float e = expf(ldf(a.a_log + h));
+		g = make_float4(expf(-e * softplusf_(z.x + ldf(bp))), expf(-e * softplusf_(z.y + ldf(bp + 1))), expf(-e * softplusf_(z.z + ldf(bp + 2))), expf(-e * softplusf_(z.w + ldf(bp + 3))));
+		*dt = g;
+	}
+	*(float4*)(ks[w] + i) = k, *(float4*)(qs[w] + i) = q, *(float4*)(gs[w] + i) = g;
+	if (lane == 0) beta[w] = w < nt ? sigmoidf_(a.proj[n * a.ldp + a.bcol + h]) : 0.f;
+	__syncthreads();
+	// warp w: column s = w of A and B; its key decays on its way through the later tokens
+	float v[2 * T];
+#pragma unroll
+	for (int t = 0; t < T; ++t) {
+		v[t] = v[T + t] = 0.f;
+		if (t < w) continue;
+		const float4 kt = *(const float4*)(ks[t] + i), qt = *(const float4*)(qs[t] + i);
+		if (t > w) {
+			const float4 gt = *(const float4*)(gs[t] + i);
+			k.x *= gt.x, k.y *= gt.y, k.z *= gt.z, k.w *= gt.w;
+			v[t] = fmaf(kt.x, k.x, kt.y * k.y) + fmaf(kt.z, k.z, kt.w * k.w);
+		}
+		v[T + t] = fmaf(qt.x, k.x, qt.y * k.y) + fmaf(qt.z, k.z, qt.w * k.w);
+	}
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) { // lane l ends with the sum of value l
+		const bool up = lane & o;
+#pragma unroll
+		for (int j = 0; j < o; ++j) {
+			const float other = __shfl_xor_sync(0xffffffffu, up ? v[j] : v[j + o], o);
+			v[j] = (up ? v[j + o] : v[j]) + other;
+		}
+	}
+	(lane < T ? A[lane] : Bm[lane - T])[w] = v[0];
+	__syncthreads();
+	if (tid < T) { // column `tid` of X by forward substitution
+		float x[T];
+#pragma unroll
+		for (int t = 0; t < T; ++t) {
+			float r = t == tid ? 1.f : 0.f;
+#pragma unroll
+			for (int s = 0; s < t; ++s) r = fmaf(-A[t][s], x[s], r);
+			x[t] = beta[t] * r;
+			X[t][tid] = x[t];
+		}
+	}
+	__syncthreads();
+	if (tid < T * T) {
+		const int t = tid / T, j = tid % T;
+		float r = 0.f;
+		for (int s = j; s <= t; ++s) r = fmaf(Bm[t][s], X[s][j], r);
+		float* out = c.sys + ((size_t)(sb.sstart[b] / T + b + blk) * a.heads + h) * 2 * T * T + tid;
+		out[0] = X[t][j], out[T * T] = r;
+	}
+}
+// One CTA of four warps per (sequence, head, DELTA_VC value columns).  16 lanes share four columns and hold eight key channels of each.
+__host__ __device__ constexpr int delta_block_floats() { return 3 * DELTA_BK * 128 + DELTA_BK * DELTA_VC + 2 * DELTA_BK * DELTA_BK; } // k, q, decay, v, X, B X
+__host__ __device__ constexpr size_t delta_block_smem() { return (size_t)(2 * delta_block_floats() + 3 * DELTA_BK * DELTA_VC + 128) * sizeof(float); }
+__global__ void __launch_bounds__(128) k_seq_delta_blocks(DeltaArgs a, DeltaBlocks c, SeqBatch sb) {
+	pdl_enter(); // programmatic dependent launch: let the next kernel's launch overlap this one, then wait for the previous one
+	constexpr int D = 128, T = DELTA_BK, VC = DELTA_VC, BUF = delta_block_floats();
+	extern __shared__ __align__(16) float sm[];
+	float* const rest = sm + 2 * BUF; // V - (K G) S, then
+	float* const read = rest + T * VC; // (Q G) S and
+	float* const corr = read + T * VC; // U, [token][column] each
+	float* const last = corr + T * VC; // [D] G_T
+	const int b = blockIdx.x, h = blockIdx.y, V = a.vdim, v0 = blockIdx.z * VC, kh = h / (a.heads / a.kv_heads);
+	const int tid = threadIdx.x, part = tid & 15, cl = (tid >> 4) * 4;
+	const int start = sb.sstart[b], cnt = sb.scount[b], nblk = (cnt + T - 1) / T;
+	const bool live = v0 + cl < V; // (V is a multiple of 4) lanes past the last column run along on the last ones
+	float* const Sg = a.state + ((size_t)sb.sslot[b] * a.heads + h) * D * V + (live ? v0 + cl : V - 4);
+	auto channel = [&](int e) { return (e >> 2) * (D / 2) + 4 * part + (e & 3); }; // this lane's channel e of 8
+	float2 S[4][4]; // [column][pair of channels]
+#pragma unroll
+	for (int p = 0; p < 4; ++p) {
+		const float4 x = *(const float4*)(Sg + (size_t)channel(2 * p) * V), y = *(const float4*)(Sg + (size_t)channel(2 * p + 1) * V);
+		S[0][p] = make_float2(x.x, y.x), S[1][p] = make_float2(x.y, y.y), S[2][p] = make_float2(x.z, y.z), S[3][p] = make_float2(x.w, y.w);
+	}
+	auto issue = [&](int blk) { // a block's inputs in 16-byte pieces; tokens past the portion: zero keys, queries and values, decays of one
+		float* const to = sm + (blk & 1) * BUF;
+		const int nt = min(T, cnt - blk * T);
+		const size_t n0 = (size_t)start + blk * T;
+		for (int e = tid; e < 3 * T * D / 4; e += 128) {
+			const int which = e / (T * D / 4), t = e / (D / 4) % T, i = 4 * (e % (D / 4));
+			float* const d = to + 4 * e;
+			if (t < nt) cp_async16(d, which == 2 ? c.dt + ((n0 + t) * a.heads + h) * D + i : (which == 0 ? a.k : a.q) + ((n0 + t) * a.kv_heads + kh) * D + i);
+			else *(float4*)d = which == 2 ? make_float4(1.f, 1.f, 1.f, 1.f) : make_float4(0.f, 0.f, 0.f, 0.f);
+		}
+		float* const vt = to + 3 * T * D;
+		{
+			const int t = tid / (VC / 4), i = 4 * (tid % (VC / 4)); // T * VC / 4 = 128 pieces
+			if (t < nt && v0 + i < V) cp_async16(vt + 4 * tid, a.v + ((n0 + t) * a.heads + h) * V + v0 + i);
+			else *(float4*)(vt + 4 * tid) = make_float4(0.f, 0.f, 0.f, 0.f);
+		}
+		cp_async16(vt + T * VC + 4 * tid, c.sys + ((size_t)(start / T + b + blk) * a.heads + h) * 2 * T * T + 4 * tid); // 2 T T / 4 = 128 pieces
+		asm volatile("cp.async.commit_group;" ::: "memory");
+	};
+	static_assert(T * VC / 4 == 128 && 2 * T * T / 4 == 128 && D == 128, "one piece of v and of the system, and one channel, per thread");
+	issue(0);
+	for (int blk = 0; blk < nblk; ++blk) {
+		float* const ks = sm + (blk & 1) * BUF;
+		float *const qs = ks + T * D, *const gs = qs + T * D, *const vs = gs + T * D;
+		const float *const X = vs + T * VC, *const BX = X + T * T;
+		if (blk + 1 < nblk) {
+			issue(blk + 1); // into the half that the block before has been done with since its last barrier
+			asm volatile("cp.async.wait_group 1;" ::: "memory");
+		} else asm volatile("cp.async.wait_group 0;" ::: "memory");
+		__syncthreads();
+		{ // in place, a channel per thread: decay -> k G, q -> q G, k -> D(T, s) k
+			float g[T], G = 1.f;
+#pragma unroll
+			for (int t = 0; t < T; ++t) g[t] = gs[t * D + tid];
+#pragma unroll
+			for (int t = 0; t < T; ++t) G *= g[t], gs[t * D + tid] = ks[t * D + tid] * G, qs[t * D + tid] *= G;
+			last[tid] = G, G = 1.f;
+#pragma unroll
+			for (int t = T - 1; t >= 0; --t) ks[t * D + tid] *= G, G *= g[t];
+		}
+		__syncthreads();
+#pragma unroll 1
+		for (int t0 = 0; t0 < T; t0 += 4) { // (K G) S and (Q G) S, four tokens' shares at a time
+			float r[32]; // [token][K, Q][column]
+#pragma unroll
+			for (int x = 0; x < 8; ++x) {
+				const float* at = (x & 1 ? qs : gs) + (t0 + x / 2) * D + 4 * part;
+				const float4 lo = *(const float4*)at, hi = *(const float4*)(at + D / 2);
+				const float2 y[4] = {make_float2(lo.x, lo.y), make_float2(lo.z, lo.w), make_float2(hi.x, hi.y), make_float2(hi.z, hi.w)};
+#pragma unroll
+				for (int j = 0; j < 4; ++j) {
+					float2 z = __fmul2_rn(y[0], S[j][0]);
+#pragma unroll
+					for (int p = 1; p < 4; ++p) z = __ffma2_rn(y[p], S[j][p], z);
+					r[4 * x + j] = z.x + z.y;
+				}
+			}
+#pragma unroll
+			for (int o = 8, left = 16; o > 0; o >>= 1, left >>= 1) { // over the 16 lanes, each keeping half of the values: lane `part` ends with two
+				const bool up = part & o;
+#pragma unroll
+				for (int i = 0; i < left; ++i) {
+					const float other = __shfl_xor_sync(0xffffffffu, up ? r[i] : r[i + left], o);
+					r[i] = (up ? r[i + left] : r[i]) + other;
+				}
+			}
+			const int at = (t0 + (part >> 2)) * VC + cl + 2 * (part & 1);
+			if (part & 2) *(float2*)(read + at) = make_float2(r[0], r[1]);
+			else {
+				const float2 v = *(const float2*)(vs + at);
+				*(float2*)(rest + at) = make_float2(v.x - r[0], v.y - r[1]);
+			}
+		}
+		__syncthreads();
+		{ // four tokens of one column per thread: U and the read-outs
+			const int col = tid & (VC - 1), r0 = 4 * (tid / VC);
+			float u[4] = {}, o[4];
+#pragma unroll
+			for (int j = 0; j < 4; ++j) o[j] = read[(r0 + j) * VC + col];
+#pragma unroll 1
+			for (int s0 = 0; s0 <= r0; s0 += 4) { // both matrices are lower triangular
+				float x[4];
+#pragma unroll
+				for (int i = 0; i < 4; ++i) x[i] = rest[(s0 + i) * VC + col];
+#pragma unroll
+				for (int j = 0; j < 4; ++j) {
+					const float4 p = *(const float4*)(X + (r0 + j) * T + s0), q = *(const float4*)(BX + (r0 + j) * T + s0);
+					u[j] = fmaf(p.x, x[0], u[j]), u[j] = fmaf(p.y, x[1], u[j]), u[j] = fmaf(p.z, x[2], u[j]), u[j] = fmaf(p.w, x[3], u[j]);
+					o[j] = fmaf(q.x, x[0], o[j]), o[j] = fmaf(q.y, x[1], o[j]), o[j] = fmaf(q.z, x[2], o[j]), o[j] = fmaf(q.w, x[3], o[j]);
+				}
+			}
+#pragma unroll
+			for (int j = 0; j < 4; ++j) {
+				corr[(r0 + j) * VC + col] = u[j];
+				const int t = blk * T + r0 + j;
+				if (t < cnt && v0 + col < V) a.o[((size_t)(start + t) * a.heads + h) * V + v0 + col] = o[j];
+			}
+		}
+		__syncthreads();
+		{
+			const float4 lo = *(const float4*)(last + 4 * part), hi = *(const float4*)(last + D / 2 + 4 * part);
+			const float2 G[4] = {make_float2(lo.x, lo.y), make_float2(lo.z, lo.w), make_float2(hi.x, hi.y), make_float2(hi.z, hi.w)};
+#pragma unroll
+			for (int j = 0; j < 4; ++j)
+#pragma unroll
+				for (int p = 0; p < 4; ++p) S[j][p] = __fmul2_rn(S[j][p], G[p]);
+		}
+#pragma unroll 4
+		for (int t = 0; t < T; ++t) {
+			const float4 lo = *(const float4*)(ks + t * D + 4 * part), hi = *(const float4*)(ks + t * D + D / 2 + 4 * part), u4 = *(const float4*)(corr + t * VC + cl);
+			const float2 y[4] = {make_float2(lo.x, lo.y), make_float2(lo.z, lo.w), make_float2(hi.x, hi.y), make_float2(hi.z, hi.w)};
+			const float u[4] = {u4.x, u4.y, u4.z, u4.w};
+#pragma unroll
+			for (int j = 0; j < 4; ++j)
+#pragma unroll
+				for (int p = 0; p < 4; ++p) S[j][p] = __ffma2_rn(y[p], make_float2(u[j], u[j]), S[j][p]);
+		}
+		__syncthreads(); // the block's buffer, its corrections and G_T have been read
+	}
+	if (live) {
+#pragma unroll
+		for (int p = 0; p < 4; ++p) {
+			*(float4*)(Sg + (size_t)channel(2 * p) * V) = make_float4(S[0][p].x, S[1][p].x, S[2][p].x, S[3][p].x);
+			*(float4*)(Sg + (size_t)channel(2 * p + 1) * V) = make_float4(S[0][p].y, S[1][p].y, S[2][p].y, S[3][p].y);
+		}
+	}
+}
 // read-out: o / rms(o) (per head) * w * sigmoid(gate); one warp per (token, head)
 // (the gate goes through a sigmoid, or through SiLU when silu_gate is set; it is read at gate[token * ldg + head * vdim + i])
 template <typename AT>

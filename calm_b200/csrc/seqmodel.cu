@@ -82,8 +82,8 @@ struct Seq {
 	size_t w_rope = 0;
 	float2* carry = nullptr;                          // SEQ_MINGRU: chunk maps of a step's longer portions
 	size_t carry_cap = 0;
-	float* gla = nullptr;                             // gated linear attention: states and decays of a step's chunks
-	size_t gla_cap = 0;
+	float* scan_ws = nullptr;                         // gated linear attention: states and decays of a step's chunks; delta rule: the systems of its blocks
+	size_t scan_cap = 0;
 	void* ah = nullptr;                               // parallel blocks: a dense unit's hidden activations, written by the mixer's input product
 	size_t w_ah = 0;
 	float* mo = nullptr;                              // parallel blocks: the mixer's output until the feed-forward's is added with it; hyper blocks: a sublayer's output
@@ -835,15 +835,17 @@ void out_product(Seq& s, const AT* X, const void* Wt, int N, int K, const OutEpi
 	gemm(s, X, K, 0, Wt, K, 0, oe.dst, s.m.width, 0, N, s.m.width, K, 1, oe.epi, oe.nrm, -1, true, &gx);
 }
 
-void ensure_gla(Seq& s, size_t need) {
-	if (need <= s.gla_cap) return;
+void ensure_scan(Seq& s, size_t need) {
+	if (need <= s.scan_cap) return;
 	CUDA_CHECK(cudaStreamSynchronize(s.stream));
-	cudaFree(s.gla); // decode graphs (one token per sequence) never read it
-	s.gla = (float*)dalloc(need * sizeof(float)), s.gla_cap = need;
+	cudaFree(s.scan_ws); // decode graphs (one token per sequence) never read it
+	s.scan_ws = (float*)dalloc(need * sizeof(float)), s.scan_cap = need;
 }
 // Portions from this many tokens on are cut into chunks.  Scan against chunks, us a layer of 128 x 128: 16 heads, 200 tokens 57, 36; 256 66, 38; 2048 468, 140; two
 // sequences of 256 85, 52; 8 heads, 128 tokens 26, 27; 256 45, 31; 2048 298, 83.
 const int kGlaChunksMin = 160;
+// ... and run through the delta rule in blocks
+const int kDeltaBlocksMin = 32;
 
 // the gated-linear-attention scan over a step's tokens: S <- diag(decay) S + k v^T, o = S^T q * qscale per (sequence, head); g names
 // the inputs (columns of a matrix with row stride ld), the state and the output
@@ -860,8 +862,8 @@ void gla_launch(Seq& s, GlaArgs& g, const SeqBatch& sb, int ld) {
 		GlaChunks c;
 		c.len = (cdiv(longest, room) + GLC_TB - 1) / GLC_TB * GLC_TB, c.count = cdiv(longest, c.len);
 		const size_t units = (size_t)sb.B * c.count * H;
-		ensure_gla(s, units * D * (Dv + 1));
-		c.add = s.gla, c.keep = s.gla + units * D * Dv;
+		ensure_scan(s, units * D * (Dv + 1));
+		c.add = s.scan_ws, c.keep = s.scan_ws + units * D * Dv;
 		const double bytes = (double)N * H * (3.0 * D + 2.0 * Dv) * 4 + 2.0 * sb.B * H * D * Dv * 4, flops = (double)N * H * D * Dv * 4.0;
 		auto go = [&](auto local, auto starts, auto apply) {
 			run_kernel(s, KD_GLA, 0, 0, [&] { launch_k(s, local, dim3(sb.B * c.count, H, cdiv(Dv, 128)), 2 * D, glc_smem(D), g, c, sb); });
@@ -983,8 +985,18 @@ void mixer_typed(Seq& s, const SeqLayer& L, RunState& r, const SeqBatch& sb, dou
 		const size_t smem = ((size_t)D * Dv + 3 * D) * sizeof(float);
 		const int threads = std::max(64, cdiv(Dv, 32) * 32);
 		const bool reg = (D == 32 || D == 64 || D == 128) && Dv <= 128 && Dv % 4 == 0 && !getenv("CALM_B200_SEQ_DELTA_SMEM");
+		int longest_portion = 0;
+		for (int b = 0; b < sb.B; ++b) longest_portion = std::max(longest_portion, s.hb_count[b]);
+		const bool blocks = reg && D == 128 && longest_portion >= kDeltaBlocksMin;
+		DeltaBlocks db{nullptr, s.f[3], cdiv(longest_portion, DELTA_BK)};
+		if (blocks) {
+			ensure_scan(s, (size_t)(N / DELTA_BK + sb.B) * H * 2 * DELTA_BK * DELTA_BK);
+			db.sys = s.scan_ws;
+			run_kernel(s, KD_DELTA, 0, 0, [&] { launch_k(s, k_seq_delta_system, dim3(sb.B * db.count, H), 512, 0, d, db, sb); });
+		}
 		run_kernel(s, KD_DELTA, (double)N * H * (3.0 * D + 2.0 * Dv) * 4 + 2.0 * sb.B * H * D * Dv * 4, (double)N * H * D * Dv * 6.0, [&] {
 			const dim3 grid(sb.B, H, cdiv(Dv, DELTA_VC));
+			if (blocks) return launch_k(s, k_seq_delta_blocks, grid, 128, delta_block_smem(), d, db, sb);
 			if (reg && D == 32) launch_k(s, k_seq_delta_scan_reg<32>, grid, 128, 0, d, sb);
 			else if (reg && D == 64) launch_k(s, k_seq_delta_scan_reg<64>, grid, 128, 0, d, sb);
 			else if (reg && D == 128) launch_k(s, k_seq_delta_scan_reg<128>, grid, 128, 0, d, sb);
@@ -1545,6 +1557,7 @@ extern "C" void* calm_b200_seq_prepare(const struct SeqModel* model) {
 		constexpr int R = decltype(r)::value, P = decltype(p)::value;
 		CUDA_CHECK(cudaFuncSetAttribute(k_seq_gla_scan<R, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gla_smem(R, P)));
 	});
+	CUDA_CHECK(cudaFuncSetAttribute(k_seq_delta_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)delta_block_smem()));
 	CUDA_CHECK(cudaFuncSetAttribute(k_seq_gla_local<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)glc_smem(128)));
 	CUDA_CHECK(cudaFuncSetAttribute(k_seq_gla_local<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)glc_smem(64)));
 	CUDA_CHECK(cudaFuncSetAttribute(k_seq_attn_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
@@ -1643,7 +1656,7 @@ extern "C" void calm_b200_seq_release(void* handle) {
 		for (RunState& q : r.sub) drop(q);
 	};
 	for (RunState& r : s->runs) drop(r);
-	cudaFree(s->lin), cudaFree(s->fsh), cudaFree(s->hist), cudaFree(s->carry), cudaFree(s->gla), cudaFree(s->rope_cs);
+	cudaFree(s->lin), cudaFree(s->fsh), cudaFree(s->hist), cudaFree(s->carry), cudaFree(s->scan_ws), cudaFree(s->rope_cs);
 	cudaFree(s->table_dev), cudaFree(s->meta_dev), cudaFreeHost(s->meta), cudaFreeHost(s->picks), cudaFree(s->logits), cudaFree(s->hW);
 	cudaFree(s->part), cudaFree(s->a3), cudaFree(s->att_kb), cudaFree(s->att_vt), cudaFree(s->att_s), cudaFree(s->att_p), cudaFree(s->x), cudaFree(s->x0), cudaFree(s->proj), cudaFree(s->hA), cudaFree(s->a1), cudaFree(s->a2), cudaFree(s->trace_buf);
 	for (float* p : s->f) cudaFree(p);

@@ -1,0 +1,37 @@
+"""The delta rule over longer portions, in blocks of tokens (k_seq_delta_system, k_seq_delta_blocks), against the plain float64 statement: value columns around a
+CTA's 32, portions that end inside a block, of one token beside a long one, key heads shared by several heads, keys that repeat (a token of a portion fed again and
+again, where the corrections inside a block matter most), and a state that is carried on into a second portion and a decoded token."""
+import os
+import sys
+
+import numpy as np
+import pytest
+
+sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
+import test_vimulorn_gpu as tv  # noqa: E402
+import vimulorn_plain  # noqa: E402
+
+from calm_b200 import vimulorn  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("heads,kv,vdim,counts", [(2, 1, 4, (32,)), (4, 2, 36, (33, 1)), (2, 2, 128, (47, 5, 64)), (3, 3, 32, (16, 113)), (1, 1, 100, (300,))])
+def test_blocks(dtype, heads, kv, vdim, counts):
+    cfg = tv.config([tv.delta(heads=heads, kv_heads=kv, dim=128, vdim=vdim, conv=2)])
+    t, toks = tv.weights(cfg, 8), tv.tokens(cfg, max(counts) + 60)
+    toks[5:25] = [toks[5]] * 20
+    ref = vimulorn_plain.forward(cfg, tv.as_f64(t), toks)
+    with vimulorn.from_tensors(cfg, t, dtype, max_tokens=900, max_seqs=3, page=8) as m:
+        slots = [m.open() for _ in counts]
+        at = np.cumsum((0,) + counts)
+        out = m.step(slots, [toks[:n] for n in counts], list(range(sum(counts))))
+        for i, n in enumerate(counts):
+            assert tv.rel_err(out[at[i]:at[i + 1]], ref[:n]) < tv.TOL[dtype], n
+        out = m.step(slots, [toks[n:n + 59] for n in counts], list(range(59 * len(counts))))
+        for i, n in enumerate(counts):
+            assert tv.rel_err(out[59 * i:59 * (i + 1)], ref[n:n + 59]) < tv.TOL[dtype], n
+        out = m.step(slots, [toks[n + 59:n + 60] for n in counts], list(range(len(counts))))
+        for i, n in enumerate(counts):
+            assert tv.rel_err(out[i:i + 1], ref[n + 59:n + 60]) < tv.TOL[dtype], n
