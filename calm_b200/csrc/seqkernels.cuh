@@ -7,6 +7,7 @@
 #pragma once
 
 #include <cuda_bf16.h>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tc05.cuh"
@@ -1632,18 +1633,23 @@ __global__ void __launch_bounds__(128) k_seq_delta_blocks(DeltaArgs a, DeltaBloc
 			float u[4] = {}, o[4];
 #pragma unroll
 			for (int j = 0; j < 4; ++j) o[j] = read[(r0 + j) * VC + col];
-#pragma unroll 1
-			for (int s0 = 0; s0 <= r0; s0 += 4) { // both matrices are lower triangular
+			// both matrices are lower triangular; on the diagonal their zeros are left out: times a later token's NaN or infinity they would not be zero
+			auto four = [&](int s0, auto diagonal) {
 				float x[4];
 #pragma unroll
 				for (int i = 0; i < 4; ++i) x[i] = rest[(s0 + i) * VC + col];
 #pragma unroll
 				for (int j = 0; j < 4; ++j) {
-					const float4 p = *(const float4*)(X + (r0 + j) * T + s0), q = *(const float4*)(BX + (r0 + j) * T + s0);
-					u[j] = fmaf(p.x, x[0], u[j]), u[j] = fmaf(p.y, x[1], u[j]), u[j] = fmaf(p.z, x[2], u[j]), u[j] = fmaf(p.w, x[3], u[j]);
-					o[j] = fmaf(q.x, x[0], o[j]), o[j] = fmaf(q.y, x[1], o[j]), o[j] = fmaf(q.z, x[2], o[j]), o[j] = fmaf(q.w, x[3], o[j]);
+					const float4 p4 = *(const float4*)(X + (r0 + j) * T + s0), q4 = *(const float4*)(BX + (r0 + j) * T + s0);
+					const float p[4] = {p4.x, p4.y, p4.z, p4.w}, q[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+					for (int i = 0; i < 4; ++i)
+						if (!decltype(diagonal)::value || i <= j) u[j] = fmaf(p[i], x[i], u[j]), o[j] = fmaf(q[i], x[i], o[j]);
 				}
-			}
+			};
+#pragma unroll 1
+			for (int s0 = 0; s0 < r0; s0 += 4) four(s0, std::false_type{});
+			four(r0, std::true_type{});
 #pragma unroll
 			for (int j = 0; j < 4; ++j) {
 				corr[(r0 + j) * VC + col] = u[j];

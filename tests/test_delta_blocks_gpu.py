@@ -35,3 +35,16 @@ def test_blocks(dtype, heads, kv, vdim, counts):
         out = m.step(slots, [toks[n + 59:n + 60] for n in counts], list(range(len(counts))))
         for i, n in enumerate(counts):
             assert tv.rel_err(out[i:i + 1], ref[n + 59:n + 60]) < tv.TOL[dtype], n
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("bad", [16, 17, 22, 35, 43])  # first, second, third and last of a block's four tokens that a thread takes together, and in the last block
+def test_no_later_value_reaches_an_earlier_token(dtype, bad):
+    cfg = tv.config([tv.delta(heads=2, kv_heads=1, dim=128, vdim=36, conv=2)])
+    t, toks = tv.weights(cfg, 8), [x % 90 for x in tv.tokens(cfg, 44)]
+    ref = vimulorn_plain.forward(cfg, tv.as_f64(t), toks)
+    t["embed"][95] = float("nan")
+    toks[bad] = 95
+    with vimulorn.from_tensors(cfg, t, dtype, max_tokens=64, max_seqs=1, page=8) as m:
+        out = m.step([m.open()], [toks], list(range(44)))
+    assert tv.rel_err(out[:bad], ref[:bad]) < tv.TOL[dtype] and np.isnan(out[bad:]).all()
