@@ -261,11 +261,12 @@ __global__ void __launch_bounds__(TG_THREADS, 2) k_seq_gemm_tc(const __grid_cons
 #define TP_THREADS 320 // a copying and a multiplying warp, eight that read results
 #define TP_SMEM (TP_STAGES * TP_STAGE_BYTES + 1024)
 template <int E>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1) k_seq_gemm_pair(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const GemmArgs a, int* err) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1) k_seq_gemm_pair(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const GemmArgs a, int* err, unsigned tries) {
 	extern __shared__ unsigned char smem_dyn[];
 	__shared__ __align__(8) uint64_t full[TP_STAGES], empty[TP_STAGES], acc_full[2], acc_empty[2]; // full, acc_empty: rank 0's are used
 	__shared__ uint32_t tmem_base_s;
-	__shared__ int asked[2], multiplied_s; // rank 0: stages that each CTA's copies got to, stages multiplied (read when a wait has given up)
+	// rank 0's, read when a wait has given up: whether one did in each CTA, stages that its copies got to, stages multiplied, accumulators handed over
+	__shared__ int gave_up_s[2], asked[2], multiplied_s, handed_s;
 	unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = (int)cluster_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
 	const int nkb = (a.K + TG_BK - 1) / TG_BK, tok_tiles = (a.N + TP_BN - 1) / TP_BN, tiles = (a.M + TP_BM - 1) / TP_BM * tok_tiles;
@@ -277,7 +278,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1) k_seq
 	if (tid == 0) {
 		for (int s = 0; s < TP_STAGES; ++s) mbar_init(&full[s], 1), mbar_init(&empty[s], 1);
 		for (int s = 0; s < 2; ++s) mbar_init(&acc_full[s], 1), mbar_init(&acc_empty[s], 16);
-		asked[0] = asked[1] = multiplied_s = 0;
+		asked[0] = asked[1] = multiplied_s = handed_s = 0;
 		mbar_init_fence();
 	}
 	if (warp == 1) pair_tmem_alloc(&tmem_base_s, 512);
@@ -293,7 +294,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1) k_seq
 			const int m0 = t / tok_tiles * TP_BM + rank * 128, n0 = t % tok_tiles * TP_BN, n1 = n0 + rank * (width(n0) / 2);
 			for (int kb = 0; kb < nkb; ++kb, ++it) {
 				const int s = it % TP_STAGES;
-				ok = mbar_wait_warp(&empty[s], ((it / TP_STAGES) & 1) ^ 1);
+				ok = mbar_wait_warp(&empty[s], ((it / TP_STAGES) & 1) ^ 1, tries);
 				if (!ok) break;
 				if (elect_one()) {
 					const uint32_t bar = cluster_addr(&full[s], 0);
@@ -306,21 +307,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1) k_seq
 		}
 		if (lane == 0) {
 			if (!ok) atomicExch(err, 1);
-			asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(&asked[rank], 0)), "r"(it) : "memory");
+			cluster_store(cluster_addr(&asked[rank], 0), it);
 		}
 		// the stages' last releases arrive in this CTA: they do before it ends
-		for (int i = max(0, it - TP_STAGES); i < it && ok; ++i) ok = mbar_wait_warp(&empty[i % TP_STAGES], (i / TP_STAGES) & 1);
+		for (int i = max(0, it - TP_STAGES); i < it && ok; ++i) ok = mbar_wait_warp(&empty[i % TP_STAGES], (i / TP_STAGES) & 1, tries);
 	} else if (warp == 1) {
 		if (rank == 0) {
-			int it = 0, n = 0;
+			int it = 0, n = 0, handed = 0;
 			for (int t = pair; t < tiles && ok; t += pairs, ++n) {
 				const int buf = n & 1;
 				const uint32_t d = tmem_base + buf * 256, idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(width(t % tok_tiles * TP_BN) >> 3) << 17) | ((uint32_t)(TP_BM >> 4) << 24);
-				ok = mbar_wait_warp(&acc_empty[buf], ((n >> 1) & 1) ^ 1);
+				ok = mbar_wait_warp(&acc_empty[buf], ((n >> 1) & 1) ^ 1, tries);
 				tc_fence_after();
 				for (int kb = 0; kb < nkb && ok; ++kb, ++it) {
 					const int s = it % TP_STAGES;
-					ok = mbar_wait_warp(&full[s], (it / TP_STAGES) & 1);
+					ok = mbar_wait_warp(&full[s], (it / TP_STAGES) & 1, tries);
 					if (!ok) break;
 					if (elect_one()) {
 						const uint64_t da = umma_desc_sw128(a_tile(s)), db = umma_desc_sw128(b_tile(s));
@@ -331,9 +332,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1) k_seq
 					}
 					__syncwarp();
 				}
+				handed += ok;
 			}
 			if (!ok && lane == 0) atomicExch(err, 2);
-			if (lane == 0) multiplied_s = it;
+			if (lane == 0) multiplied_s = it, handed_s = handed;
 		}
 	} else {
 		const int q4 = warp & 3, half = (warp - 2) / 4 * (TP_BN / 2); // the TMEM lane quarter this warp may read, and its half of the tokens
@@ -346,7 +348,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1) k_seq
 					asm volatile("prefetch.global.L2 [%0];" ::"l"((const float*)a.Y + (size_t)i * a.ldy + m0 + q4 * 32));
 					if (E == EPI_RES && a.res) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.res + (size_t)i * a.ldy + m0 + q4 * 32));
 				}
-			ok = mbar_wait_warp(&acc_full[buf], (n >> 1) & 1);
+			ok = mbar_wait_warp(&acc_full[buf], (n >> 1) & 1, tries);
 			if (!ok) break;
 			tc_fence_after();
 			tg_epilogue<E>(a, 0, gr, n0, half, half + TP_BN / 2, m0 + q4 * 32 + lane, lane, tmem_base + buf * 256 + ((uint32_t)(q4 * 32) << 16));
@@ -357,13 +359,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1) k_seq
 		if (!ok && lane == 0) atomicExch(err, 3);
 	}
 	const int gave_up = __syncthreads_or(!ok);
+	if (tid == 0) cluster_store(cluster_addr(&gave_up_s[rank], 0), gave_up);
 	cluster_sync();
-	// a wait gave up: copies that are on their way end before the CTAs do (a stage that one CTA alone asked for never fills: that wait runs out), and
-	// so do the MMAs on the stages multiplied last
-	if (rank == 0 && gave_up && tid == 0) {
-		const int most = max(asked[0], asked[1]);
+	// a wait gave up, in either CTA: what is on its way ends before the CTAs do.  Copies are counted in rank 0 (a stage that one CTA alone asked for never
+	// fills: that wait runs out); what the MMAs release and hand over arrives in both, and each CTA waits for its own arrivals
+	if (tid == 0 && (cluster_load(cluster_addr(&gave_up_s[0], 0)) | cluster_load(cluster_addr(&gave_up_s[1], 0)))) {
+		const int multiplied = cluster_load(cluster_addr(&multiplied_s, 0)), handed = cluster_load(cluster_addr(&handed_s, 0)), most = rank == 0 ? max(asked[0], asked[1]) : 0;
 		for (int i = max(0, most - TP_STAGES); i < most; ++i) mbar_wait_bounded(&full[i % TP_STAGES], (i / TP_STAGES) & 1, MBAR_SPINS / 16);
-		for (int i = max(0, multiplied_s - TP_STAGES); i < multiplied_s; ++i) mbar_wait_bounded(&empty[i % TP_STAGES], (i / TP_STAGES) & 1, MBAR_SPINS / 16);
+		for (int i = max(0, multiplied - TP_STAGES); i < multiplied; ++i) mbar_wait_bounded(&empty[i % TP_STAGES], (i / TP_STAGES) & 1, MBAR_SPINS / 16);
+		for (int i = max(0, handed - 2); i < handed; ++i) mbar_wait_bounded(&acc_full[i & 1], (i >> 1) & 1, MBAR_SPINS / 16);
 	}
 	cluster_sync();
 	if (warp == 1) {
@@ -380,6 +384,7 @@ struct TgState {
 	int* err_host = nullptr; // pinned + mapped
 	int* err_dev = nullptr;
 	int pairs = 0; // clusters of two CTAs that the device holds at a time
+	unsigned tries = MBAR_SPINS; // of a wait in the pairs' kernel
 	std::map<std::tuple<const void*, long, long, long, long, int>, CUtensorMap> maps;
 };
 static TgState g_tg;
@@ -408,6 +413,7 @@ static inline void gemm_tc_setup() {
 	});
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3(2 * 74), cfg.blockDim = dim3(TP_THREADS), cfg.dynamicSmemBytes = TP_SMEM;
+	if (const char* e = getenv("CALM_B200_SEQ_WAIT")) g_tg.tries = (unsigned)atol(e); // tests make the waits run out
 	CUDA_CHECK(cudaOccupancyMaxActiveClusters(&g_tg.pairs, k_seq_gemm_pair<EPI_F32>, &cfg));
 }
 // a stalled pipeline leaves its code here; read after the stream has been synchronised
@@ -469,7 +475,7 @@ static inline bool gemm_tc_launch(const GemmArgs& a, int batch, cudaStream_t str
 	tg_each([&](auto e) {
 		constexpr int E = decltype(e)::value;
 		if (E != kind) return;
-		if (pair) CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_seq_gemm_pair<E>, *mw, *mx, a, g_tg.err_dev));
+		if (pair) CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_seq_gemm_pair<E>, *mw, *mx, a, g_tg.err_dev, g_tg.tries));
 		else CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_seq_gemm_tc<E>, *mw, *mx, a, (int)(a.wbs != 0 && batch > 1), (int)(a.xbs != 0 && batch > 1), g_tg.err_dev));
 	});
 	return true;

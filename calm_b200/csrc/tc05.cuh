@@ -106,6 +106,14 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
 	asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
 	return a;
 }
+__device__ __forceinline__ void cluster_store(uint32_t addr, int v) { // a variable named by cluster_addr; read after a cluster_sync
+	asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ int cluster_load(uint32_t addr) {
+	int v;
+	asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+	return v;
+}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) { // a barrier named by cluster_addr
 	asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
