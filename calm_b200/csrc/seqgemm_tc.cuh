@@ -305,12 +305,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1) k_seq
 				__syncwarp();
 			}
 		}
-		if (lane == 0) {
-			if (!ok) atomicExch(err, 1);
-			cluster_store(cluster_addr(&asked[rank], 0), it);
-		}
+		if (lane == 0) cluster_store(cluster_addr(&asked[rank], 0), it);
 		// the stages' last releases arrive in this CTA: they do before it ends
+		const bool copied = ok;
 		for (int i = max(0, it - TP_STAGES); i < it && ok; ++i) ok = mbar_wait_warp(&empty[i % TP_STAGES], (i / TP_STAGES) & 1, tries);
+		if (!ok && lane == 0) atomicExch(err, copied ? 4 : 1);
 	} else if (warp == 1) {
 		if (rank == 0) {
 			int it = 0, n = 0, handed = 0;
