@@ -448,14 +448,27 @@ static inline bool gemm_tc_maps(const GemmArgs& a, int batch, const CUtensorMap*
 	return mw && mx;
 }
 // Products that run on pairs of CTAs, by estimated cycles: a 64-deep step takes a 256 x 256 tile 590 and a 128 x 128 tile 900 (two CTAs to an SM, or one), and
-// larger tiles bring 9000 more of launch, first loads and epilogue.  K = 2048, us with tiles of 128 / on pairs: 13888 rows, 2048 tokens 118 / 83; 700 tokens
-// 58 / 43; 6400 rows, 640 tokens 22.6 / 29.8 (75 tiles on 74 pairs), 2048 rows 20.1 / 20.0; K = 64: 20.3 / 21.3; K = 512: 7.4 / 9.1; K = 1024, 5632 rows, 640 tokens
-// 14.3 / 15.2, 1000 tokens 23.5 / 21.6.
+// larger tiles bring 9000 more of launch, first loads and epilogue, more where the epilogue reads what it adds to: nothing runs over the epilogues of a single wave,
+// and the smaller tiles' are half as long and, two to an SM, run over each other's products.  us alone with tiles of 128 / on pairs, K = 2048 unless given:
+//   plain, 13888 rows, 2048 tokens 118 / 83; 700 tokens 58 / 43; 8192 rows, 64 tokens 16.9 / 13.7, 128 17.6 / 14.9, 512 21.3 / 20.6; K = 1024 10.1 / 9.8, 11.0 / 10.7,
+//   13.6 / 14.3; 3072 rows, K = 1024, 256 tokens 10.7 / 13.2; gated units, 11264 rows, 64 tokens 23.5 / 20.1, 256 29.5 / 26.9, 2048 130.5 / 84.3;
+//   Dynamic Tanh added to the stream, 2048 rows, 256 tokens 24.2 / 26.3, 1024 28.0 / 28.1, 2048 32.2 / 30.3; K = 5632 43.7 / 38.3, 46.5 / 41.1, 51.6 / 45.2;
+//   added to the stream, 2048 rows, 64 tokens 17.4 / 17.5, 128 21.1 / 23.0, 256 22.3 / 26.8, 2048 26.2 / 30.4; K = 5632 38.5 / 29.5, 41.9 / 34.9, 42.6 / 43.8, 54.6 / 54.2;
+//   8192 rows, 512 tokens 30.2 / 34.2, 1024 (two waves) 60.4 / 53.4; 4096 rows, K = 1024, 2048 tokens (two waves) 41.9 / 43.8.
+// Between other launches a pair's start is hidden: by whole steps, the pairs' last column is 1 to 5 us lower where the products are deep (2048 rows added to the stream,
+// 256 / 1024 / 2048 tokens: K = 5632 4.2 less, 1.3 more, 2.4 less a product than with the smaller tiles; K = 2048, 512 / 1024 / 2048 tokens 5.1, 8.5, 2.5 more).
+static inline bool tg_pairs_pay(long M, long N, long K, int epi, long pairs) {
+	const long steps = (K + TG_BK - 1) / TG_BK, slots = 4 * pairs; // CTAs of the smaller tiles at a time
+	const long small = ((M + TG_BM - 1) / TG_BM) * ((N + TG_BN - 1) / TG_BN), large = ((M + TP_BM - 1) / TP_BM) * ((N + TP_BN - 1) / TP_BN);
+	const bool alone = small <= 5 * pairs / 2; // the smaller tiles are about one to an SM
+	long more = 9000;
+	if (epi == EPI_RES) more = large > pairs ? 14000 : N <= 224 ? 9000 + 30 * N : alone ? 24000 : 20000;
+	else if (epi == EPI_DYT_RES && N > 224 && alone) more = 15500;
+	return (large + pairs - 1) / pairs * steps * 590 + more < (small + slots - 1) / slots * steps * 900;
+}
 static inline bool tg_pairs(const GemmArgs& a, int batch) {
 	if (batch > 1 || a.seg || a.band_mode || g_tg.pairs < 1) return false;
-	const long steps = (a.K + TG_BK - 1) / TG_BK, slots = 4 * g_tg.pairs; // CTAs of the smaller tiles at a time
-	const long small = (long)((a.M + TG_BM - 1) / TG_BM) * ((a.N + TG_BN - 1) / TG_BN), large = (long)((a.M + TP_BM - 1) / TP_BM) * ((a.N + TP_BN - 1) / TP_BN);
-	return (large + g_tg.pairs - 1) / g_tg.pairs * steps * 590 + 9000 < (small + slots - 1) / slots * steps * 900;
+	return tg_pairs_pay(a.M, a.N, a.K, a.epi, g_tg.pairs);
 }
 // false: nothing was launched
 static inline bool gemm_tc_launch(const GemmArgs& a, int batch, cudaStream_t stream, bool pdl) {

@@ -1452,6 +1452,7 @@ extern "C" void* calm_b200_seq_upload(const void* host, size_t size) {
 }
 extern "C" void calm_b200_seq_free(void* p) { cudaFree(p); }
 extern "C" uint64_t calm_b200_seq_launch_count(void) { return g_seq_launches; }
+extern "C" int calm_b200_seq_pairs_pay(int rows, int tokens, int k, int epi, int pairs) { return tg_pairs_pay(rows, tokens, k, epi, pairs); }
 
 extern "C" void* calm_b200_seq_prepare(const struct SeqModel* model) {
 	int count = 0;

@@ -293,6 +293,9 @@ int calm_b200_seq_layer_runs(void* handle);
 void calm_b200_seq_read_trace(void* handle, int run, float* out);
 
 uint64_t calm_b200_seq_launch_count(void);
+/* whether a product of `rows` weight rows of k columns over `tokens` tokens with the epilogue `epi` runs on pairs of CTAs, on a device that holds
+   `pairs` of them at a time; for tests */
+int calm_b200_seq_pairs_pay(int rows, int tokens, int k, int epi, int pairs);
 void calm_b200_seq_timer_start(void* handle);
 float calm_b200_seq_timer_stop(void* handle);
 /* per-kernel-kind device time of the steps since set_perf(handle, 1): events around every launch (slow; for the bench's

@@ -54,3 +54,30 @@ def test_more_tiles_than_pairs():  # 74 x 2 tiles of logits, two to a pair
     with bovinex.from_tensors(cfg, t, "bfloat16", max_tokens=600, max_seqs=1, page=8) as m:
         got = m.step([m.open()], [toks], list(range(500)))
     assert tb.rel_err(got, bovinex_plain.forward(cfg, tb.as_f64(t), toks)) < tb.TOL["bfloat16"]
+
+
+# residual epilogues: deep products of one wave, with tiles that are full of tokens and that are not
+@pytest.mark.parametrize("n", [64, 127, 200, 257, 300])
+def test_two_addends(n):
+    cfg = tb.config([tb.attn(mlp={"ff": 6000, "kind": "dense"}), tb.gla(mlp={"ff": 6000, "kind": "dense"})], width=2040)
+    t, toks = tb.weights(cfg, 6), tb.tokens(cfg, n)
+    with bovinex.from_tensors(cfg, t, "bfloat16", max_tokens=400, max_seqs=1, page=8) as m:
+        got = m.step([m.open()], [toks], list(range(n)))
+    assert tb.rel_err(got, bovinex_plain.forward(cfg, tb.as_f64(t), toks)) < tb.TOL["bfloat16"]
+
+
+def test_two_addends_over_two_waves():  # 20 x 4 tiles
+    cfg = tb.config([tb.gla(mlp={"ff": 2048, "kind": "dense"})], width=5112)
+    t, toks = tb.weights(cfg, 6), tb.tokens(cfg, 1000)
+    with bovinex.from_tensors(cfg, t, "bfloat16", max_tokens=1100, max_seqs=1, page=8) as m:
+        got = m.step([m.open()], [toks], list(range(1000)))
+    assert tb.rel_err(got, bovinex_plain.forward(cfg, tb.as_f64(t), toks)) < tb.TOL["bfloat16"]
+
+
+@pytest.mark.parametrize("n", [65, 160, 287])
+def test_dynamic_tanh_of_deep_products(n):
+    cfg = tv.config([tv.window(mlp={"ff": 3500, "kind": "dense", "limit": 4.0}), tv.window(mlp={"ff": 3500, "kind": "dense", "limit": 4.0})], width=2040)
+    t, toks = tv.weights(cfg, 6), tv.tokens(cfg, n)
+    with vimulorn.from_tensors(cfg, t, "bfloat16", max_tokens=400, max_seqs=1, page=8) as m:
+        got = m.step([m.open()], [toks], list(range(n)))
+    assert tv.rel_err(got, vimulorn_plain.forward(cfg, tv.as_f64(t), toks)) < tv.TOL["bfloat16"]
