@@ -265,8 +265,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1) k_seq
 	extern __shared__ unsigned char smem_dyn[];
 	__shared__ __align__(8) uint64_t full[TP_STAGES], empty[TP_STAGES], acc_full[2], acc_empty[2]; // full, acc_empty: rank 0's are used
 	__shared__ uint32_t tmem_base_s;
-	// rank 0's, read when a wait has given up: whether one did in each CTA, stages that its copies got to, stages multiplied, accumulators handed over
-	__shared__ int gave_up_s[2], asked[2], multiplied_s, handed_s;
+	__shared__ int gave_up_s[2]; // whether a wait gave up in each of the CTAs
+	__shared__ int asked[2], multiplied_s, handed_s; // rank 0's, read when one did: stages that each CTA's copies got to, stages multiplied, accumulators handed over
 	unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = (int)cluster_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
 	const int nkb = (a.K + TG_BK - 1) / TG_BK, tok_tiles = (a.N + TP_BN - 1) / TP_BN, tiles = (a.M + TP_BM - 1) / TP_BM * tok_tiles;
@@ -358,11 +358,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1) k_seq
 		if (!ok && lane == 0) atomicExch(err, 3);
 	}
 	const int gave_up = __syncthreads_or(!ok);
-	if (tid == 0) cluster_store(cluster_addr(&gave_up_s[rank], 0), gave_up);
+	if (tid < 2) cluster_store(cluster_addr(&gave_up_s[rank], tid), gave_up);
 	cluster_sync();
 	// a wait gave up, in either CTA: what is on its way ends before the CTAs do.  Copies are counted in rank 0 (a stage that one CTA alone asked for never
 	// fills: that wait runs out); what the MMAs release and hand over arrives in both, and each CTA waits for its own arrivals
-	if (tid == 0 && (cluster_load(cluster_addr(&gave_up_s[0], 0)) | cluster_load(cluster_addr(&gave_up_s[1], 0)))) {
+	if (tid == 0 && (gave_up_s[0] | gave_up_s[1])) {
 		const int multiplied = cluster_load(cluster_addr(&multiplied_s, 0)), handed = cluster_load(cluster_addr(&handed_s, 0)), most = rank == 0 ? max(asked[0], asked[1]) : 0;
 		for (int i = max(0, most - TP_STAGES); i < most; ++i) mbar_wait_bounded(&full[i % TP_STAGES], (i / TP_STAGES) & 1, MBAR_SPINS / 16);
 		for (int i = max(0, multiplied - TP_STAGES); i < multiplied; ++i) mbar_wait_bounded(&empty[i % TP_STAGES], (i / TP_STAGES) & 1, MBAR_SPINS / 16);
