@@ -1456,7 +1456,8 @@ __global__ void __launch_bounds__(128) k_seq_delta_scan_reg(DeltaArgs a, SeqBatc
 // so the corrections of a block are one triangular system, U = X (V - (K G) S) with X = (1 + diag(beta) A)^-1 diag(beta), and the read-outs are (Q G) S + (B X) (V - (K G) S).
 // X and B X depend on no value: k_seq_delta_system forms them for all blocks side by side (and turns the raw decay inputs into decays, in place), and
 // k_seq_delta_blocks walks the state from block to block with products whose terms do not wait for one another.  The scan's chain of a token (dot, shuffles,
-// update: 0.75 us) becomes a block's: 3 x 700 tokens of 16 heads of 128 x 128 522 us, now DELTA_NOW.
+// update: 0.6 us, 1.7 where the CTAs take three waves) becomes a block's, 4.5 us, or 10 for three CTAs to an SM: 3 x 700 tokens of 16 heads of 128 x 128 504 -> 313 us, one
+// sequence of 2048 1263 -> 598, sixteen of 128 340 -> 211 (both kernels, timed apart).
 #define DELTA_BK 16
 struct DeltaBlocks {
 	float* sys; // [block][heads][2][DELTA_BK][DELTA_BK]: X, B X; block j of sequence b is number sstart[b] / DELTA_BK + b + j (one more than fit a portion at most)

@@ -841,11 +841,21 @@ void ensure_scan(Seq& s, size_t need) {
 	cudaFree(s.scan_ws); // decode graphs (one token per sequence) never read it
 	s.scan_ws = (float*)dalloc(need * sizeof(float)), s.scan_cap = need;
 }
-// Portions from this many tokens on are cut into chunks.  Scan against chunks, us a layer of 128 x 128: 16 heads, 200 tokens 57, 36; 256 66, 38; 2048 468, 140; two
-// sequences of 256 85, 52; 8 heads, 128 tokens 26, 27; 256 45, 31; 2048 298, 83.
+// Portions from this many tokens on are cut into chunks while every sequence gets two or more.  Scan against chunks, us a layer of 128 x 128: 16 heads, 128 tokens 38, 36; 160 43, 36;
+// 256 66, 41; 2048 467, 148; two sequences of 256 85, 59; three 138, 73 (three chunks each); four 139, 93 (two); one of 512 and three of 1 266, 135; 8 heads, 128 tokens 27, 34;
+// 160 31, 31; 256 44, 33; 2048 298, 91; 16 heads of 64 x 64, 160 tokens 27, 28; four of 160 37, 39; four of 256 56, 46; 132 value columns (a normaliser's beside 128), 160 tokens 44, 41;
+// 256 66, 52; three of 256 139, 110 (two chunks).  In whole steps the two further launches are hidden and every one of these gains: 128 tokens 14 to 22 us a layer, four of 160 of
+// 64 x 64 25.
 const int kGlaChunksMin = 160;
-// ... and run through the delta rule in blocks
+// The delta rule runs in blocks when the step's longest portion has this many tokens, and more while there are `few` portions with fewer, which a block costs as much as a
+// whole one: about 20 tokens for every wave of their CTAs (three to an SM).  Scan against blocks, us a layer of 16 heads of 128 x 128: one sequence of 16 tokens 18, 25; 32 27, 28;
+// 48 37, 31; 128 84, 53; four of 32 32, 32; sixteen of 32 97, 70.  A portion of 32 and fifteen of 1 40, 50; of 64 63, 66; of 128 107, 91; 32 heads, of 64 81, 98; of 128 133, 131; of 300
+// 267, 217; 16 heads, of 64 and sixty-three of 1 100, 150; of 300 269, 257 (whole steps, where the second launch is hidden, are 5 to 11 us a layer kinder to blocks).
 const int kDeltaBlocksMin = 32;
+bool delta_blocks_pay(int longest, int few, int heads, int vdim, int sms) {
+	const long ctas = (long)few * heads * cdiv(vdim, DELTA_VC);
+	return longest >= kDeltaBlocksMin && longest >= 20 + 20 * ctas / (3L * sms);
+}
 
 // the gated-linear-attention scan over a step's tokens: S <- diag(decay) S + k v^T, o = S^T q * qscale per (sequence, head); g names
 // the inputs (columns of a matrix with row stride ld), the state and the output
@@ -985,9 +995,9 @@ void mixer_typed(Seq& s, const SeqLayer& L, RunState& r, const SeqBatch& sb, dou
 		const size_t smem = ((size_t)D * Dv + 3 * D) * sizeof(float);
 		const int threads = std::max(64, cdiv(Dv, 32) * 32);
 		const bool reg = (D == 32 || D == 64 || D == 128) && Dv <= 128 && Dv % 4 == 0 && !getenv("CALM_B200_SEQ_DELTA_SMEM");
-		int longest_portion = 0;
-		for (int b = 0; b < sb.B; ++b) longest_portion = std::max(longest_portion, s.hb_count[b]);
-		const bool blocks = reg && D == 128 && longest_portion >= kDeltaBlocksMin;
+		int longest_portion = 0, few = 0;
+		for (int b = 0; b < sb.B; ++b) longest_portion = std::max(longest_portion, s.hb_count[b]), few += s.hb_count[b] < kDeltaBlocksMin;
+		const bool blocks = reg && D == 128 && delta_blocks_pay(longest_portion, few, H, Dv, s.sms);
 		DeltaBlocks db{nullptr, s.f[3], cdiv(longest_portion, DELTA_BK)};
 		if (blocks) {
 			ensure_scan(s, (size_t)(N / DELTA_BK + sb.B) * H * 2 * DELTA_BK * DELTA_BK);
@@ -1452,6 +1462,7 @@ extern "C" void* calm_b200_seq_upload(const void* host, size_t size) {
 }
 extern "C" void calm_b200_seq_free(void* p) { cudaFree(p); }
 extern "C" uint64_t calm_b200_seq_launch_count(void) { return g_seq_launches; }
+extern "C" int calm_b200_seq_delta_blocks_pay(int longest, int few, int heads, int vdim, int sms) { return delta_blocks_pay(longest, few, heads, vdim, sms); }
 extern "C" int calm_b200_seq_pairs_pay(int rows, int tokens, int k, int epi, int pairs) { return tg_pairs_pay(rows, tokens, k, epi, pairs); }
 
 extern "C" void* calm_b200_seq_prepare(const struct SeqModel* model) {

@@ -293,6 +293,9 @@ int calm_b200_seq_layer_runs(void* handle);
 void calm_b200_seq_read_trace(void* handle, int run, float* out);
 
 uint64_t calm_b200_seq_launch_count(void);
+/* whether the delta rule of a step runs in blocks of tokens: its longest portion, how many portions have fewer tokens than the least that blocks pay
+   for, heads, value columns of a head, SMs; for tests */
+int calm_b200_seq_delta_blocks_pay(int longest, int few, int heads, int vdim, int sms);
 /* whether a product of `rows` weight rows of k columns over `tokens` tokens with the epilogue `epi` runs on pairs of CTAs, on a device that holds
    `pairs` of them at a time; for tests */
 int calm_b200_seq_pairs_pay(int rows, int tokens, int k, int epi, int pairs);
