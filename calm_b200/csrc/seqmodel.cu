@@ -20,6 +20,7 @@
 namespace {
 
 uint64_t g_seq_launches = 0;
+uint64_t g_seq_routes[32] = {}; // by SEQ_ROUTE_*
 
 enum Kind { KD_EMBED, KD_NORM, KD_GEMM, KD_GEMM_TC, KD_GEMM_SKINNY, KD_CONV, KD_ATTN_LATENT, KD_ATTN_WINDOW, KD_DELTA, KD_ELEMENT, KD_QK, KD_GLA, KD_ROUTE, KD_HYPER, KD_LINPREP, KD_MINGRU, KD_COUNT };
 const char* const kKindNames[KD_COUNT] = {"embed", "norm", "gemm", "gemm_tcgen05", "gemm_skinny", "conv", "attention_latent", "attention_window", "delta_scan", "elementwise",
@@ -383,12 +384,12 @@ void drop_graphs(Seq& s) {
 void reserve_tokens(Seq& s, int N, int B, int W) {
 	const size_t meta = (size_t)6 * N + 4 * B + W;
 	if (meta > s.cap_meta || N > s.cap_tokens || W > s.cap_want) drop_graphs(s); // captured launches hold the old addresses
-	if (meta > s.cap_meta) {
+	if (meta > s.cap_meta) { // at least twice as much: steps that want a row more each time would move it every time, and with it all captured launches
 		CUDA_CHECK(cudaStreamSynchronize(s.stream));
 		cudaFree(s.meta_dev), cudaFreeHost(s.meta);
-		s.meta_dev = (int*)dalloc(meta * sizeof(int));
-		CUDA_CHECK(cudaHostAlloc((void**)&s.meta, meta * sizeof(int), cudaHostAllocDefault));
-		s.cap_meta = meta;
+		s.cap_meta = std::max(meta, 2 * s.cap_meta);
+		s.meta_dev = (int*)dalloc(s.cap_meta * sizeof(int));
+		CUDA_CHECK(cudaHostAlloc((void**)&s.meta, s.cap_meta * sizeof(int), cudaHostAllocDefault));
 	}
 	if (W > s.cap_want) {
 		CUDA_CHECK(cudaStreamSynchronize(s.stream));
@@ -1439,6 +1440,7 @@ void forward_decode_graph(Seq& s, const SeqBatch& sb, int n_want, double kv_rows
 		const uint64_t before = g_seq_launches;
 		cudaGraph_t graph = nullptr;
 		cudaGraphExec_t exec = nullptr;
+		++g_seq_routes[SEQ_ROUTE_CAPTURE];
 		CUDA_CHECK(cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal));
 		forward(s, sb, n_want, kv_rows, longest);
 		CUDA_CHECK(cudaStreamEndCapture(s.stream, &graph));
@@ -1462,6 +1464,7 @@ extern "C" void* calm_b200_seq_upload(const void* host, size_t size) {
 }
 extern "C" void calm_b200_seq_free(void* p) { cudaFree(p); }
 extern "C" uint64_t calm_b200_seq_launch_count(void) { return g_seq_launches; }
+extern "C" uint64_t calm_b200_seq_route_count(int route) { return route >= 0 && route < 32 ? g_seq_routes[route] : 0; }
 extern "C" int calm_b200_seq_delta_blocks_pay(int longest, int few, int heads, int vdim, int sms) { return delta_blocks_pay(longest, few, heads, vdim, sms); }
 extern "C" int calm_b200_seq_pairs_pay(int rows, int tokens, int k, int epi, int pairs) { return tg_pairs_pay(rows, tokens, k, epi, pairs); }
 

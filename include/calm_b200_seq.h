@@ -293,6 +293,9 @@ int calm_b200_seq_layer_runs(void* handle);
 void calm_b200_seq_read_trace(void* handle, int run, float* out);
 
 uint64_t calm_b200_seq_launch_count(void);
+/* how often a way through the runtime has been taken since the library was loaded; for tests */
+enum { SEQ_ROUTE_CAPTURE = 0 /* a decode step was captured */ };
+uint64_t calm_b200_seq_route_count(int route);
 /* whether the delta rule of a step runs in blocks of tokens: its longest portion, how many portions have fewer tokens than the least that blocks pay
    for, heads, value columns of a head, SMs; for tests */
 int calm_b200_seq_delta_blocks_pay(int longest, int few, int heads, int vdim, int sms);
