@@ -1382,8 +1382,20 @@ static void pf_tail(int tiles, int nkb, int sms, int na, int bn, int& tail_out, 
 		if (gain > best) best = gain, tail_out = tail, splits_out = sp;
 	}
 }
+// what is launched: pf_tiles' choice, with all tiles in slices (the tail is all of them) or the last ones only
+static int pf_cut(int mode, int rows, int n, int nkb, int sms, int& na, int& bn, int& tail, int& splits) {
+	pf_tiles(mode, rows, n, nkb, sms, na, bn, splits);
+	const int tiles = (mode == PF_UP ? rows / PF_BM : cdiv(rows / PF_BM, na)) * cdiv(n, bn);
+	if (splits > 1) tail = tiles;
+	else pf_tail(tiles, nkb, sms, na, bn, tail, splits);
+	return tiles;
+}
+static int pf_mode(int product) { return product == 0 ? PF_QKV : product == 1 ? PF_RES : PF_UP; }
 extern "C" void calm_b200_prefill_tiles(int product, int rows, int n, int k, int sms, int* out3) {
-	pf_tiles(product == 0 ? PF_QKV : product == 1 ? PF_RES : PF_UP, rows, n, k / PF_BK, sms, out3[0], out3[1], out3[2]);
+	pf_tiles(pf_mode(product), rows, n, k / PF_BK, sms, out3[0], out3[1], out3[2]);
+}
+extern "C" void calm_b200_prefill_cut(int product, int rows, int n, int k, int sms, int* out5) {
+	out5[0] = pf_cut(pf_mode(product), rows, n, k / PF_BK, sms, out5[1], out5[2], out5[3], out5[4]);
 }
 
 template <int MODE, int DBITS>
@@ -1392,10 +1404,7 @@ static void pf_gemm(const CUtensorMap (&tx)[3][2], const CUtensorMap* tw, PfGemm
 	static bool opted = false;
 	if (!opted) smem_optin(k_pf_gemm<MODE, DBITS>, limit), opted = true;
 	same_carveout((const void*)k_pf_gemm<MODE, DBITS>);
-	pf_tiles(MODE, rows, n, a.K / PF_BK, g.sms, a.na, a.bn, a.splits);
-	const int tiles = (MODE == PF_UP ? rows / PF_BM : cdiv(rows / PF_BM, a.na)) * cdiv(n, a.bn);
-	a.tail = a.splits > 1 ? tiles : 0;
-	if (a.splits == 1) pf_tail(tiles, a.K / PF_BK, g.sms, a.na, a.bn, a.tail, a.splits);
+	const int tiles = pf_cut(MODE, rows, n, a.K / PF_BK, g.sms, a.na, a.bn, a.tail, a.splits);
 	PfMaps m;
 	memcpy(m.x, tx[a.bn / 128], sizeof(m.x)); // 64, 128, 256 -> 0, 1, 2
 	memcpy(m.w, tw, (MODE == PF_QKV ? 3 : MODE == PF_UP ? 2 : 1) * sizeof(CUtensorMap));

@@ -30,6 +30,7 @@ SYMBOLS = [
     "calm_b200_tp_unique_id", "calm_b200_tp_init", "calm_b200_tp_world", "calm_b200_tp_mode",
     "calm_b200_decode_sample", "calm_b200_forward_sample", "calm_b200_read_device_logits", "calm_b200_sample_logits",
     "calm_b200_prefill_tiles",
+    "calm_b200_prefill_cut",
 ]
 
 _lib = None
@@ -79,7 +80,8 @@ def load() -> C.CDLL:
     L.calm_b200_read_device_logits.argtypes, L.calm_b200_read_device_logits.restype = [_fptr], None
     L.calm_b200_sample_logits.argtypes = [_fptr, C.c_int, C.c_float, C.c_float, C.POINTER(C.c_ulonglong), _fptr]
     L.calm_b200_sample_logits.restype = C.c_int
-    L.calm_b200_prefill_tiles.argtypes, L.calm_b200_prefill_tiles.restype = [C.c_int] * 5 + [C.POINTER(C.c_int)], None
+    for f in (L.calm_b200_prefill_tiles, L.calm_b200_prefill_cut):
+        f.argtypes, f.restype = [C.c_int] * 5 + [C.POINTER(C.c_int)], None
     _lib = L
     return L
 

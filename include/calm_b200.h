@@ -106,6 +106,9 @@ int forward_prefill_cuda(struct Transformer* transformer, const int* tokens, int
 /* How a product of the pass over n tokens is cut on a GPU of `sms` SMs (no GPU needed; for tests and measurements): product 0 q/k/v, 1 wo and w2, 2 FFN
  * up (rows of one of its matrices); out3 = row tiles of 128 per item, tokens per item, slices of k. */
 void calm_b200_prefill_tiles(int product, int rows, int n, int k, int sms, int* out3);
+/* the same with what becomes of the tiles past the last whole wave: out5 = {tiles, row tiles per item, tokens per item, tiles that are cut into K-slices
+ * (all of them, the last ones, none), slices of each} */
+void calm_b200_prefill_cut(int product, int rows, int n, int k, int sms, int* out5);
 
 /* forward + device-side greedy sample.  Returns argmax(logits) with the
  * reference's tie rule (lowest index, sampler.c:34-42).  The logits are still

@@ -1,5 +1,6 @@
-"""How the products of a prompt are cut (calm_b200_prefill_tiles) and that every cut it makes computes the same: each combination of row tiles and tokens per item
-and sliced or whole k that the rule picks anywhere in the range is run by one of the shapes here or in test_prefill_tiles_gpu.py."""
+"""How the products of a prompt are cut (calm_b200_prefill_cut) and that every cut it makes computes the same: each combination of row tiles and tokens per item
+and tiles that are whole, in K-slices, or whole with a tail in slices that the rules pick anywhere in the range is run by one of the shapes here, in
+test_prefill_tiles_gpu.py or in test_prefill_tails_gpu.py."""
 import ctypes as C
 import os
 import sys
@@ -10,6 +11,7 @@ import torch
 
 sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
 from test_prefill_gpu import _both, _check  # noqa: E402
+from test_prefill_tails_gpu import TAILS  # noqa: E402
 
 from calm_b200 import build as cbuild  # noqa: E402
 from calm_b200 import lib  # noqa: E402
@@ -17,27 +19,27 @@ from calm_b200 import modelgen as mg  # noqa: E402
 
 SMS = 148
 # dim, heads, kv heads, head_dim, hidden, tokens, and the cuts that only this shape reaches
-SHAPES = [(896, 14, 2, 64, 4864, 449, {("res", 1, 128, True)}), (896, 14, 2, 64, 4864, 1537, {("qkv", 2, 64, False), ("res", 1, 256, True), ("res", 2, 64, False)}),
-          (768, 6, 2, 128, 2688, 1550, {("res", 2, 128, True)}), (384, 3, 3, 128, 384, 1900, {("qkv", 1, 128, False)}), (896, 7, 7, 128, 896, 1717, {("qkv", 1, 256, False)}),
-          (1536, 12, 12, 128, 1536, 1595, {("qkv", 2, 128, False), ("res", 2, 128, False)}), (3072, 24, 8, 128, 6144, 67, {("up", 2, 128, True)}),
-          (4096, 32, 32, 128, 1024, 70, {("qkv", 2, 128, True), ("up", 2, 64, True)})]
-ELSEWHERE = [(384, 384, 128, 1152, 1), (896, 896, 128, 2432, 61), (1024, 1024, 256, 3456, 65), (2048, 2048, 512, 5504, 257), (4096, 4096, 1024, 14336, 130)]
+SHAPES = [(896, 14, 2, 64, 4864, 449, {("res", 1, 128, "slices")}), (896, 14, 2, 64, 4864, 1537, {("qkv", 2, 64, "whole"), ("res", 1, 256, "slices"), ("res", 2, 64, "whole")}),
+          (768, 6, 2, 128, 2688, 1550, {("res", 2, 128, "slices")}), (384, 3, 3, 128, 384, 1900, {("qkv", 1, 128, "whole")}), (896, 7, 7, 128, 896, 1717, {("qkv", 1, 256, "whole")}),
+          (1536, 12, 12, 128, 1536, 1595, {("qkv", 2, 128, "whole"), ("res", 2, 128, "whole")}), (3072, 24, 8, 128, 6144, 67, {("up", 2, 128, "slices")}),
+          (4096, 32, 32, 128, 1024, 70, {("qkv", 2, 128, "slices"), ("up", 2, 64, "slices")})]
+ELSEWHERE = [(dim, dim, dim, hidden, n) for dim, hidden, n, _ in TAILS] + [(384, 384, 128, 1152, 1), (896, 896, 128, 2432, 61), (1024, 1024, 256, 3456, 65), (2048, 2048, 512, 5504, 257), (4096, 4096, 1024, 14336, 130)]
 
 
 @pytest.fixture(scope="module")
 def cuts():
     cbuild.build()
-    L, out = lib.load(), (C.c_int * 3)()
+    L, out = lib.load(), (C.c_int * 5)()
 
     def of(dim, q_dim, kv_dim, hidden, n):
         got = set()
         for name, product, rows, k in (("qkv", 0, q_dim + 2 * kv_dim, dim), ("res", 1, dim, q_dim), ("up", 2, hidden, dim), ("res", 1, dim, hidden)):
-            L.calm_b200_prefill_tiles(product, rows, n, k, SMS, out)
-            na, bn, sp = out
-            items = (rows // 128 if name == "up" else -(-rows // 128 // na)) * -(-n // bn)
+            L.calm_b200_prefill_cut(product, rows, n, k, SMS, out)
+            tiles, na, bn, tail, sp = out
             # the accumulators fit half of TMEM; a slice is not empty; partial sums and counters of sliced products have one place per SM
-            assert na in (1, 2) and bn in (64, 128, 256) and na * bn <= 256 and (name != "up" or na == 2) and 1 <= sp <= k // 64 and (sp == 1 or items * sp <= SMS)
-            got.add((name, na, bn, sp > 1))
+            assert na in (1, 2) and bn in (64, 128, 256) and na * bn <= 256 and (name != "up" or na == 2) and 1 <= sp <= k // 64
+            assert tiles == (rows // 128 if name == "up" else -(-rows // 128 // na)) * -(-n // bn) and tail * sp <= SMS and (tail == 0) == (sp == 1) and tail in (0, tiles, tiles % SMS)
+            got.add((name, na, bn, "whole" if tail == 0 else "slices" if tail == tiles else "tail"))
         return got
 
     return of
