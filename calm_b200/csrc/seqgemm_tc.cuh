@@ -45,6 +45,7 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
 // unrolled TG_ANY, 743 in instances of their own, 652 without conditions per element, 545 with the large ones on pairs of CTAs (below).
 #define TG_ANY (-1)
 #define TG_ACT_GATE 100 // EPI_ACT times sigmoid(gate)
+#define TG_EPILOGUES 8  // EPI_*
 // Tokens [c0, c1) of the tile.  A run of 32 tokens that are all there, for 32 rows that are all there, takes a path without a condition per element: with
 // them a warp stored one token in a hundred cycles, and a 256 x 256 tile's epilogue took as long as its products (K = 2048).
 template <int E>
@@ -383,6 +384,7 @@ struct TgState {
 	int* err_host = nullptr; // pinned + mapped
 	int* err_dev = nullptr;
 	int pairs = 0; // clusters of two CTAs that the device holds at a time
+	uint64_t pair_launches[TG_EPILOGUES] = {}; // by EPI_*
 	unsigned tries = MBAR_SPINS; // of a wait in the pairs' kernel
 	std::map<std::tuple<const void*, long, long, long, long, int>, CUtensorMap> maps;
 };
@@ -484,6 +486,7 @@ static inline bool gemm_tc_launch(const GemmArgs& a, int batch, cudaStream_t str
 	at[0].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = at, cfg.numAttrs = pdl ? 1 : 0;
 	const int kind = tg_kind(a);
+	if (pair) ++g_tg.pair_launches[a.epi];
 	tg_each([&](auto e) {
 		constexpr int E = decltype(e)::value;
 		if (E != kind) return;

@@ -20,7 +20,7 @@
 namespace {
 
 uint64_t g_seq_launches = 0;
-uint64_t g_seq_routes[32] = {}; // by SEQ_ROUTE_*
+uint64_t g_seq_routes[SEQ_ROUTE_PAIRS] = {}; // by SEQ_ROUTE_*
 
 enum Kind { KD_EMBED, KD_NORM, KD_GEMM, KD_GEMM_TC, KD_GEMM_SKINNY, KD_CONV, KD_ATTN_LATENT, KD_ATTN_WINDOW, KD_DELTA, KD_ELEMENT, KD_QK, KD_GLA, KD_ROUTE, KD_HYPER, KD_LINPREP, KD_MINGRU, KD_COUNT };
 const char* const kKindNames[KD_COUNT] = {"embed", "norm", "gemm", "gemm_tcgen05", "gemm_skinny", "conv", "attention_latent", "attention_window", "delta_scan", "elementwise",
@@ -875,6 +875,7 @@ void gla_launch(Seq& s, GlaArgs& g, const SeqBatch& sb, int ld) {
 		const size_t units = (size_t)sb.B * c.count * H;
 		ensure_scan(s, units * D * (Dv + 1));
 		c.add = s.scan_ws, c.keep = s.scan_ws + units * D * Dv;
+		++g_seq_routes[SEQ_ROUTE_GLA_CHUNKS];
 		const double bytes = (double)N * H * (3.0 * D + 2.0 * Dv) * 4 + 2.0 * sb.B * H * D * Dv * 4, flops = (double)N * H * D * Dv * 4.0;
 		auto go = [&](auto local, auto starts, auto apply) {
 			run_kernel(s, KD_GLA, 0, 0, [&] { launch_k(s, local, dim3(sb.B * c.count, H, cdiv(Dv, 128)), 2 * D, glc_smem(D), g, c, sb); });
@@ -1003,6 +1004,7 @@ void mixer_typed(Seq& s, const SeqLayer& L, RunState& r, const SeqBatch& sb, dou
 		if (blocks) {
 			ensure_scan(s, (size_t)(N / DELTA_BK + sb.B) * H * 2 * DELTA_BK * DELTA_BK);
 			db.sys = s.scan_ws;
+			++g_seq_routes[SEQ_ROUTE_DELTA_BLOCKS];
 			run_kernel(s, KD_DELTA, 0, 0, [&] { launch_k(s, k_seq_delta_system, dim3(sb.B * db.count, H), 512, 0, d, db, sb); });
 		}
 		run_kernel(s, KD_DELTA, (double)N * H * (3.0 * D + 2.0 * Dv) * 4 + 2.0 * sb.B * H * D * Dv * 4, (double)N * H * D * Dv * 6.0, [&] {
@@ -1464,7 +1466,7 @@ extern "C" void* calm_b200_seq_upload(const void* host, size_t size) {
 }
 extern "C" void calm_b200_seq_free(void* p) { cudaFree(p); }
 extern "C" uint64_t calm_b200_seq_launch_count(void) { return g_seq_launches; }
-extern "C" uint64_t calm_b200_seq_route_count(int route) { return route >= 0 && route < 32 ? g_seq_routes[route] : 0; }
+extern "C" uint64_t calm_b200_seq_route_count(int route) { return route >= SEQ_ROUTE_PAIRS ? (route < SEQ_ROUTE_PAIRS + TG_EPILOGUES ? g_tg.pair_launches[route - SEQ_ROUTE_PAIRS] : 0) : route >= 0 ? g_seq_routes[route] : 0; }
 extern "C" int calm_b200_seq_delta_blocks_pay(int longest, int few, int heads, int vdim, int sms) { return delta_blocks_pay(longest, few, heads, vdim, sms); }
 extern "C" int calm_b200_seq_pairs_pay(int rows, int tokens, int k, int epi, int pairs) { return tg_pairs_pay(rows, tokens, k, epi, pairs); }
 

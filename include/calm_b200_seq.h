@@ -294,7 +294,12 @@ void calm_b200_seq_read_trace(void* handle, int run, float* out);
 
 uint64_t calm_b200_seq_launch_count(void);
 /* how often a way through the runtime has been taken since the library was loaded; for tests */
-enum { SEQ_ROUTE_CAPTURE = 0 /* a decode step was captured */ };
+enum {
+	SEQ_ROUTE_CAPTURE = 0,      /* a decode step was captured */
+	SEQ_ROUTE_GLA_CHUNKS = 1,   /* a layer's gated linear attention ran as chunks of tokens */
+	SEQ_ROUTE_DELTA_BLOCKS = 2, /* a layer's delta rule ran in blocks of tokens */
+	SEQ_ROUTE_PAIRS = 16        /* + epilogue: a product was launched (or captured) on pairs of CTAs */
+};
 uint64_t calm_b200_seq_route_count(int route);
 /* whether the delta rule of a step runs in blocks of tokens: its longest portion, how many portions have fewer tokens than the least that blocks pay
    for, heads, value columns of a head, SMs; for tests */

@@ -11,9 +11,13 @@ sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
 import test_vimulorn_gpu as tv  # noqa: E402
 import vimulorn_plain  # noqa: E402
 
-from calm_b200 import vimulorn  # noqa: E402
+from calm_b200 import seqlib, vimulorn  # noqa: E402
 
 pytestmark = pytest.mark.gpu
+
+
+def in_blocks():  # layers that ran in blocks so far (SEQ_ROUTE_DELTA_BLOCKS)
+    return seqlib.load().calm_b200_seq_route_count(2)
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
@@ -24,7 +28,7 @@ def test_blocks(dtype, heads, kv, vdim, counts):
     toks[5:25] = [toks[5]] * 20
     ref = vimulorn_plain.forward(cfg, tv.as_f64(t), toks)
     with vimulorn.from_tensors(cfg, t, dtype, max_tokens=900, max_seqs=3, page=8) as m:
-        slots = [m.open() for _ in counts]
+        slots, ran = [m.open() for _ in counts], in_blocks()
         at = np.cumsum((0,) + counts)
         out = m.step(slots, [toks[:n] for n in counts], list(range(sum(counts))))
         for i, n in enumerate(counts):
@@ -32,7 +36,9 @@ def test_blocks(dtype, heads, kv, vdim, counts):
         out = m.step(slots, [toks[n:n + 59] for n in counts], list(range(59 * len(counts))))
         for i, n in enumerate(counts):
             assert tv.rel_err(out[59 * i:59 * (i + 1)], ref[n:n + 59]) < tv.TOL[dtype], n
+        assert in_blocks() == ran + 2
         out = m.step(slots, [toks[n + 59:n + 60] for n in counts], list(range(len(counts))))
+        assert in_blocks() == ran + 2
         for i, n in enumerate(counts):
             assert tv.rel_err(out[i:i + 1], ref[n + 59:n + 60]) < tv.TOL[dtype], n
 
@@ -46,5 +52,7 @@ def test_no_later_value_reaches_an_earlier_token(dtype, bad):
     t["embed"][95] = float("nan")
     toks[bad] = 95
     with vimulorn.from_tensors(cfg, t, dtype, max_tokens=64, max_seqs=1, page=8) as m:
+        ran = in_blocks()
         out = m.step([m.open()], [toks], list(range(44)))
+        assert in_blocks() == ran + 1
     assert tv.rel_err(out[:bad], ref[:bad]) < tv.TOL[dtype] and np.isnan(out[bad:]).all()
