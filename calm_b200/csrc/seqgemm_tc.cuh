@@ -389,6 +389,9 @@ struct TgState {
 	std::map<std::tuple<const void*, long, long, long, long, int>, CUtensorMap> maps;
 };
 static TgState g_tg;
+// the pairs' kernel has no instances for the epilogues of products per head, of a decay's low rank and of rows that are all squared rectifiers (a shared unit
+// without gate and router rows): none of the families has large ones of them
+static constexpr bool tg_pair_instance(int kind) { return kind != EPI_SPLIT3 && kind != TG_ACT_GATE && kind != EPI_DECAY && kind != EPI_ACT_RELU2; }
 // f(instance) for every instance of the kernels
 template <typename F>
 static inline void tg_each(F&& f) {
@@ -410,7 +413,7 @@ static inline void gemm_tc_setup() {
 	tg_each([&](auto e) {
 		constexpr int E = decltype(e)::value;
 		CUDA_CHECK(cudaFuncSetAttribute(k_seq_gemm_tc<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, TG_SMEM));
-		CUDA_CHECK(cudaFuncSetAttribute(k_seq_gemm_pair<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM));
+		if constexpr (tg_pair_instance(E)) CUDA_CHECK(cudaFuncSetAttribute(k_seq_gemm_pair<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM));
 	});
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3(2 * 74), cfg.blockDim = dim3(TP_THREADS), cfg.dynamicSmemBytes = TP_SMEM;
@@ -469,7 +472,7 @@ static inline bool tg_pairs_pay(long M, long N, long K, int epi, long pairs) {
 	return (large + pairs - 1) / pairs * steps * 590 + more < (small + slots - 1) / slots * steps * 900;
 }
 static inline bool tg_pairs(const GemmArgs& a, int batch) {
-	if (batch > 1 || a.seg || a.band_mode || g_tg.pairs < 1) return false;
+	if (batch > 1 || a.seg || a.band_mode || g_tg.pairs < 1 || !tg_pair_instance(tg_kind(a))) return false;
 	return tg_pairs_pay(a.M, a.N, a.K, a.epi, g_tg.pairs);
 }
 // false: nothing was launched
@@ -490,8 +493,12 @@ static inline bool gemm_tc_launch(const GemmArgs& a, int batch, cudaStream_t str
 	tg_each([&](auto e) {
 		constexpr int E = decltype(e)::value;
 		if (E != kind) return;
-		if (pair) CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_seq_gemm_pair<E>, *mw, *mx, a, g_tg.err_dev, g_tg.tries));
-		else CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_seq_gemm_tc<E>, *mw, *mx, a, (int)(a.wbs != 0 && batch > 1), (int)(a.xbs != 0 && batch > 1), g_tg.err_dev));
+		if constexpr (tg_pair_instance(E))
+			if (pair) {
+				CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_seq_gemm_pair<E>, *mw, *mx, a, g_tg.err_dev, g_tg.tries));
+				return;
+			}
+		CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_seq_gemm_tc<E>, *mw, *mx, a, (int)(a.wbs != 0 && batch > 1), (int)(a.xbs != 0 && batch > 1), g_tg.err_dev));
 	});
 	return true;
 }

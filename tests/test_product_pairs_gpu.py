@@ -20,7 +20,7 @@ pytestmark = pytest.mark.gpu
 
 FF = {"ff": 2000, "kind": "dense"}
 CAPTURE, PAIRS = 0, 16  # SEQ_ROUTE_*
-F32, DYT, RES, GLU = 0, 2, 3, 7  # EPI_*
+F32, ACT, DYT, RES, GLU = 0, 1, 2, 3, 7  # EPI_*
 
 
 @pytest.fixture
@@ -98,6 +98,15 @@ def test_dynamic_tanh_of_deep_products(n, on_pairs):
         got = m.step([m.open()], [toks], list(range(n)))
     assert tv.rel_err(got, vimulorn_plain.forward(cfg, tv.as_f64(t), toks)) < tv.TOL["bfloat16"]
     assert on_pairs(DYT) >= 2
+
+
+def test_queries_from_a_deep_latent(on_pairs):
+    cfg = tv.config([tv.latent(heads=3, dim=24, q_rank=2048, mlp=None)], width=64)
+    t, toks = tv.weights(cfg, 6), tv.tokens(cfg, 100)
+    with vimulorn.from_tensors(cfg, t, "bfloat16", max_tokens=400, max_seqs=1, page=8) as m:
+        got = m.step([m.open()], [toks], list(range(100)))
+    assert tv.rel_err(got, vimulorn_plain.forward(cfg, tv.as_f64(t), toks)) < tv.TOL["bfloat16"]
+    assert on_pairs(ACT) >= 1
 
 
 def test_shallow_products_stay_on_one_cta(on_pairs):
