@@ -22,9 +22,10 @@ namespace {
 uint64_t g_seq_launches = 0;
 uint64_t g_seq_routes[SEQ_ROUTE_PAIRS] = {}; // by SEQ_ROUTE_*
 
-enum Kind { KD_EMBED, KD_NORM, KD_GEMM, KD_GEMM_TC, KD_GEMM_SKINNY, KD_CONV, KD_ATTN_LATENT, KD_ATTN_WINDOW, KD_DELTA, KD_ELEMENT, KD_QK, KD_GLA, KD_ROUTE, KD_HYPER, KD_LINPREP, KD_MINGRU, KD_COUNT };
+enum Kind { KD_EMBED, KD_NORM, KD_GEMM, KD_GEMM_TC, KD_GEMM_SKINNY, KD_CONV, KD_ATTN_LATENT, KD_ATTN_WINDOW, KD_DELTA, KD_ELEMENT, KD_QK, KD_GLA, KD_ROUTE, KD_HYPER, KD_LINPREP, KD_MINGRU, KD_GLA_CHUNKS, KD_DELTA_BLOCKS, KD_COUNT };
 const char* const kKindNames[KD_COUNT] = {"embed", "norm", "gemm", "gemm_tcgen05", "gemm_skinny", "conv", "attention_latent", "attention_window", "delta_scan", "elementwise",
-                                          "qk_prep", "gla_scan", "moe_route", "hyper", "lin_prep", "mingru_scan"};
+                                          "qk_prep", "gla_scan", "moe_route", "hyper", "lin_prep", "mingru_scan",
+                                          "gla_chunks", "delta_blocks"}; // (three and two launches a layer, the layer's bytes and operations with the last)
 
 // what one run of a layer owns (a looped layer has one of these per pass)
 struct RunState {
@@ -93,7 +94,7 @@ struct Seq {
 	float* lin = nullptr;                             // scan input of the linear recurrences served by the gated-linear-attention scan: rows [q | k | v]
 	size_t w_lin = 0;
 	int streams = 1;
-	bool h_ready = false;                             // hyper blocks: hA already holds the next sublayer's normed input (the last write formed it)
+	bool h_ready = false;                             // hyper, sandwich and serial blocks: hA already holds the next layer's normed input (what last wrote the stream formed it)
 	// routed experts: choices and weights per token, groups, and the grouped activations of max_top choices per token
 	int max_top = 0, max_experts = 0;
 	size_t w_moe_ff = 0;
@@ -878,9 +879,9 @@ void gla_launch(Seq& s, GlaArgs& g, const SeqBatch& sb, int ld) {
 		++g_seq_routes[SEQ_ROUTE_GLA_CHUNKS];
 		const double bytes = (double)N * H * (3.0 * D + 2.0 * Dv) * 4 + 2.0 * sb.B * H * D * Dv * 4, flops = (double)N * H * D * Dv * 4.0;
 		auto go = [&](auto local, auto starts, auto apply) {
-			run_kernel(s, KD_GLA, 0, 0, [&] { launch_k(s, local, dim3(sb.B * c.count, H, cdiv(Dv, 128)), 2 * D, glc_smem(D), g, c, sb); });
-			run_kernel(s, KD_GLA, 0, 0, [&] { launch_k(s, starts, dim3(cdiv((long)H * Dv * D / 4, 128), sb.B), 128, 0, g, c, sb); });
-			run_kernel(s, KD_GLA, bytes, flops, [&] { launch_k(s, apply, dim3(sb.B * c.count, H, nv), 128, 0, g, c, sb); });
+			run_kernel(s, KD_GLA_CHUNKS, 0, 0, [&] { launch_k(s, local, dim3(sb.B * c.count, H, cdiv(Dv, 128)), 2 * D, glc_smem(D), g, c, sb); });
+			run_kernel(s, KD_GLA_CHUNKS, 0, 0, [&] { launch_k(s, starts, dim3(cdiv((long)H * Dv * D / 4, 128), sb.B), 128, 0, g, c, sb); });
+			run_kernel(s, KD_GLA_CHUNKS, bytes, flops, [&] { launch_k(s, apply, dim3(sb.B * c.count, H, nv), 128, 0, g, c, sb); });
 		};
 		if (D == 128) go(k_seq_gla_local<128>, k_seq_gla_starts<128>, k_seq_gla_apply<128>);
 		else go(k_seq_gla_local<64>, k_seq_gla_starts<64>, k_seq_gla_apply<64>);
@@ -1005,9 +1006,9 @@ void mixer_typed(Seq& s, const SeqLayer& L, RunState& r, const SeqBatch& sb, dou
 			ensure_scan(s, (size_t)(N / DELTA_BK + sb.B) * H * 2 * DELTA_BK * DELTA_BK);
 			db.sys = s.scan_ws;
 			++g_seq_routes[SEQ_ROUTE_DELTA_BLOCKS];
-			run_kernel(s, KD_DELTA, 0, 0, [&] { launch_k(s, k_seq_delta_system, dim3(sb.B * db.count, H), 512, 0, d, db, sb); });
+			run_kernel(s, KD_DELTA_BLOCKS, 0, 0, [&] { launch_k(s, k_seq_delta_system, dim3(sb.B * db.count, H), 512, 0, d, db, sb); });
 		}
-		run_kernel(s, KD_DELTA, (double)N * H * (3.0 * D + 2.0 * Dv) * 4 + 2.0 * sb.B * H * D * Dv * 4, (double)N * H * D * Dv * 6.0, [&] {
+		run_kernel(s, blocks ? KD_DELTA_BLOCKS : KD_DELTA, (double)N * H * (3.0 * D + 2.0 * Dv) * 4 + 2.0 * sb.B * H * D * Dv * 4, (double)N * H * D * Dv * 6.0, [&] {
 			const dim3 grid(sb.B, H, cdiv(Dv, DELTA_VC));
 			if (blocks) return launch_k(s, k_seq_delta_blocks, grid, 128, delta_block_smem(), d, db, sb);
 			if (reg && D == 32) launch_k(s, k_seq_delta_scan_reg<32>, grid, 128, 0, d, sb);
