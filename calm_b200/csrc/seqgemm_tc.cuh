@@ -460,14 +460,15 @@ static inline bool gemm_tc_maps(const GemmArgs& a, int batch, const CUtensorMap*
 //   Dynamic Tanh added to the stream, 2048 rows, 256 tokens 24.2 / 26.3, 1024 28.0 / 28.1, 2048 32.2 / 30.3; K = 5632 43.7 / 38.3, 46.5 / 41.1, 51.6 / 45.2;
 //   added to the stream, 2048 rows, 64 tokens 17.4 / 17.5, 128 21.1 / 23.0, 256 22.3 / 26.8, 2048 26.2 / 30.4; K = 5632 38.5 / 29.5, 41.9 / 34.9, 42.6 / 43.8, 54.6 / 54.2;
 //   8192 rows, 512 tokens 30.2 / 34.2, 1024 (two waves) 60.4 / 53.4; 4096 rows, K = 1024, 2048 tokens (two waves) 41.9 / 43.8.
-// Between other launches a pair's start is hidden: by whole steps, the pairs' last column is 1 to 5 us lower where the products are deep (2048 rows added to the stream,
-// 256 / 1024 / 2048 tokens: K = 5632 4.2 less, 1.3 more, 2.4 less a product than with the smaller tiles; K = 2048, 512 / 1024 / 2048 tokens 5.1, 8.5, 2.5 more).
+// Between other launches a pair's start is hidden.  us more on pairs a product in whole steps, added to the stream, 64 / 128 / 200 / 256 / 512 / 1024 / 2048 tokens:
+//   2048 rows, K = 2048 -2.3, -1.3, 3.5, 2.4, 4.0, 4.1, 1.8; K = 5632 -11.4, -9.1, -4.4, 0.0, 1.9, -4.0, -2.3; 1024 rows, K = 2816 -8.3, -3.5, -2.0, 5.4, 3.9, 1.8, 0.3;
+//   4096 rows, K = 4096 -6.1, -2.6, -2.5, 0.7, -0.5, -0.3, -20.5 (two waves); K = 2048 -2.1, 2.5, -0.8, 3.5, 1.4, 2.4, -5.8.
 static inline bool tg_pairs_pay(long M, long N, long K, int epi, long pairs) {
 	const long steps = (K + TG_BK - 1) / TG_BK, slots = 4 * pairs; // CTAs of the smaller tiles at a time
 	const long small = ((M + TG_BM - 1) / TG_BM) * ((N + TG_BN - 1) / TG_BN), large = ((M + TP_BM - 1) / TP_BM) * ((N + TP_BN - 1) / TP_BN);
 	const bool alone = small <= 5 * pairs / 2; // the smaller tiles are about one to an SM
 	long more = 9000;
-	if (epi == EPI_RES) more = large > pairs ? 14000 : N <= 224 ? 9000 + 30 * N : alone ? 24000 : 20000;
+	if (epi == EPI_RES) more = large > pairs ? 14000 : N <= 128 ? 9000 : N <= 224 ? 13000 : alone ? 24000 : 20000;
 	else if (epi == EPI_DYT_RES && N > 224 && alone) more = 15500;
 	return (large + pairs - 1) / pairs * steps * 590 + more < (small + slots - 1) / slots * steps * 900;
 }
