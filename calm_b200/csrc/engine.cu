@@ -1352,12 +1352,14 @@ static bool pf_supported() {
 
 // Row tiles and tokens per item and K-slices of a product of `rows` weight rows over n tokens: the choice with the least estimated time, in cycles.
 // Kernel time over k-stages, 4096 x 4096 x 2047 tokens, in cycles at 1.965 GHz, for 64 / 128 / 256 tokens of one row tile and 64 / 128 of two: fp8
-// 1180 / 1280 / 1960 and 1770 / 2070 (269 / 167 / 128 and 231 / 135 us), fp16 950 / 1190 / 2220 and 1280 / 1810 (217 / 155 / 145 and 166 / 118 us);
-// the estimate has 970 / 1290 / 1930 and 1290 / 1930 for all formats.  So wide items win while every SM has one, two row tiles (half the
-// activation bytes) first; K is sliced only while an item per SM is left over, and a slice pays for its way through memory.
-// Where it misses: two row tiles and 64 tokens of weights that are widened cost a third more than estimated, and two K-slices more than the
-// fold's share (FFN up 14336 x 4096, 130 tokens, fp8: 171 us, 127 with 128 tokens a tile; q/k/v 6144 x 4096, 333 tokens, gf4: 90 us, 67 unsliced);
-// over 48 products of four models the choice is within a tenth of the best in 39.
+// 1090 / 1270 / 1880 and 1490 / 2100 (248 / 165 / 122 and 194 / 137 us), gf4 1290 / 1470 / 2060 and 1680 / 2220 (294 / 192 / 134 and 218 / 145 us), fp16
+// 870 / 1140 / 2240 and 1420 / 1890 (199 / 148 / 146 and 184 / 123 us); the estimate has 970 / 1290 / 1930 and 1290 / 1930 for all formats, also where one operand of hi
+// and lo (pf_side) or a tail in slices (pf_tail) makes it faster.  So wide items win while every SM has one, two row tiles (half the activation bytes) first; K is sliced
+// only while an item per SM is left over, and a slice pays for its way through memory.
+// Where it misses, of 72 products of four models 9 by more than a tenth: one row tile of 256 tokens or 128 in one operand against two of 128 (q/k/v 6144 x 4096: gf4,
+// 2047 tokens 206 us, 184; fp8, 1000 tokens 147, 106 with a tail; fp16, 333 tokens in two slices 58, 48 whole), and two of 64 against two of 128 with a tail (FFN up
+// 14336 x 4096, 300 tokens, fp8: 191, 160).  The fold's price of 15 a column and slice is low where whole tiles are folded (pf_tail has 40: 4096 x 14336, 60 tokens, fp16 in
+// nine slices of two row tiles 48 us, in four of one 37), about right where half of a tile's tokens are there (20 tokens, fp8: 33, 39).
 static void pf_tiles(int mode, int rows, int n, int nkb, int sms, int& na_out, int& bn_out, int& splits_out) {
 	long best = -1;
 	for (int na = 2; na >= (mode == PF_UP ? 2 : 1); --na)
@@ -1371,8 +1373,9 @@ static void pf_tiles(int mode, int rows, int n, int nkb, int sms, int& na_out, i
 		}
 }
 // More tiles than SMs: the ones past the last whole wave, `tail` of them, are cut into K-slices when the stages that saves outweigh the fold (about 40 cycles a
-// column and slice, four warps reading; 16 slices of 8 tiles made FFN up with 1000 tokens slower, 425 -> 458 us).  FFN up 14336 x 4096 with tails of 40 tiles:
-// fp8 135 tokens 150 -> 134 us, fp16 180 tokens 143 -> 131, gf4 333 tokens 209 -> 194.
+// column and slice, four warps reading; 16 slices of 8 tiles made FFN up with 1000 tokens slower, 425 -> 458 us, three to six take 382 to 386).  Whole against tails in slices,
+// FFN up 14336 x 4096: fp8 135 tokens 144 -> 123 us, 777 342 -> 324, 2047 745 -> 733; fp16 180 tokens 139 -> 120; gf4 333 tokens 195 -> 173; q/k/v 6144 x 4096 fp8 860 tokens
+// 145 -> 124; w2 4096 x 14336 fp8 1300 tokens 471 -> 383.
 static void pf_tail(int tiles, int nkb, int sms, int na, int bn, int& tail_out, int& splits_out) {
 	const int tail = tiles > sms ? tiles % sms : 0;
 	long best = 0;

@@ -1861,7 +1861,7 @@ __global__ void __launch_bounds__(128) k_seq_gla_scan(GlaArgs a, SeqBatch sb) {
 // state and the product of its decays, (2) k_seq_gla_starts walks a state element through the chunks, leaving every chunk's first state in place
 // of what it adds, and updates the slot's state, (3) k_seq_gla_apply runs each chunk's tokens from there for the read-outs.
 // k_seq_gla_scan is a chain over all tokens on as many SMs as sequences x heads x columns give (2048 tokens of 16 heads of 128 x 128: 469 us,
-// 230 ns a token whatever the arithmetic); here (1) and (3) fill the SMs: 140 us, each launch alone with cold caches 47 + 16 + 94.
+// 230 ns a token whatever the arithmetic); here (1) and (3) fill the SMs: 148 us, each launch alone with cold caches 47 + 18 + 94.
 struct GlaChunks {
 	float* add;  // [B][count][heads][vdim][dim]: what a chunk adds, then the state it starts from
 	float* keep; // [B][count][heads][dim]: product of the chunk's decays
