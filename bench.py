@@ -390,7 +390,7 @@ def main():
             except Exception:
                 tpeak = 1400.0
             prefill = {"tokens": n_pf, "ms": pf_ms, "tok_s": n_pf / (pf_ms / 1e3), "tflops": tf, "frac_of_bf16_sustained": tf / tpeak,
-                       "path": "tcgen05 GEMMs (f16 hi + lo activations: two MMAs per k-step) + block-causal attention" if served else "fed token by token (shape not served by the batched pass)",
+                       "path": "tcgen05 GEMMs (f16 hi + lo activations, both multiplied) + block-causal attention" if served else "fed token by token (shape not served by the batched pass)",
                        "vs_serial_prompt": (n_pf / (pf_ms / 1e3)) / value}
         except Exception as e:
             prefill = {"unavailable": str(e)}
