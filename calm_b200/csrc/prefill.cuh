@@ -6,7 +6,7 @@
 //   k_pf_gemm   D[128 weight rows][<= 256 tokens] = W_tile . X_tile^T with tcgen05.mma (kind::f16, cta_group::1), fp32
 //               accumulators in TMEM.  A = the weight tile, widened ON THE FLY from the model's own format (fp16 / e5m2 /
 //               gf4: all exact in f16); B = the activations as TWO f16 matrices hi + lo (x = hi + lo to 22 bits, so the
-//               result carries fp32-grade inputs: two MMAs per k-step into the same accumulator).  The epilogue applies
+//               result carries fp32-grade inputs), multiplied as one operand of both or one after the other (pf_side).  The epilogue applies
 //               what the decode kernels apply: bias / clip / RoPE / KV-cache append (QKV), residual add (wo, w2),
 //               act(w1 x) * (w3 x) with both accumulators side by side in TMEM (FFN up).
 //   k_pf_attn   causal attention of the block against the cache (online softmax in fp32; reference infer.c:238-267), scores and
