@@ -15,7 +15,7 @@ CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(HERE, "..", "include")
 TARGETS = {
     "engine": {"lib": os.path.join(HERE, "libcalm_b200.so"), "sources": ["engine.cu"],
-               "deps": ["attn.cuh", "common.cuh", "tc05.cuh", "prefill.cuh", "ring.cuh", "stages.cuh", os.path.join(INCLUDE, "calm_b200.h"), os.path.join(INCLUDE, "calm_model.h")]},
+               "deps": ["attn.cuh", "common.cuh", "tc05.cuh", "prefill.cuh", "ring.cuh", "cols.cuh", "stages.cuh", os.path.join(INCLUDE, "calm_b200.h"), os.path.join(INCLUDE, "calm_model.h")]},
     "seq": {"lib": os.path.join(HERE, "libcalm_b200_seq.so"), "sources": ["seqmodel.cu"],
             "deps": ["common.cuh", "tc05.cuh", "seqkernels.cuh", "seqgemm_tc.cuh", os.path.join(INCLUDE, "calm_b200_seq.h")]},
 }

@@ -12,14 +12,22 @@
 #include <math.h>
 #include <string.h>
 
+#include <type_traits>
 #include <vector>
 
 #include "stages.cuh"
 #include "attn.cuh"
 #include "ring.cuh"
+#include "cols.cuh"
 #include "prefill.cuh"
 
 namespace {
+
+struct ColsPlan {
+	int n = 0; // chunks of a row or tiles of a CTA
+	int steps = 0, chunk_steps = 0, grid = 0;
+	bool alone = false; // shared memory for one CTA per SM (COLS_ALONE)
+};
 
 #define MAX_STAMPS (2 + 5 * MAX_LAYERS)
 #define TP_MAX_CAND 2048 // greedy candidates (classifier CTAs) per rank in the tensor-parallel gather area
@@ -59,6 +67,7 @@ struct Engine {
 	unsigned pf_wait_limit = MBAR_SPINS; // tries of a wait in the prompt products
 	// attention launch shape
 	int attn_hg = 1, attn_hg2 = 1 /* k_attn2: padded to what it is instantiated for */, attn_qgroups = 1, attn_nsplit = 1, attn_lpp = 1;
+	ColsPlan cols_qkv, cols_wo, cols_up, cols_down; // matvecs on the tensor cores (cols.cuh); n == 0: the stage keeps its other kernels
 	// TMA-ring matvec kernels (ring.cuh): slots per warp / CTAs per SM for FFN-up and for wo / w2; u = 512-byte units per row and chunk (0: not used)
 	int ring_up_ns = 2, ring_up_cps = 2, ring_res_ns = 2, ring_res_warps = 16; // measured: 16 consuming warps per SM are needed
 	int ring_up_u = 0, ring_wo_u = 0, ring_down_u = 0, ring_wo_s = 1, ring_down_s = 1;
@@ -396,6 +405,17 @@ size_t attn_smem(int hg, int head_dim, int nsplit) {
 	return smem2 > smem ? smem2 : smem;
 }
 
+// Kernels that are to be resident side by side need one L1 / shared-memory split: all of it shared memory.  (Not the classifier: its loads want L1, 45 us against
+// 59 for the 151936 x 896 one.)
+template <typename F>
+void side_by_side(F kernel, bool yes = true) { // (an attribute outlives the model that was prepared with it)
+	if (!getenv("CALM_B200_CARVEOUT"))
+		CUDA_CHECK(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributePreferredSharedMemoryCarveout, yes ? cudaSharedmemCarveoutMaxShared : cudaSharedmemCarveoutDefault));
+}
+template <typename F>
+void cols_attr(F kernel, size_t smem) {
+	smem_optin(kernel, smem), side_by_side(kernel);
+}
 // nl == NULL: only opt in to the shared-memory size (prepare time, outside stream capture; head_dim 256 with 8 query heads
 // per kv head needs 66 KB)
 template <typename KVT, int HG>
@@ -413,6 +433,7 @@ template <typename KVT, int HG, int LPP>
 void launch_attn2(const AttnArgs& a, int nunits, int* nl) {
 	if (!nl) { // prepare time: opt-ins, and whether the cluster form can be scheduled at all
 		smem_optin(k_attn2<KVT, HG, LPP, false>, g.attn2_smem);
+		side_by_side(k_attn2<KVT, HG, LPP, false>, g.w.dbits != 4 && g.cfg.n_experts == 0);
 		{ // the cell fold polls its peers: the whole grid must fit on the device at once
 			int per_sm = 0;
 			CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_attn2<KVT, HG, LPP, false>, ATTN_THREADS, g.attn2_smem));
@@ -514,6 +535,44 @@ void ring_res_dispatch(const MatResArgs& a, int u, int S, int grid, size_t smem,
 	}
 }
 
+// cols.cuh kernels are instantiated by the chunks of a row (q/k/v, FFN up: up to 8192 weights) or the tiles of a CTA (wo, w2)
+template <int MOST, typename F>
+void cols_switch(int n, F f) {
+	if constexpr (MOST >= 1) {
+		if (n == MOST) return f(std::integral_constant<int, MOST>());
+		return cols_switch<MOST - 1>(n, f);
+	}
+	CALM_FATAL("no kernel for %d chunks or tiles", n);
+}
+template <int DBITS>
+constexpr int cols_chunks() {
+	return DBITS / 2; // 8192 weights
+}
+ColsRun cols_run(const ColsPlan& p) {
+	return ColsRun{p.steps, p.chunk_steps, 2 * cdiv(p.chunk_steps, 2 * COLS_WARPS), g.dev_err};
+}
+template <int DBITS, typename KVT>
+void cols_qkv(const QkvArgs<KVT>& a, const ColsPlan& p, bool attr_only) {
+	cols_switch<cols_chunks<DBITS>()>(p.n, [&](auto n) {
+		if (attr_only) cols_attr(k_qkv_cols<DBITS, n, KVT>, COLS_SMEM);
+		else launch_pdl(k_qkv_cols<DBITS, n, KVT>, p.grid, COLS_THREADS, COLS_SMEM, a, cols_run(p));
+	});
+}
+template <int DBITS>
+void cols_res(const MatResArgs& a, const ColsPlan& p, bool attr_only) {
+	cols_switch<COLS_TILES>(p.n, [&](auto n) {
+		if (attr_only) cols_attr(k_matres_cols<DBITS, n>, COLS_ALONE);
+		else launch_pdl(k_matres_cols<DBITS, n>, p.grid, COLS_THREADS, p.alone ? COLS_ALONE : COLS_SMEM, a, cols_run(p));
+	});
+}
+template <int DBITS>
+void cols_up(const FfnUpArgs& a, const ColsPlan& p, bool attr_only) {
+	cols_switch<cols_chunks<DBITS>()>(p.n, [&](auto n) {
+		if (attr_only) cols_attr(k_ffn_up_cols<DBITS, n>, COLS_SMEM);
+		else launch_pdl(k_ffn_up_cols<DBITS, n>, p.grid, COLS_THREADS, COLS_SMEM, a, cols_run(p));
+	});
+}
+
 // first `budget` bytes of the (w1, w3) row interleave that k_ffn_up walks: half from each matrix (row prefixes)
 static void pf_up_prefix(Prefetch& pf, int slot, const void* w1, const void* w3, size_t skip, size_t budget, size_t matrix_bytes) {
 	size_t off = (skip / 2) & ~(size_t)15, len = (budget / 2) & ~(size_t)15;
@@ -568,7 +627,10 @@ int run_token(int mode) {
 			a.eps = c.norm_eps, a.clip = c.qkv_clip, a.ln = c.norm_ln;
 			a.stamp = t.slot;
 			if (g.pf_kv && (l == 0 || !g.pf_down_qkv)) kv_prefix(a.pf, l); // later layers: requested by the previous w2 kernel
-			launch_pdl(k_qkv<DBITS, KVT>, g.grid_qkv, QKV_THREADS, g.smem_dim, a);
+			bool done = false;
+			if constexpr (DBITS != 4)
+				if (g.cols_qkv.n) cols_qkv<DBITS, KVT>(a, g.cols_qkv, false), done = true;
+			if (!done) launch_pdl(k_qkv<DBITS, KVT>, g.grid_qkv, QKV_THREADS, g.smem_dim, a);
 			++nl;
 		}
 		{
@@ -595,7 +657,11 @@ int run_token(int mode) {
 			if (dense && g.pf_wo_up) pf_up_prefix(a.pf, 0, w.w1[l], w.w3[l], g.pf_attn_up, g.pf_wo_up, up_bytes);
 			if (g.tp_fused) tp_fill(a.tpx, 2 * l); // partial over this rank's heads, summed over the ranks in the kernel
 			else if (g.tp_world > 1) a.y = g.xpart, a.accumulate = 0;
-			if (g.ring_wo_u) ring_res_dispatch<DBITS>(a, g.ring_wo_u, g.ring_wo_s, g.grid_wo_ring, g.smem_wo_ring, false);
+			bool done = false;
+			if constexpr (DBITS != 4)
+				if (g.cols_wo.n) cols_res<DBITS>(a, g.cols_wo, false), done = true;
+			if (done) {
+			} else if (g.ring_wo_u) ring_res_dispatch<DBITS>(a, g.ring_wo_u, g.ring_wo_s, g.grid_wo_ring, g.smem_wo_ring, false);
 			else launch_pdl(k_matres<DBITS>, g.grid_wo, 256, g.smem_qdim, a);
 			++nl;
 			if (g.tp_world > 1 && !g.tp_fused) {
@@ -615,7 +681,9 @@ int run_token(int mode) {
 			a.stamp = t.slot;
 			if (dense && g.pf_up_down) a.pf.p[0] = w.w2[l], a.pf.bytes[0] = (g.pf_up_down < down_bytes ? g.pf_up_down : down_bytes) & ~(size_t)15;
 			bool done = false;
-			if (g.ring_up_u) ring_up_dispatch<DBITS>(a, false), done = true;
+			if constexpr (DBITS != 4)
+				if (g.cols_up.n) cols_up<DBITS>(a, g.cols_up, false), done = true;
+			if (!done && g.ring_up_u) ring_up_dispatch<DBITS>(a, false), done = true;
 			if (!done) launch_pdl(k_ffn_up<DBITS>, g.grid_up, 256, g.smem_dim, a);
 			++nl;
 		}
@@ -631,7 +699,11 @@ int run_token(int mode) {
 			}
 			if (g.tp_fused) tp_fill(a.tpx, 2 * l + 1); // partial over this rank's FFN rows
 			else if (g.tp_world > 1) a.y = g.xpart, a.accumulate = 0;
-			if (g.ring_down_u) ring_res_dispatch<DBITS>(a, g.ring_down_u, g.ring_down_s, g.grid_down_ring, g.smem_down_ring, false);
+			bool done = false;
+			if constexpr (DBITS != 4)
+				if (g.cols_down.n) cols_res<DBITS>(a, g.cols_down, false), done = true;
+			if (done) {
+			} else if (g.ring_down_u) ring_res_dispatch<DBITS>(a, g.ring_down_u, g.ring_down_s, g.grid_down_ring, g.smem_down_ring, false);
 			else launch_pdl(k_matres<DBITS>, g.grid_down, 256, g.smem_hidden, a);
 			++nl;
 			if (g.tp_world > 1 && !g.tp_fused) {
@@ -666,7 +738,7 @@ int run_token(int mode) {
 		}
 		// Not early behind a kernel that fills the SMs' shared memory: CTAs that came while it ran would find the SMs split as it needs them, and the loads of the
 		// classifier's rows, which live on L1, run at 5.7 TB/s instead of 6.7 (128256 x 4096 fp16 182 -> 157 us, fp8 96 -> 84).  gf4 unpacks as fast either way.
-		const bool early = DBITS == 4 || !g.ring_down_u;
+		const bool early = DBITS == 4 || !(g.ring_down_u || g.cols_down.n);
 		launch_1d(early, k_output<DBITS>, grid, 256, g.smem_dim, a);
 		++nl;
 		if (split) {
@@ -739,6 +811,20 @@ void tp_shard_model() {
 	c.n_heads /= N, c.n_kv_heads /= N, c.hidden_dim = hl;
 }
 
+// How a matvec of `units` pieces of rows of n weights is cut (cols.cuh), or no plan.  tiles: the second order, one row a unit.
+template <int DBITS>
+ColsPlan plan_cols(int n, int units, bool tiles) {
+	ColsPlan p;
+	if (n % 128) return p;
+	p.steps = n / ColsStep<DBITS>::K;
+	const int chunks = cdiv(p.steps, COLS_CHUNK / 64);
+	p.chunk_steps = 2 * cdiv(p.steps, 2 * chunks);
+	p.grid = imin(g.sms, units);
+	p.n = tiles ? cdiv(cdiv(units, p.grid), 8) : chunks;
+	if (p.chunk_steps * (chunks - 1) >= p.steps || p.n > (tiles ? COLS_TILES : cols_chunks<DBITS>())) p.n = 0;
+	return p;
+}
+
 // Fix grid sizes and shared-memory opt-ins for this model (called once from prepare_cuda).
 template <int DBITS, typename KVT>
 void make_plan() {
@@ -770,6 +856,17 @@ void make_plan() {
 	}
 	// (measured: for the long FFN-up stage a full 4-CTA/SM grid with uneven rounds beats a balanced 3-CTA/SM one)
 	g.grid_up = imin(max_ctas(k_ffn_up<DBITS>, 256, g.smem_dim), cdiv(g.nact * c.hidden_dim, 8));
+	if constexpr (DBITS != 4) {
+		if (c.n_experts == 0) { // (the expert rows of a routed model are known only after the router)
+			if (!c.norm_ln) g.cols_qkv = plan_cols<DBITS>(c.dim, (g.q_dim + 2 * g.kv_dim) / 2, false);
+			if (!c.norm_ln || c.norm_par) g.cols_up = plan_cols<DBITS>(c.dim, c.hidden_dim, false);
+			g.cols_wo = plan_cols<DBITS>(g.q_dim, c.dim, true), g.cols_wo.alone = true, g.cols_down = plan_cols<DBITS>(c.hidden_dim, c.dim, true);
+			if (g.cols_qkv.n) cols_qkv<DBITS, KVT>(QkvArgs<KVT>(), g.cols_qkv, true);
+			if (g.cols_up.n) cols_up<DBITS>(FfnUpArgs(), g.cols_up, true);
+			if (g.cols_wo.n) cols_res<DBITS>(MatResArgs(), g.cols_wo, true);
+			if (g.cols_down.n) cols_res<DBITS>(MatResArgs(), g.cols_down, true);
+		}
+	}
 	// TMA-ring kernels for the dense single-GPU stages whose rows are whole 1 KB / 2 KB chunks (ring.cuh)
 	g.ring_up_u = g.ring_wo_u = g.ring_down_u = 0;
 	{ // weights are read once per token: L2::evict_first on the ring's bulk copies measured 2 % faster than the default policy
@@ -781,7 +878,7 @@ void make_plan() {
 	const bool ring_up_on = ring_ok && g.ring_up_ns >= 2 && g.ring_up_ns <= RING_MAX_NS; // (row shards of w1 / w3 under tensor parallelism are fine)
 	const bool ring_res_on = ring_ok && (g.tp_world == 1 || g.tp_fused) /* the ring kernels carry the in-kernel exchange too */ && g.ring_res_ns >= 2 && g.ring_res_ns <= RING_MAX_NS && (g.ring_res_warps == 8 || g.ring_res_warps == 16); // (gf4 too: 2.384 vs 2.467 ms per Mistral-7B token, profiles/r02_sweep_gf4_rows_per_slot.jsonl)
 	auto chunk_units = [](size_t rowbytes) { return rowbytes % 2048 == 0 ? 4 : (rowbytes % 1024 == 0 ? 2 : 0); };
-	if (ring_up_on) {
+	if (ring_up_on && !g.cols_up.n) {
 		const int u = chunk_units((size_t)c.dim * DBITS / 8);
 		if (u) {
 			g.smem_up_ring = ring_smem_bytes<DBITS>(c.dim, u, g.ring_up_ns, 8);
@@ -814,8 +911,8 @@ void make_plan() {
 		// ONE shared-memory attribute per kernel instantiation: wo and w2 may share one (same U): opt in to the larger first
 		int uw = 0, ud = 0, sw = 1, sd = 1, gw = 0, gd = 0;
 		size_t mw = 0, md = 0;
-		plan_res(g.q_dim, uw, sw, gw, mw);
-		plan_res(c.hidden_dim, ud, sd, gd, md);
+		if (!g.cols_wo.n) plan_res(g.q_dim, uw, sw, gw, mw);
+		if (!g.cols_down.n) plan_res(c.hidden_dim, ud, sd, gd, md);
 		if (uw && ud && uw == ud) { // same instantiation: its attribute must cover both launches
 			MatResArgs ma = {};
 			ring_res_dispatch<DBITS>(ma, uw, 1, 1, mw > md ? mw : md, true);
@@ -1152,6 +1249,7 @@ static void sync_stream() {
 		fprintf(stderr, "calm_b200: device failure: %s (%s); watchdog code %d\n", cudaGetErrorString(e), cudaGetErrorName(e), code);
 		abort();
 	}
+	if (g.dev_err && *(volatile int*)g.dev_err) CALM_FATAL("a wait inside a token gave up (code %d)", *(volatile int*)g.dev_err); // 9300 / 9301: cols.cuh
 }
 
 static void check_call(struct Transformer* transformer, int token, int pos) {
@@ -1407,6 +1505,11 @@ extern "C" void calm_b200_prefill_tiles(int product, int rows, int n, int k, int
 }
 extern "C" void calm_b200_prefill_cut(int product, int rows, int n, int k, int sms, int* out5) {
 	out5[0] = pf_cut(pf_mode(product), rows, n, k / PF_BK, sms, out5[1], out5[2], out5[3], out5[4]);
+}
+
+extern "C" int calm_b200_token_plan(int stage) {
+	const ColsPlan* p[4] = {&g.cols_qkv, &g.cols_wo, &g.cols_up, &g.cols_down};
+	return g.ready && stage >= 0 && stage < 4 ? p[stage]->n : 0;
 }
 
 template <int MODE, int DBITS>

@@ -110,6 +110,10 @@ void calm_b200_prefill_tiles(int product, int rows, int n, int k, int sms, int* 
  * (all of them, the last ones, none), slices of each} */
 void calm_b200_prefill_cut(int product, int rows, int n, int k, int sms, int* out5);
 
+/* How the prepared model's token runs a stage (0 q/k/v, 1 wo, 2 FFN up, 3 FFN down; for tests): pieces of a row (0, 2) or tiles of rows of a CTA (1, 3) of
+ * the tensor-core matvecs, 0 when the stage has its general kernels. */
+int calm_b200_token_plan(int stage);
+
 /* forward + device-side greedy sample.  Returns argmax(logits) with the
  * reference's tie rule (lowest index, sampler.c:34-42).  The logits are still
  * written to state.logits. */
