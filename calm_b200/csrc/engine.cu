@@ -1466,6 +1466,12 @@ static bool pf_supported() {
 // 2047 tokens 206 us, 184; fp8, 1000 tokens 147, 106 with a tail; fp16, 333 tokens in two slices 58, 48 whole), and two of 64 against two of 128 with a tail (FFN up
 // 14336 x 4096, 300 tokens, fp8: 191, 160).  The fold's price of 15 a column and slice is low where whole tiles are folded (pf_tail has 40: 4096 x 14336, 60 tokens, fp16 in
 // nine slices of two row tiles 48 us, in four of one 37), about right where half of a tile's tokens are there (20 tokens, fp8: 33, 39).
+// All tiles in slices, few enough slices for one thread-block cluster, and all clusters at one time: the CTAs take an SM each and a GPC's SMs hold this many clusters
+// (cudaOccupancyMaxActiveClusters on a B200).
+static bool pf_cluster(int tail, int tiles, int splits) {
+	static const int most[9] = {0, 0, 74, 45, 33, 26, 22, 15, 15};
+	return tail == tiles && splits > 1 && splits <= 8 && tiles <= most[splits];
+}
 static void pf_tiles(int mode, int rows, int n, int nkb, int sms, int& na_out, int& bn_out, int& splits_out) {
 	long best = -1;
 	for (int na = 2; na >= (mode == PF_UP ? 2 : 1); --na)
@@ -1477,6 +1483,14 @@ static void pf_tiles(int mode, int rows, int n, int nkb, int sms, int& na_out, i
 				if (best < 0 || cost < best) best = cost, na_out = na, bn_out = bn, splits_out = sp;
 			}
 		}
+	{ // folded inside a cluster: other slices, or slices where the fold through memory does not pay
+		const int na = na_out, bn = bn_out, cols = n < bn ? 32 * cdiv(n, 32) : bn, tiles = (mode == PF_UP ? rows / PF_BM : cdiv(rows / PF_BM, na)) * cdiv(n, bn), stage = 650 + na * bn * 5;
+		best = (long)cdiv(tiles * splits_out, sms) * cdiv(nkb, splits_out) * stage + (splits_out > 1 ? 5000 + na * cols * (20 + 15 * splits_out) : 0);
+		for (int sp = 2; sp <= 8 && tiles * sp <= sms && sp * 2 <= nkb; ++sp) {
+			const long cost = (long)cdiv(nkb, sp) * stage + 2500 + na * cols * 30;
+			if (pf_cluster(tiles, tiles, sp) && cost <= best) best = cost, splits_out = sp;
+		}
+	}
 }
 // More tiles than SMs: the ones past the last whole wave, `tail` of them, are cut into K-slices when the stages that saves outweigh the fold (about 40 cycles a
 // column and slice, four warps reading; 16 slices of 8 tiles made FFN up with 1000 tokens slower, 425 -> 458 us, three to six take 382 to 386).  Whole against tails in slices,
@@ -1499,6 +1513,7 @@ static int pf_cut(int mode, int rows, int n, int nkb, int sms, int& na, int& bn,
 	else pf_tail(tiles, nkb, sms, na, bn, tail, splits);
 	return tiles;
 }
+// all tiles in slices, few enough of each for one thread-block cluster
 static int pf_mode(int product) { return product == 0 ? PF_QKV : product == 1 ? PF_RES : PF_UP; }
 extern "C" void calm_b200_prefill_tiles(int product, int rows, int n, int k, int sms, int* out3) {
 	pf_tiles(pf_mode(product), rows, n, k / PF_BK, sms, out3[0], out3[1], out3[2]);
@@ -1516,8 +1531,7 @@ template <int MODE, int DBITS>
 static void pf_gemm(const CUtensorMap (&tx)[3][2], const CUtensorMap* tw, PfGemmArgs a, int rows, int n) {
 	constexpr size_t fixed = pf_fixed_bytes<DBITS>(), limit = 226 * 1024;
 	static bool opted = false;
-	if (!opted) smem_optin(k_pf_gemm<MODE, DBITS>, limit), opted = true;
-	same_carveout((const void*)k_pf_gemm<MODE, DBITS>);
+	if (!opted) smem_optin(k_pf_gemm<MODE, DBITS, false>, limit), smem_optin(k_pf_gemm<MODE, DBITS, true>, limit), opted = true;
 	const int tiles = pf_cut(MODE, rows, n, a.K / PF_BK, g.sms, a.na, a.bn, a.tail, a.splits);
 	PfMaps m;
 	memcpy(m.x, tx[a.bn / 128], sizeof(m.x)); // 64, 128, 256 -> 0, 1, 2
@@ -1527,11 +1541,16 @@ static void pf_gemm(const CUtensorMap (&tx)[3][2], const CUtensorMap* tw, PfGemm
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3(imin(g.sms, tiles - a.tail + a.tail * a.splits)), cfg.blockDim = dim3(pf_threads<DBITS>()), cfg.stream = g.stream;
 	cfg.dynamicSmemBytes = fixed + a.stages * pf_stage_bytes(a.na, a.bn);
-	cudaLaunchAttribute at[1];
+	cudaLaunchAttribute at[2];
 	at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
 	at[0].val.programmaticStreamSerializationAllowed = g.use_pdl ? 1 : 0;
-	cfg.attrs = at, cfg.numAttrs = 1;
-	CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_pf_gemm<MODE, DBITS>, m, a));
+	at[1].id = cudaLaunchAttributeClusterDimension;
+	at[1].val.clusterDim.x = a.splits, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
+	const bool cluster = pf_cluster(a.tail, tiles, a.splits);
+	const auto kernel = cluster ? k_pf_gemm<MODE, DBITS, true> : k_pf_gemm<MODE, DBITS, false>;
+	same_carveout((const void*)kernel);
+	cfg.attrs = at, cfg.numAttrs = cluster ? 2 : 1;
+	CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, m, a));
 	++g_launches;
 }
 
