@@ -499,7 +499,9 @@ void gemm(Seq& s, const void* X, long ldx, long xbs, const void* W, long ldw, lo
 	if (a.band_mode == 2) CALM_FATAL("seq: a banded value product needs the tcgen05 kernel"); // what the band leaves out of its input was never written
 	if (gemm_skinny_fits(s, X, ldx, xbs, W, ldw, wbs, N, K)) {
 		const dim3 grid(cdiv(M, 16), 1, batch);
-		const bool few = (long)cdiv(M, 16) * batch < 3L * s.sms && K >= 1024; // few CTAs: twice the warps per CTA keep as many bytes in flight
+		// At most a CTA per SM: twice the warps per CTA keep as many bytes in flight (2048 x 5632, 16 tokens: 7.1 us, 9.6 with eight).  More CTAs than that would run one
+		// after the other, since 16 warps take more than half of an SM's registers (5632 x 1024, one token: 6.0 us, 2.9 with eight; 3216 x 1024 3.8 and 2.1).
+		const bool few = (long)cdiv(M, 16) * batch <= s.sms && K >= 1024;
 		run_kernel(s, kind_as >= 0 ? kind_as : KD_GEMM_SKINNY, bytes, flops, [&] {
 			if (few) {
 				if (N <= 8) launch_k(s, k_seq_gemm_skinny<1, 16>, grid, 512, 0, a);
