@@ -373,6 +373,62 @@ __global__ void k_seq_conv_state(float* state, const float* proj, int ldp, int t
 	}
 }
 
+// One token per sequence (decode): both at once.  A channel's state is read by one warp only, which puts the new one in its place; the taps' weights are requested before
+// the previous kernel has ended, all values of a head vector at a time, and stay in registers (the two kernels above: 9.0 and 4.7 us for 768 and 1536 channels of one
+// token, mostly one load waiting for another).  Vectors of up to 32 C channels, two to four taps.
+template <int C>
+__global__ void __launch_bounds__(128) k_seq_conv_step(ConvArgs a, SeqBatch sb, float* state) {
+	pdl_launch_next();
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n = blockIdx.x, T1 = a.taps - 1;
+	int u = blockIdx.y * (blockDim.x >> 5) + warp, s = 0;
+	while (s < 3 && u >= a.seg[s].heads) u -= a.seg[s].heads, ++s;
+	if (s == 3) return;
+	const ConvSeg sg = a.seg[s];
+	const int ch0 = sg.col + u * sg.hd;
+	float w[C][4], b[C];
+#pragma unroll
+	for (int i = 0; i < C; ++i) {
+		const int e = lane + 32 * i;
+#pragma unroll
+		for (int j = 0; j < 4; ++j) w[i][j] = e < sg.hd && j < a.taps ? ldf(a.w + (size_t)(ch0 + e) * a.taps + j) : 0.f;
+		b[i] = e < sg.hd && a.bias ? ldf(a.bias + ch0 + e) : 0.f;
+	}
+	pdl_wait_prev();
+	const int slot = sb.tslot[n], pos = sb.tpos[n];
+	float* st = state + (size_t)slot * T1 * a.channels + ch0;
+	const float* pr = a.proj + (size_t)n * a.ldp + a.pcol + ch0;
+	float* d = sg.dst + (sg.to_cache ? cache_row(sb, slot, pos) : (long)n) * (sg.heads * sg.hd) + u * sg.hd;
+	float v[C][4]; // the values of the taps, oldest first
+#pragma unroll
+	for (int i = 0; i < C; ++i) {
+		const int e = lane + 32 * i;
+#pragma unroll
+		for (int j = 0; j < 4; ++j) v[i][j] = e < sg.hd && j < a.taps ? (j < T1 ? st[(size_t)j * a.channels + e] : pr[e]) : 0.f;
+	}
+	float y[C], ss = 0.f;
+#pragma unroll
+	for (int i = 0; i < C; ++i) {
+		const int e = lane + 32 * i;
+		y[i] = 0.f;
+#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			if (j < a.taps) y[i] += w[i][j] * v[i][j];
+			if (j > 0 && j < a.taps && e < sg.hd) st[(size_t)(j - 1) * a.channels + e] = v[i][j];
+		}
+		if (a.bias) y[i] += b[i];
+		if (sg.act) y[i] = y[i] * sigmoidf_(y[i]);
+		if (e < sg.hd) ss += y[i] * y[i];
+	}
+	float r = 1.f;
+	if (sg.norm) {
+		ss = warp_sum(ss);
+		r = (sg.norm == 1 ? 1.f / sqrtf(ss + 1e-6f) : 1.f / sqrtf(ss / (float)sg.hd + a.eps)) * sg.mul;
+	}
+#pragma unroll
+	for (int i = 0; i < C; ++i)
+		if (lane + 32 * i < sg.hd) d[lane + 32 * i] = sg.norm ? y[i] * r : y[i];
+}
+
 // ---------------------------------------------------------------- attention over the paged cache
 // One CTA per (token, tile of query heads that share one key/value head).  Keys: `kd` floats at column kcol of the K cache
 // rows, values: `vd` floats at column vcol of the V cache rows (latent attention: both are the cached latent).  Softmax in
@@ -1855,6 +1911,62 @@ __global__ void __launch_bounds__(128) k_seq_gla_scan(GlaArgs a, SeqBatch sb) {
 #pragma unroll
 		for (int i = 0; i < R; i += 4) *(float4*)(Sg + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
 	}
+}
+
+// One token per sequence (decode): the recurrence is a stream over the states.  A warp takes COLS value columns, a lane 4 NV of their key channels, so a column
+// travels as whole 512-byte lines and all of a warp's columns are on their way at once; the read-outs of its columns are transposed and
+// folded together.  (The scan's lane holds R channels of one column: 16 bytes of 32 lines per request, 19 us a layer of 16 sequences x 16 heads of
+// 128 x 128, whose 33.5 MB take 5.1 at the memory's rate.)
+template <int NV>
+__global__ void __launch_bounds__(128) k_seq_gla_step(GlaArgs a, SeqBatch sb) {
+	pdl_enter(); // programmatic dependent launch: let the next kernel's launch overlap this one, then wait for the previous one
+	constexpr int COLS = 16 / NV;
+	const int b = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, v0 = (blockIdx.z * 4 + (threadIdx.x >> 5)) * COLS, n = sb.sstart[b];
+	if (v0 >= a.vdim) return;
+	float* const Sg = a.state + (((size_t)sb.sslot[b] * a.heads + h) * a.vdim + v0) * a.ldstate;
+	const float* const row = a.proj + (size_t)n * a.ldp;
+	const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+	float4 S[COLS][NV], k4[NV], q4[NV], g4[NV];
+#pragma unroll
+	for (int i = 0; i < COLS; ++i)
+#pragma unroll
+		for (int j = 0; j < NV; ++j) S[i][j] = v0 + i < a.vdim && 4 * lane + 128 * j < a.dim ? *(const float4*)(Sg + (size_t)i * a.ldstate + 4 * lane + 128 * j) : none;
+#pragma unroll
+	for (int j = 0; j < NV; ++j) {
+		const int c = 4 * lane + 128 * j;
+		const bool in = c < a.dim;
+		k4[j] = in ? *(const float4*)(row + a.kcol + h * a.dim + c) : none, q4[j] = in ? *(const float4*)(row + a.qcol + h * a.dim + c) : none;
+		g4[j] = in ? *(const float4*)(a.decay + ((size_t)n * a.heads + h) * a.dim + c) : none;
+	}
+	const float mine = lane < COLS && v0 + lane < a.vdim ? row[a.vcol + h * a.vdim + v0 + lane] : 0.f;
+	float o[COLS];
+#pragma unroll
+	for (int i = 0; i < COLS; ++i) {
+		const float v = __shfl_sync(0xffffffffu, mine, i);
+		float o0 = 0.f, o1 = 0.f;
+#pragma unroll
+		for (int j = 0; j < NV; ++j) {
+			float4& t = S[i][j];
+			t.x = fmaf(g4[j].x, t.x, k4[j].x * v), t.y = fmaf(g4[j].y, t.y, k4[j].y * v), t.z = fmaf(g4[j].z, t.z, k4[j].z * v), t.w = fmaf(g4[j].w, t.w, k4[j].w * v);
+			o0 = fmaf(t.x, q4[j].x, o0), o1 = fmaf(t.y, q4[j].y, o1), o0 = fmaf(t.z, q4[j].z, o0), o1 = fmaf(t.w, q4[j].w, o1);
+			if (v0 + i < a.vdim && 4 * lane + 128 * j < a.dim) *(float4*)(Sg + (size_t)i * a.ldstate + 4 * lane + 128 * j) = t;
+		}
+		o[i] = o0 + o1;
+	}
+	int col = 0; // of this lane in the end
+#pragma unroll
+	for (int half = COLS / 2, m = 16; half >= 1; half >>= 1, m >>= 1) {
+		const bool up = lane & m;
+#pragma unroll
+		for (int i = 0; i < half; ++i) {
+			const float send = up ? o[i] : o[i + half];
+			o[i] = (up ? o[i + half] : o[i]) + __shfl_xor_sync(0xffffffffu, send, m);
+		}
+		col += up ? half : 0;
+	}
+#pragma unroll
+	for (int m = 16 / COLS; m >= 1; m >>= 1) o[0] += __shfl_xor_sync(0xffffffffu, o[0], m);
+	if (!(lane & (32 / COLS - 1)) && v0 + col < a.vdim) a.o[((size_t)n * a.heads + h) * a.vdim + v0 + col] = o[0] * a.qscale;
 }
 
 // The same recurrence for long portions, cut into chunks of tokens that run side by side: (1) k_seq_gla_local forms what a chunk adds to a zero

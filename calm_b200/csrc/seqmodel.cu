@@ -775,6 +775,17 @@ void conv(Seq& s, const SeqLayer& L, RunState& r, ConvArgs& ca, const SeqBatch& 
 	ca.proj = proj, ca.ldp = ldp, ca.w = (const bf16*)L.conv, ca.taps = L.taps, ca.channels = conv_channels(L), ca.state = r.conv, ca.eps = s.m.eps;
 	ca.bias = (const bf16*)L.conv_b, ca.pcol = L.type == SEQ_MAMBA2 ? L.heads * L.vdim : 0; // Mamba-2: the channels start behind z
 	const double bytes = (double)sb.N * ca.channels * 8;
+	const int widest = std::max({ca.seg[0].heads ? ca.seg[0].hd : 0, ca.seg[1].heads ? ca.seg[1].hd : 0, ca.seg[2].heads ? ca.seg[2].hd : 0});
+	if (sb.N == sb.B && L.taps >= 2 && L.taps <= 4 && widest <= 256) { // one token per sequence
+		++g_seq_routes[SEQ_ROUTE_CONV_STEPS];
+		run_kernel(s, KD_CONV, bytes, 0, [&] {
+			const dim3 grid(sb.N, cdiv(units, 4));
+			if (widest <= 64) launch_k(s, k_seq_conv_step<2>, grid, 128, 0, ca, sb, r.conv);
+			else if (widest <= 128) launch_k(s, k_seq_conv_step<4>, grid, 128, 0, ca, sb, r.conv);
+			else launch_k(s, k_seq_conv_step<8>, grid, 128, 0, ca, sb, r.conv);
+		});
+		return;
+	}
 	run_kernel(s, KD_CONV, bytes, 0, [&] { launch_k(s, k_seq_conv_heads, dim3(sb.N, cdiv(units, 4)), 128, 0, ca, sb); });
 	if (L.taps > 1)
 		run_kernel(s, KD_CONV, 0, 0, [&] { launch_k(s, k_seq_conv_state, dim3(cdiv(ca.channels, 128), sb.B), 128, 0, r.conv, proj, ca.ldp, L.taps, ca.channels, sb, ca.pcol); });
@@ -887,6 +898,14 @@ void gla_launch(Seq& s, GlaArgs& g, const SeqBatch& sb, int ld) {
 		};
 		if (D == 128) go(k_seq_gla_local<128>, k_seq_gla_starts<128>, k_seq_gla_apply<128>);
 		else go(k_seq_gla_local<64>, k_seq_gla_starts<64>, k_seq_gla_apply<64>);
+		return;
+	}
+	if (N == sb.B && g.vec && D <= 256) { // one token per sequence: a stream over the states
+		++g_seq_routes[SEQ_ROUTE_GLA_STEPS];
+		run_kernel(s, KD_GLA, (double)N * H * (3.0 * D + 2.0 * Dv) * 4 + 2.0 * sb.B * H * D * Dv * 4, (double)N * H * D * Dv * 4.0, [&] {
+			if (D <= 128) launch_k(s, k_seq_gla_step<1>, dim3(sb.B, H, cdiv(Dv, 64)), 128, 0, g, sb);
+			else launch_k(s, k_seq_gla_step<2>, dim3(sb.B, H, cdiv(Dv, 32)), 128, 0, g, sb);
+		});
 		return;
 	}
 	// lanes per value column: more of them while sequences x heads x columns alone would leave SMs without a CTA

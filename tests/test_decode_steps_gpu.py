@@ -1,0 +1,56 @@
+"""Steps of one token per sequence: gated linear attention as a stream over the states (k_seq_gla_step: key channels that fill part of a lane's four, one and two
+groups of 128, value columns that end inside a warp's share) and the convolution with its state in one kernel (k_seq_conv_step: two to four taps, head vectors of each
+instance and with a rest), against the plain float64 statement, from states that a prompt left behind; which of them ran is asserted, and what keeps the other kernels."""
+import os
+import sys
+
+import pytest
+
+sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
+import bovinex_plain  # noqa: E402
+import test_bovinex_gpu as tb  # noqa: E402
+import test_vimulorn_gpu as tv  # noqa: E402
+import vimulorn_plain  # noqa: E402
+
+from calm_b200 import bovinex, seqlib, vimulorn  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+def ran(route):
+    return seqlib.load().calm_b200_seq_route_count(route)
+
+
+def decode(mod, plain, t, cfg, dtype, route, steps=11):
+    """Prompts of three lengths, decoded tokens of all, then of the two outer ones: (largest relative error, layers that ran as steps)."""
+    weights, counts = t.weights(cfg, 5), [5, 2, 9]
+    toks = [t.tokens(cfg, n + steps + 3, 3 + i) for i, n in enumerate(counts)]
+    refs, worst, before = [plain.forward(cfg, t.as_f64(weights), x) for x in toks], 0.0, ran(route)
+    with mod.from_tensors(cfg, weights, dtype, max_tokens=256, max_seqs=4, page=16) as m:
+        slots = [m.open() for _ in counts]
+        m.step(slots, [x[:n] for x, n in zip(toks, counts)], [0])
+        assert ran(route) == before
+        for k in range(steps + 3):
+            who = [0, 1, 2] if k < steps else [2, 0]
+            out = m.step([slots[i] for i in who], [[toks[i][counts[i] + k]] for i in who], list(range(len(who))))
+            worst = max(worst, *(t.rel_err(out[j:j + 1], refs[i][counts[i] + k:counts[i] + k + 1]) for j, i in enumerate(who)))
+    return worst, ran(route) - before
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("heads,dim,vdim,steps", [(3, 16, 24, True), (2, 64, 20, True), (1, 128, 132, True), (4, 96, 68, True), (2, 132, 36, True), (1, 256, 64, True), (2, 64, 21, False)])
+def test_gated_linear_attention(dtype, heads, dim, vdim, steps):
+    cfg = tb.config([tb.gla(heads=heads, dim=dim, vdim=vdim, a_rank=8), tb.gla(heads=heads, dim=dim, vdim=vdim, a_rank=8)])
+    err, layers = decode(bovinex, bovinex_plain, tb, cfg, dtype, 3)
+    assert err < tb.TOL[dtype]
+    assert layers >= 2 and layers % 2 == 0 if steps else layers == 0
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("layer,steps", [(tv.delta(dim=64, vdim=64, conv=4), True), (tv.delta(dim=16, vdim=200, conv=3), True), (tv.window(dim=128, vdim=120, conv=2), True),
+                                         (tv.window(dim=48, vdim=20, conv=4), True), (tv.delta(conv=5), False)], ids=["delta64", "delta16-200", "window128", "window48", "five taps"])
+def test_convolution(dtype, layer, steps):
+    cfg = tv.config([layer, layer])
+    err, layers = decode(vimulorn, vimulorn_plain, tv, cfg, dtype, 4)
+    assert err < tv.TOL[dtype]
+    assert layers >= 2 and layers % 2 == 0 if steps else layers == 0
