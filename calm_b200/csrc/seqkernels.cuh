@@ -134,9 +134,14 @@ __device__ __forceinline__ float cta_sum(float v, float* red) {
 #define RMS_KEEP 16
 template <typename AT, bool LN = false>
 __global__ void __launch_bounds__(256) k_seq_rms(AT* out, const float* x, const int* rows, const bf16* w, float offset, float eps, int R, int width) {
-	pdl_enter(); // programmatic dependent launch: let the next kernel's launch overlap this one, then wait for the previous one
+	pdl_launch_next();
 	__shared__ float red[8], redm[8];
 	const int tid = threadIdx.x, nt = blockDim.x, r = blockIdx.x;
+	bf16 wk[RMS_KEEP]; // the weights are there before the previous kernel has ended
+#pragma unroll
+	for (int i = 0; i < RMS_KEEP; ++i)
+		if (i * nt + tid < width) wk[i] = w[i * nt + tid];
+	pdl_wait_prev();
 	const float* src = x + (size_t)(rows ? rows[r] : r) * width;
 	float keep[RMS_KEEP];
 	float ss = 0.f, mean = 0.f;
@@ -169,7 +174,7 @@ __global__ void __launch_bounds__(256) k_seq_rms(AT* out, const float* x, const 
 #pragma unroll
 	for (int i = 0; i < RMS_KEEP; ++i) {
 		const int c = i * nt + tid;
-		if (c < width) d[c] = to_act<AT>(keep[i] * rinv * (ldf(w + c) + offset));
+		if (c < width) d[c] = to_act<AT>(keep[i] * rinv * (__bfloat162float(wk[i]) + offset));
 	}
 	for (int c = RMS_KEEP * nt + tid; c < width; c += nt) d[c] = to_act<AT>((src[c] - mean) * rinv * (ldf(w + c) + offset));
 }
@@ -2236,10 +2241,12 @@ struct QkArgs {
 	bf16* qb = nullptr; // given: the queries leave in the activation type for the product path instead, as they are (qsplit 0) or as
 	int qsplit = 0;     //        [hi | hi | lo] rows of `dim` columns each per head (see k_seq_split_q)
 };
-__global__ void __launch_bounds__(256) k_seq_qk_rope(QkArgs a, SeqBatch sb) {
+// TH threads: 1024 where few tokens have a CTA each (16 tokens, 16 + 4 heads of 128 normed as a whole: 15.5 us with 256, most of it ten steps of two loads one after the other)
+template <int TH>
+__global__ void __launch_bounds__(TH) k_seq_qk_rope(QkArgs a, SeqBatch sb) {
 	pdl_enter(); // programmatic dependent launch: let the next kernel's launch overlap this one, then wait for the previous one
 	extern __shared__ float cs[]; // [rot_dims/2] cos, [rot_dims/2] sin, then (per_head) [heads + kv_heads] reciprocal root mean squares
-	__shared__ float red[2][8];
+	__shared__ float red[2][TH / 32];
 	const int n = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 	const int Q = a.heads * a.dim, K = a.kv_heads * a.dim, Vn = a.vheads * a.vdim, half = a.rot_dims / 2;
 	const float* pr = a.proj + (size_t)n * a.ldp;

@@ -1054,7 +1054,10 @@ void mixer_typed(Seq& s, const SeqLayer& L, RunState& r, const SeqBatch& sb, dou
 		// few tokens: their heads are shared out over several CTAs (a norm over the whole projection keeps them in one)
 		const int slices = L.q_norm && !L.qk_per_head ? 1 : std::max(1, std::min(cdiv(H + G, 8), 2 * s.sms / N));
 		const size_t qk_smem = ((size_t)2 * std::max(L.rot_dims / 2, 1) + H + G) * sizeof(float);
-		run_kernel(s, KD_QK, (double)N * ((H + G) * D * 4.0 + Vn * 4.0 + H * D * (direct ? 2.0 * (L.scores_f32 ? 3 : 1) : 4.0) + (G * D + Gv * Dv) * 4.0), 0, [&] { launch_k(s, k_seq_qk_rope, dim3(N, slices), 256, qk_smem, qa, sb); });
+		run_kernel(s, KD_QK, (double)N * ((H + G) * D * 4.0 + Vn * 4.0 + H * D * (direct ? 2.0 * (L.scores_f32 ? 3 : 1) : 4.0) + (G * D + Gv * Dv) * 4.0), 0, [&] {
+			if (slices == 1 && 2 * N <= s.sms) launch_k(s, k_seq_qk_rope<1024>, N, 1024, qk_smem, qa, sb);
+			else launch_k(s, k_seq_qk_rope<256>, dim3(N, slices), 256, qk_smem, qa, sb);
+		});
 		AttArgs a;
 		a.q = s.f[0], a.kc = r.cache_a, a.vc = r.cache_b, a.kld = G * D, a.vld = Gv * Dv, a.heads = H, a.group = H / G, a.kd = D, a.vd = Dv, a.vshare = maps;
 		a.window = L.window, a.keep_first = L.window > 0 ? L.keep_first : 0, a.scale = L.scale, a.sink = nullptr;
