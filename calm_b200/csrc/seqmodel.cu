@@ -160,14 +160,22 @@ void run_kernel(Seq& s, int kind, double bytes, double flops, F&& launch) {
 // Every kernel goes out with programmatic stream serialization allowed: it may be launched while its predecessor still runs and
 // parks in pdl_enter() until that one has completed and flushed (a no-op attribute-less launch when CALM_B200_SEQ_PDL=0).
 template <typename... KArgs, typename... Args>
-void launch_k(Seq& s, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
+void launch_c(Seq& s, int cluster_z, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) { // clusters of cluster_z CTAs along z
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = s.stream;
-	cudaLaunchAttribute at[1];
-	at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-	at[0].val.programmaticStreamSerializationAllowed = 1;
-	cfg.attrs = at, cfg.numAttrs = s.pdl ? 1 : 0;
+	cudaLaunchAttribute at[2];
+	int n = 0;
+	if (s.pdl) at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization, at[n++].val.programmaticStreamSerializationAllowed = 1;
+	if (cluster_z > 1) {
+		at[n].id = cudaLaunchAttributeClusterDimension;
+		at[n].val.clusterDim.x = 1, at[n].val.clusterDim.y = 1, at[n++].val.clusterDim.z = cluster_z;
+	}
+	cfg.attrs = at, cfg.numAttrs = n;
 	CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
+}
+template <typename... KArgs, typename... Args>
+void launch_k(Seq& s, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
+	launch_c(s, 1, kernel, grid, block, smem, args...);
 }
 
 // attention maps per head (SEQ_GQA: 2 for differential attention); latent attention: query columns in front of the latent, gate rows
@@ -563,7 +571,7 @@ void hc_read(Seq& s, void* out, const int* rows, const void* in, const SeqNorm& 
 // head tile) when few tokens look back over a long context.  bf16 mode takes the tensor-core kernel wherever its shared memory and registers
 // hold the heads' width.
 struct AttnPlan {
-	bool mma;
+	bool mma, cluster = false;
 	int tile, nsplit;
 	size_t smem;
 };
@@ -573,7 +581,7 @@ int round_split(int n) {
 	while (v < n) v = v < 4 ? v + 1 : (v & (v - 1)) ? v / 3 * 4 : v / 2 * 3; // 1 2 3 4 6 8 12 16 24 ...
 	return v;
 }
-AttnPlan attn_plan(const Seq& s, int group, int kd, int vd, bool shared_kv, int heads, int live_tokens, int span, int longest) {
+AttnPlan attn_plan(const Seq& s, int group, int kd, int vd, bool shared_kv, int heads, int live_tokens, int span, int longest, bool parts = false) {
 	AttnPlan p;
 	p.smem = atm_smem(kd, vd, shared_kv);
 	p.mma = s.attn_mma && !s.m.exact && p.smem <= 220 * 1024 && vd <= 8 * 8 * ATM_TILES;
@@ -581,8 +589,14 @@ AttnPlan attn_plan(const Seq& s, int group, int kd, int vd, bool shared_kv, int 
 	if (p.mma) {
 		p.tile = std::min(group, 16);
 		while (group % p.tile) --p.tile;
-		const int ctas = live_tokens * (heads / p.tile), room = s.sms * std::max(1, std::min(4, (int)(227 * 1024 / (p.smem + 1024))));
+		const int per_sm = std::max(1, std::min(4, (int)(227 * 1024 / (p.smem + 1024)))), ctas = live_tokens * (heads / p.tile), room = s.sms * per_sm;
 		p.nsplit = ctas >= room ? 1 : std::max(1, std::min({round_split(cdiv(keys, ATM_KC)), room / ctas, ATT_MAXSPLIT}));
+		// Up to twelve shares run as at most eight, which a thread-block cluster folds: a second 32 keys for some of them cost less than the merge's launch.  The sums of a
+		// share go where its keys were, and all clusters are to run at one time (the GPCs hold this many of a size with a CTA per SM).
+		static const int most[9] = {0, 0, 74, 45, 33, 26, 22, 15, 15};
+		const int shares = std::min(p.nsplit, 8);
+		p.cluster = !parts && p.nsplit > 1 && p.nsplit <= 12 && ctas <= most[shares] * per_sm && (size_t)p.tile * vd <= (size_t)2 * ATM_KC * (atm_pad(kd) + (shared_kv ? 0 : atm_pad(vd)));
+		if (p.cluster) p.nsplit = shares;
 	} else {
 		p.tile = attn_tile(group, kd, vd), p.smem = attn_smem(p.tile, kd);
 		const int ctas = live_tokens * (heads / p.tile);
@@ -743,8 +757,9 @@ void attention(Seq& s, int kind, AttArgs a, void* out, const SeqBatch& sb, doubl
 	int span = a.window > 0 ? a.window + a.keep_first : 0;
 	if (a.chunk > 0) span = span > 0 ? std::min(span, a.chunk) : a.chunk;
 	const bool shared_kv = a.kc == a.vc;
-	const AttnPlan p = attn_plan(s, a.group, a.kd, a.vd, shared_kv, a.heads, live, span, longest);
-	a.tile = p.tile, a.nsplit = p.nsplit;
+	const AttnPlan p = attn_plan(s, a.group, a.kd, a.vd, shared_kv, a.heads, live, span, longest, diff != nullptr);
+	a.tile = p.tile, a.nsplit = p.nsplit, a.cluster = p.cluster;
+	if (a.cluster) ++g_seq_routes[SEQ_ROUTE_ATTN_CLUSTERS];
 	ensure_part(s, (size_t)sb.N * a.heads * a.nsplit * (a.vd + 2));
 	a.part = s.part;
 	const dim3 grid(sb.N, a.heads / a.tile, a.nsplit);
@@ -752,7 +767,7 @@ void attention(Seq& s, int kind, AttArgs a, void* out, const SeqBatch& sb, doubl
 	const double flops = 2.0 * kv_rows * a.heads * (a.kd + a.vd);
 	run_kernel(s, kind, a.skip ? 0 : bytes, a.skip ? 0 : flops, [&] {
 		auto al4 = [](long v) { return v % 4 == 0; };
-		if (p.mma) launch_k(s, k_seq_attn_mma, grid, 256, p.smem, a, (bf16*)out, sb, shared_kv ? 1 : 0, al4(a.kd) && al4(a.kld) && (shared_kv || (al4(a.vd) && al4(a.vld))) ? 1 : 0);
+		if (p.mma) launch_c(s, a.cluster ? a.nsplit : 1, k_seq_attn_mma, grid, 256, p.smem, a, (bf16*)out, sb, shared_kv ? 1 : 0, al4(a.kd) && al4(a.kld) && (shared_kv || (al4(a.vd) && al4(a.vld))) ? 1 : 0);
 		else if (s.m.exact) launch_k(s, k_seq_attention<float>, grid, ATT_THREADS, p.smem, a, (float*)out, sb);
 		else launch_k(s, k_seq_attention<bf16>, grid, ATT_THREADS, p.smem, a, (bf16*)out, sb);
 	});
@@ -762,7 +777,7 @@ void attention(Seq& s, int kind, AttArgs a, void* out, const SeqBatch& sb, doubl
 			if (s.m.exact) launch_k(s, k_seq_attn_diff_merge<float>, mg, 128, 0, a, *diff, (float*)out);
 			else launch_k(s, k_seq_attn_diff_merge<bf16>, mg, 128, 0, a, *diff, (bf16*)out);
 		});
-	else if (a.nsplit > 1)
+	else if (a.nsplit > 1 && !a.cluster)
 		run_kernel(s, kind, 0, 0, [&] {
 			const dim3 mg(sb.N, a.heads, cdiv(a.vd, 128));
 			if (s.m.exact) launch_k(s, k_seq_attention_merge<float>, mg, 128, 0, a, (float*)out);
@@ -1451,7 +1466,7 @@ void forward_decode_graph(Seq& s, const SeqBatch& sb, int n_want, double kv_rows
 		if (L.type != SEQ_LATENT && L.type != SEQ_WINDOW && L.type != SEQ_GQA) return; // recurrent mixers: nothing to share out
 		const bool lat = L.type == SEQ_LATENT;
 		const int group = lat ? L.heads : L.heads / L.kv_heads, kd = lat ? L.kv_rank + L.rot_dims : L.dim, vd = lat ? L.kv_rank : L.vdim;
-		const int heads = L.heads * att_maps(L), ns = attn_plan(s, group, kd, vd, lat, heads, sb.N, attn_span(L), longest).nsplit;
+		const int heads = L.heads * att_maps(L), ns = attn_plan(s, group, kd, vd, lat, heads, sb.N, attn_span(L), longest, att_maps(L) > 1).nsplit;
 		key.push_back(ns);
 		part_need = std::max(part_need, (size_t)sb.N * heads * ns * (vd + 2));
 	};

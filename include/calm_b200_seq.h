@@ -300,6 +300,7 @@ enum {
 	SEQ_ROUTE_DELTA_BLOCKS = 2, /* a layer's delta rule ran in blocks of tokens */
 	SEQ_ROUTE_GLA_STEPS = 3,    /* a layer's gated linear attention ran as one token per sequence (counted when it is captured, too) */
 	SEQ_ROUTE_CONV_STEPS = 4,   /* so did a layer's convolution */
+	SEQ_ROUTE_ATTN_CLUSTERS = 5, /* a layer's shares of the keys were folded inside thread-block clusters */
 	SEQ_ROUTE_PAIRS = 16        /* + epilogue: a product was launched (or captured) on pairs of CTAs */
 };
 uint64_t calm_b200_seq_route_count(int route);

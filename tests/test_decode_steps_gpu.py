@@ -54,3 +54,22 @@ def test_convolution(dtype, layer, steps):
     err, layers = decode(vimulorn, vimulorn_plain, tv, cfg, dtype, 4)
     assert err < tv.TOL[dtype]
     assert layers >= 2 and layers % 2 == 0 if steps else layers == 0
+
+
+# keys of a decoded token: 32 a share up to eight shares, twelve shares as eight, more as before
+@pytest.mark.parametrize("n,clusters", [(40, True), (95, True), (161, True), (255, True), (300, True), (383, True), (420, False)])
+@pytest.mark.parametrize("layer", [tv.latent(), tv.latent(heads=16, dim=64, vdim=128, kv_rank=96), tv.window(size=1000), tb.attn(size=0), tb.attn(heads=8, kv_heads=1, dim=64, vdim=128, size=600, keep=5)],
+                         ids=["latent", "latent16", "sinks", "groups", "eight heads"])
+def test_shares_in_clusters(layer, n, clusters):
+    t, mod, plain = (tb, bovinex, bovinex_plain) if layer["mixer"].get("rot") else (tv, vimulorn, vimulorn_plain)
+    cfg = t.config([layer])
+    weights, toks = t.weights(cfg, 5), t.tokens(cfg, n + 3)
+    ref, before = plain.forward(cfg, t.as_f64(weights), toks), ran(5)
+    with mod.from_tensors(cfg, weights, "bfloat16", max_tokens=512, max_seqs=2, page=16) as m:
+        slot = m.open()
+        m.step([slot], [toks[:n]], [0])
+        at = ran(5)
+        for k in range(3):
+            out = m.step([slot], [[toks[n + k]]], [0])
+            assert t.rel_err(out, ref[n + k:n + k + 1]) < t.TOL["bfloat16"], k
+    assert at == before and (ran(5) > at) == clusters
