@@ -24,7 +24,7 @@
 // rows after the other with one accumulator per tile and the vector's pieces made as they are needed (wo, w2: few rows, long ones).
 //
 // Measured, a whole token: Qwen2-0.5B fp16 at 131 positions 895 -> 648 us, Llama-3-8B fp8 at 4095 2200 -> 2144 us; tokens of six layers between those
-// widths 1.01 to 1.27 times as fast (k_qkv, k_matres, ring.cuh before).  By stage, Llama-3-8B fp8: q/k/v 8.6 -> 6.7 us, wo 7.4 -> 6.9, FFN up 19.8 -> 21, w2 13.9 -> 13.3; 0.5B: 4.1 ->
+// widths 1.00 to 1.28 times as fast (k_qkv, k_matres, ring.cuh before).  By stage, Llama-3-8B fp8: q/k/v 8.6 -> 6.7 us, wo 7.4 -> 6.9, FFN up 19.8 -> 21, w2 13.9 -> 13.3; 0.5B: 4.1 ->
 // 1.8, 3.4 -> 1.5, 6.8 -> 4.2, 7.7 -> 3.6.  What bounds it now: about 2 us from the last store of a stage to the first product of the next (the grid's end is seen after 1.1 us,
 // the vector's way to the registers and its pieces take the rest), then the memory's rate.
 #pragma once

@@ -1,4 +1,5 @@
-// ring.cuh -- the two largest matvec stages (FFN up, FFN down; and wo) fed by warp-private bulk-TMA rings.
+// ring.cuh -- the two largest matvec stages (FFN up, FFN down; and wo) fed by warp-private bulk-TMA rings: gf4 models, and stages of fp8 and fp16
+// models that plan_cols finds no plan for (cols.cuh serves the others).
 //
 // Why: the register-fed stage kernels keep their bytes in flight in registers --
 // a warp requests one batch (8 x 16 B per lane), waits a DRAM round trip, consumes it, and only then requests the next --
