@@ -63,6 +63,7 @@ struct ColsRun {
 	int steps, chunk_steps; // 64-byte steps of a row, and of its pieces in a stage (the last may have fewer)
 	int own;                // of a piece's steps, those of a warp: 2 or 4
 	int* err;               // mapped host word: a wait that gave up
+	unsigned tries;         // of a wait before it gives up
 };
 
 struct ColsShared {
@@ -94,9 +95,24 @@ __device__ __forceinline__ void cols_wait_prev(bool polls) {
 	asm volatile("bar.sync 1, %0;" ::"n"(COLS_THREADS) : "memory");
 }
 
+// Every wait is bounded: a role whose wait gives up leaves its loop with a code, and the others' waits then run out too.
+__device__ __forceinline__ bool cols_gave_up(ColsShared* sh, int code) {
+	if ((threadIdx.x & 31) == 0) sh->gave_up = code;
+	return false;
+}
+// The end of a CTA's roles.  issued: the first of this copying warp's stages that it did not request (0: another warp).  Whichever role gave up, and however far the copies had come
+// by then: nothing may be in flight into this CTA's shared memory when it exits.
+__device__ __forceinline__ void cols_finish(ColsShared* sh, const ColsRun& r, int issued) {
+	__syncthreads();
+	if (!sh->gave_up) return;
+	for (int k = issued - 2; k >= max(0, issued - COLS_STAGES); k -= 2) mbar_wait_warp(&sh->full[k % COLS_STAGES], (k / COLS_STAGES) & 1); // the last stage of each of its slots
+	if (threadIdx.x == 0) *reinterpret_cast<volatile int*>(r.err) = sh->gave_up;
+}
+
 // A copying warp (of two: they take the stages in turn).  order(i, tile, chunk): what stage i holds; row(tile, slot): where the weights of the tile's row `slot` begin, NULL: no such row.
+// Returns the first of its stages that it did not request.
 template <typename OrderFn, typename RowFn>
-__device__ __forceinline__ void cols_produce(ColsShared* sh, const ColsRun& r, unsigned char* ring, int nst, OrderFn order, RowFn row) {
+__device__ __forceinline__ int cols_produce(ColsShared* sh, const ColsRun& r, unsigned char* ring, int nst, OrderFn order, RowFn row) {
 	const int lane = threadIdx.x & 31, which = (threadIdx.x >> 5) - COLS_WARPS;
 	const uint64_t policy = l2_policy_evict_first();
 	bool waited = false;
@@ -105,7 +121,10 @@ __device__ __forceinline__ void cols_produce(ColsShared* sh, const ColsRun& r, u
 		const int slot = i % COLS_STAGES;
 		if (i >= COLS_STAGES) {
 			if (!waited) cols_wait_prev(which == 0), waited = true; // no stage is free before the others have activations
-			if (!mbar_wait_warp(&sh->empty[slot], ((i / COLS_STAGES) & 1) ^ 1)) break;
+			if (!mbar_wait_warp(&sh->empty[slot], ((i / COLS_STAGES) & 1) ^ 1, r.tries)) {
+				cols_gave_up(sh, 9401);
+				break;
+			}
 		}
 		int tile, chunk;
 		order(i, tile, chunk);
@@ -117,10 +136,7 @@ __device__ __forceinline__ void cols_produce(ColsShared* sh, const ColsRun& r, u
 		if (src) tma_load_1d_hint(ring + slot * COLS_STAGE + lane * COLS_PITCH, src + (size_t)chunk * r.chunk_steps * 64, bytes, &sh->full[slot], policy);
 	}
 	if (!waited) cols_wait_prev(which == 0);
-	if (i < nst) { // a warp gave up: nothing may be in flight into this CTA's shared memory when it exits
-		if (lane == 0) sh->gave_up = 9301;
-		for (int k = i - 2; k >= max(0, i - COLS_STAGES); k -= 2) mbar_wait_warp(&sh->full[k % COLS_STAGES], (k / COLS_STAGES) & 1);
-	}
+	return i;
 }
 
 __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -230,13 +246,13 @@ __device__ __forceinline__ void cols_multiply(const unsigned char* stage, const 
 }
 
 // this warp's sums of a tile's 8 rows: columns 0 - 2 of rows 0 - 7 and columns 3 - 5 of rows 8 - 15
-__device__ __forceinline__ bool cols_hand_over(ColsShared* sh, float* part, const ColsLane& l, int tile, const float (&acc)[4], float unscale) {
+__device__ __forceinline__ bool cols_hand_over(ColsShared* sh, const ColsRun& r, float* part, const ColsLane& l, int tile, const float (&acc)[4], float unscale) {
 	float v = (l.t == 2 ? acc[2] : acc[0]) + (l.t == 0 ? acc[1] : acc[3]);
 	v = l.t == 3 ? 0.f : v;
 	v += __shfl_xor_sync(0xffffffffu, v, 1);
 	v += __shfl_xor_sync(0xffffffffu, v, 2);
 	const int buf = tile % COLS_PARTS;
-	if (tile >= COLS_PARTS && !mbar_wait_warp(&sh->part_empty[buf], ((tile / COLS_PARTS) & 1) ^ 1)) return false;
+	if (tile >= COLS_PARTS && !mbar_wait_warp(&sh->part_empty[buf], ((tile / COLS_PARTS) & 1) ^ 1, r.tries)) return cols_gave_up(sh, 9402);
 	if (l.t == 0) part[(buf * COLS_WARPS + l.warp) * 8 + l.g] = v * unscale;
 	__syncwarp();
 	if (l.lane == 0) mbar_arrive(&sh->part_full[buf]);
@@ -245,12 +261,12 @@ __device__ __forceinline__ bool cols_hand_over(ColsShared* sh, float* part, cons
 
 // The epilogue's warp: emit(tile, slot, v) with row slot lane % 8 and its sum in every eight lanes.
 template <typename EmitFn>
-__device__ __forceinline__ void cols_epilogue(ColsShared* sh, const float* part, int tiles, EmitFn emit) {
+__device__ __forceinline__ void cols_epilogue(ColsShared* sh, const ColsRun& r, const float* part, int tiles, EmitFn emit) {
 	const int lane = threadIdx.x & 31, row = lane & 7, quarter = lane >> 3;
 	for (int tile = 0; tile < tiles; ++tile) {
 		const int buf = tile % COLS_PARTS;
-		if (!mbar_wait_warp(&sh->part_full[buf], (tile / COLS_PARTS) & 1)) {
-			if (lane == 0) sh->gave_up = 9302;
+		if (!mbar_wait_warp(&sh->part_full[buf], (tile / COLS_PARTS) & 1, r.tries)) {
+			cols_gave_up(sh, 9403);
 			return;
 		}
 		const float* p = part + (buf * COLS_WARPS + quarter * (COLS_WARPS / 4)) * 8 + row;
@@ -328,10 +344,7 @@ struct ColsTiles {
 		int slot = 0, parity = 0;
 		const int whole = l.own(r, 0), rest = l.own(r, NC - 1);
 		auto stage = [&](int c, float (&acc)[4]) {
-			if (!mbar_wait_warp(&sh->full[slot], parity)) {
-				if (l.lane == 0) sh->gave_up = 9300;
-				return false;
-			}
+			if (!mbar_wait_warp(&sh->full[slot], parity, r.tries)) return cols_gave_up(sh, 9400);
 			cols_multiply<DBITS>(ring + slot * COLS_STAGE, r, l, c < NC - 1 ? whole : rest, x[c], acc);
 			__syncwarp(); // every lane has read its weights
 			if (l.lane == 0) mbar_arrive(&sh->empty[slot]);
@@ -344,13 +357,13 @@ struct ColsTiles {
 			x[c].make(buf, l, f[c]);
 			if (!stage(c, acc)) return;
 		}
-		if (!cols_hand_over(sh, part, l, 0, acc, unscale)) return;
+		if (!cols_hand_over(sh, r, part, l, 0, acc, unscale)) return;
 		for (int tile = 1; tile < tiles; ++tile) {
 			acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
 #pragma unroll
 			for (int c = 0; c < NC; ++c)
 				if (!stage(c, acc)) return;
-			if (!cols_hand_over(sh, part, l, tile, acc, unscale)) return;
+			if (!cols_hand_over(sh, r, part, l, tile, acc, unscale)) return;
 		}
 	}
 };
@@ -368,10 +381,11 @@ __global__ void __maxnreg__((ColsTiles<DBITS, NC>::REGS)) k_qkv_cols(const QkvAr
 	const int nrows = a.q_dim + 2 * a.kv_dim;
 	const int row0 = 2 * cols_share(nrows / 2, blockIdx.x), rows = 2 * cols_share(nrows / 2, blockIdx.x + 1) - row0, tiles = (rows + 7) / 8;
 	const ColsLane l;
+	int issued = 0;
 	cols_init(&sh);
 	if (l.warp == COLS_WARPS || l.warp == COLS_WARPS + 1) {
 		const size_t rowbytes = (size_t)r.steps * 64;
-		cols_produce(&sh, r, smem_raw, tiles * NC, [&](int i, int& tile, int& chunk) { tile = i / NC, chunk = i % NC; },
+		issued = cols_produce(&sh, r, smem_raw, tiles * NC, [&](int i, int& tile, int& chunk) { tile = i / NC, chunk = i % NC; },
 		             [&](int tile, int slot) -> const unsigned char* {
 			             const int j = row0 + 8 * tile + slot;
 			             if (j >= row0 + rows) return nullptr;
@@ -396,7 +410,7 @@ __global__ void __maxnreg__((ColsTiles<DBITS, NC>::REGS)) k_qkv_cols(const QkvAr
 		__syncwarp();
 		const int kv_pos = a.tp->kv_pos;
 		float post = 1.f;
-		cols_epilogue(&sh, part, tiles, [&](int tile, int slot, float v) {
+		cols_epilogue(&sh, r, part, tiles, [&](int tile, int slot, float v) {
 			if (tile == 0 && a.normw) post = cols_rms(&sh, a.dim, a.eps);
 			v *= post;
 			const float other = __shfl_xor_sync(0xffffffffu, v, 1);
@@ -421,12 +435,11 @@ __global__ void __maxnreg__((ColsTiles<DBITS, NC>::REGS)) k_qkv_cols(const QkvAr
 			}
 		});
 	}
-	__syncthreads();
+	cols_finish(&sh, r, issued);
 	if (a.xb_out && blockIdx.x == 0 && l.warp < COLS_WARPS) { // norm_par: the FFN reads the normalised vector
 		const float post = a.normw ? cols_rms(&sh, a.dim, a.eps) : 1.f;
 		for (int i = threadIdx.x; i < a.dim; i += 32 * COLS_WARPS) a.xb_out[i] = __ldcg(a.x + i) * (a.normw ? a.normw[i] : 1.f) * post;
 	}
-	if (threadIdx.x == 0 && sh.gave_up) *reinterpret_cast<volatile int*>(r.err) = sh.gave_up;
 	stamp_end(a.stamp);
 }
 
@@ -442,10 +455,11 @@ __global__ void __maxnreg__((ColsTiles<DBITS, NC>::REGS)) k_ffn_up_cols(const Ff
 	uint32_t* buf = reinterpret_cast<uint32_t*>(part + COLS_PARTS * COLS_WARPS * 8);
 	const int i0 = cols_share(a.hidden, blockIdx.x), n = cols_share(a.hidden, blockIdx.x + 1) - i0, tiles = (n + 3) / 4;
 	const ColsLane l;
+	int issued = 0;
 	cols_init(&sh);
 	if (l.warp == COLS_WARPS || l.warp == COLS_WARPS + 1) {
 		const size_t rowbytes = (size_t)r.steps * 64;
-		cols_produce(&sh, r, smem_raw, tiles * NC, [&](int i, int& tile, int& chunk) { tile = i / NC, chunk = i % NC; },
+		issued = cols_produce(&sh, r, smem_raw, tiles * NC, [&](int i, int& tile, int& chunk) { tile = i / NC, chunk = i % NC; },
 		             [&](int tile, int slot) -> const unsigned char* {
 			             const int i = 4 * tile + (slot & 3);
 			             return i >= n ? nullptr : (const unsigned char*)(slot < 4 ? a.w1 : a.w3) + (size_t)(i0 + i) * rowbytes;
@@ -459,7 +473,7 @@ __global__ void __maxnreg__((ColsTiles<DBITS, NC>::REGS)) k_ffn_up_cols(const Ff
 	} else {
 		cols_wait_prev(false);
 		float post = 1.f;
-		cols_epilogue(&sh, part, tiles, [&](int tile, int slot, float v) {
+		cols_epilogue(&sh, r, part, tiles, [&](int tile, int slot, float v) {
 			if (tile == 0 && a.normw) post = cols_rms(&sh, a.dim, a.eps);
 			v *= post;
 			const float u3 = __shfl_xor_sync(0xffffffffu, v, 4);
@@ -467,8 +481,7 @@ __global__ void __maxnreg__((ColsTiles<DBITS, NC>::REGS)) k_ffn_up_cols(const Ff
 			if (l.lane < 4 && i < n) a.hb[i0 + i] = (a.gelu ? act_gelu(v) : act_silu(v)) * u3;
 		});
 	}
-	__syncthreads();
-	if (threadIdx.x == 0 && sh.gave_up) *reinterpret_cast<volatile int*>(r.err) = sh.gave_up;
+	cols_finish(&sh, r, issued);
 	stamp_end(a.stamp);
 }
 
@@ -485,10 +498,11 @@ __global__ void __maxnreg__((cols_regs(2 * ColsStep<DBITS>::B + 4 * T))) k_matre
 	const int row0 = cols_share(a.d, blockIdx.x), rows = cols_share(a.d, blockIdx.x + 1) - row0;
 	const int chunks = (r.steps + r.chunk_steps - 1) / r.chunk_steps;
 	const ColsLane l;
+	int issued = 0;
 	cols_init(&sh);
 	if (l.warp == COLS_WARPS || l.warp == COLS_WARPS + 1) {
 		const size_t rowbytes = (size_t)r.steps * 64;
-		cols_produce(&sh, r, smem_raw, T * chunks, [&](int i, int& tile, int& chunk) { tile = i % T, chunk = i / T; },
+		issued = cols_produce(&sh, r, smem_raw, T * chunks, [&](int i, int& tile, int& chunk) { tile = i % T, chunk = i / T; },
 		             [&](int tile, int slot) -> const unsigned char* {
 			             const int j = 8 * tile + slot;
 			             return j >= rows ? nullptr : (const unsigned char*)a.w + (size_t)(row0 + j) * rowbytes;
@@ -532,9 +546,8 @@ __global__ void __maxnreg__((cols_regs(2 * ColsStep<DBITS>::B + 4 * T))) k_matre
 			const int n = l.own(r, c);
 #pragma unroll
 			for (int t = 0; t < T; ++t) {
-				if (!mbar_wait_warp(&sh.full[slot], parity)) {
-					if (l.lane == 0) sh.gave_up = 9300;
-					ok = false;
+				if (!mbar_wait_warp(&sh.full[slot], parity, r.tries)) {
+					ok = cols_gave_up(&sh, 9400);
 					break;
 				}
 				cols_multiply<DBITS>(smem_raw + slot * COLS_STAGE, r, l, n, x, acc[t]);
@@ -545,22 +558,21 @@ __global__ void __maxnreg__((cols_regs(2 * ColsStep<DBITS>::B + 4 * T))) k_matre
 		}
 #pragma unroll
 		for (int t = 0; t < T; ++t)
-			if (ok) ok = cols_hand_over(&sh, part, l, t, acc[t], cols_unscale(e));
+			if (ok) ok = cols_hand_over(&sh, r, part, l, t, acc[t], cols_unscale(e));
 	} else {
 		cols_wait_prev(false);
 		for (int j = l.lane; j < rows; j += 32) sh.rows[j] = a.accumulate && a.tpx.world <= 1 ? __ldcg(a.y + row0 + j) : 0.f;
 		__syncwarp();
-		cols_epilogue(&sh, part, T, [&](int tile, int slot, float v) {
+		cols_epilogue(&sh, r, part, T, [&](int tile, int slot, float v) {
 			const int j = 8 * tile + slot;
 			if (l.lane >= 8 || j >= rows) return;
 			if (a.tpx.world > 1) sh.rows[j] = v;
 			else a.y[row0 + j] = sh.rows[j] + v;
 		});
 	}
-	__syncthreads();
+	cols_finish(&sh, r, issued);
 	if (a.tpx.world > 1) { // the matvec -> all-reduce fusion of stages.cuh TpExchange
 		tp_exchange_rows(a.tpx, sh.rows, row0, rows, a.y, a.d);
 	}
-	if (threadIdx.x == 0 && sh.gave_up) *reinterpret_cast<volatile int*>(r.err) = sh.gave_up;
 	stamp_end(a.stamp);
 }

@@ -65,6 +65,7 @@ struct Engine {
 	int ncand = 0;
 
 	unsigned pf_wait_limit = MBAR_SPINS; // tries of a wait in the prompt products
+	unsigned token_wait_limit = MBAR_SPINS; // ... in a token's matvecs (cols.cuh)
 	// attention launch shape
 	int attn_hg = 1, attn_hg2 = 1 /* k_attn2: padded to what it is instantiated for */, attn_qgroups = 1, attn_nsplit = 1, attn_lpp = 1;
 	ColsPlan cols_qkv, cols_wo, cols_up, cols_down; // matvecs on the tensor cores (cols.cuh); n == 0: the stage keeps its other kernels
@@ -549,7 +550,7 @@ constexpr int cols_chunks() {
 	return DBITS / 2; // 8192 weights
 }
 ColsRun cols_run(const ColsPlan& p) {
-	return ColsRun{p.steps, p.chunk_steps, 2 * cdiv(p.chunk_steps, 2 * COLS_WARPS), g.dev_err};
+	return ColsRun{p.steps, p.chunk_steps, 2 * cdiv(p.chunk_steps, 2 * COLS_WARPS), g.dev_err, g.token_wait_limit};
 }
 template <int DBITS, typename KVT>
 void cols_qkv(const QkvArgs<KVT>& a, const ColsPlan& p, bool attr_only) {
@@ -1057,6 +1058,7 @@ extern "C" void prepare_cuda(struct Transformer* transformer) {
 	g.use_pdl = !(getenv("CALM_B200_PDL") && atoi(getenv("CALM_B200_PDL")) == 0);
 	g.carveout = getenv("CALM_B200_CARVEOUT") ? atoi(getenv("CALM_B200_CARVEOUT")) : -1;
 	if (const char* e = getenv("CALM_B200_PREFILL_WAIT")) g.pf_wait_limit = (unsigned)atoi(e);
+	if (const char* e = getenv("CALM_B200_TOKEN_WAIT")) g.token_wait_limit = (unsigned)atoi(e);
 	g.debug = getenv("CALM_B200_DEBUG") && atoi(getenv("CALM_B200_DEBUG"));
 	if (g.debug) g.use_graph = false;
 	g.perf = (getenv("CALM_B200_PERF") && atoi(getenv("CALM_B200_PERF"))) || getenv("CUDA_INJECTION64_PATH");
@@ -1241,6 +1243,11 @@ extern "C" void calm_b200_release(struct Transformer* transformer) {
 	}
 }
 
+// Ends the process when a kernel's wait has given up: 93xx k_pf_gemm, 94xx cols.cuh (also in a token whose call did not synchronise), 92xx k_attn2's fold, which stops its kernel.
+static void check_waits() {
+	const int code = g.dev_err ? *(volatile int*)g.dev_err : 0;
+	if (code) CALM_FATAL("%s gave up (code %d)", code / 100 == 93 ? "prompt pass: a wait inside a product" : code / 100 == 94 ? "a wait inside a matvec of a token" : "a wait", code);
+}
 static void sync_stream() {
 	cudaError_t e = cudaStreamSynchronize(g.stream);
 	if (e != cudaSuccess) {
@@ -1249,7 +1256,7 @@ static void sync_stream() {
 		fprintf(stderr, "calm_b200: device failure: %s (%s); watchdog code %d\n", cudaGetErrorString(e), cudaGetErrorName(e), code);
 		abort();
 	}
-	if (g.dev_err && *(volatile int*)g.dev_err) CALM_FATAL("a wait inside a token gave up (code %d)", *(volatile int*)g.dev_err); // 9300 / 9301: cols.cuh
+	check_waits();
 }
 
 static void check_call(struct Transformer* transformer, int token, int pos) {
@@ -1639,7 +1646,7 @@ extern "C" int forward_prefill_cuda(struct Transformer* transformer, const int* 
 		default: pf_run<4, uint8_t>(m, pos0 + o); break;
 		}
 		CUDA_CHECK(cudaStreamSynchronize(g.stream)); // `tokens` is the caller's memory (pageable): the copy above must have left it
-		if (*(volatile int*)g.dev_err) CALM_FATAL("prompt pass: a wait inside a product gave up (code %d)", *(volatile int*)g.dev_err);
+		check_waits();
 	}
 	CUDA_CHECK(cudaGetLastError());
 	return 1;

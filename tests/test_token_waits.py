@@ -1,0 +1,47 @@
+"""Waits of a token's tensor-core matvecs (cols.cuh) that run out: whichever role gives up, the kernel ends with a code that the host reports, with no warp split and
+nothing left on its way into the shared memory of a CTA that has ended."""
+import os
+import re
+import subprocess
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+# 512 x 1024: a CTA's copying warps have requested all of their stages before the first is used
+CHILD = """
+from dataclasses import replace
+from calm_b200 import lib, modelgen as mg
+spec = replace(mg.SPECS["pf-tiny-hd128"], name="waits", dtype="%s", dim=%d, hidden_dim=%d, n_layers=2)
+with lib.DeviceModel(spec, mg.generate(spec, seed=3)) as dm:
+    assert all(lib.load().calm_b200_token_plan(s) for s in range(4))
+    dm.forward(5, 0)
+print("done")
+"""
+
+
+def test_copies_end_before_their_cta_whichever_role_gave_up():
+    """A multiplying warp can give up on a stage behind which the copying warps have nothing left to request: they cannot learn of it inside their loop."""
+    src = open(os.path.join(ROOT, "calm_b200", "csrc", "cols.cuh")).read()
+    waits = re.findall(r"mbar_wait_warp\(&sh(?:\.|->)\w+\[.*?\], .*?\)\)", src)
+    assert "mbar_wait_bounded(" not in src  # whole warps give up
+    assert len(waits) >= 5 and all(w.endswith("r.tries))") for w in waits), waits
+    finish = src[src.index("void cols_finish("):]
+    finish = finish[:finish.index("\n}\n")]
+    assert finish.index("__syncthreads()") < finish.index("gave_up") < finish.index("mbar_wait_warp(&sh->full[")
+    for kernel in ("k_qkv_cols", "k_ffn_up_cols", "k_matres_cols"):
+        body = src[src.index(kernel + "(const"):]
+        body = body[:body.index("\n}\n")]
+        assert "issued = cols_produce(" in body and body.index("cols_epilogue(") < body.index("\n\tcols_finish(&sh, r, issued);")
+        assert not re.search(r"\n\t{1,3}return;", body)  # every thread comes to the end
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,dim,hidden", [("fp8", 512, 1024), ("fp16", 512, 1024), ("fp8", 2048, 8192), ("fp16", 2048, 8192)])
+@pytest.mark.parametrize("tries", [0, 1])  # none: no role gets a stage; one: the ring is filled, what waits for a copy that has not landed gives up
+def test_reported(dtype, dim, hidden, tries):
+    env = dict(os.environ, CALM_B200_TOKEN_WAIT=str(tries), PYTHONPATH=ROOT)
+    r = subprocess.run([sys.executable, "-c", CHILD % (dtype, dim, hidden)], env=env, cwd=ROOT, capture_output=True, text=True, timeout=300)
+    gave_up = re.search(r"a wait inside a matvec of a token gave up \(code 94\d\d\)", r.stdout + r.stderr)
+    assert r.returncode != 0 and gave_up if tries == 0 else bool(gave_up) != ("done" in r.stdout), r.stdout + r.stderr
