@@ -37,6 +37,12 @@ def test_copies_end_before_their_cta_whichever_role_gave_up():
         assert not re.search(r"\n\t{1,3}return;", body)  # every thread comes to the end
 
 
+def test_a_wait_gives_up_within_seconds():
+    """A try of mbarrier.try_wait that does not succeed takes 3.95 us on a B200."""
+    src = open(os.path.join(ROOT, "calm_b200", "csrc", "tc05.cuh")).read()
+    assert 1 <= (1 << int(re.search(r"#define MBAR_SPINS \(1u << (\d+)\)", src).group(1))) * 3.95e-6 <= 10
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype,dim,hidden", [("fp8", 512, 1024), ("fp16", 512, 1024), ("fp8", 2048, 8192), ("fp16", 2048, 8192)])
 @pytest.mark.parametrize("tries", [0, 1])  # none: no role gets a stage; one: the ring is filled, what waits for a copy that has not landed gives up
