@@ -63,7 +63,7 @@ struct ColsRun {
 	int steps, chunk_steps; // 64-byte steps of a row, and of its pieces in a stage (the last may have fewer)
 	int own;                // of a piece's steps, those of a warp: 2 or 4
 	int* err;               // mapped host word: a wait that gave up
-	unsigned tries;         // of a wait before it gives up
+	unsigned tries;         // of a wait before it gives up (the multiplying warps of k_matres_cols: none if this is 0, else MBAR_SPINS; a limit in a register cost 0.3 us a launch there)
 };
 
 struct ColsShared {
@@ -95,24 +95,21 @@ __device__ __forceinline__ void cols_wait_prev(bool polls) {
 	asm volatile("bar.sync 1, %0;" ::"n"(COLS_THREADS) : "memory");
 }
 
-// Every wait is bounded: a role whose wait gives up leaves its loop with a code, and the others' waits then run out too.
-__device__ __forceinline__ bool cols_gave_up(ColsShared* sh, int code) {
+// Every wait is bounded: a role whose wait gives up leaves its loop with a code, and the others' waits then run out too.  Nearly all waits end with their first try; what follows
+// is kept out of the way, since a kernel's code is read anew in every launch and most launches are short (q/k/v and FFN up of Llama-3-8B fp8 6.9 and 19.8 us; with the loop in place 7.3 and 21.7).
+static __device__ __noinline__ bool cols_wait_on(ColsShared* sh, uint64_t* bar, uint32_t parity, unsigned tries, int code) {
+	if (mbar_wait_warp(bar, parity, tries)) return true;
 	if ((threadIdx.x & 31) == 0) sh->gave_up = code;
 	return false;
 }
-// The end of a CTA's roles.  issued: the first of this copying warp's stages that it did not request (0: another warp).  Whichever role gave up, and however far the copies had come
-// by then: nothing may be in flight into this CTA's shared memory when it exits.
-__device__ __forceinline__ void cols_finish(ColsShared* sh, const ColsRun& r, int issued) {
-	__syncthreads();
-	if (!sh->gave_up) return;
-	for (int k = issued - 2; k >= max(0, issued - COLS_STAGES); k -= 2) mbar_wait_warp(&sh->full[k % COLS_STAGES], (k / COLS_STAGES) & 1); // the last stage of each of its slots
-	if (threadIdx.x == 0) *reinterpret_cast<volatile int*>(r.err) = sh->gave_up;
+__device__ __forceinline__ bool cols_wait(ColsShared* sh, uint64_t* bar, uint32_t parity, const ColsRun& r, int code) {
+	return __all_sync(0xffffffffu, mbar_try_wait(bar, parity) && r.tries) || cols_wait_on(sh, bar, parity, r.tries, code);
 }
 
 // A copying warp (of two: they take the stages in turn).  order(i, tile, chunk): what stage i holds; row(tile, slot): where the weights of the tile's row `slot` begin, NULL: no such row.
-// Returns the first of its stages that it did not request.
+// Whichever role gives up, nothing is in flight into this CTA's shared memory when it exits: these warps wait for their last copies themselves, at a time when others need those too.
 template <typename OrderFn, typename RowFn>
-__device__ __forceinline__ int cols_produce(ColsShared* sh, const ColsRun& r, unsigned char* ring, int nst, OrderFn order, RowFn row) {
+__device__ __forceinline__ void cols_produce(ColsShared* sh, const ColsRun& r, unsigned char* ring, int nst, OrderFn order, RowFn row) {
 	const int lane = threadIdx.x & 31, which = (threadIdx.x >> 5) - COLS_WARPS;
 	const uint64_t policy = l2_policy_evict_first();
 	bool waited = false;
@@ -121,10 +118,7 @@ __device__ __forceinline__ int cols_produce(ColsShared* sh, const ColsRun& r, un
 		const int slot = i % COLS_STAGES;
 		if (i >= COLS_STAGES) {
 			if (!waited) cols_wait_prev(which == 0), waited = true; // no stage is free before the others have activations
-			if (!mbar_wait_warp(&sh->empty[slot], ((i / COLS_STAGES) & 1) ^ 1, r.tries)) {
-				cols_gave_up(sh, 9401);
-				break;
-			}
+			if (!cols_wait(sh, &sh->empty[slot], ((i / COLS_STAGES) & 1) ^ 1, r, 9401)) break;
 		}
 		int tile, chunk;
 		order(i, tile, chunk);
@@ -136,7 +130,7 @@ __device__ __forceinline__ int cols_produce(ColsShared* sh, const ColsRun& r, un
 		if (src) tma_load_1d_hint(ring + slot * COLS_STAGE + lane * COLS_PITCH, src + (size_t)chunk * r.chunk_steps * 64, bytes, &sh->full[slot], policy);
 	}
 	if (!waited) cols_wait_prev(which == 0);
-	return i;
+	for (int k = i - 2; k >= max(0, i - COLS_STAGES); k -= 2) mbar_wait_warp(&sh->full[k % COLS_STAGES], (k / COLS_STAGES) & 1); // the last stage of each of its slots
 }
 
 __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -216,16 +210,18 @@ struct ColsFragments {
 	}
 };
 
-// n steps of one stage's 8 rows
+// n steps of one stage's 8 rows; the stage is free for its next copy once they are in registers
 template <int DBITS>
-__device__ __forceinline__ void cols_multiply(const unsigned char* stage, const ColsRun& r, const ColsLane& l, int n, const ColsFragments<DBITS>& x, float (&acc)[4]) {
-	const unsigned char* p = stage + l.g * COLS_PITCH + l.warp * r.own * 64 + l.t * 16;
+__device__ __forceinline__ void cols_multiply(ColsShared* sh, const unsigned char* ring, int slot, const ColsRun& r, const ColsLane& l, int n, const ColsFragments<DBITS>& x, float (&acc)[4]) {
+	const unsigned char* p = ring + slot * COLS_STAGE + l.g * COLS_PITCH + l.warp * r.own * 64 + l.t * 16;
 	uint4 lo[2], up[2];
 #pragma unroll
 	for (int s = 0; s < 2; ++s) {
 		lo[s] = 2 * s < n ? *reinterpret_cast<const uint4*>(p + 128 * s) : make_uint4(0, 0, 0, 0);
 		up[s] = 2 * s + 1 < n ? *reinterpret_cast<const uint4*>(p + 128 * s + 64) : make_uint4(0, 0, 0, 0);
 	}
+	__syncwarp(); // every lane has its weights
+	if (l.lane == 0) mbar_arrive(&sh->empty[slot]);
 #pragma unroll
 	for (int s = 0; s < 2; ++s) {
 		if (2 * s >= n) break;
@@ -252,7 +248,7 @@ __device__ __forceinline__ bool cols_hand_over(ColsShared* sh, const ColsRun& r,
 	v += __shfl_xor_sync(0xffffffffu, v, 1);
 	v += __shfl_xor_sync(0xffffffffu, v, 2);
 	const int buf = tile % COLS_PARTS;
-	if (tile >= COLS_PARTS && !mbar_wait_warp(&sh->part_empty[buf], ((tile / COLS_PARTS) & 1) ^ 1, r.tries)) return cols_gave_up(sh, 9402);
+	if (tile >= COLS_PARTS && !cols_wait(sh, &sh->part_empty[buf], ((tile / COLS_PARTS) & 1) ^ 1, r, 9402)) return false;
 	if (l.t == 0) part[(buf * COLS_WARPS + l.warp) * 8 + l.g] = v * unscale;
 	__syncwarp();
 	if (l.lane == 0) mbar_arrive(&sh->part_full[buf]);
@@ -265,10 +261,7 @@ __device__ __forceinline__ void cols_epilogue(ColsShared* sh, const ColsRun& r, 
 	const int lane = threadIdx.x & 31, row = lane & 7, quarter = lane >> 3;
 	for (int tile = 0; tile < tiles; ++tile) {
 		const int buf = tile % COLS_PARTS;
-		if (!mbar_wait_warp(&sh->part_full[buf], (tile / COLS_PARTS) & 1, r.tries)) {
-			cols_gave_up(sh, 9403);
-			return;
-		}
+		if (!cols_wait(sh, &sh->part_full[buf], (tile / COLS_PARTS) & 1, r, 9403)) return;
 		const float* p = part + (buf * COLS_WARPS + quarter * (COLS_WARPS / 4)) * 8 + row;
 		float v = p[0];
 #pragma unroll
@@ -344,10 +337,8 @@ struct ColsTiles {
 		int slot = 0, parity = 0;
 		const int whole = l.own(r, 0), rest = l.own(r, NC - 1);
 		auto stage = [&](int c, float (&acc)[4]) {
-			if (!mbar_wait_warp(&sh->full[slot], parity, r.tries)) return cols_gave_up(sh, 9400);
-			cols_multiply<DBITS>(ring + slot * COLS_STAGE, r, l, c < NC - 1 ? whole : rest, x[c], acc);
-			__syncwarp(); // every lane has read its weights
-			if (l.lane == 0) mbar_arrive(&sh->empty[slot]);
+			if (!cols_wait(sh, &sh->full[slot], parity, r, 9400)) return false;
+			cols_multiply<DBITS>(sh, ring, slot, r, l, c < NC - 1 ? whole : rest, x[c], acc);
 			if (++slot == COLS_STAGES) slot = 0, parity ^= 1;
 			return true;
 		};
@@ -381,11 +372,10 @@ __global__ void __maxnreg__((ColsTiles<DBITS, NC>::REGS)) k_qkv_cols(const QkvAr
 	const int nrows = a.q_dim + 2 * a.kv_dim;
 	const int row0 = 2 * cols_share(nrows / 2, blockIdx.x), rows = 2 * cols_share(nrows / 2, blockIdx.x + 1) - row0, tiles = (rows + 7) / 8;
 	const ColsLane l;
-	int issued = 0;
 	cols_init(&sh);
 	if (l.warp == COLS_WARPS || l.warp == COLS_WARPS + 1) {
 		const size_t rowbytes = (size_t)r.steps * 64;
-		issued = cols_produce(&sh, r, smem_raw, tiles * NC, [&](int i, int& tile, int& chunk) { tile = i / NC, chunk = i % NC; },
+		cols_produce(&sh, r, smem_raw, tiles * NC, [&](int i, int& tile, int& chunk) { tile = i / NC, chunk = i % NC; },
 		             [&](int tile, int slot) -> const unsigned char* {
 			             const int j = row0 + 8 * tile + slot;
 			             if (j >= row0 + rows) return nullptr;
@@ -435,11 +425,12 @@ __global__ void __maxnreg__((ColsTiles<DBITS, NC>::REGS)) k_qkv_cols(const QkvAr
 			}
 		});
 	}
-	cols_finish(&sh, r, issued);
+	__syncthreads();
 	if (a.xb_out && blockIdx.x == 0 && l.warp < COLS_WARPS) { // norm_par: the FFN reads the normalised vector
 		const float post = a.normw ? cols_rms(&sh, a.dim, a.eps) : 1.f;
 		for (int i = threadIdx.x; i < a.dim; i += 32 * COLS_WARPS) a.xb_out[i] = __ldcg(a.x + i) * (a.normw ? a.normw[i] : 1.f) * post;
 	}
+	if (threadIdx.x == 0 && sh.gave_up) *reinterpret_cast<volatile int*>(r.err) = sh.gave_up;
 	stamp_end(a.stamp);
 }
 
@@ -455,11 +446,10 @@ __global__ void __maxnreg__((ColsTiles<DBITS, NC>::REGS)) k_ffn_up_cols(const Ff
 	uint32_t* buf = reinterpret_cast<uint32_t*>(part + COLS_PARTS * COLS_WARPS * 8);
 	const int i0 = cols_share(a.hidden, blockIdx.x), n = cols_share(a.hidden, blockIdx.x + 1) - i0, tiles = (n + 3) / 4;
 	const ColsLane l;
-	int issued = 0;
 	cols_init(&sh);
 	if (l.warp == COLS_WARPS || l.warp == COLS_WARPS + 1) {
 		const size_t rowbytes = (size_t)r.steps * 64;
-		issued = cols_produce(&sh, r, smem_raw, tiles * NC, [&](int i, int& tile, int& chunk) { tile = i / NC, chunk = i % NC; },
+		cols_produce(&sh, r, smem_raw, tiles * NC, [&](int i, int& tile, int& chunk) { tile = i / NC, chunk = i % NC; },
 		             [&](int tile, int slot) -> const unsigned char* {
 			             const int i = 4 * tile + (slot & 3);
 			             return i >= n ? nullptr : (const unsigned char*)(slot < 4 ? a.w1 : a.w3) + (size_t)(i0 + i) * rowbytes;
@@ -481,7 +471,8 @@ __global__ void __maxnreg__((ColsTiles<DBITS, NC>::REGS)) k_ffn_up_cols(const Ff
 			if (l.lane < 4 && i < n) a.hb[i0 + i] = (a.gelu ? act_gelu(v) : act_silu(v)) * u3;
 		});
 	}
-	cols_finish(&sh, r, issued);
+	__syncthreads();
+	if (threadIdx.x == 0 && sh.gave_up) *reinterpret_cast<volatile int*>(r.err) = sh.gave_up;
 	stamp_end(a.stamp);
 }
 
@@ -498,11 +489,10 @@ __global__ void __maxnreg__((cols_regs(2 * ColsStep<DBITS>::B + 4 * T))) k_matre
 	const int row0 = cols_share(a.d, blockIdx.x), rows = cols_share(a.d, blockIdx.x + 1) - row0;
 	const int chunks = (r.steps + r.chunk_steps - 1) / r.chunk_steps;
 	const ColsLane l;
-	int issued = 0;
 	cols_init(&sh);
 	if (l.warp == COLS_WARPS || l.warp == COLS_WARPS + 1) {
 		const size_t rowbytes = (size_t)r.steps * 64;
-		issued = cols_produce(&sh, r, smem_raw, T * chunks, [&](int i, int& tile, int& chunk) { tile = i % T, chunk = i / T; },
+		cols_produce(&sh, r, smem_raw, T * chunks, [&](int i, int& tile, int& chunk) { tile = i % T, chunk = i / T; },
 		             [&](int tile, int slot) -> const unsigned char* {
 			             const int j = 8 * tile + slot;
 			             return j >= rows ? nullptr : (const unsigned char*)a.w + (size_t)(row0 + j) * rowbytes;
@@ -525,7 +515,7 @@ __global__ void __maxnreg__((cols_regs(2 * ColsStep<DBITS>::B + 4 * T))) k_matre
 		stamp_begin(a.stamp);
 		fetch(0);
 		int slot = 0, parity = 0, e = 8;
-		bool ok = true;
+		bool ok = r.tries != 0;
 		for (int c = 0; c < chunks && ok; ++c) {
 			float most = 0.f;
 #pragma unroll
@@ -546,19 +536,18 @@ __global__ void __maxnreg__((cols_regs(2 * ColsStep<DBITS>::B + 4 * T))) k_matre
 			const int n = l.own(r, c);
 #pragma unroll
 			for (int t = 0; t < T; ++t) {
-				if (!mbar_wait_warp(&sh.full[slot], parity, r.tries)) {
-					ok = cols_gave_up(&sh, 9400);
+				if (!mbar_wait_warp(&sh.full[slot], parity)) {
+					ok = false;
 					break;
 				}
-				cols_multiply<DBITS>(smem_raw + slot * COLS_STAGE, r, l, n, x, acc[t]);
-				__syncwarp(); // every lane has read its weights
-				if (l.lane == 0) mbar_arrive(&sh.empty[slot]);
+				cols_multiply<DBITS>(&sh, smem_raw, slot, r, l, n, x, acc[t]);
 				if (++slot == COLS_STAGES) slot = 0, parity ^= 1;
 			}
 		}
 #pragma unroll
 		for (int t = 0; t < T; ++t)
 			if (ok) ok = cols_hand_over(&sh, r, part, l, t, acc[t], cols_unscale(e));
+		if (!ok && l.lane == 0) sh.gave_up = 9400;
 	} else {
 		cols_wait_prev(false);
 		for (int j = l.lane; j < rows; j += 32) sh.rows[j] = a.accumulate && a.tpx.world <= 1 ? __ldcg(a.y + row0 + j) : 0.f;
@@ -570,9 +559,10 @@ __global__ void __maxnreg__((cols_regs(2 * ColsStep<DBITS>::B + 4 * T))) k_matre
 			else a.y[row0 + j] = sh.rows[j] + v;
 		});
 	}
-	cols_finish(&sh, r, issued);
+	__syncthreads();
 	if (a.tpx.world > 1) { // the matvec -> all-reduce fusion of stages.cuh TpExchange
 		tp_exchange_rows(a.tpx, sh.rows, row0, rows, a.y, a.d);
 	}
+	if (threadIdx.x == 0 && sh.gave_up) *reinterpret_cast<volatile int*>(r.err) = sh.gave_up;
 	stamp_end(a.stamp);
 }

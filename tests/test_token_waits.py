@@ -22,18 +22,19 @@ print("done")
 
 
 def test_copies_end_before_their_cta_whichever_role_gave_up():
-    """A multiplying warp can give up on a stage behind which the copying warps have nothing left to request: they cannot learn of it inside their loop."""
+    """A multiplying warp can give up on a stage behind which the copying warps have nothing left to request: they wait for what they requested in any case."""
     src = open(os.path.join(ROOT, "calm_b200", "csrc", "cols.cuh")).read()
-    waits = re.findall(r"mbar_wait_warp\(&sh(?:\.|->)\w+\[.*?\], .*?\)\)", src)
     assert "mbar_wait_bounded(" not in src  # whole warps give up
-    assert len(waits) >= 5 and all(w.endswith("r.tries))") for w in waits), waits
-    finish = src[src.index("void cols_finish("):]
-    finish = finish[:finish.index("\n}\n")]
-    assert finish.index("__syncthreads()") < finish.index("gave_up") < finish.index("mbar_wait_warp(&sh->full[")
+    produce = src[src.index("void cols_produce("):]
+    produce = produce[:produce.index("\n}\n")]
+    loop, end = produce[:produce.index("\n\t}\n")], produce[produce.index("\n\t}\n") + 4:]
+    assert "return" not in produce and "break" in loop
+    drain = re.search(r"for \(int k = i - 2; k >= max\(0, i - COLS_STAGES\); k -= 2\) mbar_wait_warp\(&sh->full\[k % COLS_STAGES\], \(k / COLS_STAGES\) & 1\);", end)
+    assert drain and not re.search(r"\bif\b(?! \(!waited\))", end)
     for kernel in ("k_qkv_cols", "k_ffn_up_cols", "k_matres_cols"):
         body = src[src.index(kernel + "(const"):]
         body = body[:body.index("\n}\n")]
-        assert "issued = cols_produce(" in body and body.index("cols_epilogue(") < body.index("\n\tcols_finish(&sh, r, issued);")
+        assert body.index("cols_produce(") < body.index("cols_epilogue(") < body.index("\n\t__syncthreads();") < body.index("r.err) = sh.gave_up")
         assert not re.search(r"\n\t{1,3}return;", body)  # every thread comes to the end
 
 
