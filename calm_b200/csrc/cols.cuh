@@ -15,9 +15,9 @@
 // contiguous bytes for a step and takes their k in the order they lie in -- B has the same order.  An SM starts one such product every two cycles (measured,
 // 16 warps).  Dot products of packed FP32 FMA in this frame took 4.3 instructions a weight at 60 % of the issue slots (conversions, a transposing
 // reduction per row: FFN up 25.6 us against 24).
-// The tensor core truncates where it aligns and adds.  With fp16 weights (products of 22 bits) the first piece therefore has 8 bits and two products add up in it before an FP32 addition: whole tokens,
-// 32 seeds, median distance from 64 bits 0.53e-6 (896 wide, 6 layers) and 0.83e-6 (1536 wide, 12), 0.78 and 1.35 without, 0.74 and 1.05 with the FP32 dot products of k_qkv and ring.cuh; it costs 0.7 % of a token of
-// Qwen2-0.5B (643 -> 648 us) and 1 to 2 % of 16 layers of Llama-3-8B.  With fp8 weights (14 bits) it is not needed: 0.67e-6 and 1.04e-6 (1024 and 1536 wide) against 0.79 and 1.12.
+// The tensor core truncates where it aligns and adds, so the first piece has 8 bits and two products (fp16) or those of a stage, eight at most (fp8), add up in it before an FP32 addition.
+// Distance from 64 bits, as a share of that of the FP32 dot products of ring.cuh (1.3 to 1.7e-7 for a row of w2, 2 to 3e-7 for FFN up): fp8 rows of 4096, 14336 and 28672 weights, normal
+// and gated activations, 0.48 to 0.71, FFN up 0.55 and 0.68 (2048); fp16 0.84 to 0.98, FFN up 0.63 and 0.86 (1024).  Whole rows of fp8 in the tensor core were 1.5 (4096) to 11 times (28672) as far off as the ring's.
 // The 8 warps' sums of a tile of 8 rows go through shared memory to one more warp, which adds them in order (deterministic) and applies the
 // stage's epilogue while the others are at the next tile (left to the last of the 8, this held up the slowest one: FFN up 29 us instead of 24).
 //
@@ -161,12 +161,10 @@ struct ColsLane {
 };
 
 // The pieces of 64 activations (f0, f1: elements 2 lane and 2 lane + 1, scaled) into 384 bytes of the warp's own.
-template <int DBITS>
 __device__ __forceinline__ void cols_split(uint32_t* buf, int lane, float f0, float f1) {
-	// fp16: the first piece is 8 bits, not 11: a product of 16 terms aligns them to the largest and drops what falls off its end, which is less the shorter they are
+	// The first piece is 8 bits, not 11: a product of 16 terms aligns them to the largest and drops what falls off its end, which is less the shorter they are
 	// (8 + 11 + 11 bits still hold all 24).
-	constexpr uint32_t mask = DBITS == 16 ? 0xffff0000u : 0xffffffffu;
-	const __half2 hi = __floats2half2_rn(__uint_as_float(__float_as_uint(f0) & mask), __uint_as_float(__float_as_uint(f1) & mask));
+	const __half2 hi = __floats2half2_rn(__uint_as_float(__float_as_uint(f0) & 0xffff0000u), __uint_as_float(__float_as_uint(f1) & 0xffff0000u));
 	float r0 = f0 - __low2float(hi), r1 = f1 - __high2float(hi);
 	r0 = fabsf(f0) <= FLT_MAX ? r0 : 0.f, r1 = fabsf(f1) <= FLT_MAX ? r1 : 0.f; // an infinity has no remainder
 	const __half2 mid = __floats2half2_rn(r0, r1);
@@ -194,8 +192,8 @@ struct ColsFragments {
 #pragma unroll
 		for (int k = 0; k < F / 2; k += 2) { // 128 activations at a time
 			__syncwarp(); // the previous pieces have been read
-			cols_split<DBITS>(buf, l.lane, f[2 * k], f[2 * k + 1]);
-			cols_split<DBITS>(buf + 96, l.lane, f[2 * k + 2], f[2 * k + 3]);
+			cols_split(buf, l.lane, f[2 * k], f[2 * k + 1]);
+			cols_split(buf + 96, l.lane, f[2 * k + 2], f[2 * k + 3]);
 			__syncwarp();
 #pragma unroll
 			for (int h = 0; h < 2; ++h) {
@@ -222,23 +220,25 @@ __device__ __forceinline__ void cols_multiply(ColsShared* sh, const unsigned cha
 	}
 	__syncwarp(); // every lane has its weights
 	if (l.lane == 0) mbar_arrive(&sh->empty[slot]);
+	float d[4] = {0.f, 0.f, 0.f, 0.f}; // a few products only add up in the tensor core, which truncates
+	auto add = [&] { acc[0] += d[0], acc[1] += d[1], acc[2] += d[2], acc[3] += d[3]; };
 #pragma unroll
 	for (int s = 0; s < 2; ++s) {
 		if (2 * s >= n) break;
 		const uint32_t wl[4] = {lo[s].x, lo[s].y, lo[s].z, lo[s].w}, wu[4] = {up[s].x, up[s].y, up[s].z, up[s].w};
 		const uint32_t(&b)[ColsStep<DBITS>::B] = x.b[s];
 		if constexpr (DBITS == 16) {
-			float d[4] = {0.f, 0.f, 0.f, 0.f}; // a few products only add up in the tensor core, which truncates
+			d[0] = d[1] = d[2] = d[3] = 0.f;
 			mma16816(d, wl[0], wu[0], wl[1], wu[1], b[0], b[1]);
 			mma16816(d, wl[2], wu[2], wl[3], wu[3], b[2], b[3]);
-#pragma unroll
-			for (int i = 0; i < 4; ++i) acc[i] += d[i];
+			add();
 		} else {
 #pragma unroll
 			for (int m = 0; m < 4; ++m)
-				mma16816(acc, __byte_perm(wl[m], 0, 0x1404), __byte_perm(wu[m], 0, 0x1404), __byte_perm(wl[m], 0, 0x3424), __byte_perm(wu[m], 0, 0x3424), b[2 * m], b[2 * m + 1]);
+				mma16816(d, __byte_perm(wl[m], 0, 0x1404), __byte_perm(wu[m], 0, 0x1404), __byte_perm(wl[m], 0, 0x3424), __byte_perm(wu[m], 0, 0x3424), b[2 * m], b[2 * m + 1]);
 		}
 	}
+	if constexpr (DBITS != 16) add();
 }
 
 // this warp's sums of a tile's 8 rows: columns 0 - 2 of rows 0 - 7 and columns 3 - 5 of rows 8 - 15
