@@ -8,7 +8,9 @@
 // CTA IS resident while the previous kernel still runs (programmatic dependent launch), and the ring is full when the dependency wait returns.
 //
 // Arithmetic: mma.m16n8k16, f16 x f16 -> f32, 8 rows of weights at a time.  Weights are exact in f16 (e5m2: a byte permute), the
-// activations are three f16 pieces of a value scaled by a power of two (30 bits: nothing of the 24 is lost).  A row of weights goes through a product
+// activations are three f16 pieces of a value scaled by the power of two that brings a warp's largest one (of a row; of a piece of it in wo and w2) to 2^14: all 24 bits down to 2^-34 of
+// it, steps of 2^-58 of it below (with the pieces at one scale and 2^7 the 24 bits ended at 2^-9, and rows whose weights met only entries of 2^-20 of the largest were 3e-5 off, of 2^-26
+// 4e-3; 1e-7 now).  A row of weights goes through a product
 // twice at once: rows g of A are 64 bytes (a step) of row g, rows g + 8 the next step of the same row, columns 0 - 2 of B the pieces of the first step's activations
 // and columns 3 - 5 of the second's; the sums wanted are those of rows 0 - 7 in columns 0 - 2 and of rows 8 - 15 in columns 3 - 5.  So no product is
 // spent on padding rows and a warp's activations take half the registers.  A warp of 8 owns two or four steps of every 2 KB of a row; lane (g, t) reads 16
@@ -58,6 +60,10 @@ struct ColsStep { // 64 bytes of a row
 // free first would take two of its CTAs, the last ones none, and every kernel behind it would inherit that (FFN up of Llama-3-8B fp8: 27 us, 20 evenly).
 // wo asks for this much shared memory: two of its CTAs do not fit an SM, one beside one of FFN up's does.
 #define COLS_ALONE 115200
+
+// An activation is three f16 pieces: its first 8 bits, what they leave times COLS_MID, what that leaves times COLS_LO (a piece has columns, and so sums, of its own)
+#define COLS_MID 256.f
+#define COLS_LO 524288.f
 
 struct ColsRun {
 	int steps, chunk_steps; // 64-byte steps of a row, and of its pieces in a stage (the last may have fewer)
@@ -139,13 +145,22 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
 	             : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// power of two that brings values of magnitude m (its biased exponent) to [2^7, 2^8), and its inverse
-__device__ __forceinline__ int cols_exponent(float m) {
-	const int e = (int)(__float_as_uint(m) >> 23);
-	return e == 255 ? 134 : max(e, 8); // infinities keep their value
+// biased exponent of the largest magnitude, and the power of two that brings it to [2^14, 2^15)
+__device__ __forceinline__ int cols_exponent(float m) { return max((int)(__float_as_uint(m) >> 23), 37); } // (below 2^-90 the third piece's steps are FP32's)
+__device__ __forceinline__ float cols_scale(int e) { return __uint_as_float((uint32_t)(268 - e) << 23); }
+__device__ __forceinline__ float cols_unscale(int e) { return __uint_as_float((uint32_t)(e - 14) << 23); }
+// a warp's activations at the scale that their largest magnitude asks for; returns what undoes it
+template <int N>
+__device__ __forceinline__ float cols_to_scale(float (&f)[N]) {
+	float most = 0.f;
+#pragma unroll
+	for (int k = 0; k < N; ++k) most = fmaxf(most, fabsf(f[k]));
+	const int e = cols_exponent(warp_max(most));
+	const float scale = cols_scale(e);
+#pragma unroll
+	for (int k = 0; k < N; ++k) f[k] *= scale;
+	return cols_unscale(e);
 }
-__device__ __forceinline__ float cols_scale(int e) { return __uint_as_float((uint32_t)(261 - e) << 23); }
-__device__ __forceinline__ float cols_unscale(int e) { return __uint_as_float((uint32_t)(e - 7) << 23); }
 
 struct ColsLane {
 	int lane, warp, g, t;
@@ -156,6 +171,10 @@ struct ColsLane {
 		return max(0, min(r.own, steps - r.own * warp));
 	}
 	// its first activation there
+	__device__ __forceinline__ float2 worth(float unscale) const { // of a sum in either of its two columns (pieces 0 1 | 2 0 | 1 2)
+		constexpr float mid = 1.f / COLS_MID, lo = 1.f / COLS_LO;
+		return make_float2(unscale * (t == 0 ? 1.f : t == 1 ? lo : mid), unscale * (t == 0 ? mid : t == 1 ? 1.f : lo));
+	}
 	template <int DBITS>
 	__device__ __forceinline__ size_t at(const ColsRun& r, int c) const { return (size_t)(c * r.chunk_steps + r.own * warp) * ColsStep<DBITS>::K; }
 };
@@ -167,8 +186,10 @@ __device__ __forceinline__ void cols_split(uint32_t* buf, int lane, float f0, fl
 	const __half2 hi = __floats2half2_rn(__uint_as_float(__float_as_uint(f0) & 0xffff0000u), __uint_as_float(__float_as_uint(f1) & 0xffff0000u));
 	float r0 = f0 - __low2float(hi), r1 = f1 - __high2float(hi);
 	r0 = fabsf(f0) <= FLT_MAX ? r0 : 0.f, r1 = fabsf(f1) <= FLT_MAX ? r1 : 0.f; // an infinity has no remainder
+	r0 *= COLS_MID, r1 *= COLS_MID;
 	const __half2 mid = __floats2half2_rn(r0, r1);
-	const __half2 lo = __floats2half2_rn(r0 - __low2float(mid), r1 - __high2float(mid));
+	constexpr float next = COLS_LO / COLS_MID;
+	const __half2 lo = __floats2half2_rn((r0 - __low2float(mid)) * next, (r1 - __high2float(mid)) * next);
 	buf[lane] = *reinterpret_cast<const uint32_t*>(&hi), buf[32 + lane] = *reinterpret_cast<const uint32_t*>(&mid), buf[64 + lane] = *reinterpret_cast<const uint32_t*>(&lo);
 }
 // A warp's activations of one chunk as B fragments: f[2 k], f[2 k + 1] are elements 64 k + 2 lane, + 1, scaled.
@@ -177,7 +198,7 @@ struct ColsFragments {
 	static constexpr int B = ColsStep<DBITS>::B, F = ColsStep<DBITS>::F;
 	uint32_t b[2][B];
 
-	__device__ __forceinline__ void make(uint32_t* buf, const ColsLane& l, const float (&f)[F]) {
+	__device__ __forceinline__ void make(uint32_t* buf, const ColsLane& l, const float* f) {
 		const int which = l.g >= 3, piece = l.g - 3 * which; // lanes of g = 6, 7 hold nothing
 		auto take = [&](uint32_t* d, const uint32_t* from, int at, bool on) { // eight halves
 			if (on && l.g < 6) {
@@ -208,9 +229,9 @@ struct ColsFragments {
 	}
 };
 
-// n steps of one stage's 8 rows; the stage is free for its next copy once they are in registers
+// n steps of one stage's 8 rows; the stage is free for its next copy once they are in registers.  u: what sums in this lane's two columns are worth
 template <int DBITS>
-__device__ __forceinline__ void cols_multiply(ColsShared* sh, const unsigned char* ring, int slot, const ColsRun& r, const ColsLane& l, int n, const ColsFragments<DBITS>& x, float (&acc)[4]) {
+__device__ __forceinline__ void cols_multiply(ColsShared* sh, const unsigned char* ring, int slot, const ColsRun& r, const ColsLane& l, int n, const ColsFragments<DBITS>& x, float2 u, float (&acc)[4]) {
 	const unsigned char* p = ring + slot * COLS_STAGE + l.g * COLS_PITCH + l.warp * r.own * 64 + l.t * 16;
 	uint4 lo[2], up[2];
 #pragma unroll
@@ -221,7 +242,7 @@ __device__ __forceinline__ void cols_multiply(ColsShared* sh, const unsigned cha
 	__syncwarp(); // every lane has its weights
 	if (l.lane == 0) mbar_arrive(&sh->empty[slot]);
 	float d[4] = {0.f, 0.f, 0.f, 0.f}; // a few products only add up in the tensor core, which truncates
-	auto add = [&] { acc[0] += d[0], acc[1] += d[1], acc[2] += d[2], acc[3] += d[3]; };
+	auto add = [&] { acc[0] = fmaf(d[0], u.x, acc[0]), acc[1] = fmaf(d[1], u.y, acc[1]), acc[2] = fmaf(d[2], u.x, acc[2]), acc[3] = fmaf(d[3], u.y, acc[3]); };
 #pragma unroll
 	for (int s = 0; s < 2; ++s) {
 		if (2 * s >= n) break;
@@ -242,14 +263,14 @@ __device__ __forceinline__ void cols_multiply(ColsShared* sh, const unsigned cha
 }
 
 // this warp's sums of a tile's 8 rows: columns 0 - 2 of rows 0 - 7 and columns 3 - 5 of rows 8 - 15
-__device__ __forceinline__ bool cols_hand_over(ColsShared* sh, const ColsRun& r, float* part, const ColsLane& l, int tile, const float (&acc)[4], float unscale) {
+__device__ __forceinline__ bool cols_hand_over(ColsShared* sh, const ColsRun& r, float* part, const ColsLane& l, int tile, const float (&acc)[4]) {
 	float v = (l.t == 2 ? acc[2] : acc[0]) + (l.t == 0 ? acc[1] : acc[3]);
 	v = l.t == 3 ? 0.f : v;
 	v += __shfl_xor_sync(0xffffffffu, v, 1);
 	v += __shfl_xor_sync(0xffffffffu, v, 2);
 	const int buf = tile % COLS_PARTS;
 	if (tile >= COLS_PARTS && !cols_wait(sh, &sh->part_empty[buf], ((tile / COLS_PARTS) & 1) ^ 1, r, 9402)) return false;
-	if (l.t == 0) part[(buf * COLS_WARPS + l.warp) * 8 + l.g] = v * unscale;
+	if (l.t == 0) part[(buf * COLS_WARPS + l.warp) * 8 + l.g] = v;
 	__syncwarp();
 	if (l.lane == 0) mbar_arrive(&sh->part_full[buf]);
 	return true;
@@ -290,11 +311,12 @@ template <int DBITS, int NC>
 struct ColsTiles {
 	static constexpr int F = ColsStep<DBITS>::F, REGS = cols_regs(2 * NC * ColsStep<DBITS>::B);
 	ColsFragments<DBITS> x[NC];
-	float f[NC][F], unscale;
+	float f[NC * F];
+	float2 u;
 
 	// x (times the norm's weights, with the sum of its squares into sh->ss)
 	__device__ __forceinline__ void load(ColsShared* sh, const ColsRun& r, const ColsLane& l, const float* __restrict__ xin, const float* __restrict__ normw) {
-		float ss = 0.f, most = 0.f;
+		float ss = 0.f;
 #pragma unroll
 		for (int c = 0; c < NC; ++c) {
 			const int n = l.own(r, c) * ColsStep<DBITS>::K; // this warp's activations of the chunk
@@ -302,7 +324,7 @@ struct ColsTiles {
 #pragma unroll
 			for (int k = 0; k < F / 2; ++k) {
 				const float2 v = 64 * k < n ? __ldcg(p + 32 * k) : make_float2(0.f, 0.f);
-				f[c][2 * k] = v.x, f[c][2 * k + 1] = v.y;
+				f[c * F + 2 * k] = v.x, f[c * F + 2 * k + 1] = v.y;
 			}
 		}
 		if (normw) {
@@ -313,48 +335,38 @@ struct ColsTiles {
 #pragma unroll
 				for (int k = 0; k < F / 2; ++k) {
 					const float2 w = 64 * k < n ? __ldg(p + 32 * k) : make_float2(0.f, 0.f);
-					ss = fmaf(f[c][2 * k], f[c][2 * k], ss), ss = fmaf(f[c][2 * k + 1], f[c][2 * k + 1], ss);
-					f[c][2 * k] *= w.x, f[c][2 * k + 1] *= w.y;
+					float &f0 = f[c * F + 2 * k], &f1 = f[c * F + 2 * k + 1];
+					ss = fmaf(f0, f0, ss), ss = fmaf(f1, f1, ss);
+					f0 *= w.x, f1 *= w.y;
 				}
 			}
 			ss = warp_sum(ss);
 			if (l.lane == 0) sh->ss[l.warp] = ss; // (read behind the first tile's barrier)
 		}
-#pragma unroll
-		for (int c = 0; c < NC; ++c)
-#pragma unroll
-			for (int k = 0; k < F; ++k) most = fmaxf(most, fabsf(f[c][k]));
-		const int e = cols_exponent(warp_max(most));
-		const float scale = cols_scale(e);
-		unscale = cols_unscale(e);
-#pragma unroll
-		for (int c = 0; c < NC; ++c) {
-#pragma unroll
-			for (int k = 0; k < F; ++k) f[c][k] *= scale;
-		}
+		u = l.worth(cols_to_scale(f));
 	}
 	__device__ __forceinline__ void run(ColsShared* sh, const ColsRun& r, const ColsLane& l, uint32_t* buf, const unsigned char* ring, float* part, int tiles) {
 		int slot = 0, parity = 0;
 		const int whole = l.own(r, 0), rest = l.own(r, NC - 1);
 		auto stage = [&](int c, float (&acc)[4]) {
 			if (!cols_wait(sh, &sh->full[slot], parity, r, 9400)) return false;
-			cols_multiply<DBITS>(sh, ring, slot, r, l, c < NC - 1 ? whole : rest, x[c], acc);
+			cols_multiply<DBITS>(sh, ring, slot, r, l, c < NC - 1 ? whole : rest, x[c], u, acc);
 			if (++slot == COLS_STAGES) slot = 0, parity ^= 1;
 			return true;
 		};
 		float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
 		for (int c = 0; c < NC; ++c) { // the first tile: a chunk's pieces are made when it is used, so that the first stages are free early
-			x[c].make(buf, l, f[c]);
+			x[c].make(buf, l, f + c * F);
 			if (!stage(c, acc)) return;
 		}
-		if (!cols_hand_over(sh, r, part, l, 0, acc, unscale)) return;
+		if (!cols_hand_over(sh, r, part, l, 0, acc)) return;
 		for (int tile = 1; tile < tiles; ++tile) {
 			acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
 #pragma unroll
 			for (int c = 0; c < NC; ++c)
 				if (!stage(c, acc)) return;
-			if (!cols_hand_over(sh, r, part, l, tile, acc, unscale)) return;
+			if (!cols_hand_over(sh, r, part, l, tile, acc)) return;
 		}
 	}
 };
@@ -514,22 +526,10 @@ __global__ void __maxnreg__((cols_regs(2 * ColsStep<DBITS>::B + 4 * T))) k_matre
 		cols_wait_prev(false);
 		stamp_begin(a.stamp);
 		fetch(0);
-		int slot = 0, parity = 0, e = 8;
+		int slot = 0, parity = 0;
 		bool ok = r.tries != 0;
 		for (int c = 0; c < chunks && ok; ++c) {
-			float most = 0.f;
-#pragma unroll
-			for (int k = 0; k < F; ++k) most = fmaxf(most, fabsf(f[k]));
-			const int now = cols_exponent(warp_max(most));
-			if (c == 0 || now > e + 7) { // values above 2^15: the sums so far go to the new scale (exact)
-				const float by = c == 0 ? 1.f : cols_unscale(e) * cols_scale(now);
-#pragma unroll
-				for (int t = 0; t < T; ++t) acc[t][0] *= by, acc[t][1] *= by, acc[t][2] *= by, acc[t][3] *= by;
-				e = now;
-			}
-			const float scale = cols_scale(e);
-#pragma unroll
-			for (int k = 0; k < F; ++k) f[k] *= scale;
+			const float2 u = l.worth(cols_to_scale(f));
 			ColsFragments<DBITS> x;
 			x.make(buf + l.warp * 192, l, f);
 			fetch(c + 1);
@@ -540,13 +540,13 @@ __global__ void __maxnreg__((cols_regs(2 * ColsStep<DBITS>::B + 4 * T))) k_matre
 					ok = false;
 					break;
 				}
-				cols_multiply<DBITS>(&sh, smem_raw, slot, r, l, n, x, acc[t]);
+				cols_multiply<DBITS>(&sh, smem_raw, slot, r, l, n, x, u, acc[t]);
 				if (++slot == COLS_STAGES) slot = 0, parity ^= 1;
 			}
 		}
 #pragma unroll
 		for (int t = 0; t < T; ++t)
-			if (ok) ok = cols_hand_over(&sh, r, part, l, t, acc[t], cols_unscale(e));
+			if (ok) ok = cols_hand_over(&sh, r, part, l, t, acc[t]);
 		if (!ok && l.lane == 0) sh.gave_up = 9400;
 	} else {
 		cols_wait_prev(false);

@@ -63,3 +63,38 @@ def test_sums_of_long_rows(dtype, hidden):
         got, _, v = _first_token(spec, t, 5)
         err.append(_rel(got, _reference(spec, t, 5, v)[0]))
     assert np.median(err) < 4.5e-7, err
+
+
+@pytest.mark.parametrize("dtype", ["fp8", "fp16"])
+@pytest.mark.parametrize("dim,hidden", [(512, 1024), (2176, 4864)])  # one piece of a row, several
+def test_small_activations_beside_large_ones(dtype, dim, hidden):
+    """Every stage's input has entries of some 2^26 times the others (2^12 in front of wo, whose input is held in f16), first, in the middle and last, met by weights of zero: the
+    result is made of the small ones.  FP32 products are exact to 2^-24 whatever lies beside them; 2e-6 leaves the four stages' and the classifier's sums 3e-7 each.
+    Fixed point with 32 bits below the largest entry was 2e-3 to 1e-2 off."""
+    spec = replace(mg.SPECS["pf-tiny-hd128"], name="outliers", dtype=dtype, dim=dim, hidden_dim=hidden, n_heads=dim // 128, n_kv_heads=dim // 128, n_layers=1, qkv_bias=False)
+    t, g = mg.generate(spec, seed=4), torch.Generator().manual_seed(1)
+    get = lambda n: _values(t[n], dtype)
+    at, up = [0, dim // 2 + 1, dim - 1], [0, hidden // 2 + 1, hidden - 1]
+    x = torch.randn(spec.vocab_size, dim, generator=g).double() * 2.0**-11
+    x[:, at] = 2.0**15
+    _store(t, "model.embed.weight", x, dtype)
+    for n in ("attn.norm.weight", "mlp.norm.weight"):
+        t[L0 + n] *= 2.0**22  # the small ones leave the norm as values of about 0.1
+    for n in (L0 + "attn.wq.weight", L0 + "attn.wk.weight", L0 + "attn.wv.weight", L0 + "mlp.w1.weight", L0 + "mlp.w3.weight", "model.output.weight"):
+        w = get(n)
+        w[:, at] = 0
+        if ".w1." in n or ".w3." in n:
+            w[up] *= 2.0**13
+        if ".wv." in n:
+            w[at] *= 2.0**12
+        _store(t, n, w, dtype)
+    for n, zero in (("attn.wo.weight", at), ("mlp.w2.weight", up)):
+        w = get(L0 + n)
+        w[:, zero] = 0
+        w[at] = 0  # (the large entries of the residual stay as they are)
+        _store(t, L0 + n, w, dtype)
+    got, k, v = _first_token(spec, t, 5)
+    ref, rk, rv = _reference(spec, t, 5, v)
+    for a, b in ((k, rk), (v, rv)):
+        assert (np.abs(a - b) <= 2.0**-10 * np.abs(b) + 2.0**-24).all()  # the next f16 value at most
+    assert _rel(got, ref) < 2e-6
