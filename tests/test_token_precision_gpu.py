@@ -98,3 +98,27 @@ def test_small_activations_beside_large_ones(dtype, dim, hidden):
     for a, b in ((k, rk), (v, rv)):
         assert (np.abs(a - b) <= 2.0**-10 * np.abs(b) + 2.0**-24).all()  # the next f16 value at most
     assert _rel(got, ref) < 2e-6
+
+
+@pytest.mark.parametrize("dtype", ["fp8", "fp16"])
+def test_infinite_weights(dtype):
+    """A row with an infinite weight gives that infinity with the activation's sign, not a NaN of its pieces; rows beside it are untouched.  Seen in the cache, where a value row's
+    result goes by itself (a NaN would end at the lower limit of the clip, as one infinity)."""
+    spec = replace(mg.SPECS["pf-tiny-hd128"], name="infinite", dtype=dtype, n_layers=1, qkv_bias=False)
+    t = mg.generate(spec, seed=6)
+    xn = _values(t["model.embed.weight"], dtype)[5] * t[L0 + "attn.norm.weight"].double()
+    wv = _values(t[L0 + "attn.wv.weight"], dtype)
+    rows = range(3, spec.kv_dim, 5)
+    for i, r in enumerate(rows):
+        c = (i * 37) % spec.dim
+        wv[r, c] = float("inf") if i % 2 else float("-inf")
+        if i % 3 == 0:  # another one of the same effect
+            o = (c + 200) % spec.dim
+            wv[r, o] = wv[r, c] * torch.sign(xn[c] * xn[o])
+    _store(t, L0 + "attn.wv.weight", wv, dtype)
+    _, _, v = _first_token(spec, t, 5)
+    ref = _reference(spec, t, 5, np.zeros(spec.kv_dim))[2]
+    assert np.isinf(ref[rows]).all() and (ref[rows] > 0).any() and (ref[rows] < 0).any()
+    assert (v[rows] == ref[rows]).all()
+    rest = np.setdiff1d(np.arange(spec.kv_dim), rows)
+    assert (np.abs(v[rest] - ref[rest]) <= 2.0**-10 * np.abs(ref[rest]) + 2.0**-24).all()
