@@ -305,9 +305,11 @@ __device__ __forceinline__ float cols_rms(const ColsShared* sh, int n, float eps
 	return 1.0f / sqrtf(ss / n + eps);
 }
 
-// Registers of a thread: two kernels of the chain share an SM's 65536 (2 x 352 threads x 88), unless rows are longer or more than usual
+// Registers of a thread: two kernels of the chain share an SM's 65536 (2 x 352 threads x 88) unless rows are longer than usual.  Where 88 do not hold the vector's pieces they are kept in
+// local memory, which costs more than the early start gives: FFN up 13824 x 5120 and 16384 x 6144 fp8 (three pieces of 16) 31.1 -> 26.5 us and 36.3 -> 31.9 with 168, 14336 x 5632 fp16
+// (six of 8) 509 -> 500 us for a token of four layers.
 constexpr int cols_regs(int pieces_and_sums) {
-	return pieces_and_sums <= 48 ? 88 : 168;
+	return pieces_and_sums <= 40 ? 88 : 168;
 }
 
 // ---- first order: tile by tile, NC chunks a row, the vector's pieces in registers

@@ -434,7 +434,7 @@ template <typename KVT, int HG, int LPP>
 void launch_attn2(const AttnArgs& a, int nunits, int* nl) {
 	if (!nl) { // prepare time: opt-ins, and whether the cluster form can be scheduled at all
 		smem_optin(k_attn2<KVT, HG, LPP, false>, g.attn2_smem);
-		side_by_side(k_attn2<KVT, HG, LPP, false>, g.w.dbits != 4 && g.cfg.n_experts == 0);
+		side_by_side(k_attn2<KVT, HG, LPP, false>, g.cols_qkv.n || g.cols_wo.n || g.cols_up.n || g.cols_down.n);
 		{ // the cell fold polls its peers: the whole grid must fit on the device at once
 			int per_sm = 0;
 			CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_attn2<KVT, HG, LPP, false>, ATTN_THREADS, g.attn2_smem));
@@ -837,6 +837,19 @@ void make_plan() {
 	if (smem_res > 227 * 1024 || g.smem_dim > 227 * 1024) CALM_FATAL("activation vector does not fit in shared memory (dim %d, hidden %d)", c.dim, c.hidden_dim);
 	smem_optin(k_qkv<DBITS, KVT>, g.smem_dim), smem_optin(k_ffn_up<DBITS>, g.smem_dim), smem_optin(k_output<DBITS>, g.smem_dim);
 	smem_optin(k_matres<DBITS>, smem_res); // ONE attribute per kernel: the larger of its two launch shapes (wo, w2)
+	if constexpr (DBITS != 4) {
+		if (c.n_experts == 0) { // (the expert rows of a routed model are known only after the router)
+			const int stages = getenv("CALM_B200_COLS") ? atoi(getenv("CALM_B200_COLS")) : 15; // (experiments) 1 q/k/v, 2 wo, 4 FFN up, 8 FFN down
+			if (stages & 1 && !c.norm_ln) g.cols_qkv = plan_cols<DBITS>(c.dim, (g.q_dim + 2 * g.kv_dim) / 2, false);
+			if (stages & 2) g.cols_wo = plan_cols<DBITS>(g.q_dim, c.dim, true), g.cols_wo.alone = true;
+			if (stages & 4 && (!c.norm_ln || c.norm_par)) g.cols_up = plan_cols<DBITS>(c.dim, c.hidden_dim, false);
+			if (stages & 8) g.cols_down = plan_cols<DBITS>(c.hidden_dim, c.dim, true);
+			if (g.cols_qkv.n) cols_qkv<DBITS, KVT>(QkvArgs<KVT>(), g.cols_qkv, true);
+			if (g.cols_up.n) cols_up<DBITS>(FfnUpArgs(), g.cols_up, true);
+			if (g.cols_wo.n) cols_res<DBITS>(MatResArgs(), g.cols_wo, true);
+			if (g.cols_down.n) cols_res<DBITS>(MatResArgs(), g.cols_down, true);
+		}
+	}
 	{
 		// k_attn2 when the shape is instantiated and the CTA's share of the context fits in shared memory
 		g.attn_nbmax = cdiv(cdiv(c.seq_len, ATTN2_BP), g.attn_nsplit);
@@ -857,17 +870,6 @@ void make_plan() {
 	}
 	// (measured: for the long FFN-up stage a full 4-CTA/SM grid with uneven rounds beats a balanced 3-CTA/SM one)
 	g.grid_up = imin(max_ctas(k_ffn_up<DBITS>, 256, g.smem_dim), cdiv(g.nact * c.hidden_dim, 8));
-	if constexpr (DBITS != 4) {
-		if (c.n_experts == 0) { // (the expert rows of a routed model are known only after the router)
-			if (!c.norm_ln) g.cols_qkv = plan_cols<DBITS>(c.dim, (g.q_dim + 2 * g.kv_dim) / 2, false);
-			if (!c.norm_ln || c.norm_par) g.cols_up = plan_cols<DBITS>(c.dim, c.hidden_dim, false);
-			g.cols_wo = plan_cols<DBITS>(g.q_dim, c.dim, true), g.cols_wo.alone = true, g.cols_down = plan_cols<DBITS>(c.hidden_dim, c.dim, true);
-			if (g.cols_qkv.n) cols_qkv<DBITS, KVT>(QkvArgs<KVT>(), g.cols_qkv, true);
-			if (g.cols_up.n) cols_up<DBITS>(FfnUpArgs(), g.cols_up, true);
-			if (g.cols_wo.n) cols_res<DBITS>(MatResArgs(), g.cols_wo, true);
-			if (g.cols_down.n) cols_res<DBITS>(MatResArgs(), g.cols_down, true);
-		}
-	}
 	// TMA-ring kernels for the dense single-GPU stages whose rows are whole 1 KB / 2 KB chunks (ring.cuh)
 	g.ring_up_u = g.ring_wo_u = g.ring_down_u = 0;
 	{ // weights are read once per token: L2::evict_first on the ring's bulk copies measured 2 % faster than the default policy
