@@ -1533,7 +1533,8 @@ extern "C" void calm_b200_prefill_cut(int product, int rows, int n, int k, int s
 
 extern "C" int calm_b200_token_plan(int stage) {
 	const ColsPlan* p[4] = {&g.cols_qkv, &g.cols_wo, &g.cols_up, &g.cols_down};
-	return g.ready && stage >= 0 && stage < 4 ? p[stage]->n : 0;
+	const int ring[4] = {0, g.ring_wo_u, g.ring_up_u, g.ring_down_u};
+	return !g.ready || stage < 0 || stage > 7 ? 0 : stage < 4 ? p[stage]->n : p[stage - 4]->n ? 0 : ring[stage - 4];
 }
 
 template <int MODE, int DBITS>

@@ -47,7 +47,7 @@ class ModelSpec:
     n_experts_active: int = 0
     norm_eps: float = 1e-5
     act_type: str = "silu"  # silu | gelu
-    norm_type: str = "rmsnorm"  # rmsnorm | layernorm | layernorm_par
+    norm_type: str = "rmsnorm"  # rmsnorm | layernorm, either with _par: one norm for attention and FFN
     qkv_clip: Optional[float] = None
     qkv_bias: bool = False
     tied: bool = False  # no model.output.weight: classifier = embedding
@@ -192,7 +192,7 @@ def tensor_plan(spec: ModelSpec):
     for l in range(s.n_layers):
         p = f"model.layers.{l}."
         plan.append((p + "attn.norm.weight", (s.dim,), "n"))
-        if s.norm_type != "layernorm_par":
+        if not s.norm_type.endswith("_par"):
             plan.append((p + "mlp.norm.weight", (s.dim,), "n"))
         plan.append((p + "attn.wq.weight", (s.q_dim, s.dim), "w"))
         plan.append((p + "attn.wk.weight", (s.kv_dim, s.dim), "w"))
@@ -338,7 +338,7 @@ def fill_transformer(spec: ModelSpec, ptr_of, seq_len: Optional[int] = None, kvb
     c.norm_eps = spec.norm_eps
     c.act_gelu = spec.act_type == "gelu"
     c.norm_ln = spec.norm_type.startswith("layernorm")
-    c.norm_par = spec.norm_type == "layernorm_par"
+    c.norm_par = spec.norm_type.endswith("_par")
     c.qkv_clip = spec.qkv_clip if spec.qkv_clip is not None else FLT_MAX
 
     w = t.weights

@@ -110,15 +110,18 @@ def test_fp8_kv_cache_teacher_forced_vs_oracle(oracle_pkg, name):
 
 
 @pytest.mark.parametrize("dtype", ["gf4", "fp8", "fp16"])
-def test_ring_fed_kernels_vs_oracle(oracle_pkg, dtype):
+def test_ring_fed_kernels_vs_oracle(oracle_pkg, dtype, monkeypatch):
     """Shapes the ring-fed stage kernels of ring.cuh serve (rows of whole 1 KB / 2 KB chunks, K-slices folded in shared memory;
-    for gf4 with the staged group sums) against the CPU oracle, teacher-forced."""
-    spec = replace(mg.SPECS["pf-tiny-hd128"], name="ring-" + dtype, dtype=dtype, dim=2048, hidden_dim=4096, n_heads=8, n_kv_heads=2, n_layers=2)
+    for gf4 with the staged group sums; fp8 and fp16 where the tensor-core matvecs leave them the stage) against the CPU oracle, teacher-forced."""
+    monkeypatch.setenv("CALM_B200_COLS", "0")
+    spec = replace(mg.SPECS["pf-tiny-hd128"], name="ring-" + dtype, dtype=dtype, dim=2048, hidden_dim=4096, n_heads=16, n_kv_heads=4, n_layers=2)
     toks = mg.teacher_tokens(spec.vocab_size, 20)
     host = mg.HostModel(spec, seed=7)
     ck = oracle_pkg.Checker("port")
     ref = oracle_pkg.teacher_forced(ck, host, toks)
     with lib.DeviceModel(spec, host.tensors) as dm:
+        plan = [lib.load().calm_b200_token_plan(s) for s in range(8)]
+        assert plan[:4] == [0, 0, 0, 0] and all(plan[5:]), plan
         got = np.stack([dm.forward(t, i) for i, t in enumerate(toks)])
     ck.release(host)
     sigma = float(ref.std())

@@ -24,10 +24,10 @@ def _gpus():
     return torch.cuda.device_count()
 
 
-def _run_world(tmp_path, name, world, fused, tokens, greedy=12):
+def _run_world(tmp_path, name, world, fused, tokens, greedy=12, cols="15"):
     out = str(tmp_path / "tp")
     idfile = str(tmp_path / "nccl.id")
-    env = dict(os.environ, PYTHONPATH=ROOT, CALM_B200_QUIET="1", CALM_B200_TP_FUSED=str(fused))
+    env = dict(os.environ, PYTHONPATH=ROOT, CALM_B200_QUIET="1", CALM_B200_TP_FUSED=str(fused), CALM_B200_COLS=cols)
     procs = [subprocess.Popen([sys.executable, "-m", "calm_b200.tp", "--spec", name, "--rank", str(r), "--world", str(world), "--idfile", idfile,
                                "--tokens", str(tokens), "--out", out, "--greedy", str(greedy)], cwd=ROOT, env=env,
                               stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True) for r in range(world)]
@@ -48,15 +48,18 @@ CASES = [("tiny-fp8", 2, 1), ("tiny-gf4", 2, 1), ("tiny-bias2", 2, 1), ("tiny-ln
          ("tiny-moe", 2, 1), ("ring-tp", 2, 1), ("tiny-tp8", 2, 1), ("ring-tp", 4, 1), ("tiny-tp8", 4, 1), ("tiny-tp8-moe", 4, 1), ("tiny-tp8", 4, 0), ("tiny-tp8", 8, 1), ("tiny-tp8-moe", 8, 1), ("tiny-tp8", 8, 0)]
 
 
+@pytest.mark.parametrize("cols", ["15", "0"])
 @pytest.mark.parametrize("name,world,fused", CASES)
-def test_ranks_match_single_device_reference(tmp_path, name, world, fused):
-    """fused=1: partial sums exchanged inside k_matres over peer memory, classifier split by vocabulary;
+def test_ranks_match_single_device_reference(tmp_path, name, world, fused, cols):
+    """fused=1: partial sums exchanged inside k_matres_cols (cols=0: k_matres, k_matres_ring) over peer memory, classifier split by vocabulary;
     fused=0: ncclAllReduce between kernels, replicated classifier."""
+    if cols == "0" and name not in ("ring-tp", "tiny-fp8"):
+        pytest.skip("one of the other kernels' models")
     if _gpus() < world:
         pytest.skip(f"needs {world} GPUs")
     spec = mg.SPECS[name]
     g = golden(name)
-    res = _run_world(tmp_path, name, world, fused, len(g["tokens"]))
+    res = _run_world(tmp_path, name, world, fused, len(g["tokens"]), cols=cols)
     r0 = res[0]
     assert int(r0["world"]) == world
     for r in res:
