@@ -478,6 +478,14 @@ struct GemmExtra {
 	AttBand band = {};
 };
 bool al8(long v) { return v % 8 == 0; }
+// Warps of a CTA in the weight-streaming kernel.  Twice the warps keep as many bytes in flight where every CTA has an SM (2048 x 5632, 16 tokens: 7.1 us, 9.6 with eight).  More CTAs than
+// that would run one after the other, since 16 warps take more than half of an SM's registers (5632 x 1024, one token: 6.0 us, 2.9 with eight; 3216 x 1024 3.8 and 2.1).
+// groups > 1 with rows: a product grouped by expert, most of whose CTAs find no row and leave; they cost more with 16 warps, so rows are to be longer and CTAs fewer than three an SM (two rows
+// for eight experts: 512 x 2048 4.5 -> 3.8 us, 512 x 1024 3.1 -> 3.5, 2048 x 1024 4.4 -> 7.1; four for sixteen: 512 x 2048 5.1 -> 5.4).
+int skinny_warps(int M, int K, int groups, int rows, int sms) {
+	const long ctas = (long)cdiv(M, 16) * groups, working = rows > 0 ? (long)cdiv(M, 16) * std::min(groups, rows) : ctas;
+	return working <= sms && ctas < 3L * sms && K >= (ctas > sms ? 2048 : 1024) ? 16 : 8;
+}
 // products of few rows that the weight-streaming kernel takes
 bool gemm_skinny_fits(const Seq& s, const void* X, long ldx, long xbs, const void* W, long ldw, long wbs, int N, int K) {
 	return !s.m.exact && N <= 32 && al8(K) && al8(ldx) && al8(ldw) && al8(xbs) && al8(wbs) && ((uintptr_t)X & 15) == 0 && ((uintptr_t)W & 15) == 0;
@@ -507,9 +515,7 @@ void gemm(Seq& s, const void* X, long ldx, long xbs, const void* W, long ldw, lo
 	if (a.band_mode == 2) CALM_FATAL("seq: a banded value product needs the tcgen05 kernel"); // what the band leaves out of its input was never written
 	if (gemm_skinny_fits(s, X, ldx, xbs, W, ldw, wbs, N, K)) {
 		const dim3 grid(cdiv(M, 16), 1, batch);
-		// At most a CTA per SM: twice the warps per CTA keep as many bytes in flight (2048 x 5632, 16 tokens: 7.1 us, 9.6 with eight).  More CTAs than that would run one
-		// after the other, since 16 warps take more than half of an SM's registers (5632 x 1024, one token: 6.0 us, 2.9 with eight; 3216 x 1024 3.8 and 2.1).
-		const bool few = (long)cdiv(M, 16) * batch <= s.sms && K >= 1024;
+		const bool few = skinny_warps(M, K, batch, ex->seg ? ex->x_rows : 0, s.sms) == 16;
 		run_kernel(s, kind_as >= 0 ? kind_as : KD_GEMM_SKINNY, bytes, flops, [&] {
 			if (few) {
 				if (N <= 8) launch_k(s, k_seq_gemm_skinny<1, 16>, grid, 512, 0, a);
@@ -1507,6 +1513,7 @@ extern "C" void* calm_b200_seq_upload(const void* host, size_t size) {
 extern "C" void calm_b200_seq_free(void* p) { cudaFree(p); }
 extern "C" uint64_t calm_b200_seq_launch_count(void) { return g_seq_launches; }
 extern "C" uint64_t calm_b200_seq_route_count(int route) { return route >= SEQ_ROUTE_PAIRS ? (route < SEQ_ROUTE_PAIRS + TG_EPILOGUES ? g_tg.pair_launches[route - SEQ_ROUTE_PAIRS] : 0) : route >= 0 ? g_seq_routes[route] : 0; }
+extern "C" int calm_b200_seq_skinny_warps(int m, int k, int groups, int rows, int sms) { return skinny_warps(m, k, groups, rows, sms); }
 extern "C" int calm_b200_seq_delta_blocks_pay(int longest, int few, int heads, int vdim, int sms) { return delta_blocks_pay(longest, few, heads, vdim, sms); }
 extern "C" int calm_b200_seq_pairs_pay(int rows, int tokens, int k, int epi, int pairs) { return tg_pairs_pay(rows, tokens, k, epi, pairs); }
 

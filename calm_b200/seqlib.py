@@ -89,6 +89,7 @@ def load() -> C.CDLL:
     L.calm_b200_seq_launch_count.argtypes, L.calm_b200_seq_launch_count.restype = [], C.c_uint64
     L.calm_b200_seq_pairs_pay.argtypes, L.calm_b200_seq_pairs_pay.restype = [C.c_int] * 5, C.c_int
     L.calm_b200_seq_delta_blocks_pay.argtypes, L.calm_b200_seq_delta_blocks_pay.restype = [C.c_int] * 5, C.c_int
+    L.calm_b200_seq_skinny_warps.argtypes, L.calm_b200_seq_skinny_warps.restype = [C.c_int] * 5, C.c_int
     L.calm_b200_seq_route_count.argtypes, L.calm_b200_seq_route_count.restype = [C.c_int], C.c_uint64
     L.calm_b200_seq_timer_start.argtypes, L.calm_b200_seq_timer_start.restype = [C.c_void_p], None
     L.calm_b200_seq_timer_stop.argtypes, L.calm_b200_seq_timer_stop.restype = [C.c_void_p], C.c_float

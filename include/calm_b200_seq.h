@@ -307,6 +307,9 @@ uint64_t calm_b200_seq_route_count(int route);
 /* whether the delta rule of a step runs in blocks of tokens: its longest portion, how many portions have fewer tokens than the least that blocks pay
    for, heads, value columns of a head, SMs; for tests */
 int calm_b200_seq_delta_blocks_pay(int longest, int few, int heads, int vdim, int sms);
+/* warps of a CTA in a product of at most 32 tokens (m weight rows of k columns, in each of `groups` matrices; rows: over all groups of a product grouped by
+ * expert, 0: not grouped); for tests */
+int calm_b200_seq_skinny_warps(int m, int k, int groups, int rows, int sms);
 /* whether a product of `rows` weight rows of k columns over `tokens` tokens with the epilogue `epi` runs on pairs of CTAs, on a device that holds
    `pairs` of them at a time; for tests */
 int calm_b200_seq_pairs_pay(int rows, int tokens, int k, int epi, int pairs);
