@@ -58,6 +58,7 @@ struct Seq {
 	std::map<const SeqLayer*, std::pair<double*, float>> rot; // per SEQ_GQA / SEQ_LATENT record (a layer's, or one of a pair's): angle step of every rotated pair (device), factor on cos and sin
 	cudaStream_t stream = nullptr;
 	int sms = 0;
+	std::map<std::pair<size_t, int>, int> attn_clusters; // shared memory, CTAs of a cluster -> clusters of k_seq_attn_mma that the device holds at a time
 	bool tc = false; // tcgen05 products available (bf16 mode)
 
 	// state manager
@@ -587,7 +588,20 @@ int round_split(int n) {
 	while (v < n) v = v < 4 ? v + 1 : (v & (v - 1)) ? v / 3 * 4 : v / 2 * 3; // 1 2 3 4 6 8 12 16 24 ...
 	return v;
 }
-AttnPlan attn_plan(const Seq& s, int group, int kd, int vd, bool shared_kv, int heads, int live_tokens, int span, int longest, bool parts = false) {
+int attn_clusters(Seq& s, size_t smem, int ctas) {
+	const auto at = s.attn_clusters.emplace(std::make_pair(smem, ctas), 0);
+	if (at.second) {
+		cudaLaunchConfig_t cfg = {};
+		cfg.gridDim = dim3(1, 1, ctas), cfg.blockDim = 256, cfg.dynamicSmemBytes = smem;
+		cudaLaunchAttribute size;
+		size.id = cudaLaunchAttributeClusterDimension;
+		size.val.clusterDim.x = size.val.clusterDim.y = 1, size.val.clusterDim.z = ctas;
+		cfg.attrs = &size, cfg.numAttrs = 1;
+		CUDA_CHECK(cudaOccupancyMaxActiveClusters(&at.first->second, k_seq_attn_mma, &cfg));
+	}
+	return at.first->second;
+}
+AttnPlan attn_plan(Seq& s, int group, int kd, int vd, bool shared_kv, int heads, int live_tokens, int span, int longest, bool parts = false) {
 	AttnPlan p;
 	p.smem = atm_smem(kd, vd, shared_kv);
 	p.mma = s.attn_mma && !s.m.exact && p.smem <= 220 * 1024 && vd <= 8 * 8 * ATM_TILES;
@@ -597,11 +611,17 @@ AttnPlan attn_plan(const Seq& s, int group, int kd, int vd, bool shared_kv, int 
 		while (group % p.tile) --p.tile;
 		const int per_sm = std::max(1, std::min(4, (int)(227 * 1024 / (p.smem + 1024)))), ctas = live_tokens * (heads / p.tile), room = s.sms * per_sm;
 		p.nsplit = ctas >= room ? 1 : std::max(1, std::min({round_split(cdiv(keys, ATM_KC)), room / ctas, ATT_MAXSPLIT}));
-		// Up to twelve shares run as at most eight, which a thread-block cluster folds: a second 32 keys for some of them cost less than the merge's launch.  The sums of a
-		// share go where its keys were, and all clusters are to run at one time (the GPCs hold this many of a size with a CTA per SM).
-		static const int most[9] = {0, 0, 74, 45, 33, 26, 22, 15, 15};
+		// Up to twelve shares run as at most eight, which a thread-block cluster folds: a second 32 keys for some of them cost less than the merge's launch.  The sums of a share go where
+		// its keys were.  All clusters are to run at one time, and large ones in three quarters of the places the device has for them, or they wait for the previous kernel's last CTAs to
+		// free eight in one GPC; and a CTA is to read no more than 2048 sums of the others.  Captured steps of four layers, us with the merge and with clusters: 16 heads of 128, four
+		// for keys, one sequence of 40 / 250 positions 143 -> 131, 165 -> 152, six of 250 166 -> 168, six of 380 181 -> 167, eight of 250 (32 clusters of eight, 33 fit) 168 -> 188, of 380 178 -> 201;
+		// 16 heads on latents of 128 at 250 164 -> 147, eight on 256 157 -> 150, sixteen on 256 at 40 154 -> 153, six sequences 157 -> 168, on 512 165 -> 177.
 		const int shares = std::min(p.nsplit, 8);
-		p.cluster = !parts && p.nsplit > 1 && p.nsplit <= 12 && ctas <= most[shares] * per_sm && (size_t)p.tile * vd <= (size_t)2 * ATM_KC * (atm_pad(kd) + (shared_kv ? 0 : atm_pad(vd)));
+		p.cluster = !parts && p.nsplit > 1 && p.nsplit <= 12 && p.tile * vd <= 2048 && (size_t)p.tile * vd <= (size_t)2 * ATM_KC * (atm_pad(kd) + (shared_kv ? 0 : atm_pad(vd)));
+		if (p.cluster) {
+			const int fit = attn_clusters(s, p.smem, shares);
+			p.cluster = ctas <= (shares > 4 ? fit * 3 / 4 : fit);
+		}
 		if (p.cluster) p.nsplit = shares;
 	} else {
 		p.tile = attn_tile(group, kd, vd), p.smem = attn_smem(p.tile, kd);

@@ -73,3 +73,24 @@ def test_shares_in_clusters(layer, n, clusters):
             out = m.step([slot], [[toks[n + k]]], [0])
             assert t.rel_err(out, ref[n + k:n + k + 1]) < t.TOL["bfloat16"], k
     assert at == before and (ran(5) > at) == clusters
+
+
+# what keeps the merge: 32 clusters of eight where 33 fit, 4096 sums to read, wide latents; and next to them what does not
+@pytest.mark.parametrize("layer,batch,n,clusters", [(tb.attn(heads=8, kv_heads=2, dim=128, vdim=128, size=0), 16, 250, False), (tb.attn(heads=8, kv_heads=2, dim=128, vdim=128, size=0), 8, 250, True),
+                                                    (tb.attn(heads=8, kv_heads=2, dim=128, vdim=128, size=0), 16, 70, True), (tb.attn(heads=16, kv_heads=4, dim=64, vdim=64, size=0), 10, 300, False),
+                                                    (tv.latent(heads=16, dim=16, vdim=16, kv_rank=256), 2, 70, False), (tv.latent(heads=8, dim=16, vdim=16, kv_rank=256), 2, 70, True)])
+def test_clusters_where_they_pay(layer, batch, n, clusters):
+    t, mod, plain = (tb, bovinex, bovinex_plain) if layer["mixer"].get("rot") else (tv, vimulorn, vimulorn_plain)
+    cfg = t.config([layer])
+    weights, toks = t.weights(cfg, 5), t.tokens(cfg, n + 2)
+    ref = plain.forward(cfg, t.as_f64(weights), toks)
+    with mod.from_tensors(cfg, weights, "bfloat16", max_tokens=batch * (n + 64), max_seqs=batch, page=16) as m:
+        slots = [m.open() for _ in range(batch)]
+        for s in slots:
+            m.step([s], [toks[:n]], [0])
+        before = ran(5)
+        for k in range(2):
+            out = m.step(slots, [[toks[n + k]]] * batch, list(range(batch)))
+            for row in out:
+                assert t.rel_err(row[None], ref[n + k:n + k + 1]) < t.TOL["bfloat16"], k
+    assert (ran(5) > before) == clusters
