@@ -26,24 +26,12 @@
 #pragma once
 
 #include "stages.cuh"
+#include "tc05.cuh"
 
 #define ATTN2_BP 16   // positions per block (one bulk copy of K, one of V)
 #define ATTN2_MAXB 32 // blocks per CTA
 
-// ---- thread-block cluster helpers (the CTAs of a unit form one cluster when CLUSTER: nsplit <= 16)
-__device__ __forceinline__ void cluster_sync_all() { // every thread of every CTA of the cluster; release / acquire at cluster scope
-	asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-	asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float ld_dsmem(const float* local_ptr, uint32_t cta_rank) { // the same shared-memory location in CTA `cta_rank` of this cluster
-	uint32_t raddr;
-	float v;
-	asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(raddr) : "r"(smem_u32(local_ptr)), "r"(cta_rank));
-	asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(raddr) : "memory");
-	return v;
-}
-
-#define ATTN2_MAX_CLUSTER 16
+#define ATTN2_MAX_CLUSTER 16 // the CTAs of a unit form one cluster when CLUSTER
 
 // shared memory: K blocks | V blocks | q [HG][head_dim] | merge scratch | this CTA's merged record [HG][head_dim + 2]
 template <typename KVT>
@@ -322,10 +310,10 @@ __global__ void __launch_bounds__(ATTN_THREADS) k_attn2(const AttnArgs a) {
 		__shared__ float mls[ATTN2_MAX_CLUSTER][HG][2]; // (m, l) of every slice, then (coefficient, -) in place
 		__shared__ float invl[HG];
 		attn_cta_merge<HG>(a, HG, 0, HG, warp, NW, m, l, acc, scratch, myrec);
-		cluster_sync_all(); // every CTA's record is complete and visible cluster-wide
+		cluster_sync(); // every CTA's record is complete and visible cluster-wide
 		for (int i = tid; i < nsplit * HG; i += ATTN_THREADS) {
 			const int s = i / HG, h = i % HG;
-			mls[s][h][0] = ld_dsmem(myrec + h * REC + HD, s), mls[s][h][1] = ld_dsmem(myrec + h * REC + HD + 1, s);
+			mls[s][h][0] = cluster_load_f32(cluster_addr(myrec + h * REC + HD, s)), mls[s][h][1] = cluster_load_f32(cluster_addr(myrec + h * REC + HD + 1, s));
 		}
 		__syncthreads();
 		if (tid < HG) {
@@ -348,12 +336,12 @@ __global__ void __launch_bounds__(ATTN_THREADS) k_attn2(const AttnArgs a) {
 			float v = 0.f;
 			if (o < o_end) {
 				const int h = o / HD, e = o % HD;
-				for (int s = sg; s < nsplit; s += 8) v = fmaf(ld_dsmem(myrec + h * REC + e, s), mls[s][h][0], v);
+				for (int s = sg; s < nsplit; s += 8) v = fmaf(cluster_load_f32(cluster_addr(myrec + h * REC + e, s)), mls[s][h][0], v);
 			}
 			v += __shfl_xor_sync(0xffffffffu, v, 1), v += __shfl_xor_sync(0xffffffffu, v, 2), v += __shfl_xor_sync(0xffffffffu, v, 4);
 			if (o < o_end && sg == 0) __stcg(a.out + (size_t)hbase * HD + o, v * invl[o / HD]);
 		}
-		cluster_sync_all(); // no CTA may exit (and free its shared memory) while a peer still reads its record
+		cluster_sync(); // no CTA may exit (and free its shared memory) while a peer still reads its record
 	} else {
 		constexpr int REC = HD + 2;
 		__shared__ float mls[ATTN2_MAXB + 4][HG][2]; // (m, l) of every slice, then the coefficient in place  (nsplit <= 36)

@@ -1465,6 +1465,13 @@ static bool pf_supported() {
 	       (c.head_dim == 64 || c.head_dim == 128) && !(getenv("CALM_B200_PREFILL") && atoi(getenv("CALM_B200_PREFILL")) == 0);
 }
 
+// All tiles in slices, few enough slices for one thread-block cluster, and all clusters at one time: the CTAs take an SM each and a GPC's SMs hold this many clusters
+// (cudaOccupancyMaxActiveClusters on a B200; the rule has no device to ask where its tests run).
+static bool pf_cluster(int tail, int tiles, int splits) {
+	static const int most[9] = {0, 0, 74, 45, 33, 26, 22, 15, 15};
+	return tail == tiles && splits > 1 && splits <= 8 && tiles <= most[splits];
+}
+
 // Row tiles and tokens per item and K-slices of a product of `rows` weight rows over n tokens: the choice with the least estimated time, in cycles.
 // Kernel time over k-stages, 4096 x 4096 x 2047 tokens, in cycles at 1.965 GHz, for 64 / 128 / 256 tokens of one row tile and 64 / 128 of two: fp8
 // 1090 / 1270 / 1880 and 1490 / 2100 (248 / 165 / 122 and 194 / 137 us), gf4 1290 / 1470 / 2060 and 1680 / 2220 (294 / 192 / 134 and 218 / 145 us), fp16
@@ -1475,12 +1482,7 @@ static bool pf_supported() {
 // 2047 tokens 206 us, 184; fp8, 1000 tokens 147, 106 with a tail; fp16, 333 tokens in two slices 58, 48 whole), and two of 64 against two of 128 with a tail (FFN up
 // 14336 x 4096, 300 tokens, fp8: 191, 160).  The fold's price of 15 a column and slice is low where whole tiles are folded (pf_tail has 40: 4096 x 14336, 60 tokens, fp16 in
 // nine slices of two row tiles 48 us, in four of one 37), about right where half of a tile's tokens are there (20 tokens, fp8: 33, 39).
-// All tiles in slices, few enough slices for one thread-block cluster, and all clusters at one time: the CTAs take an SM each and a GPC's SMs hold this many clusters
-// (cudaOccupancyMaxActiveClusters on a B200).
-static bool pf_cluster(int tail, int tiles, int splits) {
-	static const int most[9] = {0, 0, 74, 45, 33, 26, 22, 15, 15};
-	return tail == tiles && splits > 1 && splits <= 8 && tiles <= most[splits];
-}
+// Row tiles and tokens are chosen by the price of the fold through memory; what a cluster's fold costs decides the slices of that choice only.
 static void pf_tiles(int mode, int rows, int n, int nkb, int sms, int& na_out, int& bn_out, int& splits_out) {
 	long best = -1;
 	for (int na = 2; na >= (mode == PF_UP ? 2 : 1); --na)
@@ -1522,13 +1524,18 @@ static int pf_cut(int mode, int rows, int n, int nkb, int sms, int& na, int& bn,
 	else pf_tail(tiles, nkb, sms, na, bn, tail, splits);
 	return tiles;
 }
-// all tiles in slices, few enough of each for one thread-block cluster
 static int pf_mode(int product) { return product == 0 ? PF_QKV : product == 1 ? PF_RES : PF_UP; }
 extern "C" void calm_b200_prefill_tiles(int product, int rows, int n, int k, int sms, int* out3) {
 	pf_tiles(pf_mode(product), rows, n, k / PF_BK, sms, out3[0], out3[1], out3[2]);
 }
 extern "C" void calm_b200_prefill_cut(int product, int rows, int n, int k, int sms, int* out5) {
 	out5[0] = pf_cut(pf_mode(product), rows, n, k / PF_BK, sms, out5[1], out5[2], out5[3], out5[4]);
+}
+
+extern "C" int calm_b200_prefill_clusters(int product, int rows, int n, int k, int sms) {
+	int na, bn, tail, splits;
+	const int tiles = pf_cut(pf_mode(product), rows, n, k / PF_BK, sms, na, bn, tail, splits);
+	return pf_cluster(tail, tiles, splits);
 }
 
 extern "C" int calm_b200_token_plan(int stage) {

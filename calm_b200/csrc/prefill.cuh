@@ -279,22 +279,6 @@ __device__ __forceinline__ void pf_epilogue(const PfGemmArgs& a, int gr, int lan
 	}
 }
 
-// ---- the CTAs of a cluster
-__device__ __forceinline__ void pf_cluster_sync() { // every thread of every CTA; release / acquire at cluster scope
-	asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-	asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t pf_peer(const float* own, int rank) { // the same place in the shared memory of CTA `rank`
-	uint32_t r;
-	asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(own)), "r"(rank));
-	return r;
-}
-__device__ __forceinline__ float pf_peer_load(uint32_t addr) {
-	float v;
-	asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-	return v;
-}
-
 // named barrier of `threads` threads that also tells whether `p` held for all of them
 __device__ __forceinline__ bool bar_and(int id, int threads, bool p) {
 	int all;
@@ -617,7 +601,7 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 	}
 	if constexpr (CLUSTER) { // each CTA of a tile adds up, in slice order, and finishes its share of the tile's tokens
 		pdl_wait_prev(); // (roles that touch nothing of the previous kernel have not waited for it)
-		pf_cluster_sync();
+		cluster_sync();
 		const Item t = item_of(blockIdx.x);
 		const int cols = min(bn, a.n_tokens - t.tok0), rank = blockIdx.x % splits;
 		const int lo = cols * rank / splits, hi = cols * (rank + 1) / splits, groups = pf_threads<DBITS>() / PF_BM, lr = tid % PF_BM;
@@ -626,17 +610,17 @@ __global__ void __launch_bounds__(pf_threads<DBITS>(), 1) k_pf_gemm(const __grid
 				float v[4] = {0.f, 0.f, 0.f, 0.f}, v3[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
 				for (int sp = 0; sp < splits; ++sp) {
-					const uint32_t peer = pf_peer(partial + (size_t)(i * bn + c) * PF_BM + lr, sp);
+					const uint32_t peer = cluster_addr(partial + (size_t)(i * bn + c) * PF_BM + lr, sp);
 #pragma unroll
 					for (int j = 0; j < 4; ++j)
 						if (c + j < hi) {
-							v[j] += pf_peer_load(peer + j * PF_BM * 4);
-							if (MODE == PF_UP) v3[j] += pf_peer_load(peer + (bn + j) * PF_BM * 4);
+							v[j] += cluster_load_f32(peer + j * PF_BM * 4);
+							if (MODE == PF_UP) v3[j] += cluster_load_f32(peer + (bn + j) * PF_BM * 4);
 						}
 				}
 				pf_epilogue<MODE, 4>(a, t.row0 + i * PF_BM + lr, lane, t.tok0 + c, hi - c, v, v3);
 			}
-		pf_cluster_sync(); // no CTA leaves while another reads its sums
+		cluster_sync(); // no CTA leaves while another reads its sums
 	}
 	if (warp == 1) {
 		tc_fence_after();

@@ -699,21 +699,6 @@ __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
 __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
 	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
-// the CTAs of a cluster
-__device__ __forceinline__ void seq_cluster_sync() { // every thread of every CTA; release / acquire at cluster scope
-	asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-	asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t seq_peer(const float* own, int rank) { // the same place in the shared memory of CTA `rank`
-	uint32_t r;
-	asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(own)), "r"(rank));
-	return r;
-}
-__device__ __forceinline__ float seq_peer_load(uint32_t addr) {
-	float v;
-	asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-	return v;
-}
 __global__ void __launch_bounds__(256) k_seq_attn_mma(AttArgs a, bf16* out, SeqBatch sb, int shared_kv, int vec) {
 	pdl_enter(); // programmatic dependent launch: let the next kernel's launch overlap this one, then wait for the previous one
 	extern __shared__ __align__(16) float sm[];
@@ -872,17 +857,17 @@ __global__ void __launch_bounds__(256) k_seq_attn_mma(AttArgs a, bf16* out, SeqB
 				const int r = g + (e >> 1) * 8, d = (warp + 8 * i) * 8 + 2 * t + (e & 1);
 				if (r < R && d < vd) own[r * vd + d] = acc[i][e];
 			}
-		seq_cluster_sync();
+		cluster_sync();
 		__shared__ float wz[8][16], inv[16];
 		if (tid < 16) {
 			float m[8], l = 0.f, mx = -INFINITY;
 #pragma unroll
-			for (int k = 0; k < 8; ++k) m[k] = k < ns ? seq_peer_load(seq_peer(mrow + tid, k)) : -INFINITY, mx = fmaxf(mx, m[k]);
+			for (int k = 0; k < 8; ++k) m[k] = k < ns ? cluster_load_f32(cluster_addr(mrow + tid, k)) : -INFINITY, mx = fmaxf(mx, m[k]);
 #pragma unroll
 			for (int k = 0; k < 8; ++k)
 				if (k < ns) {
 					const float w = m[k] != -INFINITY ? expf(m[k] - mx) : 0.f; // a share without keys counts nothing
-					wz[k][tid] = w, l = fmaf(w, seq_peer_load(seq_peer(lrow + tid, k)), l);
+					wz[k][tid] = w, l = fmaf(w, cluster_load_f32(cluster_addr(lrow + tid, k)), l);
 				}
 			inv[tid] = 1.f / l;
 		}
@@ -894,10 +879,10 @@ __global__ void __launch_bounds__(256) k_seq_attn_mma(AttArgs a, bf16* out, SeqB
 			const float gt = a.gate ? sigmoidf_(a.gate[(size_t)n * a.ldg + (size_t)(h0 + r) * a.ghs + (size_t)d * a.ges]) : 1.f;
 			float v = 0.f;
 #pragma unroll 8
-			for (int k = 0; k < ns; ++k) v = fmaf(seq_peer_load(seq_peer(own + e, k)), wz[k][r], v);
+			for (int k = 0; k < ns; ++k) v = fmaf(cluster_load_f32(cluster_addr(own + e, k)), wz[k][r], v);
 			out[o * vd + d] = __float2bfloat16_rn(v * (gt * inv[r]));
 		}
-		seq_cluster_sync(); // no CTA leaves while another reads its sums
+		cluster_sync(); // no CTA leaves while another reads its sums
 		return;
 	}
 #pragma unroll

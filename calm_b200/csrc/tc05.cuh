@@ -89,15 +89,13 @@ __device__ __forceinline__ bool elect_one() { // one lane of a converged warp
 	return p != 0;
 }
 
-// ---------------------------------------------------------------- two CTAs of a cluster on one tile (cta_group::2)
-// Both hold their own 128 rows of A and half of B's rows at the same offsets of their shared memory; rank 0 issues the MMAs, and each finds its 128 rows of D
-// in its own TMEM.
+// ---------------------------------------------------------------- the CTAs of a cluster
 __device__ __forceinline__ uint32_t cluster_rank() {
 	uint32_t r;
 	asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
 	return r;
 }
-__device__ __forceinline__ void cluster_sync() { // every thread of both CTAs, warps converged
+__device__ __forceinline__ void cluster_sync() { // every thread of every CTA; release / acquire at cluster scope
 	__syncwarp();
 	asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -107,6 +105,15 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
 	asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
 	return a;
 }
+__device__ __forceinline__ float cluster_load_f32(uint32_t addr) { // named by cluster_addr
+	float v;
+	asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+	return v;
+}
+
+// ---------------------------------------------------------------- two CTAs of a cluster on one tile (cta_group::2)
+// Both hold their own 128 rows of A and half of B's rows at the same offsets of their shared memory; rank 0 issues the MMAs, and each finds its 128 rows of D
+// in its own TMEM.
 __device__ __forceinline__ void cluster_store(uint32_t addr, int v) { // a variable named by cluster_addr; read after a cluster_sync
 	asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }

@@ -31,6 +31,7 @@ SYMBOLS = [
     "calm_b200_decode_sample", "calm_b200_forward_sample", "calm_b200_read_device_logits", "calm_b200_sample_logits",
     "calm_b200_prefill_tiles",
     "calm_b200_prefill_cut",
+    "calm_b200_prefill_clusters",
     "calm_b200_token_plan",
 ]
 
@@ -82,6 +83,7 @@ def load() -> C.CDLL:
     L.calm_b200_sample_logits.argtypes = [_fptr, C.c_int, C.c_float, C.c_float, C.POINTER(C.c_ulonglong), _fptr]
     L.calm_b200_sample_logits.restype = C.c_int
     L.calm_b200_token_plan.argtypes, L.calm_b200_token_plan.restype = [C.c_int], C.c_int
+    L.calm_b200_prefill_clusters.argtypes, L.calm_b200_prefill_clusters.restype = [C.c_int] * 5, C.c_int
     for f in (L.calm_b200_prefill_tiles, L.calm_b200_prefill_cut):
         f.argtypes, f.restype = [C.c_int] * 5 + [C.POINTER(C.c_int)], None
     _lib = L

@@ -110,6 +110,9 @@ void calm_b200_prefill_tiles(int product, int rows, int n, int k, int sms, int* 
  * (all of them, the last ones, none), slices of each} */
 void calm_b200_prefill_cut(int product, int rows, int n, int k, int sms, int* out5);
 
+/* 1 when the slices of that cut's tiles are folded inside thread-block clusters, 0: through memory, or no slices */
+int calm_b200_prefill_clusters(int product, int rows, int n, int k, int sms);
+
 /* How the prepared model's token runs a stage (0 q/k/v, 1 wo, 2 FFN up, 3 FFN down; for tests): pieces of a row (0, 2) or tiles of rows of a CTA (1, 3) of
  * the tensor-core matvecs, 0 when the stage has its other kernels; 4 + stage: 512-byte units of a row and chunk of the ring-fed kernel, 0 when the stage has none. */
 int calm_b200_token_plan(int stage);

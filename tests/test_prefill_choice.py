@@ -1,6 +1,6 @@
 """How the products of a prompt are cut (calm_b200_prefill_cut) and that every cut it makes computes the same: each combination of row tiles and tokens per item
-and tiles that are whole, in K-slices, or whole with a tail in slices that the rules pick anywhere in the range is run by one of the shapes here, in
-test_prefill_tiles_gpu.py or in test_prefill_tails_gpu.py."""
+and tiles that are whole, in K-slices folded through memory, in K-slices folded inside clusters, or whole with a tail in slices that the rules pick anywhere in the range is run by one of the shapes here, in
+test_prefill_tiles_gpu.py, test_prefill_tails_gpu.py or test_prefill_clusters_gpu.py."""
 import ctypes as C
 import os
 import sys
@@ -11,6 +11,7 @@ import torch
 
 sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
 from test_prefill_gpu import _both, _check  # noqa: E402
+from test_prefill_clusters_gpu import CLUSTERS  # noqa: E402
 from test_prefill_tails_gpu import TAILS  # noqa: E402
 
 from calm_b200 import build as cbuild  # noqa: E402
@@ -19,11 +20,12 @@ from calm_b200 import modelgen as mg  # noqa: E402
 
 SMS = 148
 # dim, heads, kv heads, head_dim, hidden, tokens, and the cuts that only this shape reaches
-SHAPES = [(896, 14, 2, 64, 4864, 449, {("res", 1, 128, "slices")}), (896, 14, 2, 64, 4864, 1537, {("qkv", 2, 64, "whole"), ("res", 1, 256, "slices"), ("res", 2, 64, "whole")}),
-          (768, 6, 2, 128, 2688, 1550, {("res", 2, 128, "slices")}), (384, 3, 3, 128, 384, 1900, {("qkv", 1, 128, "whole")}), (896, 7, 7, 128, 896, 1717, {("qkv", 1, 256, "whole")}),
-          (1536, 12, 12, 128, 1536, 1595, {("qkv", 2, 128, "whole"), ("res", 2, 128, "whole")}), (3072, 24, 8, 128, 6144, 67, {("up", 2, 128, "slices")}),
-          (4096, 32, 32, 128, 1024, 70, {("qkv", 2, 128, "slices"), ("up", 2, 64, "slices")})]
-ELSEWHERE = [(dim, dim, dim, hidden, n) for dim, hidden, n, _ in TAILS] + [(384, 384, 128, 1152, 1), (896, 896, 128, 2432, 61), (1024, 1024, 256, 3456, 65), (2048, 2048, 512, 5504, 257), (4096, 4096, 1024, 14336, 130)]
+SHAPES = [(896, 14, 2, 64, 4864, 449, {("res", 1, 128, "clusters")}), (896, 14, 2, 64, 4864, 1537, {("qkv", 2, 64, "whole"), ("res", 1, 256, "memory"), ("res", 2, 64, "whole")}),
+          (768, 6, 2, 128, 2688, 1550, {("res", 2, 128, "clusters")}), (384, 3, 3, 128, 384, 1900, {("qkv", 1, 128, "whole")}), (896, 7, 7, 128, 896, 1717, {("qkv", 1, 256, "whole")}),
+          (1536, 12, 12, 128, 1536, 1595, {("qkv", 2, 128, "whole"), ("res", 2, 128, "whole")}), (3072, 24, 8, 128, 6144, 67, {("up", 2, 128, "memory")}),
+          (4096, 32, 32, 128, 1024, 70, {("qkv", 2, 128, "memory")}), (2048, 16, 4, 128, 2048, 73, {("qkv", 1, 64, "memory")}), (3072, 24, 12, 128, 3072, 73, {("qkv", 2, 64, "memory"), ("up", 2, 64, "memory")}),
+          (3072, 24, 3, 128, 3072, 313, {("qkv", 2, 128, "clusters")}), (896, 7, 1, 128, 2304, 801, {("res", 1, 128, "memory")}), (4096, 32, 4, 128, 4096, 130, {("up", 2, 128, "clusters")})]
+ELSEWHERE = [(dim, heads * hd, kv * hd, hidden, n) for dim, heads, kv, hd, hidden, n, _ in CLUSTERS] + [(dim, dim, dim, hidden, n) for dim, hidden, n, _ in TAILS] + [(384, 384, 128, 1152, 1), (896, 896, 128, 2432, 61), (1024, 1024, 256, 3456, 65), (2048, 2048, 512, 5504, 257), (4096, 4096, 1024, 14336, 130)]
 
 
 @pytest.fixture(scope="module")
@@ -39,7 +41,7 @@ def cuts():
             # the accumulators fit half of TMEM; a slice is not empty; partial sums and counters of sliced products have one place per SM
             assert na in (1, 2) and bn in (64, 128, 256) and na * bn <= 256 and (name != "up" or na == 2) and 1 <= sp <= k // 64
             assert tiles == (rows // 128 if name == "up" else -(-rows // 128 // na)) * -(-n // bn) and tail * sp <= SMS and (tail == 0) == (sp == 1) and tail in (0, tiles, tiles % SMS)
-            got.add((name, na, bn, "whole" if tail == 0 else "slices" if tail == tiles else "tail"))
+            got.add((name, na, bn, "whole" if tail == 0 else "tail" if tail != tiles else "clusters" if L.calm_b200_prefill_clusters(product, rows, n, k, SMS) else "memory"))
         return got
 
     return of
