@@ -28,10 +28,11 @@
 // Two orders of the pieces of a CTA's rows: tile by tile with the whole vector's pieces in registers (q/k/v, FFN up), or one piece of all
 // rows after the other with one accumulator per tile and the vector's pieces made as they are needed (wo, w2: few rows, long ones).
 //
-// Measured, a whole token: Qwen2-0.5B fp16 at 131 positions 895 -> 648 us, Llama-3-8B fp8 at 4095 2200 -> 2144 us; tokens of six layers between those
-// widths 1.00 to 1.28 times as fast (k_qkv, k_matres, ring.cuh before).  By stage, Llama-3-8B fp8: q/k/v 8.6 -> 6.7 us, wo 7.4 -> 6.9, FFN up 19.8 -> 21, w2 13.9 -> 13.3; 0.5B: 4.1 ->
-// 1.8, 3.4 -> 1.5, 6.8 -> 4.2, 7.7 -> 3.6.  What bounds it now: about 2 us from the last store of a stage to the first product of the next (the grid's end is seen after 1.1 us,
-// the vector's way to the registers and its pieces take the rest), then the memory's rate.
+// Measured, a whole token: Qwen2-0.5B fp16 at 131 positions 906 -> 639 us, Llama-3-8B fp8 at 4095 2215 -> 2149; tokens of six layers between those
+// widths 1.00 to 1.26 times as fast (k_qkv, k_matres, ring.cuh before), four layers of 5120 to 8192 wide models 1.02 to 1.32 times.  By stage, Llama-3-8B fp8: q/k/v 8.5 -> 6.9 us, wo 7.4 -> 6.9,
+// FFN up 19.9, w2 13.9 -> 14.1; 0.5B: 4.2 -> 1.8, 3.5 -> 1.5, 6.7 -> 4.2, 7.8 -> 3.6.  Rows of 4096 fp16 weights are where the ring is as good: w2 18.0 us there, 20.2 here.
+// What bounds it now: about 2 us from the last store of a stage to the first product of the next (the grid's end is seen after 1.1 us, the vector's way to the registers and its pieces take
+// the rest), then the memory's rate.
 #pragma once
 
 #include "stages.cuh"
@@ -170,11 +171,11 @@ struct ColsLane {
 		const int steps = min(r.chunk_steps, r.steps - c * r.chunk_steps);
 		return max(0, min(r.own, steps - r.own * warp));
 	}
-	// its first activation there
 	__device__ __forceinline__ float2 worth(float unscale) const { // of a sum in either of its two columns (pieces 0 1 | 2 0 | 1 2)
 		constexpr float mid = 1.f / COLS_MID, lo = 1.f / COLS_LO;
 		return make_float2(unscale * (t == 0 ? 1.f : t == 1 ? lo : mid), unscale * (t == 0 ? mid : t == 1 ? 1.f : lo));
 	}
+	// this warp's first activation in chunk c
 	template <int DBITS>
 	__device__ __forceinline__ size_t at(const ColsRun& r, int c) const { return (size_t)(c * r.chunk_steps + r.own * warp) * ColsStep<DBITS>::K; }
 };

@@ -89,7 +89,7 @@ struct Engine {
 	// L2 prefetch schedule (common.cuh Prefetch): what each stage requests for the stages after it.  Bytes, or flags.
 	// Measured: no setting beats "off" -- the stage kernels are not waiting for
 	// DRAM behind their boundaries, and requests for later stages only compete with the running one -- so the default is off;
-	// CALM_B200_PF keeps the experiment reproducible.
+	// CALM_B200_PF keeps the experiment reproducible (k_qkv, k_attn2, k_matres, ring.cuh; the stages of cols.cuh request nothing for others: CALM_B200_COLS=0 turns those off).
 	bool pf_kv = false;           // k_qkv / w2 request the KV prefix the next attention kernel reads
 	bool pf_attn_wo = false;      // k_attn requests wo
 	size_t pf_attn_up = 0;        // ... and this much of w1 + w3
