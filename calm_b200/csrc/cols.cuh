@@ -267,8 +267,8 @@ __device__ __forceinline__ void cols_multiply(ColsShared* sh, const unsigned cha
 __device__ __forceinline__ bool cols_hand_over(ColsShared* sh, const ColsRun& r, float* part, const ColsLane& l, int tile, const float (&acc)[4]) {
 	float a = l.t == 2 ? acc[2] : acc[0], b = l.t == 0 ? acc[1] : acc[3];
 	// An infinite weight: the sums of the first pieces (a of t = 0, b of t = 1) say which infinity, the other pieces may be zero or have the other sign.  (Where an activation is so far below
-	// the largest beside it, 2^-39, that its first piece is zero too, the row stays a NaN.  In this form: as comparisons of a
-	// and b, or as a vote of the warp, it cost FFN up of 4096 x 14336 fp8 1.2 and 0.5 us.)
+	// the largest beside it, 2^-39, that its first piece is zero too, the row stays a NaN.)
+	// As a difference, since comparisons of a and b cost FFN up of 4096 x 14336 fp8 1.2 us and a vote of the warp 0.5.
 	const float first = l.t == 0 ? a : l.t == 1 ? b : 0.f;
 	float v = a + b;
 	v = __fadd_rn(v, -v) == 0.f ? v : first;
